@@ -177,7 +177,6 @@ cudaError_t Denoiser::ensure(int n, int h, int w) {
     if (px <= cap_pixels_ && h == h_ && w == w_dim_ && n == n_) return cudaSuccess;
     // keep the parameters, drop the activations
     std::vector<void *> keep = {w_, g_, m_, v_, wb_, wtc_, wtcb_, zero_bias_, pack_jobs_, loss_, err_};
-    partial_ = nullptr;
     x16_ = nullptr;
     gb16_ = nullptr;
     bias_part_ = nullptr;
@@ -225,25 +224,16 @@ cudaError_t Denoiser::ensure(int n, int h, int w) {
         (e = take(gb16_, px * 128)) != cudaSuccess ||
         (e = take(bias_part_, (size_t)dn::kGradPrepBlocks * 128)) != cudaSuccess)
         return e;
-    // split-tap partial sums of the tensor-core kernel: the largest need of
-    // any forward or backward-data convolution; per-group weight-gradient sums
-    size_t partial = 0, partial_wg = 0;
+    // per-group weight-gradient sums: the largest need of any convolution
+    size_t partial_wg = 0;
     for (int i = 0; i < kNumConvs; i++) {
-        dn::TcConvPlan shape;
         const int l = kLevel[i];
-        if (dn::tc_conv_plan(shape, act_[0].x, n, h >> l, w >> l, pad16(kConvs[i][0]), kConvs[i][1], true,
-                             sm_count_) == cudaSuccess)
-            partial = std::max(partial, shape.partial_floats);
-        if (i > 0 && dn::tc_conv_plan(shape, act_[0].x, n, h >> l, w >> l, pad16(kConvs[i][1]), kConvs[i][0], false,
-                                      sm_count_) == cudaSuccess)
-            partial = std::max(partial, shape.partial_floats);
         dn::TcWgradPlan wg;
         if (dn::tc_wgrad_plan(wg, act_[0].x, n, h >> l, w >> l, kConvs[i][0], pad16(kConvs[i][0]), kConvs[i][1],
                               sm_count_) == cudaSuccess)
             partial_wg = std::max(partial_wg, wg.partial_floats);
     }
     if (partial_wg && (e = take(partial_wg_, partial_wg)) != cudaSuccess) return e;
-    if (partial && (e = take(partial_, partial)) != cudaSuccess) return e;
     cap_pixels_ = px;
     return cudaSuccess;
 }
@@ -287,7 +277,7 @@ cudaError_t Denoiser::conv_fwd(int ci, const Buf &in, __nv_bfloat16 *y, float *y
     dn::TcConvPlan *pl = nullptr;
     cudaError_t e = tc_plan(ci, in, pl);
     if (e != cudaSuccess) return e;
-    return dn::conv3x3_forward_tc(*pl, wtc_ + tc_off_[ci], bias, y, y32, partial_, err_, st, fuse, overlap);
+    return dn::conv3x3_forward_tc(*pl, wtc_ + tc_off_[ci], bias, y, y32, err_, st, fuse, overlap);
 }
 
 cudaError_t Denoiser::forward(const float *rad, const __half *feat, int n, int h, int w, cudaStream_t st,
@@ -301,7 +291,8 @@ cudaError_t Denoiser::forward(const float *rad, const __half *feat, int n, int h
     // the tensor cores read the input padded to 16 channels (x16_), also for
     // the residual and the first convolution's weight gradient: the
     // 10-channel copy is written only for the CUDA cores
-    chk(dn::pack_input(rad, feat, tensor_cores_ ? nullptr : act_[0].x, tensor_cores_ ? x16_ : nullptr, px, st));
+    chk(dn::pack_input(rad, feat, tensor_cores_ ? nullptr : act_[0].x, tensor_cores_ ? x16_ : nullptr, px, (size_t)h * w,
+                       st));
     const __nv_bfloat16 *x0 = tensor_cores_ ? x16_ : act_[0].x;
     const int x0_c = tensor_cores_ ? pad16(kConvs[0][0]) : act_[0].c;
     // On the tensor cores the poolings and the upsampling + concatenations are
@@ -362,14 +353,8 @@ cudaError_t Denoiser::forward(const float *rad, const __half *feat, int n, int h
     }
     // output convolution (no ReLU), FP32; the network predicts a correction
     // to the noisy input's log radiance (residual), and the output transform
-    // gives radiance: both in its epilogue unless it splits its taps
-    dn::TcConvPlan *pl = nullptr;
-    bool fused_out = false;
-    if (fuse && e == cudaSuccess) {
-        chk(tc_plan(conv, act_[prev], pl));
-        fused_out = pl && pl->splits == 1;
-    }
-    if (fused_out) {
+    // gives radiance: both in its epilogue on the tensor cores
+    if (fuse) {
         dn::TcFuse f;
         f.res = x0, f.res_c = x0_c;
         f.rad = out_rad, f.feat = feat;
@@ -412,7 +397,7 @@ cudaError_t Denoiser::backward(const float *target, cudaStream_t st) {
                                      c.cout, st));
             return;
         }
-        chk(dn::grad_prep(y, g, gb16_, bias_part_, db, p, c.cout, pad16(c.cout), st));
+        chk(dn::grad_prep(y, g, gb16_, bias_part_, db, p, (size_t)hh * ww, c.cout, pad16(c.cout), st));
         if (need_dx) {
             dn::TcConvPlan &pl = plans_bwd_[ci];
             if (pl.x != gb16_ || pl.n != n || pl.h != hh || pl.w != ww) {
@@ -426,8 +411,8 @@ cudaError_t Denoiser::backward(const float *target, cudaStream_t st) {
             // programmatic launch: its prologue loads the transposed weights
             // (packed after the last optimizer step) while the bias
             // gradient's final sums (the last kernel of grad_prep) run
-            chk(dn::conv3x3_forward_tc(pl, wtcb_ + tcb_off_[ci], zero_bias_, nullptr, in.g, partial_, err_, st,
-                                       nullptr, true));
+            chk(dn::conv3x3_forward_tc(pl, wtcb_ + tcb_off_[ci], zero_bias_, nullptr, in.g, err_, st, nullptr,
+                                       true));
         }
         dn::TcWgradPlan &wg = plans_wg_[ci];
         if (wg.g != gb16_ || wg.n != n || wg.h != hh || wg.w != ww) {

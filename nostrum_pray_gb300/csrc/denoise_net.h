@@ -75,10 +75,9 @@ class Denoiser {
     float *w_ = nullptr, *g_ = nullptr, *m_ = nullptr, *v_ = nullptr, *loss_ = nullptr;
     __nv_bfloat16 *wb_ = nullptr;
     // tensor-core forward: packed weights (offsets per conv), the input padded
-    // to 16 channels, split-tap partial sums, one plan per convolution
+    // to 16 channels, one plan per convolution
     __nv_bfloat16 *wtc_ = nullptr, *x16_ = nullptr;
     std::vector<size_t> tc_off_;
-    float *partial_ = nullptr;
     std::vector<dn::TcConvPlan> plans_;
     int sm_count_ = 0;
     // tensor-core backward-data: per convolution the transposed, tap-mirrored

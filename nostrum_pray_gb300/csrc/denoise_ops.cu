@@ -179,37 +179,44 @@ __global__ void k_relu_mask(const __nv_bfloat16 *y, const float *g, float *out, 
     for (size_t i = gtid(); i < n; i += gstride()) out[i] = bf(y[i]) > 0.f ? g[i] : 0.f;
 }
 
-__global__ void k_grad_bf16(const float *g, __nv_bfloat16 *out, size_t pixels, int c, int c_pad) {
-    const size_t n = pixels * (size_t)c_pad;
-    for (size_t i = gtid(); i < n; i += gstride()) {
-        const size_t p = i / (size_t)c_pad;
-        const int k = (int)(i - p * c_pad);
-        out[i] = __float2bfloat16(k < c ? g[p * c + k] : 0.f);
-    }
-}
-
-// Threads (r, k), r < rows, k < c_pad: channel k of pixels p0 + r, p0 + r +
-// rows, ... of the block's range; reads and writes are row-contiguous.
+// Threads (r, q), r < rows, q < c_pad / 8: the 8-channel chunk q of pixels p0
+// + r, p0 + r + rows, ... of the block's range. y and out are planar (images
+// of px pixels), g channels last. c = 3 or a multiple of 8.
 __global__ void k_grad_prep(const __nv_bfloat16 *y, const float *g, __nv_bfloat16 *out, float *part, size_t pixels,
-                            size_t chunk, int c, int c_pad, int rows) {
-    __shared__ float sm[256];
-    const int k = (int)threadIdx.x % c_pad, r = (int)threadIdx.x / c_pad;
+                            size_t px, size_t chunk, int c, int c_pad, int rows) {
+    __shared__ float sm[256][9];
+    const int nq = c_pad >> 3, q = (int)threadIdx.x % nq, r = (int)threadIdx.x / nq;
     const size_t p0 = (size_t)blockIdx.x * chunk, p1 = p0 + chunk < pixels ? p0 + chunk : pixels;
-    float acc = 0.f;
+    float acc[8] = {};
     for (size_t p = p0 + r; p < p1; p += rows) {
-        float v = 0.f;
-        if (k < c) {
-            v = g[p * c + k];
-            if (y && !(bf(y[p * c + k]) > 0.f)) v = 0.f;
+        const size_t img = p / px, plane = (img * nq + q) * px + (p - img * px);
+        float v[8] = {};
+        if (c & 7) {
+            for (int k = 0; k < 8; k++)
+                if (8 * q + k < c) v[k] = g[p * c + 8 * q + k];
+        } else {
+            const float4 *s = reinterpret_cast<const float4 *>(g + p * c + 8 * q);
+            const float4 a = s[0], b = s[1];
+            v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
         }
-        out[p * c_pad + k] = __float2bfloat16(v);
-        acc += v;
+        if (y) {
+            const uint4 m4 = reinterpret_cast<const uint4 *>(y)[plane];
+            const __nv_bfloat16 *m = reinterpret_cast<const __nv_bfloat16 *>(&m4);
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                if (!(bf(m[k]) > 0.f)) v[k] = 0.f;
+        }
+        __nv_bfloat16 o[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) o[k] = __float2bfloat16(v[k]), acc[k] += v[k];
+        reinterpret_cast<uint4 *>(out)[plane] = *reinterpret_cast<const uint4 *>(o);
     }
-    sm[threadIdx.x] = acc;
+#pragma unroll
+    for (int k = 0; k < 8; k++) sm[threadIdx.x][k] = acc[k];
     __syncthreads();
-    if (r == 0 && k < c) {
+    for (int k = (int)threadIdx.x; k < c; k += (int)blockDim.x) {
         float s = 0.f;
-        for (int i = 0; i < rows; i++) s += sm[i * c_pad + k];
+        for (int i = 0; i < rows; i++) s += sm[i * nq + (k >> 3)][k & 7];
         part[(size_t)blockIdx.x * c + k] = s;
     }
 }
@@ -309,9 +316,10 @@ __device__ __forceinline__ float demod(const __half *feat, size_t i) {
 
 // network input: log1p(radiance / demodulation) 3, albedo 3, normal 3, depth
 // 1 from FP16 feature buffers (radiance n x 3 floats, features n x 7 halves);
-// x16 (optional) receives the same 10 channels padded to 16 with zeros
+// x16 (optional) receives the same 10 channels padded to 16 with zeros, planar
+// (images of px pixels)
 __global__ void k_pack_input(const float *rad, const __half *feat, __nv_bfloat16 *x, __nv_bfloat16 *x16,
-                             size_t pixels) {
+                             size_t pixels, size_t px) {
     // the first convolution may launch now (its prologue overlaps this
     // kernel; it waits for this kernel's completion before reading x16)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -323,9 +331,10 @@ __global__ void k_pack_input(const float *rad, const __half *feat, __nv_bfloat16
         if (x)
             for (int k = 0; k < 10; k++) x[p * 10 + k] = v[k];
         if (x16) {
-            uint4 *o = reinterpret_cast<uint4 *>(x16 + p * 16);
+            const size_t img = p / px;
+            uint4 *o = reinterpret_cast<uint4 *>(x16) + img * px + p;  // plane 2 img, pixel p - img px
             o[0] = *reinterpret_cast<const uint4 *>(v);
-            o[1] = *reinterpret_cast<const uint4 *>(v + 8);
+            o[px] = *reinterpret_cast<const uint4 *>(v + 8);
         }
     }
 }
@@ -456,20 +465,15 @@ cudaError_t bias_grad(const float *g, float *db, size_t pixels, int c, cudaStrea
     return cudaGetLastError();
 }
 cudaError_t grad_prep(const __nv_bfloat16 *y, const float *g, __nv_bfloat16 *out, float *part, float *db,
-                      size_t pixels, int c, int c_pad, cudaStream_t st) {
-    if (c_pad < c || c_pad > 256 || (c_pad & 15) || pixels == 0) return cudaErrorInvalidValue;
-    const int rows = 256 / c_pad;
+                      size_t pixels, size_t px, int c, int c_pad, cudaStream_t st) {
+    if (c_pad < c || c_pad > 256 || (c_pad & 15) || (c != 3 && (c & 7)) || pixels == 0) return cudaErrorInvalidValue;
+    const int rows = 256 / (c_pad / 8);
     const size_t chunk = (pixels + kGradPrepBlocks - 1) / kGradPrepBlocks;
     const int blocks = (int)((pixels + chunk - 1) / chunk);
-    k_grad_prep<<<blocks, rows * c_pad, 0, st>>>(y, g, out, part, pixels, chunk, c, c_pad, rows);
+    k_grad_prep<<<blocks, rows * (c_pad / 8), 0, st>>>(y, g, out, part, pixels, px, chunk, c, c_pad, rows);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     k_bias_finalize<<<c, 256, 0, st>>>(part, db, blocks, c);
-    return cudaGetLastError();
-}
-cudaError_t grad_bf16(const float *g, __nv_bfloat16 *out, size_t pixels, int c, int c_pad, cudaStream_t st) {
-    if (c_pad < c) return cudaErrorInvalidValue;
-    k_grad_bf16<<<blocks_for(pixels * (size_t)c_pad), 256, 0, st>>>(g, out, pixels, c, c_pad);
     return cudaGetLastError();
 }
 cudaError_t avgpool(const __nv_bfloat16 *x, __nv_bfloat16 *y, int n, int h, int w, int c, cudaStream_t st) {
@@ -496,8 +500,8 @@ cudaError_t upsample_concat(const __nv_bfloat16 *low, const __nv_bfloat16 *skip,
     return cudaGetLastError();
 }
 cudaError_t pack_input(const float *rad, const __half *feat, __nv_bfloat16 *x, __nv_bfloat16 *x16, size_t pixels,
-                       cudaStream_t st) {
-    k_pack_input<<<blocks_for(pixels), 256, 0, st>>>(rad, feat, x, x16, pixels);
+                       size_t px, cudaStream_t st) {
+    k_pack_input<<<blocks_for(pixels), 256, 0, st>>>(rad, feat, x, x16, pixels, px);
     return cudaGetLastError();
 }
 cudaError_t l1_loss(const float *out, const float *target, const __half *feat, float *g, float *loss, float *part,

@@ -14,21 +14,22 @@
 namespace pray_gpu {
 namespace dn {
 
-// tcgen05 tensor-core version (denoise_tc.cu). A plan holds the input's TMA
-// tensor map (the input buffer is fixed) and the launch shape; Cin must be a
-// multiple of 16 (pack_input pads the network input), the weights packed by tc_pack_weights
-// (cin_pad = Cin of the plan). Levels with few tiles split the taps over CTAs
-// and need `partial` (partial_floats floats). *err is set to 1 if one of the
-// kernel's bounded mbarrier waits ran out.
+// tcgen05 tensor-core version (denoise_tc.cu). Its BF16 tensors are planar in
+// 8-channel chunks: [image][channel / 8][y][x][8] (the CUDA-core kernels'
+// tensors are channels last). A plan holds the input's TMA tensor map (the
+// input buffer is fixed) and the launch shape; Cin must be a multiple of 16
+// (pack_input pads the network input), the weights packed by tc_pack_weights
+// (cin_pad = Cin of the plan). *err is set to 1 if one of the kernel's bounded
+// mbarrier waits ran out.
 struct TcConvPlan {
-    alignas(64) unsigned char tmap[128];  // CUtensorMap of x: (C, W, H, N), box (8, 10, 18, 1)
+    alignas(64) unsigned char tmap[128];  // CUtensorMap of x: (8 W, H, C / 8, N), box (80, 18, C / 8, 1)
     const __nv_bfloat16 *x;
     int n, h, w, cin, cout, npad, relu;
-    int tiles_x, tiles_y, tiles, splits, taps_per_split, taps_per_stage, stages, tmem_cols;
+    int tiles_x, tiles_y, tiles, taps_per_stage, stages, tmem_cols;
     int nsplit, npad_full;  // output-channel split: nsplit CTAs per tile, npad channels each of npad_full
     int persistent, grid;  // persistent pipelined kernel (no split, weights resident) and its CTAs
     uint32_t w_off, bar_off, halo_stride;
-    size_t smem, partial_floats;
+    size_t smem;
 };
 cudaError_t tc_conv_plan(TcConvPlan &p, const __nv_bfloat16 *x, int n, int h, int w, int cin, int cout, bool relu,
                          int sm_count);
@@ -37,7 +38,7 @@ cudaError_t tc_pack_weights(const float *w, __nv_bfloat16 *packed, int cin, int 
 // Weights of the backward-data convolution of a forward convolution with
 // cin_f inputs and cout_f outputs (w[cout_f][9][cin_f]): a plan with
 // cin = cout_f rounded up to 16 and cout = cin_f runs it on the output
-// gradient (as BF16, grad_bf16) and writes the input gradient.
+// gradient (as BF16, grad_prep) and writes the input gradient.
 cudaError_t tc_pack_weights_bwd(const float *w, __nv_bfloat16 *packed, int cin_f, int cout_f, cudaStream_t st);
 // Every packing of a network's weights in one launch: job j packs w (the
 // FP32 [cout_f][9][cin_f] weights of one convolution) into out, as
@@ -64,8 +65,7 @@ cudaError_t tc_pack_all(const TcPackJob *jobs_dev, int njobs, size_t total, cuda
 //   res:  FP32 output += res[pixel * res_c + channel] (BF16);
 //   rad:  (cout 3) rad = expm1(FP32 output) * (max(albedo, 0) + kDemodFloor),
 //         the albedo from feat (7 halves per pixel).
-// pool and cat need cout a multiple of 16, res and rad the FP32 output; none
-// works with a tap split (p.splits > 1).
+// pool and cat need cout a multiple of 16, res and rad the FP32 output.
 struct TcFuse {
     __nv_bfloat16 *pool = nullptr;
     __nv_bfloat16 *cat = nullptr;
@@ -76,8 +76,10 @@ struct TcFuse {
     const __half *feat = nullptr;
 };
 cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked, const float *bias,
-                               __nv_bfloat16 *y, float *y32, float *partial, int *err, cudaStream_t st,
+                               __nv_bfloat16 *y, float *y32, int *err, cudaStream_t st,
                                const TcFuse *fuse = nullptr, bool overlap_prologue = false);
+// y: the BF16 output (planar, cout a multiple of 16), y32: the FP32 output
+// (channels last); either may be NULL.
 // overlap_prologue: launch with programmatic stream serialisation, so that the
 // kernel's prologue (barriers, tensor memory, weight copies) overlaps the
 // previous kernel of the stream; its input copies wait for that kernel to
@@ -86,13 +88,13 @@ cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked
 // dw[co][tap][ci] += sum over pixels p of g[p][co] * x[p + offset(tap)][ci],
 // a GEMM with M = output channels (padded to 128), N = input channels, K =
 // pixels. g: the output gradient as BF16 with cout_pad = cout rounded up to
-// 16 channels (grad_bf16); x: the convolution's input, read through the
+// 16 channels (grad_prep); x: the convolution's input, read through the
 // forward plan's halo tensor map (fwd: a plan over x with cin = cin_pad).
 // Each CTA accumulates the nine taps (or a group of them, as many as tensor
 // memory holds) over a group of 16 x 8 tiles and writes them to `partial`
 // (partial_floats floats); a second kernel adds the groups in order into dw.
 struct TcWgradPlan {
-    alignas(64) unsigned char gmap[128];  // CUtensorMap of g: (cout_pad, W, H, N), box (8, 8, 16, 1)
+    alignas(64) unsigned char gmap[128];  // CUtensorMap of g: (8 W, H, cout_pad / 8, N), box (64, 16, cout_pad / 8, 1)
     const __nv_bfloat16 *g;
     int n, h, w, cin, cin_pad, cout, cout_pad;
     int tiles_x, tiles_y, tiles, tiles_per_cta, groups, taps_per_pass, passes, tmem_cols, stages;
@@ -115,12 +117,11 @@ cudaError_t bias_grad(const float *g, float *db, size_t pixels, int c, cudaStrea
 // tensor-core backward: the ReLU mask of the convolution's output y (NULL:
 // no mask), the masked gradient as BF16 with c_pad >= c channels (the pad
 // zero), and the bias gradient: per-block partial sums in part
-// (kGradPrepBlocks x c floats), added in block order into db.
+// (kGradPrepBlocks x c floats), added in block order into db. y and out are
+// planar (images of px pixels), g channels last; c is 3 or a multiple of 8.
 constexpr int kGradPrepBlocks = 1024;
 cudaError_t grad_prep(const __nv_bfloat16 *y, const float *g, __nv_bfloat16 *out, float *part, float *db,
-                      size_t pixels, int c, int c_pad, cudaStream_t st);
-// g (pixels x c FP32) as BF16 with c_pad >= c channels (the pad zero)
-cudaError_t grad_bf16(const float *g, __nv_bfloat16 *out, size_t pixels, int c, int c_pad, cudaStream_t st);
+                      size_t pixels, size_t px, int c, int c_pad, cudaStream_t st);
 cudaError_t avgpool(const __nv_bfloat16 *x, __nv_bfloat16 *y, int n, int h, int w, int c, cudaStream_t st);
 cudaError_t avgpool_backward(const float *gy, float *gx, int n, int h, int w, int c, cudaStream_t st);
 cudaError_t upsample_backward(const float *gy, float *gx, int n, int h, int w, int c, int cy, cudaStream_t st);
@@ -129,9 +130,10 @@ cudaError_t split_add(const float *gy, float *gx, size_t pixels, int c, int cy, 
 // max(albedo, 0) + kDemodFloor (per channel) on the way in and in the loss's
 // target, multiplied back on the way out.
 constexpr float kDemodFloor = 0.05f;
-// x (may be NULL): 10 channels; x16 (may be NULL): the same padded to 16 channels
+// x (may be NULL): 10 channels; x16 (may be NULL): the same padded to 16
+// channels, planar (images of px pixels)
 cudaError_t pack_input(const float *rad, const __half *feat, __nv_bfloat16 *x, __nv_bfloat16 *x16, size_t pixels,
-                       cudaStream_t st);
+                       size_t px, cudaStream_t st);
 // cat = [nearest 2x upsampling of low (c channels, h x w), skip (cs channels)]
 cudaError_t upsample_concat(const __nv_bfloat16 *low, const __nv_bfloat16 *skip, __nv_bfloat16 *cat, int n, int h,
                             int w, int c, int cs, cudaStream_t st);

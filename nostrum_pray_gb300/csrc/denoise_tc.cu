@@ -1,12 +1,19 @@
 // 3x3 convolution forward on the 5th-generation tensor cores (tcgen05), BF16
 // operands, FP32 accumulation in tensor memory (TMEM).
 //
+// Activations are planar in 8-channel chunks, [image][channel / 8][y][x][8]
+// (16 bytes per pixel and chunk), which is the layout the tensor cores read
+// from shared memory, so a halo is copied as whole rows.
+//
 // Implicit GEMM without an im2col copy. One CTA (4 warps) computes a tile of
 // 16 x 8 output pixels (M = 128) x all output channels (N = Cout rounded up
-// to 16). The input halo of the tile, 18 x 10 pixels x Cin, is loaded once
-// by TMA (one 4-D tiled copy per 8-channel chunk; out-of-image pixels arrive
+// to 16). The input halo of the tile, 18 x 10 pixels x Cin, is loaded by one
+// 4-D TMA copy (rows of 160 contiguous bytes; out-of-image pixels arrive
 // as zeros, which is the convolution's padding) into planes of
-// [y][x][8 channels] (16 bytes per pixel). In that layout the A operand of
+// [y][x][8 channels]. With channels-last tensors the same halo is a box of
+// 16-byte rows, ten times as many requests: the copies, not HBM or the
+// tensor cores, bounded the wide levels (80 -> 32 channels at 8 x 512^2: 171 us
+// against PLANAR_US). In the planes the A operand of
 // tap (dy, dx) for 16 channels is the halo itself seen through a shared-memory
 // matrix descriptor: the tile's 8-pixel rows are the 8-row core-matrix
 // groups (stride 160 bytes = one halo row), the two 8-channel chunks are the
@@ -20,9 +27,7 @@
 //
 // The deep, small levels have too few tiles for 152 SMs: there each tile's
 // output channels are split over CTAs (each loads its slice of the weights
-// with one 3-D TMA box), or, for a single 16-channel chunk, the nine taps over
-// 3 or 9 CTAs, each writing FP32 partial sums that a second kernel adds in
-// split order (deterministic) with the bias and ReLU.
+// with one 3-D TMA box).
 //
 // The epilogue also performs the network's glue (TcFuse): 2 x 2 average
 // pooling, nearest 2x upsampling into a concatenation, the residual add and
@@ -50,8 +55,7 @@ namespace {
 
 constexpr int kTileW = 8, kTileH = 16;
 constexpr int kHaloW = kTileW + 2, kHaloH = kTileH + 2;
-constexpr uint32_t kChunkBytes = kHaloW * kHaloH * 16;  // one 8-channel halo plane (2880)
-constexpr uint32_t kPlaneBytes = 2944;                  // plane stride, 128-byte aligned
+constexpr uint32_t kPlaneBytes = kHaloW * kHaloH * 16;  // one 8-channel halo plane (2880), planes back to back
 constexpr uint32_t kRowBytes = kHaloW * 16;             // one halo row of one plane (160)
 constexpr uint32_t kWaitLimit = 1u << 24;
 constexpr size_t kSmemBudget = 110 * 1024;              // target per CTA (two or more CTAs per SM)
@@ -64,13 +68,11 @@ struct TcArgs {
     const float *bias;
     __nv_bfloat16 *y;
     float *y32;
-    float *partial;          // [split][M][npad] when splits > 1
     int n, h, wd, cin, cout, npad, relu;
     int tiles_x, tiles_y;
-    int taps_per_split, taps_per_stage, stages;
-    int nsplit;               // > 1: blockIdx.y picks output channels [y * npad, (y + 1) * npad), all taps,
-                              // the weight slice by TMA (wmap) from the packing of npad_full rows
-    int npad_full;
+    int taps_per_stage, stages;
+    int nsplit;               // > 1: blockIdx.y picks output channels [y * npad, (y + 1) * npad), the weight
+                              // slice by TMA (wmap) from the packing of all rows
     int tmem_cols;
     uint32_t w_off, bar_off;  // shared-memory offsets (the halo is at 0)
     uint32_t halo_stride;     // persistent kernel: distance between the halo ring's slots
@@ -128,14 +130,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     return false;
 }
 
-// One 8-channel chunk of the halo: box (8 channels, 10 x, 18 y, 1 image) at
-// (c, x, y, img); x and y may be -1 (zero fill).
-__device__ __forceinline__ void tma_halo(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c, int x, int y,
-                                         int img) {
+// A tile of a planar tensor, every chunk: box (8 * columns, rows, chunks, 1
+// image) at column x, row y; a halo starts at -1 (zero fill).
+__device__ __forceinline__ void tma_tile(uint32_t dst, const CUtensorMap *map, uint32_t bar, int x, int y, int img) {
     asm volatile(
         "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, "
         "%6}], [%2];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c), "r"(x), "r"(y), "r"(img)
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(8 * x), "r"(y), "r"(0), "r"(img)
         : "memory");
 }
 
@@ -175,18 +176,19 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 // Epilogue of one tile: the calling warp reads TMEM lanes 32q..32q+31 (q =
 // quad, the warp's lane quadrant: its warp index mod 4; tile rows m = pixel
 // (m / 8, m % 8)) from column `tmem` on, 16 columns at a time, and stores
-// bias + ReLU + BF16 (16-byte stores), FP32, or raw FP32 partials, plus the
-// extra stores of P.f. A warp holds four whole tile rows, so the 2 x 2 blocks
+// bias + ReLU as BF16 (planar: the eight pixels of a tile row are 128
+// contiguous bytes per chunk) or FP32 (channels last), plus the extra stores
+// of P.f. A warp holds four whole tile rows, so the 2 x 2 blocks
 // of the pooling are lanes (l, l + 1, l + 8, l + 9) for l with even row and
 // column, summed in the order of k_avgpool (row-major).
-__device__ __forceinline__ void epilogue(const TcArgs &P, uint32_t tmem, int img, int y0, int x0, int split,
-                                         int quad, int n0 = 0) {
+__device__ __forceinline__ void epilogue(const TcArgs &P, uint32_t tmem, int img, int y0, int x0, int quad,
+                                         int n0 = 0) {
     const int lane = (int)(threadIdx.x & 31);
     const int m = quad * 32 + lane;
     const int yy = y0 + (m >> 3), xx = x0 + (m & 7);
     const bool valid = yy < P.h && xx < P.wd;
-    const size_t M = (size_t)P.n * P.h * P.wd;
-    const size_t pix = ((size_t)img * P.h + yy) * P.wd + xx;
+    const size_t px = (size_t)P.h * P.wd, at = (size_t)yy * P.wd + xx;  // one plane, the pixel in it
+    const size_t pix = img * px + at;
     const bool vec = (P.y || P.f.pool || P.f.cat) && (P.cout & 15) == 0;
     for (int c0 = 0; c0 < P.npad; c0 += 16) {
         uint32_t r[16];
@@ -202,13 +204,8 @@ __device__ __forceinline__ void epilogue(const TcArgs &P, uint32_t tmem, int img
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         // the pooling's shuffles need every lane of the warp
         if (!valid && !(vec && P.f.pool)) continue;
-        if (P.partial) {
-            float4 *o = reinterpret_cast<float4 *>(P.partial + ((size_t)split * M + pix) * P.npad + c0);
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-                o[k] = make_float4(__uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1]),
-                                   __uint_as_float(r[4 * k + 2]), __uint_as_float(r[4 * k + 3]));
-        } else if (vec) {
+        if (vec) {
+            const int chunk = (n0 + c0) >> 3;  // this and the next 8-channel chunk of the output
             float v[16];
 #pragma unroll
             for (int k = 0; k < 16; k++) {
@@ -219,22 +216,22 @@ __device__ __forceinline__ void epilogue(const TcArgs &P, uint32_t tmem, int img
             const uint4 hi =
                 make_uint4(pack2(v[8], v[9]), pack2(v[10], v[11]), pack2(v[12], v[13]), pack2(v[14], v[15]));
             if (valid && P.y) {
-                uint4 *o = reinterpret_cast<uint4 *>(P.y + pix * P.cout + n0 + c0);
-                o[0] = lo, o[1] = hi;
+                uint4 *o = reinterpret_cast<uint4 *>(P.y) + ((size_t)img * (P.cout >> 3) + chunk) * px + at;
+                o[0] = lo, o[px] = hi;
             }
             if (valid && P.f.cat) {
-                const int ch = P.f.cat_off + n0 + c0;
+                uint4 *o = reinterpret_cast<uint4 *>(P.f.cat);
+                const size_t plane = (size_t)img * (P.f.cat_c >> 3) + (P.f.cat_off >> 3) + chunk;
                 if (P.f.cat_up) {
+                    // the pixel's 2 x 2 block: two neighbours (32 bytes) in each of two rows
                     const size_t W2 = 2 * (size_t)P.wd;
-                    const size_t b = (((size_t)img * 2 * P.h + 2 * yy) * W2 + 2 * xx) * P.f.cat_c + ch;
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        uint4 *o = reinterpret_cast<uint4 *>(P.f.cat + b + ((q >> 1) * W2 + (q & 1)) * P.f.cat_c);
-                        o[0] = lo, o[1] = hi;
-                    }
+                    o += plane * 4 * px + 2 * yy * W2 + 2 * xx;
+                    o[0] = lo, o[1] = lo, o[W2] = lo, o[W2 + 1] = lo;
+                    o += 4 * px;
+                    o[0] = hi, o[1] = hi, o[W2] = hi, o[W2 + 1] = hi;
                 } else {
-                    uint4 *o = reinterpret_cast<uint4 *>(P.f.cat + pix * P.f.cat_c + ch);
-                    o[0] = lo, o[1] = hi;
+                    o += plane * px + at;
+                    o[0] = lo, o[px] = hi;
                 }
             }
             if (P.f.pool) {
@@ -252,10 +249,11 @@ __device__ __forceinline__ void epilogue(const TcArgs &P, uint32_t tmem, int img
                 }
                 const int ho = P.h >> 1, wo = P.wd >> 1, yo = yy >> 1, xo = xx >> 1;
                 if (((lane >> 3) & 1) == 0 && (lane & 1) == 0 && yo < ho && xo < wo) {
-                    uint4 *o = reinterpret_cast<uint4 *>(P.f.pool + (((size_t)img * ho + yo) * wo + xo) * P.cout +
-                                                         n0 + c0);
+                    const size_t pp = (size_t)ho * wo;
+                    uint4 *o = reinterpret_cast<uint4 *>(P.f.pool) + ((size_t)img * (P.cout >> 3) + chunk) * pp +
+                               (size_t)yo * wo + xo;
                     o[0] = make_uint4(po[0], po[1], po[2], po[3]);
-                    o[1] = make_uint4(po[4], po[5], po[6], po[7]);
+                    o[pp] = make_uint4(po[4], po[5], po[6], po[7]);
                 }
             }
         } else {
@@ -265,8 +263,7 @@ __device__ __forceinline__ void epilogue(const TcArgs &P, uint32_t tmem, int img
                 if (co >= P.cout) break;
                 float v = __uint_as_float(r[k]) + __ldg(P.bias + co);
                 if (P.relu) v = fmaxf(v, 0.f);
-                if (P.y) P.y[pix * P.cout + co] = __float2bfloat16(v);
-                if (P.f.res) v += __bfloat162float(P.f.res[pix * P.f.res_c + co]);
+                if (P.f.res) v += __bfloat162float(P.f.res[((size_t)img * (P.f.res_c >> 3) * px + at) * 8 + co]);
                 if (P.y32) P.y32[pix * P.cout + co] = v;
                 if (P.f.rad)
                     P.f.rad[pix * 3 + co] =
@@ -292,12 +289,8 @@ __global__ void __launch_bounds__(128) k_conv_tc(const __grid_constant__ CUtenso
     const int per_img = P.tiles_x * P.tiles_y;
     const int img = blockIdx.x / per_img, rem = blockIdx.x - img * per_img;
     const int y0 = (rem / P.tiles_x) * kTileH, x0 = (rem % P.tiles_x) * kTileW;
-    // tap split (nsplit 1): blockIdx.y picks a group of taps; output-channel
-    // split: all taps, channels from n0
-    const int split = P.nsplit > 1 ? 0 : blockIdx.y;
-    const int n0 = P.nsplit > 1 ? (int)blockIdx.y * P.npad : 0;
-    const int t0 = split * P.taps_per_split;
-    const int nloads = P.taps_per_split / P.taps_per_stage;
+    const int n0 = (int)blockIdx.y * P.npad;
+    const int nloads = 9 / P.taps_per_stage;
     const int kchunks = P.cin >> 3;  // 8-channel chunks per tap (the weight map's third coordinate)
     const uint32_t wtap_bytes = (uint32_t)P.cin * P.npad * 2;
     const uint32_t stage_bytes = wtap_bytes * P.taps_per_stage;
@@ -322,22 +315,19 @@ __global__ void __launch_bounds__(128) k_conv_tc(const __grid_constant__ CUtenso
         // weights: the first `stages` loads; with the output-channel split, one
         // TMA box per load: rows n0..n0+npad of every (tap, chunk) of the stage
         int issued = 0;
-        const __nv_bfloat16 *wsrc = P.w + (size_t)t0 * P.cin * P.npad;
         auto load_weights = [&](int stage, int load) {
             mbar_expect_tx(bar(2 + stage), stage_bytes);
             if (P.nsplit > 1)
-                tma_w(wbase + stage * stage_bytes, &wmap, bar(2 + stage), n0,
-                      (t0 + load * P.taps_per_stage) * kchunks);
+                tma_w(wbase + stage * stage_bytes, &wmap, bar(2 + stage), n0, load * P.taps_per_stage * kchunks);
             else
-                bulk_copy(wbase + stage * stage_bytes, wsrc + (size_t)load * P.taps_per_stage * P.cin * P.npad,
+                bulk_copy(wbase + stage * stage_bytes, P.w + (size_t)load * P.taps_per_stage * P.cin * P.npad,
                           stage_bytes, bar(2 + stage));
         };
         for (; issued < nloads && issued < P.stages; issued++) load_weights(issued, issued);
         // the weights do not depend on the previous kernel; the input does
         grid_dependency_wait();
-        // halo: one copy per 8-channel chunk, all completing on bars[0]
-        mbar_expect_tx(bar(0), (uint32_t)nchunk * kChunkBytes);
-        for (int c = 0; c < nchunk; c++) tma_halo(halo + c * kPlaneBytes, &xmap, bar(0), 8 * c, x0 - 1, y0 - 1, img);
+        mbar_expect_tx(bar(0), (uint32_t)nchunk * kPlaneBytes);
+        tma_tile(halo, &xmap, bar(0), x0 - 1, y0 - 1, img);
         const bool halo_done = mbar_wait(bar(0), 0);
         ok = halo_done;
         const uint32_t idesc = inst_desc(128, P.npad);
@@ -351,7 +341,7 @@ __global__ void __launch_bounds__(128) k_conv_tc(const __grid_constant__ CUtenso
             consumed = j + 1;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (int q = 0; q < P.taps_per_stage; q++) {
-                const int tap = t0 + j * P.taps_per_stage + q;
+                const int tap = j * P.taps_per_stage + q;
                 const int dy = tap / 3, dx = tap - 3 * (tap / 3);
                 const uint32_t a0 = halo + (uint32_t)(dy * kHaloW + dx) * 16;
                 const uint32_t b0 = wbase + s * stage_bytes + q * wtap_bytes;
@@ -388,7 +378,7 @@ __global__ void __launch_bounds__(128) k_conv_tc(const __grid_constant__ CUtenso
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     __syncthreads();
     if (!ok && tid == 0) atomicExch(P.err, 1);
-    if (ok) epilogue(P, tmem, img, y0, x0, split, warp, n0);
+    if (ok) epilogue(P, tmem, img, y0, x0, warp, n0);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
@@ -408,7 +398,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 
 constexpr int kWsThreads = 192;  // warp 0 loads, warp 1 issues MMAs, warps 2-5 drain accumulators
 
-// Persistent, warp-specialised variant for levels that need no tap split and
+// Persistent, warp-specialised variant for levels that need no split and
 // whose weights fit in shared memory beside a ring of halos. Each CTA loads
 // the weights once and walks tiles blockIdx.x, blockIdx.x + gridDim.x, ...:
 //   warp 0 (one thread) loads tile i's halo into ring slot i % H once the
@@ -486,9 +476,8 @@ __global__ void __launch_bounds__(kWsThreads) k_conv_tc_persistent(const __grid_
                 int img, y0, x0;
                 tile_of(i, img, y0, x0);
                 const uint32_t dst = halo0 + (uint32_t)h * P.halo_stride;
-                mbar_expect_tx(bar(full0 + h), (uint32_t)nchunk * kChunkBytes);
-                for (int c = 0; c < nchunk; c++)
-                    tma_halo(dst + c * kPlaneBytes, &xmap, bar(full0 + h), 8 * c, x0 - 1, y0 - 1, img);
+                mbar_expect_tx(bar(full0 + h), (uint32_t)nchunk * kPlaneBytes);
+                tma_tile(dst, &xmap, bar(full0 + h), x0 - 1, y0 - 1, img);
                 *issued = i + 1;
             }
         }
@@ -542,7 +531,7 @@ __global__ void __launch_bounds__(kWsThreads) k_conv_tc_persistent(const __grid_
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             int img, y0, x0;
             tile_of(i, img, y0, x0);
-            epilogue(P, tmem + (uint32_t)(a * acc_stride), img, y0, x0, 0, quad);
+            epilogue(P, tmem + (uint32_t)(a * acc_stride), img, y0, x0, quad);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             mbar_arrive(bar(acce0 + a));
         }
@@ -563,8 +552,6 @@ __global__ void __launch_bounds__(kWsThreads) k_conv_tc_persistent(const __grid_
     }
 }
 
-// Sum of the split partials in split order, plus bias, ReLU, store; four
-// channels per thread when cout is a multiple of 4, else one.
 // ---- weight gradient ---------------------------------------------------------
 //
 // dw[co][tap][ci] = sum_p g[p][co] x[p + offset(tap)][ci]: per tap a GEMM with
@@ -601,16 +588,6 @@ struct WgArgs {
 
 // MN-major A and B: transpose bits of the kind::f16 instruction descriptor
 __host__ __device__ constexpr uint32_t inst_desc_mn(int m, int n) { return inst_desc(m, n) | (1u << 15) | (1u << 16); }
-
-// One plane (8 channels) of a tile of the output gradient: box (8, 8, 16, 1).
-__device__ __forceinline__ void tma_tile(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c, int x, int y,
-                                         int img) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, "
-        "%6}], [%2];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c), "r"(x), "r"(y), "r"(img)
-        : "memory");
-}
 
 __global__ void __launch_bounds__(128) k_wgrad_tc(const __grid_constant__ CUtensorMap gmap,
                                                   const __grid_constant__ CUtensorMap xmap, WgArgs P) {
@@ -653,7 +630,7 @@ __global__ void __launch_bounds__(128) k_wgrad_tc(const __grid_constant__ CUtens
     if (tid == 0) {
         bool ok = true;
         const uint32_t idesc = inst_desc_mn(128, P.cin_pad);
-        const uint32_t bytes = (uint32_t)gplanes * kGradPlaneBytes + (uint32_t)xplanes * kChunkBytes;
+        const uint32_t bytes = (uint32_t)gplanes * kGradPlaneBytes + (uint32_t)xplanes * kPlaneBytes;
         const int per_img = P.tiles_x * P.tiles_y;
         const int n = t_end > t_begin ? t_end - t_begin : 0;
         // tile i of the group goes to stage i % S; issue() starts its loads
@@ -663,9 +640,8 @@ __global__ void __launch_bounds__(128) k_wgrad_tc(const __grid_constant__ CUtens
             const int y0 = (rem / P.tiles_x) * kTileH, x0 = (rem % P.tiles_x) * kTileW;
             const uint32_t a = abase(st), b = a + P.b_off;
             mbar_expect_tx(bar(st), bytes);
-            for (int c = 0; c < gplanes; c++) tma_tile(a + c * kGradPlaneBytes, &gmap, bar(st), 8 * c, x0, y0, img);
-            for (int c = 0; c < xplanes; c++)
-                tma_halo(b + c * kPlaneBytes, &xmap, bar(st), 8 * c, x0 - 1, y0 - 1, img);
+            tma_tile(a, &gmap, bar(st), x0, y0, img);
+            tma_tile(b, &xmap, bar(st), x0 - 1, y0 - 1, img);
         };
         int issued = 0, consumed = 0, committed = 0;
         if (n > 0) issue(issued++);
@@ -788,44 +764,6 @@ __global__ void k_wgrad_finalize(const float *partial, float *dw, int groups, in
     }
 }
 
-template <int kVec>
-__global__ void k_conv_finalize(const float *partial, const float *bias, __nv_bfloat16 *y, float *y32, size_t M,
-                                int npad, int cout, int splits, int relu) {
-    const int groups = cout / kVec;
-    const size_t total = M * (size_t)groups;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t pix = i / groups;
-        const int co = kVec * (int)(i - pix * groups);
-        float v[kVec];
-#pragma unroll
-        for (int k = 0; k < kVec; k++) v[k] = partial[pix * npad + co + k];
-        for (int s = 1; s < splits; s++) {
-            const float *q = partial + ((size_t)s * M + pix) * npad + co;
-#pragma unroll
-            for (int k = 0; k < kVec; k++) v[k] = v[k] + q[k];
-        }
-#pragma unroll
-        for (int k = 0; k < kVec; k++) {
-            v[k] = v[k] + bias[co + k];
-            if (relu) v[k] = fmaxf(v[k], 0.f);
-        }
-        if (kVec == 4) {
-            if (y) {
-                uint2 o;
-                o.x = pack2(v[0], v[1 % kVec]);
-                o.y = pack2(v[2 % kVec], v[3 % kVec]);
-                *reinterpret_cast<uint2 *>(y + pix * cout + co) = o;
-            }
-            if (y32)
-                *reinterpret_cast<float4 *>(y32 + pix * cout + co) =
-                    make_float4(v[0], v[1 % kVec], v[2 % kVec], v[3 % kVec]);
-        } else {
-            if (y) y[pix * cout + co] = __float2bfloat16(v[0]);
-            if (y32) y32[pix * cout + co] = v[0];
-        }
-    }
-}
-
 // out[tap][chunk][row][8] from w[cout][9][cin] (zero rows and channels pad).
 __global__ void k_pack_weights(const float *w, __nv_bfloat16 *out, int cin, int cin_pad, int cout, int npad) {
     const int nchunk = cin_pad >> 3;
@@ -910,6 +848,23 @@ EncodeTiled encode_fn() {
     return fn;
 }
 
+// Tensor map of a planar tensor (n images of h x w, c channels, a multiple of
+// 8) for boxes of bw x bh pixels and every chunk: dimensions (8 w, h, c / 8, n).
+cudaError_t tile_map(void *out, const __nv_bfloat16 *x, int n, int h, int w, int c, int bw, int bh) {
+    EncodeTiled enc = encode_fn();
+    if (!enc) return cudaErrorNotSupported;
+    const cuuint64_t px = (cuuint64_t)h * w, chunks = (cuuint64_t)c / 8;
+    const cuuint64_t dims[4] = {(cuuint64_t)w * 8, (cuuint64_t)h, chunks, (cuuint64_t)n};
+    const cuuint64_t strides[3] = {(cuuint64_t)w * 16, px * 16, px * chunks * 16};
+    const cuuint32_t box[4] = {(cuuint32_t)bw * 8, (cuuint32_t)bh, (cuuint32_t)chunks, 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    const CUresult r = enc(static_cast<CUtensorMap *>(out), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4,
+                           const_cast<__nv_bfloat16 *>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 }  // namespace
 
 size_t tc_packed_weight_elems(int cin_pad, int cout) { return (size_t)9 * cin_pad * ((cout + 15) / 16 * 16); }
@@ -976,18 +931,7 @@ cudaError_t tc_wgrad_plan(TcWgradPlan &p, const __nv_bfloat16 *g, int n, int h, 
         if (p.smem > kSmemMax) p.smem = kSmemMax;
     }
     p.partial_floats = (size_t)p.groups * 9 * cout * cin_pad;
-    EncodeTiled enc = encode_fn();
-    if (!enc) return cudaErrorNotSupported;
-    const cuuint64_t dims[4] = {(cuuint64_t)p.cout_pad, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n};
-    const cuuint64_t strides[3] = {(cuuint64_t)p.cout_pad * 2, (cuuint64_t)w * p.cout_pad * 2,
-                                   (cuuint64_t)h * w * p.cout_pad * 2};
-    const cuuint32_t box[4] = {8, kTileW, kTileH, 1};
-    const cuuint32_t estr[4] = {1, 1, 1, 1};
-    CUtensorMap *map = reinterpret_cast<CUtensorMap *>(p.gmap);
-    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16 *>(g), dims, strides, box,
-                           estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+    return tile_map(p.gmap, g, n, h, w, p.cout_pad, kTileW, kTileH);
 }
 
 cudaError_t conv3x3_wgrad_tc(const TcWgradPlan &p, const TcConvPlan &fwd, float *dw, float *partial, int *err,
@@ -1037,43 +981,35 @@ cudaError_t tc_conv_plan(TcConvPlan &p, const __nv_bfloat16 *x, int n, int h, in
     // too few tiles to fill the GPU twice: split the output channels into
     // chunks of a multiple of 16 (each CTA all nine taps for its chunk, so no
     // partial sums), the widest chunk that still gives one CTA per SM (every
-    // chunk's CTA loads the whole input halo, so narrower chunks cost loads);
-    // with a single 16-channel chunk, split the taps instead (partial sums and
-    // a finalize pass)
-    p.splits = 1;
+    // chunk's CTA loads the whole input halo, so narrower chunks cost loads)
     p.nsplit = 1;
     p.npad_full = p.npad;
-    if (tiles < 2LL * sm_count) {
-        if (p.npad >= 32) {
-            int cw = 16;
-            for (int c = p.npad / 2 / 16 * 16; c >= 16; c -= 16)
-                if (p.npad % c == 0 && tiles * (p.npad / c) >= (long long)sm_count) {
-                    cw = c;
-                    break;
-                }
-            p.nsplit = p.npad / cw;
-            p.npad = cw;
-        } else {
-            p.splits = (tiles * 3 >= 2LL * sm_count) ? 3 : 9;
-        }
+    if (tiles < 2LL * sm_count && p.npad >= 32) {
+        int cw = 16;
+        for (int c = p.npad / 2 / 16 * 16; c >= 16; c -= 16)
+            if (p.npad % c == 0 && tiles * (p.npad / c) >= (long long)sm_count) {
+                cw = c;
+                break;
+            }
+        p.nsplit = p.npad / cw;
+        p.npad = cw;
     }
-    p.taps_per_split = 9 / p.splits;
-    const size_t halo = (size_t)(cin / 8) * kPlaneBytes;
+    const size_t halo = ((size_t)(cin / 8) * kPlaneBytes + 127) & ~(size_t)127;  // TMA destinations: 128-byte aligned
     const size_t wtap = (size_t)cin * p.npad * 2;
     // a TMA box of the weight slice spans at most 256 (tap, chunk) rows
-    const bool box_ok = p.nsplit == 1 || (size_t)p.taps_per_split * (cin / 8) <= 256;
-    if (halo + p.taps_per_split * wtap <= kSmemBudget && box_ok) {
-        p.taps_per_stage = p.taps_per_split;
+    const bool box_ok = p.nsplit == 1 || (size_t)9 * (cin / 8) <= 256;
+    if (halo + 9 * wtap <= kSmemBudget && box_ok) {
+        p.taps_per_stage = 9;
         p.stages = 1;
     } else {
         p.taps_per_stage = 1;
         size_t fit = halo < kSmemBudget ? (kSmemBudget - halo) / wtap : 0;
         if (fit < 2) fit = 2;
-        p.stages = (int)(fit < (size_t)p.taps_per_split ? fit : (size_t)p.taps_per_split);
+        p.stages = (int)(fit < 9 ? fit : 9);
     }
     if (p.nsplit > 1 && (size_t)p.taps_per_stage * (cin / 8) > 256) return cudaErrorInvalidValue;
     // persistent pipelined kernel: no split, two halos and all weights resident
-    p.persistent = p.splits == 1 && p.nsplit == 1 && 2 * halo + 9 * wtap + 64 <= kSmemPersistent;
+    p.persistent = p.nsplit == 1 && 2 * halo + 9 * wtap + 64 <= kSmemPersistent;
     size_t smem;
     int cols = 32;
     if (p.persistent) {
@@ -1119,27 +1055,14 @@ cudaError_t tc_conv_plan(TcConvPlan &p, const __nv_bfloat16 *x, int n, int h, in
     } else {
         p.grid = p.tiles;
     }
-    p.partial_floats = p.splits > 1 ? (size_t)p.splits * n * h * w * p.npad : 0;
-
-    EncodeTiled enc = encode_fn();
-    if (!enc) return cudaErrorNotSupported;
-    const cuuint64_t dims[4] = {(cuuint64_t)cin, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n};
-    const cuuint64_t strides[3] = {(cuuint64_t)cin * 2, (cuuint64_t)w * cin * 2, (cuuint64_t)h * w * cin * 2};
-    const cuuint32_t box[4] = {8, kHaloW, kHaloH, 1};
-    const cuuint32_t estr[4] = {1, 1, 1, 1};
-    CUtensorMap *map = reinterpret_cast<CUtensorMap *>(p.tmap);
-    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16 *>(x), dims, strides,
-                           box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+    return tile_map(p.tmap, x, n, h, w, cin, kHaloW, kHaloH);
 }
 
 cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked, const float *bias,
-                               __nv_bfloat16 *y, float *y32, float *partial, int *err, cudaStream_t st,
-                               const TcFuse *fuse, bool overlap_prologue) {
-    if (p.splits > 1 && !partial) return cudaErrorInvalidValue;
+                               __nv_bfloat16 *y, float *y32, int *err, cudaStream_t st, const TcFuse *fuse,
+                               bool overlap_prologue) {
+    if (y && (p.cout & 15)) return cudaErrorInvalidValue;
     if (fuse) {
-        if (p.splits > 1) return cudaErrorInvalidValue;
         if ((fuse->pool || fuse->cat) && (p.cout & 15)) return cudaErrorInvalidValue;
         if (fuse->cat && (fuse->cat_c & 7 || fuse->cat_off & 7 || fuse->cat_off + p.cout > fuse->cat_c))
             return cudaErrorInvalidValue;
@@ -1161,13 +1084,11 @@ cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked
     }
     TcArgs a;
     a.w = wpacked, a.bias = bias;
-    a.y = p.splits > 1 ? nullptr : y;
-    a.y32 = p.splits > 1 ? nullptr : y32;
-    a.partial = p.splits > 1 ? partial : nullptr;
+    a.y = y, a.y32 = y32;
     a.n = p.n, a.h = p.h, a.wd = p.w, a.cin = p.cin, a.cout = p.cout, a.npad = p.npad, a.relu = p.relu;
     a.tiles_x = p.tiles_x, a.tiles_y = p.tiles_y;
-    a.taps_per_split = p.taps_per_split, a.taps_per_stage = p.taps_per_stage, a.stages = p.stages;
-    a.nsplit = p.nsplit, a.npad_full = p.npad_full;
+    a.taps_per_stage = p.taps_per_stage, a.stages = p.stages;
+    a.nsplit = p.nsplit;
     a.tmem_cols = p.tmem_cols;
     a.w_off = p.w_off, a.bar_off = p.bar_off, a.halo_stride = p.halo_stride;
     a.err = err;
@@ -1202,19 +1123,10 @@ cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked
         cfg.gridDim = dim3((unsigned)p.grid), cfg.blockDim = dim3(kWsThreads);
         e = cudaLaunchKernelEx(&cfg, k_conv_tc_persistent, map, a);
     } else {
-        cfg.gridDim = dim3((unsigned)p.tiles, (unsigned)(p.nsplit > 1 ? p.nsplit : p.splits)), cfg.blockDim = dim3(128);
+        cfg.gridDim = dim3((unsigned)p.tiles, (unsigned)p.nsplit), cfg.blockDim = dim3(128);
         e = cudaLaunchKernelEx(&cfg, k_conv_tc, map, wmap, a);
     }
-    if (e == cudaSuccess) e = cudaGetLastError();
-    if (e != cudaSuccess || p.splits == 1) return e;
-    const size_t M = (size_t)p.n * p.h * p.w;
-    if ((p.cout & 3) == 0)
-        k_conv_finalize<4><<<grid_for(M * p.cout / 4), 256, 0, st>>>(partial, bias, y, y32, M, p.npad, p.cout,
-                                                                      p.splits, p.relu);
-    else
-        k_conv_finalize<1><<<grid_for(M * p.cout), 256, 0, st>>>(partial, bias, y, y32, M, p.npad, p.cout, p.splits,
-                                                                  p.relu);
-    return cudaGetLastError();
+    return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 }  // namespace dn
