@@ -164,6 +164,70 @@ __device__ __forceinline__ void mma(uint32_t tmem, uint64_t ad, uint64_t bd, uin
         : "memory");
 }
 
+// One lane of the (converged) warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred P;\n elect.sync _|P, 0xffffffff;\n selp.u32 %0, 1, 0, P;\n}\n" : "=r"(p));
+    return p != 0;
+}
+
+// The MMAs of ntaps taps (9, or the single tap `tap0`) over kPairs pairs of
+// 8-channel chunks, the accumulation in (tap, chunk) order. a: start of the
+// halo, b: start of the taps' packed weights, both in 16-byte units; bpair:
+// weights of a chunk pair (2 npad). Only the start addresses of the
+// descriptors change, by constants once unrolled: an MMA of N = 32 takes the
+// tensor cores 41 clocks (the 4 KB + 1 KB of operands at 128 bytes per clock),
+// which the issuing thread keeps up with only if it has little to compute per
+// MMA (rebuilding descriptors in a rolled loop took it 95 to 220 clocks per
+// MMA, whatever N).
+template <int kPairs>
+__device__ __forceinline__ void issue_taps(uint32_t tmem, uint32_t a, uint32_t b, uint32_t bpair, uint32_t idesc,
+                                           int tap0, int ntaps) {
+    constexpr uint32_t kRow = kRowBytes >> 4, kPair = 2 * (kPlaneBytes >> 4);
+    constexpr uint64_t ahi = ((uint64_t)(kPlaneBytes >> 4) << 16) | ((uint64_t)(kRowBytes >> 4) << 32) | (1ull << 46);
+    const uint64_t bhi = ((uint64_t)(bpair >> 1) << 16) | ((uint64_t)(128 >> 4) << 32) | (1ull << 46);
+    if (ntaps == 9) {
+        uint32_t acc = 0;
+#pragma unroll 1
+        for (int dy = 0; dy < 3; dy++) {
+#pragma unroll(kPairs <= 2 ? 3 : 1)
+            for (int dx = 0; dx < 3; dx++) {
+#pragma unroll
+                for (int p = 0; p < kPairs; p++) {
+                    mma(tmem, ahi | (a + dx + p * kPair), bhi | b, idesc, acc);
+                    acc = 1;
+                    b += bpair;
+                }
+            }
+            a += kRow;
+        }
+    } else {
+        a += (tap0 / 3) * kRow + tap0 % 3;
+#pragma unroll
+        for (int p = 0; p < kPairs; p++) {
+            mma(tmem, ahi | (a + p * kPair), bhi | b, idesc, (tap0 | p) != 0 ? 1u : 0u);
+            b += bpair;
+        }
+    }
+}
+
+// issue_taps for any number of channels (the network's pair counts unrolled).
+__device__ __forceinline__ void issue_taps(int pairs, uint32_t tmem, uint32_t a, uint32_t b, uint32_t bpair,
+                                           uint32_t idesc, int tap0, int ntaps) {
+    switch (pairs) {
+    case 1: return issue_taps<1>(tmem, a, b, bpair, idesc, tap0, ntaps);
+    case 2: return issue_taps<2>(tmem, a, b, bpair, idesc, tap0, ntaps);
+    case 3: return issue_taps<3>(tmem, a, b, bpair, idesc, tap0, ntaps);
+    case 4: return issue_taps<4>(tmem, a, b, bpair, idesc, tap0, ntaps);
+    case 5: return issue_taps<5>(tmem, a, b, bpair, idesc, tap0, ntaps);
+    case 6: return issue_taps<6>(tmem, a, b, bpair, idesc, tap0, ntaps);
+    case 7: return issue_taps<7>(tmem, a, b, bpair, idesc, tap0, ntaps);
+    case 8: return issue_taps<8>(tmem, a, b, bpair, idesc, tap0, ntaps);
+    case 10: return issue_taps<10>(tmem, a, b, bpair, idesc, tap0, ntaps);
+    case 14: return issue_taps<14>(tmem, a, b, bpair, idesc, tap0, ntaps);
+    }
+}
+
 __device__ __forceinline__ void commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -292,8 +356,7 @@ __global__ void __launch_bounds__(128) k_conv_tc(const __grid_constant__ CUtenso
     const int n0 = (int)blockIdx.y * P.npad;
     const int nloads = 9 / P.taps_per_stage;
     const int kchunks = P.cin >> 3;  // 8-channel chunks per tap (the weight map's third coordinate)
-    const uint32_t wtap_bytes = (uint32_t)P.cin * P.npad * 2;
-    const uint32_t stage_bytes = wtap_bytes * P.taps_per_stage;
+    const uint32_t stage_bytes = (uint32_t)P.cin * P.npad * 2 * P.taps_per_stage;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -340,17 +403,8 @@ __global__ void __launch_bounds__(128) k_conv_tc(const __grid_constant__ CUtenso
             }
             consumed = j + 1;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int q = 0; q < P.taps_per_stage; q++) {
-                const int tap = j * P.taps_per_stage + q;
-                const int dy = tap / 3, dx = tap - 3 * (tap / 3);
-                const uint32_t a0 = halo + (uint32_t)(dy * kHaloW + dx) * 16;
-                const uint32_t b0 = wbase + s * stage_bytes + q * wtap_bytes;
-                for (int p = 0; p < nchunk / 2; p++) {
-                    const uint64_t ad = smem_desc(a0 + 2 * p * kPlaneBytes, kPlaneBytes, kRowBytes);
-                    const uint64_t bd = smem_desc(b0 + 2 * p * P.npad * 16, P.npad * 16, 128);
-                    mma(tmem, ad, bd, idesc, (j | q | p) != 0 ? 1u : 0u);
-                }
-            }
+            issue_taps(nchunk / 2, tmem, halo >> 4, (wbase + s * stage_bytes) >> 4, 2 * P.npad, idesc, j,
+                       P.taps_per_stage);
             commit(bar(2 + P.stages + s));
             // refill the stage of the previous load once its MMAs are done
             // (this load's MMAs are queued behind them)
@@ -482,7 +536,7 @@ __global__ void __launch_bounds__(kWsThreads) k_conv_tc_persistent(const __grid_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && items > 0) {
+        if (items > 0 && elect_one()) {
             bool ok = mbar_wait(bar(wbar), 0);
             *w_waited = 1;
             if (!ok) *abort_flag = 1;
@@ -500,17 +554,8 @@ __global__ void __launch_bounds__(kWsThreads) k_conv_tc_persistent(const __grid_
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t acc = tmem + (uint32_t)(a * acc_stride);
-                const uint32_t hb = halo0 + (uint32_t)h * P.halo_stride;
-                for (int tap = 0; tap < 9; tap++) {
-                    const int dy = tap / 3, dx = tap - 3 * (tap / 3);
-                    const uint32_t a0 = hb + (uint32_t)(dy * kHaloW + dx) * 16;
-                    const uint32_t b0 = wbase + (uint32_t)tap * P.cin * P.npad * 2;
-                    for (int p = 0; p < nchunk / 2; p++) {
-                        const uint64_t ad = smem_desc(a0 + 2 * p * kPlaneBytes, kPlaneBytes, kRowBytes);
-                        const uint64_t bd = smem_desc(b0 + 2 * p * P.npad * 16, P.npad * 16, 128);
-                        mma(acc, ad, bd, idesc, (tap | p) != 0 ? 1u : 0u);
-                    }
-                }
+                issue_taps(nchunk / 2, acc, (halo0 + (uint32_t)h * P.halo_stride) >> 4, wbase >> 4, 2 * P.npad, idesc,
+                           0, 9);
                 commit(bar(empty0 + h));
                 commit(bar(accf0 + a));
             }
@@ -666,12 +711,11 @@ __global__ void __launch_bounds__(128) k_wgrad_tc(const __grid_constant__ CUtens
             for (int q = 0; q < ntaps; q++) {
                 const int tap = tap0 + q, dy = tap / 3, dx = tap - 3 * (tap / 3);
                 const uint32_t d = tmem + (uint32_t)(q * P.cin_pad);
-                for (int k = 0; k < kTileH / 2; k++) {
-                    const uint64_t ad = smem_desc(a + (uint32_t)k * 256u, 128u, kGradPlaneBytes);
-                    const uint64_t bd =
-                        smem_desc(b + (uint32_t)((2 * k + dy) * kHaloW + dx) * 16u, kRowBytes, kPlaneBytes);
-                    mma(d, ad, bd, idesc, (i == 0 && k == 0) ? 0u : 1u);
-                }
+                const uint64_t ad = smem_desc(a, 128u, kGradPlaneBytes);
+                const uint64_t bd = smem_desc(b + (uint32_t)(dy * kHaloW + dx) * 16u, kRowBytes, kPlaneBytes);
+#pragma unroll
+                for (int k = 0; k < kTileH / 2; k++)  // two tile rows per step
+                    mma(d, ad + k * (256u >> 4), bd + k * (2 * kRowBytes >> 4), idesc, (i == 0 && k == 0) ? 0u : 1u);
             }
             commit(bar(2 + st));
             committed = i + 1;
@@ -969,7 +1013,11 @@ cudaError_t conv3x3_wgrad_tc(const TcWgradPlan &p, const TcConvPlan &fwd, float 
 cudaError_t tc_conv_plan(TcConvPlan &p, const __nv_bfloat16 *x, int n, int h, int w, int cin, int cout, bool relu,
                          int sm_count) {
     std::memset(&p, 0, sizeof(p));
-    if (n <= 0 || h <= 0 || w <= 0 || cin <= 0 || (cin & 15) || cin > 2040 || cout <= 0) return cudaErrorInvalidValue;
+    // (the pair counts that issue_taps unrolls)
+    const int pairs = cin / 16;
+    if (n <= 0 || h <= 0 || w <= 0 || cin <= 0 || (cin & 15) || cout <= 0 ||
+        !(pairs <= 8 || pairs == 10 || pairs == 14))
+        return cudaErrorInvalidValue;
     p.x = x, p.n = n, p.h = h, p.w = w, p.cin = cin, p.cout = cout, p.relu = relu ? 1 : 0;
     p.npad = (cout + 15) / 16 * 16;
     if (p.npad > 256) return cudaErrorInvalidValue;
