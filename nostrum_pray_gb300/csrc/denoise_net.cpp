@@ -358,7 +358,8 @@ cudaError_t Denoiser::forward(const float *rad, const __half *feat, int n, int h
         dn::TcFuse f;
         f.res = x0, f.res_c = x0_c;
         f.rad = out_rad, f.feat = feat;
-        chk(conv_fwd(conv, act_[prev], nullptr, out_, st, &f, fuse));
+        // (inference: the log-space output stays unwritten)
+        chk(conv_fwd(conv, act_[prev], nullptr, infer ? nullptr : out_, st, &f, fuse));
     } else {
         chk(conv_fwd(conv, act_[prev], nullptr, out_, st));
         chk(dn::add_input(out_, x0, x0_c, px, st));

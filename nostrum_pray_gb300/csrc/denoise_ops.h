@@ -25,10 +25,12 @@ struct TcConvPlan {
     alignas(64) unsigned char tmap[128];  // CUtensorMap of x: (8 W, H, C / 8, N), box (80, 18, C / 8, 1)
     const __nv_bfloat16 *x;
     int n, h, w, cin, cout, npad, relu;
-    int tiles_x, tiles_y, tiles, taps_per_stage, stages, tmem_cols;
-    int nsplit, npad_full;  // output-channel split: nsplit CTAs per tile, npad channels each of npad_full
-    int persistent, grid;  // persistent pipelined kernel (no split, weights resident) and its CTAs
-    uint32_t w_off, bar_off, halo_stride;
+    int tiles_x, tiles_y, tiles;
+    int nsplit, npad_full;        // output-channel chunks of npad channels each, of npad_full
+    int grid, per_sm;             // persistent CTAs of each chunk, and the CTAs per SM it was planned for
+    int ring, wstages;            // halo slots; weight slots of a tap each (9: all resident)
+    int acc_slots, acc_stride, tmem_cols;
+    uint32_t halo_stride, w_off, bias_off, bar_off;
     size_t smem;
 };
 cudaError_t tc_conv_plan(TcConvPlan &p, const __nv_bfloat16 *x, int n, int h, int w, int cin, int cout, bool relu,
@@ -65,7 +67,9 @@ cudaError_t tc_pack_all(const TcPackJob *jobs_dev, int njobs, size_t total, cuda
 //   res:  FP32 output += res[pixel * res_c + channel] (BF16);
 //   rad:  (cout 3) rad = expm1(FP32 output) * (max(albedo, 0) + kDemodFloor),
 //         the albedo from feat (7 halves per pixel).
-// pool and cat need cout a multiple of 16, res and rad the FP32 output.
+// pool and cat need cout a multiple of 16; pool comes with cat at the same
+// pixel; res (cout at most 4) goes with rad or the FP32 output, which take no
+// other store.
 struct TcFuse {
     __nv_bfloat16 *pool = nullptr;
     __nv_bfloat16 *cat = nullptr;

@@ -5,29 +5,24 @@
 // (16 bytes per pixel and chunk), which is the layout the tensor cores read
 // from shared memory, so a halo is copied as whole rows.
 //
-// Implicit GEMM without an im2col copy. One CTA (4 warps) computes a tile of
-// 16 x 8 output pixels (M = 128) x all output channels (N = Cout rounded up
-// to 16). The input halo of the tile, 18 x 10 pixels x Cin, is loaded by one
+// Implicit GEMM without an im2col copy. A tile is 16 x 8 output pixels (M =
+// 128) x a chunk of the output channels (N, a multiple of 16). Its input halo,
+// 18 x 10 pixels x Cin, is loaded by one
 // 4-D TMA copy (rows of 160 contiguous bytes; out-of-image pixels arrive
 // as zeros, which is the convolution's padding) into planes of
 // [y][x][8 channels]. With channels-last tensors the same halo is a box of
-// 16-byte rows, ten times as many requests: the copies, not HBM or the
-// tensor cores, bounded the wide levels (80 -> 32 channels at 8 x 512^2: 171 us
-// against PLANAR_US). In the planes the A operand of
+// 16-byte rows, ten times as many requests (512^2 frame: 262 us against 216 us
+// planar). In the planes the A operand of
 // tap (dy, dx) for 16 channels is the halo itself seen through a shared-memory
 // matrix descriptor: the tile's 8-pixel rows are the 8-row core-matrix
 // groups (stride 160 bytes = one halo row), the two 8-channel chunks are the
 // K-direction core matrices (stride = one plane), and the start address moves
 // by (dy * 10 + dx) * 16 bytes. So all nine taps read the same halo and the
 // threads gather nothing. The weights are packed once (tc_pack_weights) as
-// [tap][8-channel chunk][row][8] BF16 — exactly the no-swizzle K-major
-// core-matrix layout — and copied with plain bulk copies, all taps at once
-// when they fit or through a ring of per-tap stages. One thread issues the
-// kind::f16 MMAs (M 128, N Npad, K 16) and commits them to mbarriers.
-//
-// The deep, small levels have too few tiles for 152 SMs: there each tile's
-// output channels are split over CTAs (each loads its slice of the weights
-// with one 3-D TMA box).
+// [tap][8-channel chunk][row][8] BF16 - exactly the no-swizzle K-major
+// core-matrix layout - and a CTA copies the rows of its channels tap by tap.
+// One thread issues the kind::f16 MMAs (M 128, N Npad, K 16) and commits them
+// to mbarriers. See k_conv_tc for the pipeline and tc_conv_plan for the split.
 //
 // The epilogue also performs the network's glue (TcFuse): 2 x 2 average
 // pooling, nearest 2x upsampling into a concatenation, the residual add and
@@ -36,6 +31,7 @@
 // Every mbarrier wait is bounded: on timeout the kernel records an error,
 // stops issuing, waits (bounded) for the copies and MMAs it issued, and frees
 // its TMEM.
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <cstring>
@@ -58,26 +54,25 @@ constexpr int kHaloW = kTileW + 2, kHaloH = kTileH + 2;
 constexpr uint32_t kPlaneBytes = kHaloW * kHaloH * 16;  // one 8-channel halo plane (2880), planes back to back
 constexpr uint32_t kRowBytes = kHaloW * 16;             // one halo row of one plane (160)
 constexpr uint32_t kWaitLimit = 1u << 24;
-constexpr size_t kSmemBudget = 110 * 1024;              // target per CTA (two or more CTAs per SM)
-constexpr size_t kSmemPersistent = 200 * 1024;          // persistent kernel: up to one CTA per SM
 constexpr size_t kSmemMax = 227 * 1024;
 constexpr size_t kSmemPerSm = 228 * 1024;
+constexpr int kTaps = 9;
 
 struct TcArgs {
-    const __nv_bfloat16 *w;  // packed weights [tap][chunk][npad][8]
-    const float *bias;
+    const __nv_bfloat16 *w;  // packed weights [tap][chunk][row][8]
+    const float *bias;       // NULL: none
     __nv_bfloat16 *y;
     float *y32;
     int n, h, wd, cin, cout, npad, relu;
     int tiles_x, tiles_y;
-    int taps_per_stage, stages;
-    int nsplit;               // > 1: blockIdx.y picks output channels [y * npad, (y + 1) * npad), the weight
-                              // slice by TMA (wmap) from the packing of all rows
-    int tmem_cols;
-    uint32_t w_off, bar_off;  // shared-memory offsets (the halo is at 0)
-    uint32_t halo_stride;     // persistent kernel: distance between the halo ring's slots
+    int ring;                // halo slots
+    int wstages;             // kTaps: every tap's weights resident; else a ring of taps
+    int nsplit;              // > 1: blockIdx.y picks output channels [y * npad, (y + 1) * npad), the weight
+                             // rows by TMA (wmap) from the packing of all rows
+    int acc_slots, acc_stride, tmem_cols;  // accumulators, TMEM columns from one to the next
+    uint32_t halo_stride, w_off, bias_off, bar_off;  // shared-memory layout (the halos are at 0)
     int *err;
-    TcFuse f;                 // extra stores of the epilogue
+    TcFuse f;                // extra stores of the epilogue
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -171,60 +166,40 @@ __device__ __forceinline__ bool elect_one() {
     return p != 0;
 }
 
-// The MMAs of ntaps taps (9, or the single tap `tap0`) over kPairs pairs of
-// 8-channel chunks, the accumulation in (tap, chunk) order. a: start of the
-// halo, b: start of the taps' packed weights, both in 16-byte units; bpair:
-// weights of a chunk pair (2 npad). Only the start addresses of the
-// descriptors change, by constants once unrolled: an MMA of N = 32 takes the
-// tensor cores 41 clocks (the 4 KB + 1 KB of operands at 128 bytes per clock),
-// which the issuing thread keeps up with only if it has little to compute per
-// MMA (rebuilding descriptors in a rolled loop took it 95 to 220 clocks per
-// MMA, whatever N).
+// The MMAs of one tap over kPairs pairs of 8-channel chunks. a: the halo at
+// the tap's offset, b: the tap's packed weights, both in 16-byte units; bpair:
+// weights of a chunk pair (2 npad); acc: 0 for the tile's first MMA. Only the
+// start addresses of the descriptors change, by constants once unrolled: an
+// MMA of N = 32 takes the tensor cores 41 clocks (4 KB + 1 KB of operands at
+// 128 bytes per clock), which the issuing thread keeps up with only if it has
+// little to compute per MMA (rebuilding descriptors in a rolled loop took it
+// 95 to 220 clocks per MMA, whatever N).
 template <int kPairs>
-__device__ __forceinline__ void issue_taps(uint32_t tmem, uint32_t a, uint32_t b, uint32_t bpair, uint32_t idesc,
-                                           int tap0, int ntaps) {
-    constexpr uint32_t kRow = kRowBytes >> 4, kPair = 2 * (kPlaneBytes >> 4);
+__device__ __forceinline__ void issue_tap(uint32_t tmem, uint32_t a, uint32_t b, uint32_t bpair, uint32_t idesc,
+                                          uint32_t acc) {
+    constexpr uint32_t kPair = 2 * (kPlaneBytes >> 4);
     constexpr uint64_t ahi = ((uint64_t)(kPlaneBytes >> 4) << 16) | ((uint64_t)(kRowBytes >> 4) << 32) | (1ull << 46);
     const uint64_t bhi = ((uint64_t)(bpair >> 1) << 16) | ((uint64_t)(128 >> 4) << 32) | (1ull << 46);
-    if (ntaps == 9) {
-        uint32_t acc = 0;
-#pragma unroll 1
-        for (int dy = 0; dy < 3; dy++) {
-#pragma unroll(kPairs <= 2 ? 3 : 1)
-            for (int dx = 0; dx < 3; dx++) {
 #pragma unroll
-                for (int p = 0; p < kPairs; p++) {
-                    mma(tmem, ahi | (a + dx + p * kPair), bhi | b, idesc, acc);
-                    acc = 1;
-                    b += bpair;
-                }
-            }
-            a += kRow;
-        }
-    } else {
-        a += (tap0 / 3) * kRow + tap0 % 3;
-#pragma unroll
-        for (int p = 0; p < kPairs; p++) {
-            mma(tmem, ahi | (a + p * kPair), bhi | b, idesc, (tap0 | p) != 0 ? 1u : 0u);
-            b += bpair;
-        }
+    for (int p = 0; p < kPairs; p++) {
+        mma(tmem, ahi | (a + p * kPair), bhi | b, idesc, acc);
+        acc = 1;
+        b += bpair;
     }
 }
 
-// issue_taps for any number of channels (the network's pair counts unrolled).
-__device__ __forceinline__ void issue_taps(int pairs, uint32_t tmem, uint32_t a, uint32_t b, uint32_t bpair,
-                                           uint32_t idesc, int tap0, int ntaps) {
-    switch (pairs) {
-    case 1: return issue_taps<1>(tmem, a, b, bpair, idesc, tap0, ntaps);
-    case 2: return issue_taps<2>(tmem, a, b, bpair, idesc, tap0, ntaps);
-    case 3: return issue_taps<3>(tmem, a, b, bpair, idesc, tap0, ntaps);
-    case 4: return issue_taps<4>(tmem, a, b, bpair, idesc, tap0, ntaps);
-    case 5: return issue_taps<5>(tmem, a, b, bpair, idesc, tap0, ntaps);
-    case 6: return issue_taps<6>(tmem, a, b, bpair, idesc, tap0, ntaps);
-    case 7: return issue_taps<7>(tmem, a, b, bpair, idesc, tap0, ntaps);
-    case 8: return issue_taps<8>(tmem, a, b, bpair, idesc, tap0, ntaps);
-    case 10: return issue_taps<10>(tmem, a, b, bpair, idesc, tap0, ntaps);
-    case 14: return issue_taps<14>(tmem, a, b, bpair, idesc, tap0, ntaps);
+// All nine taps, accumulated in (tap, chunk) order (one or two chunk pairs:
+// the taps of a row unrolled too).
+template <int kPairs>
+__device__ __forceinline__ void issue_tile(uint32_t tmem, uint32_t a, uint32_t b, uint32_t bpair, uint32_t idesc) {
+    uint32_t acc = 0;
+#pragma unroll 1
+    for (int dy = 0; dy < 3; dy++, a += kRowBytes >> 4) {
+#pragma unroll(kPairs <= 2 ? 3 : 1)
+        for (int dx = 0; dx < 3; dx++, b += kPairs * bpair) {
+            issue_tap<kPairs>(tmem, a + dx, b, bpair, idesc, acc);
+            acc = 1;
+        }
     }
 }
 
@@ -232,213 +207,195 @@ __device__ __forceinline__ void commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// The epilogue's arithmetic on pairs: FP32 add, BF16 rounding, and max(., 0)
+// of a rounded pair (the same value as rounding max(., 0): NaN gives 0).
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t pair(uint32_t lo, uint32_t hi) { return (uint64_t)hi << 32 | lo; }
+__device__ __forceinline__ uint32_t round2(uint64_t v) {
+    uint32_t d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "r"((uint32_t)(v >> 32)), "r"((uint32_t)v));
+    return d;
+}
+__device__ __forceinline__ uint32_t relu2(uint32_t v) {
+    uint32_t d;
+    asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(v), "r"(0u));
+    return d;
+}
+// The two values of a BF16 pair as FP32.
+__device__ __forceinline__ uint64_t widen2(uint32_t w) { return pair(w << 16, w & 0xFFFF0000u); }
+
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t *>(&v);
 }
 
-// Epilogue of one tile: the calling warp reads TMEM lanes 32q..32q+31 (q =
-// quad, the warp's lane quadrant: its warp index mod 4; tile rows m = pixel
-// (m / 8, m % 8)) from column `tmem` on, 16 columns at a time, and stores
-// bias + ReLU as BF16 (planar: the eight pixels of a tile row are 128
-// contiguous bytes per chunk) or FP32 (channels last), plus the extra stores
-// of P.f. A warp holds four whole tile rows, so the 2 x 2 blocks
-// of the pooling are lanes (l, l + 1, l + 8, l + 9) for l with even row and
-// column, summed in the order of k_avgpool (row-major).
-__device__ __forceinline__ void epilogue(const TcArgs &P, uint32_t tmem, int img, int y0, int x0, int quad,
-                                         int n0 = 0) {
-    const int lane = (int)(threadIdx.x & 31);
-    const int m = quad * 32 + lane;
-    const int yy = y0 + (m >> 3), xx = x0 + (m & 7);
-    const bool valid = yy < P.h && xx < P.wd;
-    const size_t px = (size_t)P.h * P.wd, at = (size_t)yy * P.wd + xx;  // one plane, the pixel in it
-    const size_t pix = img * px + at;
-    const bool vec = (P.y || P.f.pool || P.f.cat) && (P.cout & 15) == 0;
-    for (int c0 = 0; c0 < P.npad; c0 += 16) {
-        uint32_t r[16];
-        const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
+// TMEM columns [c, c + 16 kBlocks) of the warp's 32 lanes.
+template <int kBlocks>
+__device__ __forceinline__ void load_tmem(uint32_t taddr, uint32_t *r) {
+#pragma unroll
+    for (int b = 0; b < kBlocks; b++)
         asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
             "[%16];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-              "=r"(r[15])
-            : "r"(taddr)
+            : "=r"(r[16 * b]), "=r"(r[16 * b + 1]), "=r"(r[16 * b + 2]), "=r"(r[16 * b + 3]), "=r"(r[16 * b + 4]),
+              "=r"(r[16 * b + 5]), "=r"(r[16 * b + 6]), "=r"(r[16 * b + 7]), "=r"(r[16 * b + 8]),
+              "=r"(r[16 * b + 9]), "=r"(r[16 * b + 10]), "=r"(r[16 * b + 11]), "=r"(r[16 * b + 12]),
+              "=r"(r[16 * b + 13]), "=r"(r[16 * b + 14]), "=r"(r[16 * b + 15])
+            : "r"(taddr + 16 * b)
             : "memory");
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        // the pooling's shuffles need every lane of the warp
-        if (!valid && !(vec && P.f.pool)) continue;
-        if (vec) {
-            const int chunk = (n0 + c0) >> 3;  // this and the next 8-channel chunk of the output
-            float v[16];
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// What a convolution stores (a kernel instance each): the BF16 outputs; also
+// their 2 x 2 averages and a copy into a concatenation; also (or only) the
+// outputs upsampled into a concatenation; FP32 outputs (channels last), with
+// the residual and the output transform.
+enum EpiMode { kEpiY, kEpiPool, kEpiUp, kEpiF32 };
+
+// A warp's share of a tile: one pixel per lane (tile row m = pixel (m / 8,
+// m % 8)), the planes' size and where the pixel's first stores go.
+struct EpiPixel {
+    int lane;
+    bool valid, pool_valid;
+    uint32_t px, pp;       // pixels of a plane, of a pooled plane
+    uint4 *y, *cat, *pool; // the tile's chunk n0 / 8 at the lane's pixel
+    size_t pix;            // channels-last pixel
+    const __nv_bfloat16 *res;
+};
+
+// The stores of 16 channels (chunk q and q + 1 from the CTA's first;
+// accumulators r) of a lane's pixel: bias + ReLU as BF16 (planar: the eight
+// pixels of a tile row are 128 contiguous bytes per chunk) or FP32, plus the
+// extra stores of P.f. bias: the 16 channels' (shared memory); c: the first.
+template <int kMode>
+__device__ __forceinline__ void store16(const TcArgs &P, const uint32_t *r, const EpiPixel &e, int q, int c,
+                                        const float *bias) {
+    uint64_t v[8];
 #pragma unroll
-            for (int k = 0; k < 16; k++) {
-                v[k] = __uint_as_float(r[k]) + __ldg(P.bias + n0 + c0 + k);
-                if (P.relu) v[k] = fmaxf(v[k], 0.f);
-            }
-            const uint4 lo = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
-            const uint4 hi =
-                make_uint4(pack2(v[8], v[9]), pack2(v[10], v[11]), pack2(v[12], v[13]), pack2(v[14], v[15]));
-            if (valid && P.y) {
-                uint4 *o = reinterpret_cast<uint4 *>(P.y) + ((size_t)img * (P.cout >> 3) + chunk) * px + at;
-                o[0] = lo, o[px] = hi;
-            }
-            if (valid && P.f.cat) {
-                uint4 *o = reinterpret_cast<uint4 *>(P.f.cat);
-                const size_t plane = (size_t)img * (P.f.cat_c >> 3) + (P.f.cat_off >> 3) + chunk;
-                if (P.f.cat_up) {
-                    // the pixel's 2 x 2 block: two neighbours (32 bytes) in each of two rows
-                    const size_t W2 = 2 * (size_t)P.wd;
-                    o += plane * 4 * px + 2 * yy * W2 + 2 * xx;
-                    o[0] = lo, o[1] = lo, o[W2] = lo, o[W2 + 1] = lo;
-                    o += 4 * px;
-                    o[0] = hi, o[1] = hi, o[W2] = hi, o[W2 + 1] = hi;
-                } else {
-                    o += plane * px + at;
-                    o[0] = lo, o[px] = hi;
-                }
-            }
-            if (P.f.pool) {
-                const uint32_t wd[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-                uint32_t po[8];
+    for (int k = 0; k < 8; k += 2) {
+        const uint4 b = *reinterpret_cast<const uint4 *>(bias + 2 * k);
+        v[k] = add2(pair(r[2 * k], r[2 * k + 1]), pair(b.x, b.y));
+        v[k + 1] = add2(pair(r[2 * k + 2], r[2 * k + 3]), pair(b.z, b.w));
+    }
+    if (kMode == kEpiF32) {
+        if (!e.valid) return;
+        uint2 res = make_uint2(0u, 0u);  // four channels of the residual
+        if (e.res) res = *reinterpret_cast<const uint2 *>(e.res);
 #pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    const __nv_bfloat162 a2 = *reinterpret_cast<const __nv_bfloat162 *>(&wd[k]);
-                    const float a0 = __low2float(a2), a1 = __high2float(a2);
-                    const float b0 = __shfl_down_sync(0xFFFFFFFFu, a0, 1), b1 = __shfl_down_sync(0xFFFFFFFFu, a1, 1);
-                    const float c0v = __shfl_down_sync(0xFFFFFFFFu, a0, 8);
-                    const float c1v = __shfl_down_sync(0xFFFFFFFFu, a1, 8);
-                    const float d0 = __shfl_down_sync(0xFFFFFFFFu, a0, 9), d1 = __shfl_down_sync(0xFFFFFFFFu, a1, 9);
-                    po[k] = pack2(0.25f * (a0 + b0 + c0v + d0), 0.25f * (a1 + b1 + c1v + d1));
-                }
-                const int ho = P.h >> 1, wo = P.wd >> 1, yo = yy >> 1, xo = xx >> 1;
-                if (((lane >> 3) & 1) == 0 && (lane & 1) == 0 && yo < ho && xo < wo) {
-                    const size_t pp = (size_t)ho * wo;
-                    uint4 *o = reinterpret_cast<uint4 *>(P.f.pool) + ((size_t)img * (P.cout >> 3) + chunk) * pp +
-                               (size_t)yo * wo + xo;
-                    o[0] = make_uint4(po[0], po[1], po[2], po[3]);
-                    o[pp] = make_uint4(po[4], po[5], po[6], po[7]);
-                }
+        for (int k = 0; k < 16; k++) {
+            const int co = c + k;
+            if (co >= P.cout) break;
+            float u = __uint_as_float((uint32_t)(k & 1 ? v[k / 2] >> 32 : v[k / 2]));
+            if (P.relu) u = fmaxf(u, 0.f);
+            if (k < 4 && e.res) {
+                const uint32_t w = k < 2 ? res.x : res.y;
+                u += __uint_as_float(k & 1 ? w & 0xFFFF0000u : w << 16);
             }
-        } else {
+            if (P.y32) P.y32[e.pix * P.cout + co] = u;
+            if (P.f.rad)
+                P.f.rad[e.pix * 3 + co] =
+                    expm1f(u) * (fmaxf(__half2float(P.f.feat[7 * e.pix + co]), 0.f) + kDemodFloor);
+        }
+        return;
+    }
+    uint32_t w[8];
 #pragma unroll
-            for (int k = 0; k < 16; k++) {
-                const int co = n0 + c0 + k;
-                if (co >= P.cout) break;
-                float v = __uint_as_float(r[k]) + __ldg(P.bias + co);
-                if (P.relu) v = fmaxf(v, 0.f);
-                if (P.f.res) v += __bfloat162float(P.f.res[((size_t)img * (P.f.res_c >> 3) * px + at) * 8 + co]);
-                if (P.y32) P.y32[pix * P.cout + co] = v;
-                if (P.f.rad)
-                    P.f.rad[pix * 3 + co] =
-                        expm1f(v) * (fmaxf(__half2float(P.f.feat[7 * pix + co]), 0.f) + kDemodFloor);
-            }
+    for (int k = 0; k < 8; k++) w[k] = P.relu ? relu2(round2(v[k])) : round2(v[k]);
+    const uint4 lo = make_uint4(w[0], w[1], w[2], w[3]), hi = make_uint4(w[4], w[5], w[6], w[7]);
+    if (e.valid && P.y) {
+        uint4 *o = e.y + (size_t)q * e.px;
+        o[0] = lo, o[e.px] = hi;
+    }
+    if (kMode == kEpiUp && e.valid) {
+        // the pixel's 2 x 2 block: two neighbours (32 bytes) in each of two rows
+        const uint32_t W2 = 2 * (uint32_t)P.wd;
+        uint4 *o = e.cat + (size_t)q * 4 * e.px;
+        o[0] = lo, o[1] = lo, o[W2] = lo, o[W2 + 1] = lo;
+        o += 4 * e.px;
+        o[0] = hi, o[1] = hi, o[W2] = hi, o[W2 + 1] = hi;
+    }
+    if (kMode == kEpiPool) {
+        if (e.valid) {
+            uint4 *o = e.cat + (size_t)q * e.px;
+            o[0] = lo, o[e.px] = hi;
+        }
+        // A warp holds four whole tile rows: a 2 x 2 block is lanes l (even
+        // row and column), l + 1, l + 8, l + 9. Each of the four averages two
+        // of the eight channel pairs: the lanes of a column pair exchange
+        // halves, then the rows exchange quarters, both values of each row
+        // kept so that the sum is in the order of k_avgpool (row-major).
+        constexpr unsigned kFull = 0xFFFFFFFFu;
+        const bool odd = e.lane & 1, low = e.lane & 8;
+        uint32_t a[4], b[4];  // the row's left and right pixel, four pairs
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint32_t got = __shfl_xor_sync(kFull, odd ? w[k] : w[4 + k], 1);
+            a[k] = odd ? got : w[k], b[k] = odd ? w[4 + k] : got;
+        }
+        uint32_t o[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const uint32_t ga = __shfl_xor_sync(kFull, low ? a[k] : a[2 + k], 8);
+            const uint32_t gb = __shfl_xor_sync(kFull, low ? b[k] : b[2 + k], 8);
+            const uint32_t ta = low ? ga : a[k], tb = low ? gb : b[k];          // the upper row's
+            const uint32_t ba = low ? a[2 + k] : ga, bb = low ? b[2 + k] : gb;  // the lower row's
+            const uint64_t s = add2(add2(add2(widen2(ta), widen2(tb)), widen2(ba)), widen2(bb));
+            o[k] = pack2(0.25f * __uint_as_float((uint32_t)s), 0.25f * __uint_as_float((uint32_t)(s >> 32)));
+        }
+        // pairs 0-3 are the first chunk, 4-7 the second
+        if (e.pool_valid) {
+            uint2 *d = reinterpret_cast<uint2 *>(e.pool + (size_t)(q + (odd ? 1 : 0)) * e.pp) + (low ? 1 : 0);
+            *d = make_uint2(o[0], o[1]);
         }
     }
 }
 
-__global__ void __launch_bounds__(128) k_conv_tc(const __grid_constant__ CUtensorMap xmap,
-                                                 const __grid_constant__ CUtensorMap wmap, TcArgs P) {
-    extern __shared__ __align__(1024) uint8_t smem[];
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int nchunk = P.cin >> 3;
-    const uint32_t halo = smem_u32(smem), wbase = halo + P.w_off;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + P.bar_off);
-    // bars[0] halo loaded, bars[1] all MMAs done, bars[2 + s] stage s loaded,
-    // bars[2 + stages + s] stage s consumed by its MMAs
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 + 2 * P.stages);
-    int *okflag = reinterpret_cast<int *>(tmem_slot + 1);
-    auto bar = [&](int i) { return smem_u32(&bars[i]); };
-
-    const int per_img = P.tiles_x * P.tiles_y;
-    const int img = blockIdx.x / per_img, rem = blockIdx.x - img * per_img;
-    const int y0 = (rem / P.tiles_x) * kTileH, x0 = (rem % P.tiles_x) * kTileW;
-    const int n0 = (int)blockIdx.y * P.npad;
-    const int nloads = 9 / P.taps_per_stage;
-    const int kchunks = P.cin >> 3;  // 8-channel chunks per tap (the weight map's third coordinate)
-    const uint32_t stage_bytes = (uint32_t)P.cin * P.npad * 2 * P.taps_per_stage;
-
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(P.tmem_cols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+// Epilogue of one tile: the calling warp reads TMEM lanes 32q..32q+31 (q =
+// quad, the warp's lane quadrant: its warp index mod 4) from column `tmem`
+// on, 32 columns at a time.
+template <int kMode>
+__device__ __forceinline__ void epilogue(const TcArgs &P, uint32_t tmem, int img, int y0, int x0, int quad, int n0,
+                                         const float *bias) {
+    EpiPixel e;
+    e.lane = (int)(threadIdx.x & 31);
+    const int m = quad * 32 + e.lane, yy = y0 + (m >> 3), xx = x0 + (m & 7);
+    e.valid = yy < P.h && xx < P.wd;
+    e.px = (uint32_t)P.h * (uint32_t)P.wd;
+    const uint32_t at = (uint32_t)yy * (uint32_t)P.wd + (uint32_t)xx;
+    const int q0 = n0 >> 3;
+    if (kMode == kEpiF32) {
+        e.pix = (size_t)img * e.px + at;
+        e.res = P.f.res ? P.f.res + ((size_t)img * (P.f.res_c >> 3) * e.px + at) * 8 : nullptr;
+    } else {
+        e.y = reinterpret_cast<uint4 *>(P.y) + ((size_t)img * (P.cout >> 3) + q0) * e.px + at;
     }
-    if (tid == 0) {
-        for (int i = 0; i < 2 + 2 * P.stages; i++) mbar_init(bar(i));
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (kMode == kEpiPool || kMode == kEpiUp) {
+        const size_t plane = (size_t)img * (P.f.cat_c >> 3) + (P.f.cat_off >> 3) + q0;
+        e.cat = reinterpret_cast<uint4 *>(P.f.cat);
+        if (kMode == kEpiUp) e.cat += plane * 4 * e.px + 4 * (size_t)yy * P.wd + 2 * xx;
+        else e.cat += plane * e.px + at;
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
-
-    if (tid == 0) {
-        bool ok = true;
-        // weights: the first `stages` loads; with the output-channel split, one
-        // TMA box per load: rows n0..n0+npad of every (tap, chunk) of the stage
-        int issued = 0;
-        auto load_weights = [&](int stage, int load) {
-            mbar_expect_tx(bar(2 + stage), stage_bytes);
-            if (P.nsplit > 1)
-                tma_w(wbase + stage * stage_bytes, &wmap, bar(2 + stage), n0, load * P.taps_per_stage * kchunks);
-            else
-                bulk_copy(wbase + stage * stage_bytes, P.w + (size_t)load * P.taps_per_stage * P.cin * P.npad,
-                          stage_bytes, bar(2 + stage));
-        };
-        for (; issued < nloads && issued < P.stages; issued++) load_weights(issued, issued);
-        // the weights do not depend on the previous kernel; the input does
-        grid_dependency_wait();
-        mbar_expect_tx(bar(0), (uint32_t)nchunk * kPlaneBytes);
-        tma_tile(halo, &xmap, bar(0), x0 - 1, y0 - 1, img);
-        const bool halo_done = mbar_wait(bar(0), 0);
-        ok = halo_done;
-        const uint32_t idesc = inst_desc(128, P.npad);
-        int consumed = 0;
-        for (int j = 0; j < nloads && ok; j++) {
-            const int s = j % P.stages;
-            if (!mbar_wait(bar(2 + s), (uint32_t)(j / P.stages) & 1)) {
-                ok = false;
-                break;
-            }
-            consumed = j + 1;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            issue_taps(nchunk / 2, tmem, halo >> 4, (wbase + s * stage_bytes) >> 4, 2 * P.npad, idesc, j,
-                       P.taps_per_stage);
-            commit(bar(2 + P.stages + s));
-            // refill the stage of the previous load once its MMAs are done
-            // (this load's MMAs are queued behind them)
-            if (j >= 1 && issued < nloads) {
-                const int jp = j - 1, sp = jp % P.stages;
-                if (!mbar_wait(bar(2 + P.stages + sp), (uint32_t)(jp / P.stages) & 1)) {
-                    ok = false;
-                    break;
-                }
-                load_weights(sp, issued);
-                issued++;
-            }
-        }
-        // all MMAs issued so far complete on bars[1]
-        commit(bar(1));
-        if (!ok) {
-            // drain copies still in flight (bounded) before the shared memory goes away
-            if (!halo_done) mbar_wait(bar(0), 0);
-            for (int j = consumed; j < issued; j++) mbar_wait(bar(2 + j % P.stages), (uint32_t)(j / P.stages) & 1);
-        }
-        *okflag = ok ? 1 : 0;
+    if (kMode == kEpiPool) {
+        const int ho = P.h >> 1, wo = P.wd >> 1, yo = yy >> 1, xo = xx >> 1;
+        e.pool_valid = yo < ho && xo < wo;
+        e.pp = (uint32_t)ho * (uint32_t)wo;
+        e.pool = reinterpret_cast<uint4 *>(P.f.pool) + ((size_t)img * (P.cout >> 3) + q0) * e.pp + (uint32_t)yo * wo + xo;
     }
-    __syncthreads();
-    const bool ok = mbar_wait(bar(1), 0) && *okflag;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (!ok && tid == 0) atomicExch(P.err, 1);
-    if (ok) epilogue(P, tmem, img, y0, x0, warp, n0);
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 0) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(P.tmem_cols)
-                     : "memory");
+    const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16);
+    uint32_t r[32];
+    int c0 = 0;
+    for (; c0 + 32 <= P.npad; c0 += 32) {
+        load_tmem<2>(taddr + c0, r);
+        store16<kMode>(P, r, e, c0 >> 3, n0 + c0, bias + c0);
+        store16<kMode>(P, r + 16, e, (c0 >> 3) + 2, n0 + c0 + 16, bias + c0 + 16);
+    }
+    if (c0 < P.npad) {
+        load_tmem<1>(taddr + c0, r);
+        store16<kMode>(P, r, e, c0 >> 3, n0 + c0, bias + c0);
     }
 }
 
@@ -450,52 +407,139 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-constexpr int kWsThreads = 192;  // warp 0 loads, warp 1 issues MMAs, warps 2-5 drain accumulators
+constexpr int kEpiGroups = 3;  // groups of four epilogue warps
+constexpr int kConvThreads = 64 + 128 * kEpiGroups;
 
-// Persistent, warp-specialised variant for levels that need no split and
-// whose weights fit in shared memory beside a ring of halos. Each CTA loads
-// the weights once and walks tiles blockIdx.x, blockIdx.x + gridDim.x, ...:
-//   warp 0 (one thread) loads tile i's halo into ring slot i % H once the
-//     MMAs of tile i - H have released it;
-//   warp 1 (one thread) waits for the halo and for accumulator i % 2 to be
-//     drained, issues the tile's MMAs into it and commits them to the slot's
-//     "released" and the accumulator's "full" barriers;
-//   warps 2-5 (one TMEM lane quadrant each) drain accumulator i % 2 to
-//     global memory and release it.
-// So halo loads, MMAs and epilogues of consecutive tiles overlap. Every wait
+// A position in a ring of n slots and its phase (the parity of the completed
+// rounds), moved on without divisions: the roles' loops are one thread's or
+// one warp's serial chains, and the divisions by the ring sizes and the tile
+// counts took more time per tile than 9 MMAs do.
+struct Ring {
+    int n, slot = 0;
+    uint32_t phase = 0;
+    __device__ __forceinline__ explicit Ring(int slots) : n(slots) {}
+    __device__ __forceinline__ void next() {
+        if (++slot == n) slot = 0, phase ^= 1u;
+    }
+};
+
+// Every `step`-th tile from `first` on: image, row and column of tiles.
+struct TileWalk {
+    int img, ty, tx, d_img, d_ty, d_tx, tiles_x, tiles_y;
+    __device__ __forceinline__ TileWalk(int first, int step, int tx_n, int ty_n) : tiles_x(tx_n), tiles_y(ty_n) {
+        const int per = tx_n * ty_n;
+        img = first / per, d_img = step / per;
+        first -= img * per, step -= d_img * per;
+        ty = first / tx_n, tx = first - ty * tx_n;
+        d_ty = step / tx_n, d_tx = step - d_ty * tx_n;
+    }
+    __device__ __forceinline__ int x0() const { return tx * kTileW; }
+    __device__ __forceinline__ int y0() const { return ty * kTileH; }
+    __device__ __forceinline__ void next() {
+        img += d_img, ty += d_ty, tx += d_tx;
+        if (tx >= tiles_x) tx -= tiles_x, ty++;
+        if (ty >= tiles_y) ty -= tiles_y, img++;
+    }
+};
+
+// The state that the roles of a convolution's CTA share.
+struct ConvCta {
+    uint32_t halo0, wbase, bars, tmem;
+    int items;
+    volatile int *abort_flag, *h_issued, *h_waited, *w_issued, *w_waited;
+    // barriers: halo loaded [H], halo released [H], accumulator full [A],
+    // drained [A], weights loaded [S], weights released [S], final drain
+    int hfull, hfree, afull, afree, wfull, wfree, dbar;
+    __device__ __forceinline__ uint32_t bar(int i) const { return bars + 8u * (uint32_t)i; }
+};
+
+// The MMA role (one thread) for Cin = 16 kPairs.
+template <int kPairs>
+__device__ __forceinline__ void conv_mma(const TcArgs &P, const ConvCta &C) {
+    const int H = P.ring, S = P.wstages, A = P.acc_slots;
+    const bool resident = S == kTaps;
+    const uint32_t idesc = inst_desc(128, P.npad), bpair = 2 * P.npad, wtap = (uint32_t)P.cin * P.npad * 2;
+    bool ok = true;
+    Ring h(H), a(A), w(S);
+    if (resident) {
+        ok = mbar_wait(C.bar(C.wfull), 0);
+        if (ok) *C.w_waited = 1;
+    }
+    for (int i = 0; i < C.items && ok && !*C.abort_flag; i++) {
+        if (!(ok = mbar_wait(C.bar(C.hfull + h.slot), h.phase))) break;
+        *C.h_waited = i + 1;
+        if (i >= A && !(ok = mbar_wait(C.bar(C.afree + a.slot), a.phase ^ 1u))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t acc = C.tmem + (uint32_t)(a.slot * P.acc_stride);
+        const uint32_t hb = (C.halo0 + (uint32_t)h.slot * P.halo_stride) >> 4;
+        if (resident) {
+            issue_tile<kPairs>(acc, hb, C.wbase >> 4, bpair, idesc);
+        } else {
+            uint32_t ha = hb;
+#pragma unroll 1
+            for (int tap = 0; tap < kTaps; tap++) {
+                if (!(ok = mbar_wait(C.bar(C.wfull + w.slot), w.phase))) break;
+                *C.w_waited = i * kTaps + tap + 1;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                issue_tap<kPairs>(acc, ha, (C.wbase + w.slot * wtap) >> 4, bpair, idesc, tap ? 1u : 0u);
+                commit(C.bar(C.wfree + w.slot));
+                w.next();
+                ha += tap == 2 || tap == 5 ? (kRowBytes >> 4) - 2 : 1;
+            }
+            if (!ok) break;
+        }
+        commit(C.bar(C.hfree + h.slot));
+        commit(C.bar(C.afull + a.slot));
+        h.next(), a.next();
+    }
+    if (!ok) *C.abort_flag = 1;
+    // everything this thread issued completes before TMEM is freed
+    commit(C.bar(C.dbar));
+    mbar_wait(C.bar(C.dbar), 0);
+}
+
+// One convolution. A persistent, warp-specialised CTA owns a chunk of the
+// output channels (blockIdx.y) and walks tiles blockIdx.x, blockIdx.x +
+// gridDim.x, ...:
+//   warp 0 (one thread) loads weights, either all nine taps once or, where
+//     they do not fit beside the halos, tap after tap through a ring of
+//     wstages slots for every tile; and tile i's halo into slot i % ring once
+//     the MMAs of tile i - ring have released it;
+//   warp 1 (one thread) waits for the halo, for accumulator i % acc_slots to be
+//     drained and for each tap's weights, issues the tile's MMAs and commits
+//     them to the slots' "released" and the accumulator's "full" barriers;
+//   the other warps, groups of four (one TMEM lane quadrant each), drain the
+//     accumulators of the tiles in turn to global memory and release them.
+// So loads, MMAs and epilogues of consecutive tiles overlap inside a CTA, and
+// one or two CTAs per SM suffice: more of them would start up one after
+// another (their tensor memory is allocated under a lock), 8 us before the
+// last of eight per SM had loaded its first tile. Every wait
 // is bounded; a timeout sets a shared abort flag that ends every role's
 // loop, and the copies and MMAs in flight are waited for (bounded) before
 // the shared memory and TMEM are released.
-__global__ void __launch_bounds__(kWsThreads) k_conv_tc_persistent(const __grid_constant__ CUtensorMap xmap,
-                                                                   TcArgs P) {
+template <int kMode>
+__global__ void __launch_bounds__(kConvThreads, 2) k_conv_tc(const __grid_constant__ CUtensorMap xmap,
+                                                             const __grid_constant__ CUtensorMap wmap, TcArgs P) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int H = P.stages;  // halo ring slots
+    const int H = P.ring, S = P.wstages, A = P.acc_slots;
+    const bool resident = S == kTaps;
     const int nchunk = P.cin >> 3;
-    const uint32_t halo0 = smem_u32(smem), wbase = halo0 + P.w_off;
+    float *bias = reinterpret_cast<float *>(smem + P.bias_off);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + P.bar_off);
-    // bars: [0, H) halo loaded, [H, 2H) halo released, 2H + a accumulator
-    // full, 2H + 2 + a accumulator drained, 2H + 4 weights loaded, 2H + 5
-    // final drain of the MMAs
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * H + 6);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    volatile int *issued = reinterpret_cast<volatile int *>(tmem_slot + 2);    // halos loaded so far
-    volatile int *consumed = reinterpret_cast<volatile int *>(tmem_slot + 3);  // halos the MMA warp waited for
-    volatile int *w_waited = reinterpret_cast<volatile int *>(tmem_slot + 4);
-    auto bar = [&](int i) { return smem_u32(&bars[i]); };
-    const int full0 = 0, empty0 = H, accf0 = 2 * H, acce0 = 2 * H + 2, wbar = 2 * H + 4, dbar = 2 * H + 5;
-    const int per_img = P.tiles_x * P.tiles_y;
-    const int tiles = P.n * per_img;
-    const int items = tiles > (int)blockIdx.x ? (tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-    auto tile_of = [&](int i, int &img, int &y0, int &x0) {
-        const int t = (int)blockIdx.x + i * (int)gridDim.x;
-        img = t / per_img;
-        const int rem = t - img * per_img;
-        y0 = (rem / P.tiles_x) * kTileH;
-        x0 = (rem % P.tiles_x) * kTileW;
-    };
-    const uint32_t wbytes = (uint32_t)P.cin * P.npad * 2 * 9;
-    const int acc_stride = (P.npad + 31) & ~31;  // TMEM columns between the two accumulators
+    ConvCta C;
+    C.halo0 = smem_u32(smem), C.wbase = C.halo0 + P.w_off, C.bars = smem_u32(bars);
+    C.hfull = 0, C.hfree = H, C.afull = 2 * H, C.afree = C.afull + A, C.wfull = C.afree + A, C.wfree = C.wfull + S,
+    C.dbar = C.wfree + S;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + C.dbar + 1);
+    C.abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    // loads issued by warp 0 and waited for by warp 1: halos, weights
+    C.h_issued = C.abort_flag + 1, C.h_waited = C.abort_flag + 2, C.w_issued = C.abort_flag + 3,
+    C.w_waited = C.abort_flag + 4;
+    const int n0 = (int)blockIdx.y * P.npad;
+    const int first = (int)blockIdx.x, step = (int)gridDim.x;
+    const int items = (P.n * P.tiles_x * P.tiles_y - 1 - first) / step + 1;
+    C.items = items;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -503,96 +547,119 @@ __global__ void __launch_bounds__(kWsThreads) k_conv_tc_persistent(const __grid_
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (tid == 0) {
-        for (int i = 0; i < 2 * H; i++) mbar_init(bar(i));
-        mbar_init(bar(accf0)), mbar_init(bar(accf0 + 1));
-        mbar_init_count(bar(acce0), 128), mbar_init_count(bar(acce0 + 1), 128);
-        mbar_init(bar(wbar)), mbar_init(bar(dbar));
-        *abort_flag = 0, *issued = 0, *consumed = 0, *w_waited = 0;
+    if (tid == 32) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&xmap)) : "memory");
+        for (int i = 0; i < C.dbar + 1; i++) mbar_init_count(C.bar(i), i >= C.afree && i < C.wfull ? 128 : 1);
+        *C.abort_flag = 0, *C.h_issued = 0, *C.h_waited = 0, *C.w_issued = 0, *C.w_waited = 0;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    for (int i = tid - 64; i >= 0 && i < P.npad; i += kConvThreads - 64)
+        bias[i] = P.bias && n0 + i < P.cout ? __ldg(P.bias + n0 + i) : 0.f;
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
+    C.tmem = *tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0 && items > 0) {
-            mbar_expect_tx(bar(wbar), wbytes);
-            bulk_copy(wbase, P.w, wbytes, bar(wbar));
+        if (elect_one()) {
+            const uint32_t wtap = (uint32_t)P.cin * P.npad * 2;  // bytes of a tap's weights
+            // taps k and k + 1 ... k + n - 1 to consecutive slots from slot s
+            auto copy_taps = [&](int s, int tap, int n, uint32_t b) {
+                mbar_expect_tx(b, n * wtap);
+                if (P.nsplit == 1)
+                    bulk_copy(C.wbase + s * wtap, P.w + (size_t)tap * P.cin * P.npad, n * wtap, b);
+                else
+                    for (int t = 0; t < n; t++) tma_w(C.wbase + (s + t) * wtap, &wmap, b, n0, (tap + t) * nchunk);
+            };
+            Ring w(S), h(H);
+            TileWalk t(first, step, P.tiles_x, P.tiles_y);
+            int k = 0, next_tap = 0;  // taps and halos loaded so far, the next tap
+            int halos = 0;
+            auto load_tap = [&]() {
+                if (k >= S && !mbar_wait(C.bar(C.wfree + w.slot), w.phase ^ 1u)) return false;
+                copy_taps(w.slot, next_tap, 1, C.bar(C.wfull + w.slot));
+                *C.w_issued = ++k;
+                if (++next_tap == kTaps) next_tap = 0;
+                w.next();
+                return true;
+            };
+            auto load_halo = [&]() {
+                if (halos >= H && !mbar_wait(C.bar(C.hfree + h.slot), h.phase ^ 1u)) return false;
+                const uint32_t b = C.bar(C.hfull + h.slot);
+                mbar_expect_tx(b, (uint32_t)nchunk * kPlaneBytes);
+                tma_tile(C.halo0 + (uint32_t)h.slot * P.halo_stride, &xmap, b, t.x0() - 1, t.y0() - 1, t.img);
+                *C.h_issued = ++halos;
+                h.next(), t.next();
+                return true;
+            };
+            // the weights do not depend on the previous kernel; the input does
+            if (resident) copy_taps(0, 0, kTaps, C.bar(C.wfull)), *C.w_issued = 1;
+            else
+                while (k < S) load_tap();
             grid_dependency_wait();
-            for (int i = 0; i < items && !*abort_flag; i++) {
-                const int h = i % H;
-                if (i >= H && !mbar_wait(bar(empty0 + h), (uint32_t)((i / H) - 1) & 1)) {
-                    *abort_flag = 1;
-                    break;
-                }
-                int img, y0, x0;
-                tile_of(i, img, y0, x0);
-                const uint32_t dst = halo0 + (uint32_t)h * P.halo_stride;
-                mbar_expect_tx(bar(full0 + h), (uint32_t)nchunk * kPlaneBytes);
-                tma_tile(dst, &xmap, bar(full0 + h), x0 - 1, y0 - 1, img);
-                *issued = i + 1;
+            bool ok = load_halo();
+            for (int i = 0; i < items && ok && !*C.abort_flag; i++) {
+                // the next tile's halo before the rest of this one's weights
+                if (H > 1 && i + 1 < items) ok = load_halo();
+                if (!resident)
+                    while (ok && k < kTaps * (i + 1)) ok = load_tap();
+                if (H == 1 && i + 1 < items && ok) ok = load_halo();
             }
+            if (!ok) *C.abort_flag = 1;
         }
     } else if (warp == 1) {
-        if (items > 0 && elect_one()) {
-            bool ok = mbar_wait(bar(wbar), 0);
-            *w_waited = 1;
-            if (!ok) *abort_flag = 1;
-            const uint32_t idesc = inst_desc(128, P.npad);
-            for (int i = 0; i < items && ok && !*abort_flag; i++) {
-                const int h = i % H, a = i & 1;
-                if (!mbar_wait(bar(full0 + h), (uint32_t)(i / H) & 1)) {
-                    *abort_flag = 1;
-                    break;
-                }
-                *consumed = i + 1;
-                if (i >= 2 && !mbar_wait(bar(acce0 + a), (uint32_t)((i >> 1) - 1) & 1)) {
-                    *abort_flag = 1;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t acc = tmem + (uint32_t)(a * acc_stride);
-                issue_taps(nchunk / 2, acc, (halo0 + (uint32_t)h * P.halo_stride) >> 4, wbase >> 4, 2 * P.npad, idesc,
-                           0, 9);
-                commit(bar(empty0 + h));
-                commit(bar(accf0 + a));
+        if (elect_one()) {
+            switch (nchunk / 2) {  // the network's channel counts
+            case 1: conv_mma<1>(P, C); break;
+            case 2: conv_mma<2>(P, C); break;
+            case 3: conv_mma<3>(P, C); break;
+            case 4: conv_mma<4>(P, C); break;
+            case 5: conv_mma<5>(P, C); break;
+            case 6: conv_mma<6>(P, C); break;
+            case 7: conv_mma<7>(P, C); break;
+            case 8: conv_mma<8>(P, C); break;
+            case 10: conv_mma<10>(P, C); break;
+            case 14: conv_mma<14>(P, C); break;
+            default: *C.abort_flag = 1;
             }
-            // everything this thread issued completes before TMEM is freed
-            commit(bar(dbar));
-            mbar_wait(bar(dbar), 0);
         }
     } else {
-        const int quad = warp & 3;  // warps 2, 3, 4, 5 -> TMEM lane quadrants 2, 3, 0, 1
+        const int quad = warp & 3;  // the warp's TMEM lane quadrant
         // every decision warp-uniform: the TMEM loads below are warp-collective
-        for (int i = 0; i < items; i++) {
-            if (__any_sync(0xFFFFFFFFu, *abort_flag != 0)) break;
-            const int a = i & 1;
-            if (!__all_sync(0xFFFFFFFFu, mbar_wait(bar(accf0 + a), (uint32_t)(i >> 1) & 1))) {
-                if (lane == 0) *abort_flag = 1;
+        // No more groups than accumulators: a group that waits for tile i has
+        // seen tile i - groups done, so the slot's previous tile i - A is done
+        // too and its barrier is in the phase just before the one waited for
+        // (with fewer accumulators the wait could be met by the phase before
+        // that, whose parity is the same).
+        const int group = (warp - 2) >> 2, groups = A < kEpiGroups ? A : kEpiGroups;
+        TileWalk t(first + group * step, groups * step, P.tiles_x, P.tiles_y);
+        Ring acc(A);
+        for (int i = 0; i < group; i++) acc.next();
+        for (int i = group < groups ? group : items; i < items; i += groups, t.next()) {
+            if (__any_sync(0xFFFFFFFFu, *C.abort_flag != 0)) break;
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait(C.bar(C.afull + acc.slot), acc.phase))) {
+                if (lane == 0) *C.abort_flag = 1;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            int img, y0, x0;
-            tile_of(i, img, y0, x0);
-            epilogue(P, tmem + (uint32_t)(a * acc_stride), img, y0, x0, quad);
+            epilogue<kMode>(P, C.tmem + (uint32_t)(acc.slot * P.acc_stride), t.img, t.y0(), t.x0(), quad, n0, bias);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            mbar_arrive(bar(acce0 + a));
+            mbar_arrive(C.bar(C.afree + acc.slot));
+            for (int k = 0; k < groups; k++) acc.next();
         }
     }
     __syncthreads();
-    if (tid == 0 && *abort_flag) {
+    if (tid == 0 && *C.abort_flag) {
         atomicExch(P.err, 1);
         // copies still in flight (bounded) before the shared memory goes away
-        if (items > 0 && !*w_waited) mbar_wait(bar(wbar), 0);
-        for (int j = *consumed; j < *issued; j++) mbar_wait(bar(full0 + j % H), (uint32_t)(j / H) & 1);
+        for (int j = *C.h_waited; j < *C.h_issued; j++) mbar_wait(C.bar(C.hfull + j % H), (uint32_t)(j / H) & 1u);
+        for (int j = *C.w_waited; j < *C.w_issued; j++) mbar_wait(C.bar(C.wfull + j % S), (uint32_t)(j / S) & 1u);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(P.tmem_cols)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(C.tmem), "r"(P.tmem_cols)
                      : "memory");
     }
 }
@@ -1013,10 +1080,8 @@ cudaError_t conv3x3_wgrad_tc(const TcWgradPlan &p, const TcConvPlan &fwd, float 
 cudaError_t tc_conv_plan(TcConvPlan &p, const __nv_bfloat16 *x, int n, int h, int w, int cin, int cout, bool relu,
                          int sm_count) {
     std::memset(&p, 0, sizeof(p));
-    // (the pair counts that issue_taps unrolls)
-    const int pairs = cin / 16;
     if (n <= 0 || h <= 0 || w <= 0 || cin <= 0 || (cin & 15) || cout <= 0 ||
-        !(pairs <= 8 || pairs == 10 || pairs == 14))
+        !(cin <= 128 || cin == 160 || cin == 224))  // (the pair counts that issue() unrolls)
         return cudaErrorInvalidValue;
     p.x = x, p.n = n, p.h = h, p.w = w, p.cin = cin, p.cout = cout, p.relu = relu ? 1 : 0;
     p.npad = (cout + 15) / 16 * 16;
@@ -1026,83 +1091,70 @@ cudaError_t tc_conv_plan(TcConvPlan &p, const __nv_bfloat16 *x, int n, int h, in
     const long long tiles = (long long)n * p.tiles_x * p.tiles_y;
     if (tiles > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
     p.tiles = (int)tiles;
-    // too few tiles to fill the GPU twice: split the output channels into
-    // chunks of a multiple of 16 (each CTA all nine taps for its chunk, so no
-    // partial sums), the widest chunk that still gives one CTA per SM (every
-    // chunk's CTA loads the whole input halo, so narrower chunks cost loads)
-    p.nsplit = 1;
     p.npad_full = p.npad;
-    if (tiles < 2LL * sm_count && p.npad >= 32) {
-        int cw = 16;
-        for (int c = p.npad / 2 / 16 * 16; c >= 16; c -= 16)
-            if (p.npad % c == 0 && tiles * (p.npad / c) >= (long long)sm_count) {
-                cw = c;
-                break;
-            }
-        p.nsplit = p.npad / cw;
-        p.npad = cw;
-    }
+    // The split: a chunk width cw of the output channels (every CTA loads whole
+    // halos, so narrower chunks cost loads, and an MMA below N = 32 is no
+    // faster), one or two CTAs per SM, the weights resident or streamed. Taken
+    // is the one with the shortest estimate in clocks: per tile the larger of
+    // the SM's MMAs (operands at 128 bytes per clock, N / 2 clocks at least), its
+    // copies at 64 bytes per clock and its epilogue (kEpiClk), for the tiles that fall to one SM, plus the
+    // first tile's copies.
+    const int pairs = cin / 16;
+    constexpr double kEpiClk = 14.0;   // clocks per channel of a tile for one CTA's epilogue warps
+    constexpr double kRoleClk = 450.0; // what a CTA's MMA thread spends per tile besides the MMAs
     const size_t halo = ((size_t)(cin / 8) * kPlaneBytes + 127) & ~(size_t)127;  // TMA destinations: 128-byte aligned
+    double best = 0;
+    for (int cw = 16; cw <= p.npad_full; cw += 16) {
+        if (p.npad_full % cw) continue;
+        const int nsplit = p.npad_full / cw;
+        const size_t wtap = (size_t)cin * cw * 2;
+        const int stride = (cw + 31) & ~31;
+        for (int per_sm = 1; per_sm <= 2; per_sm++) {
+            const long long slots = (long long)sm_count * per_sm / nsplit;
+            if (slots < 1) continue;
+            const long long ctas = tiles < slots ? tiles : slots, items = (tiles + ctas - 1) / ctas;
+            int acc = items > 2 ? 4 : items > 1 ? 2 : 1, cols = 32;
+            while (acc > 1 && acc * stride * per_sm > 512) acc--;
+            while (cols < acc * stride) cols <<= 1;
+            if (cols * per_sm > 512) continue;
+            const size_t budget = per_sm == 2 ? kSmemPerSm / 2 - 1024 : kSmemMax;
+            const size_t misc = 4 * (size_t)cw + 8 * (2 * 4 + 2 * 4 + 2 * kTaps + 1) + 64;
+            for (int wst = kTaps; wst >= 3; wst--) {
+                const size_t rest = misc + wst * wtap;
+                if (rest + halo > budget) continue;
+                long long ring = (long long)((budget - rest) / halo);
+                if (ring > items) ring = items;
+                if (ring > 4) ring = 4;
+                const double mma = kTaps * pairs * (cw / 4 + 32 > cw / 2 ? cw / 4 + 32 : cw / 2);
+                const double load = ((double)halo + (wst < kTaps ? kTaps * wtap : 0)) / 64, epi = cw * kEpiClk;
+                double on_sm = (double)(ctas * nsplit + sm_count - 1) / sm_count;  // CTAs of the busiest SM
+                if (on_sm > per_sm) on_sm = per_sm;
+                double tile = std::max(on_sm * std::max(mma, load), std::max(mma + kRoleClk, epi));
+                if (ring == 1 && items > 1) tile += load / 2 + 600;  // nothing loaded beside the MMAs
+                double cost = items * tile + (halo + wst * wtap) / 64.0;
+                // small enough for the next kernel's CTAs to start up beside this one's
+                if (rest + ring * halo > kSmemPerSm / 2 - 1024) cost += 600;
+                if (best == 0 || cost < best) {
+                    best = cost;
+                    p.npad = cw, p.nsplit = nsplit, p.grid = (int)ctas, p.wstages = wst, p.ring = (int)ring;
+                    p.acc_slots = acc, p.acc_stride = stride, p.tmem_cols = cols;
+                    p.per_sm = per_sm;
+                }
+                break;  // fewer weight slots never help
+            }
+        }
+    }
+    if (best == 0) return cudaErrorInvalidValue;
     const size_t wtap = (size_t)cin * p.npad * 2;
-    // a TMA box of the weight slice spans at most 256 (tap, chunk) rows
-    const bool box_ok = p.nsplit == 1 || (size_t)9 * (cin / 8) <= 256;
-    if (halo + 9 * wtap <= kSmemBudget && box_ok) {
-        p.taps_per_stage = 9;
-        p.stages = 1;
-    } else {
-        p.taps_per_stage = 1;
-        size_t fit = halo < kSmemBudget ? (kSmemBudget - halo) / wtap : 0;
-        if (fit < 2) fit = 2;
-        p.stages = (int)(fit < 9 ? fit : 9);
-    }
-    if (p.nsplit > 1 && (size_t)p.taps_per_stage * (cin / 8) > 256) return cudaErrorInvalidValue;
-    // persistent pipelined kernel: no split, two halos and all weights resident
-    p.persistent = p.nsplit == 1 && 2 * halo + 9 * wtap + 64 <= kSmemPersistent;
-    size_t smem;
-    int cols = 32;
-    if (p.persistent) {
-        while (cols < 2 * ((p.npad + 31) & ~31)) cols <<= 1;
-        // a ring of three halos unless two keep more CTAs resident per SM
-        auto ring_smem = [&](int ring) {
-            const size_t bar = (ring * halo + 9 * wtap + 15) & ~(size_t)15;
-            return bar + 8 * (2 * (size_t)ring + 6) + 32;
-        };
-        auto resident = [&](int ring) {
-            const size_t by_smem = kSmemPerSm / (ring_smem(ring) + 1024), by_tmem = 512 / (size_t)cols;
-            return by_smem < by_tmem ? by_smem : by_tmem;
-        };
-        const int ring = ring_smem(3) <= kSmemPersistent && resident(3) >= resident(2) ? 3 : 2;
-        p.stages = ring;
-        p.halo_stride = (uint32_t)halo;
-        p.w_off = (uint32_t)(ring * halo);
-        p.bar_off = (uint32_t)((ring * halo + 9 * wtap + 15) & ~(size_t)15);
-        smem = ring_smem(ring);
-    } else {
-        p.halo_stride = 0;
-        p.w_off = (uint32_t)halo;
-        p.bar_off = (uint32_t)(halo + (size_t)p.stages * p.taps_per_stage * wtap);
-        p.bar_off = (p.bar_off + 15) & ~15u;
-        smem = p.bar_off + 8 * (2 + 2 * (size_t)p.stages) + 16;
-        while (cols < p.npad) cols <<= 1;
-    }
-    p.tmem_cols = cols;
+    p.halo_stride = (uint32_t)halo;
+    p.w_off = (uint32_t)(p.ring * halo);
+    p.bias_off = (uint32_t)(p.w_off + p.wstages * wtap);
+    p.bar_off = (p.bias_off + 4 * (uint32_t)p.npad + 15) & ~15u;
+    p.smem = p.bar_off + 8 * (2 * (size_t)p.ring + 2 * (size_t)p.acc_slots + 2 * (size_t)p.wstages + 1) + 32;
     // no more CTAs per SM than TMEM has columns for (tcgen05.alloc would wait)
-    const size_t max_ctas = 512 / cols;
-    if (smem > kSmemMax) return cudaErrorInvalidValue;
-    if (kSmemPerSm / (smem + 1024) > max_ctas) {
-        smem = kSmemPerSm / max_ctas - 1024 + 16;
-        if (smem > kSmemMax) smem = kSmemMax;  // one CTA per SM
-    }
-    p.smem = smem;
-    if (p.persistent) {
-        size_t per_sm = kSmemPerSm / (smem + 1024);
-        if (per_sm > max_ctas) per_sm = max_ctas;
-        if (per_sm < 1) per_sm = 1;
-        const long long slots = (long long)sm_count * (long long)per_sm;
-        p.grid = (int)(tiles < slots ? tiles : slots);
-    } else {
-        p.grid = p.tiles;
-    }
+    const size_t max_ctas = 512 / p.tmem_cols;
+    if (kSmemPerSm / (p.smem + 1024) > max_ctas) p.smem = kSmemPerSm / max_ctas - 1024 + 16;
+    if (p.smem > kSmemMax) p.smem = kSmemMax;
     return tile_map(p.tmap, x, n, h, w, cin, kHaloW, kHaloH);
 }
 
@@ -1114,7 +1166,10 @@ cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked
         if ((fuse->pool || fuse->cat) && (p.cout & 15)) return cudaErrorInvalidValue;
         if (fuse->cat && (fuse->cat_c & 7 || fuse->cat_off & 7 || fuse->cat_off + p.cout > fuse->cat_c))
             return cudaErrorInvalidValue;
-        if ((fuse->res || fuse->rad) && !y32) return cudaErrorInvalidValue;
+        // one of: pooling with the copy into a concatenation, upsampling, FP32
+        if ((fuse->pool != nullptr) != (fuse->cat && !fuse->cat_up)) return cudaErrorInvalidValue;
+        if ((y32 || fuse->rad) && (y || fuse->cat)) return cudaErrorInvalidValue;
+        if (fuse->res && (p.cout > 4 || (!y32 && !fuse->rad))) return cudaErrorInvalidValue;
         if (fuse->rad && (p.cout != 3 || !fuse->feat)) return cudaErrorInvalidValue;
     }
     // the shared-memory opt-in is a per-device setting of each kernel: once per device
@@ -1124,10 +1179,10 @@ cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked
     if (e0 != cudaSuccess) return e0;
     const uint64_t bit = dev < 64 ? 1ull << dev : 0;
     if (!bit || !(attr_set.load() & bit)) {
-        cudaError_t e = cudaFuncSetAttribute(k_conv_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_conv_tc_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
-        if (e != cudaSuccess) return e;
+        for (auto k : {k_conv_tc<kEpiY>, k_conv_tc<kEpiPool>, k_conv_tc<kEpiUp>, k_conv_tc<kEpiF32>}) {
+            const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
+            if (e != cudaSuccess) return e;
+        }
         attr_set.fetch_or(bit);
     }
     TcArgs a;
@@ -1135,10 +1190,9 @@ cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked
     a.y = y, a.y32 = y32;
     a.n = p.n, a.h = p.h, a.wd = p.w, a.cin = p.cin, a.cout = p.cout, a.npad = p.npad, a.relu = p.relu;
     a.tiles_x = p.tiles_x, a.tiles_y = p.tiles_y;
-    a.taps_per_stage = p.taps_per_stage, a.stages = p.stages;
-    a.nsplit = p.nsplit;
-    a.tmem_cols = p.tmem_cols;
-    a.w_off = p.w_off, a.bar_off = p.bar_off, a.halo_stride = p.halo_stride;
+    a.ring = p.ring, a.wstages = p.wstages, a.nsplit = p.nsplit;
+    a.acc_slots = p.acc_slots, a.acc_stride = p.acc_stride, a.tmem_cols = p.tmem_cols;
+    a.halo_stride = p.halo_stride, a.w_off = p.w_off, a.bias_off = p.bias_off, a.bar_off = p.bar_off;
     a.err = err;
     if (fuse) a.f = *fuse;
     CUtensorMap map, wmap;
@@ -1151,7 +1205,7 @@ cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked
         if (!enc) return cudaErrorNotSupported;
         const cuuint64_t dims[3] = {8, (cuuint64_t)p.npad_full, (cuuint64_t)9 * (p.cin / 8)};
         const cuuint64_t strides[2] = {16, (cuuint64_t)p.npad_full * 16};
-        const cuuint32_t box[3] = {8, (cuuint32_t)p.npad, (cuuint32_t)(p.taps_per_stage * (p.cin / 8))};
+        const cuuint32_t box[3] = {8, (cuuint32_t)p.npad, (cuuint32_t)(p.cin / 8)};  // one tap
         const cuuint32_t estr[3] = {1, 1, 1};
         const CUresult r = enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<__nv_bfloat16 *>(wpacked), dims,
                                strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -1166,14 +1220,11 @@ cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked
     cfg.stream = st;
     cfg.attrs = overlap_prologue ? attr : nullptr;
     cfg.numAttrs = overlap_prologue ? 1 : 0;
-    cudaError_t e;
-    if (p.persistent) {
-        cfg.gridDim = dim3((unsigned)p.grid), cfg.blockDim = dim3(kWsThreads);
-        e = cudaLaunchKernelEx(&cfg, k_conv_tc_persistent, map, a);
-    } else {
-        cfg.gridDim = dim3((unsigned)p.tiles, (unsigned)p.nsplit), cfg.blockDim = dim3(128);
-        e = cudaLaunchKernelEx(&cfg, k_conv_tc, map, wmap, a);
-    }
+    cfg.gridDim = dim3((unsigned)p.grid, (unsigned)p.nsplit), cfg.blockDim = dim3(kConvThreads);
+    const bool f32 = y32 || (fuse && fuse->rad), pool = fuse && fuse->pool, cat = fuse && fuse->cat;
+    const cudaError_t e = cudaLaunchKernelEx(
+        &cfg, f32 ? k_conv_tc<kEpiF32> : pool ? k_conv_tc<kEpiPool> : cat ? k_conv_tc<kEpiUp> : k_conv_tc<kEpiY>, map,
+        wmap, a);
     return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
