@@ -98,9 +98,7 @@ cudaError_t Denoiser::init(uint64_t seed) {
     if ((e = take(w_, total)) != cudaSuccess || (e = take(g_, total)) != cudaSuccess ||
         (e = take(m_, total)) != cudaSuccess || (e = take(v_, total)) != cudaSuccess ||
         (e = take(wb_, total)) != cudaSuccess || (e = take(wtc_, tc_total)) != cudaSuccess ||
-        (e = take(wtcb_, tcb_total)) != cudaSuccess || (e = take(zero_bias_, 256)) != cudaSuccess ||
-        (e = cudaMemset(zero_bias_, 0, 256 * sizeof(float))) != cudaSuccess ||
-        (e = take(loss_, 1 + dn::kL1Parts)) != cudaSuccess || (e = take(err_, 1)) != cudaSuccess ||
+        (e = take(wtcb_, tcb_total)) != cudaSuccess || (e = take(loss_, 1 + dn::kL1Parts)) != cudaSuccess || (e = take(err_, 1)) != cudaSuccess ||
         (e = cudaMemset(err_, 0, sizeof(int))) != cudaSuccess)
         return e;
     // He-normal weights, zero biases, from the seed
@@ -176,11 +174,10 @@ cudaError_t Denoiser::ensure(int n, int h, int w) {
     const size_t px = (size_t)n * h * w;
     if (px <= cap_pixels_ && h == h_ && w == w_dim_ && n == n_) return cudaSuccess;
     // keep the parameters, drop the activations
-    std::vector<void *> keep = {w_, g_, m_, v_, wb_, wtc_, wtcb_, zero_bias_, pack_jobs_, loss_, err_};
+    std::vector<void *> keep = {w_, g_, m_, v_, wb_, wtc_, wtcb_, pack_jobs_, loss_, err_};
     x16_ = nullptr;
-    gb16_ = nullptr;
-    bias_part_ = nullptr;
     partial_wg_ = nullptr;
+    backward_tc_ = backward_cc_ = false;
     plans_.assign(kNumConvs, dn::TcConvPlan{});
     plans_bwd_.assign(kNumConvs, dn::TcConvPlan{});
     plans_wg_.assign(kNumConvs, dn::TcWgradPlan{});
@@ -192,14 +189,13 @@ cudaError_t Denoiser::ensure(int n, int h, int w) {
     grad_.clear();
     n_ = n, h_ = h, w_dim_ = w;
     cudaError_t e;
-    auto act = [&](int level, int c, bool with_grad) -> cudaError_t {
+    auto act = [&](int level, int c) -> cudaError_t {
         const size_t p = (size_t)n * (h >> level) * (w >> level);
         Buf b;
         b.level = level;
         b.c = c;
         cudaError_t er = take(b.x, p * c);
         if (er != cudaSuccess) return er;
-        if (with_grad && (er = take(b.g, p * c)) != cudaSuccess) return er;
         act_.push_back(b);
         return cudaSuccess;
     };
@@ -207,34 +203,77 @@ cudaError_t Denoiser::ensure(int n, int h, int w) {
     //  0 x0(10)
     //  1 e0a 2 e0 | 3 p1 4 e1a 5 e1 | 6 p2 7 e2a 8 e2 | 9 p3 10 e3a 11 e3 | 12 p4 13 e4a 14 e4
     //  15 cat3 16 d3a 17 d3 | 18 cat2 19 d2a 20 d2 | 21 cat1 22 d1a 23 d1 | 24 cat0 25 d0a 26 d0
-    if ((e = act(0, 10, false)) != cudaSuccess) return e;
+    if ((e = act(0, 10)) != cudaSuccess) return e;
     for (int l = 0; l < 5; l++) {
-        if (l > 0 && (e = act(l, kEnc[l - 1], true)) != cudaSuccess) return e;  // pooled input
-        if ((e = act(l, kEnc[l], true)) != cudaSuccess) return e;
-        if ((e = act(l, kEnc[l], true)) != cudaSuccess) return e;
+        if (l > 0 && (e = act(l, kEnc[l - 1])) != cudaSuccess) return e;  // pooled input
+        if ((e = act(l, kEnc[l])) != cudaSuccess) return e;
+        if ((e = act(l, kEnc[l])) != cudaSuccess) return e;
     }
     for (int l = 3; l >= 0; l--) {
         const int up = (l == 3) ? kEnc[4] : kEnc[l + 1];
-        if ((e = act(l, up + kEnc[l], true)) != cudaSuccess) return e;  // concat
-        if ((e = act(l, kEnc[l], true)) != cudaSuccess) return e;
-        if ((e = act(l, kEnc[l], true)) != cudaSuccess) return e;
+        if ((e = act(l, up + kEnc[l])) != cudaSuccess) return e;  // concat
+        if ((e = act(l, kEnc[l])) != cudaSuccess) return e;
+        if ((e = act(l, kEnc[l])) != cudaSuccess) return e;
     }
-    if ((e = take(out_, px * 3)) != cudaSuccess || (e = take(gout_, px * 3)) != cudaSuccess ||
-        (e = take(gtmp_, px * 128)) != cudaSuccess || (e = take(x16_, px * pad16(kConvs[0][0]))) != cudaSuccess ||
-        (e = take(gb16_, px * 128)) != cudaSuccess ||
-        (e = take(bias_part_, (size_t)dn::kGradPrepBlocks * 128)) != cudaSuccess)
+    if ((e = take(out_, px * 3)) != cudaSuccess || (e = take(x16_, px * pad16(kConvs[0][0]))) != cudaSuccess)
         return e;
-    // per-group weight-gradient sums: the largest need of any convolution
-    size_t partial_wg = 0;
-    for (int i = 0; i < kNumConvs; i++) {
-        const int l = kLevel[i];
-        dn::TcWgradPlan wg;
-        if (dn::tc_wgrad_plan(wg, act_[0].x, n, h >> l, w >> l, kConvs[i][0], pad16(kConvs[i][0]), kConvs[i][1],
-                              sm_count_) == cudaSuccess)
-            partial_wg = std::max(partial_wg, wg.partial_floats);
-    }
-    if (partial_wg && (e = take(partial_wg_, partial_wg)) != cudaSuccess) return e;
     cap_pixels_ = px;
+    return cudaSuccess;
+}
+
+// Buffers and plans of the backward pass, made by the first one after a
+// change of size (inference needs none).
+cudaError_t Denoiser::ensure_backward() {
+    const size_t px = (size_t)n_ * h_ * w_dim_;
+    cudaError_t e = cudaSuccess;
+    if (!tensor_cores_) {
+        if (backward_cc_) return cudaSuccess;
+        for (size_t i = 1; i < act_.size(); i++)
+            if ((e = take(act_[i].g, (size_t)n_ * (h_ >> act_[i].level) * (w_dim_ >> act_[i].level) * act_[i].c)) !=
+                cudaSuccess)
+                return e;
+        if ((e = take(gout_, px * 3)) != cudaSuccess || (e = take(gtmp_, px * 128)) != cudaSuccess) return e;
+        backward_cc_ = true;
+        return cudaSuccess;
+    }
+    if (backward_tc_) return cudaSuccess;
+    auto pixels = [&](int level) { return (size_t)n_ * (h_ >> level) * (w_dim_ >> level); };
+    for (int l = 0; l < 4; l++)
+        if ((e = take(skip_g_[l], pixels(l) * kEnc[l])) != cudaSuccess) return e;
+    if ((e = take(l1_part_, (size_t)4 * dn::kL1Blocks)) != cudaSuccess) return e;
+    std::vector<dn::BiasJob> jobs;
+    size_t partial_wg = 0;
+    for (int i = kNumConvs - 1; i >= 0; i--) {
+        const Conv &c = convs_[i];
+        const int l = kLevel[i], h = h_ >> l, w = w_dim_ >> l;
+        __nv_bfloat16 *&g = gq_[i];
+        if ((e = take(g, pixels(l) * pad16(c.cout))) != cudaSuccess) return e;
+        // the output gradient of convolution i comes from the backward-data
+        // convolution of i + 1, that of the output convolution from the loss
+        dn::BiasJob j;
+        j.db = g_ + c.offset + (size_t)c.cout * 9 * c.cin;
+        j.c = c.cout;
+        if (i == kNumConvs - 1) {
+            j.part = l1_part_ + dn::kL1Blocks;
+            j.rows = dn::l1_blocks(px);
+        } else {
+            j.rows = plans_bwd_[i + 1].grid;
+            if ((e = take(bias_part_[i], (size_t)j.rows * c.cout)) != cudaSuccess) return e;
+            j.part = bias_part_[i];
+        }
+        jobs.push_back(j);
+        if (i > 0 && (e = dn::tc_conv_plan(plans_bwd_[i], g, n_, h, w, pad16(c.cout), c.cin, false, sm_count_,
+                                           true)) != cudaSuccess)
+            return e;
+        if ((e = dn::tc_wgrad_plan(plans_wg_[i], g, n_, h, w, c.cin, pad16(c.cin), c.cout, sm_count_)) != cudaSuccess)
+            return e;
+        partial_wg = std::max(partial_wg, plans_wg_[i].partial_floats);
+    }
+    if ((e = take(partial_wg_, partial_wg)) != cudaSuccess || (e = take(bias_jobs_, jobs.size())) != cudaSuccess ||
+        (e = cudaMemcpy(bias_jobs_, jobs.data(), jobs.size() * sizeof(jobs[0]), cudaMemcpyHostToDevice)) !=
+            cudaSuccess)
+        return e;
+    backward_tc_ = true;
     return cudaSuccess;
 }
 
@@ -369,6 +408,55 @@ cudaError_t Denoiser::forward(const float *rad, const __half *feat, int n, int h
 }
 
 cudaError_t Denoiser::backward(const float *target, cudaStream_t st) {
+    const cudaError_t e = ensure_backward();
+    if (e != cudaSuccess) return e;
+    return tensor_cores_ ? backward_tc(target, st) : backward_cc(target, st);
+}
+
+// On the tensor cores the input gradient of a convolution is a forward
+// convolution of its output gradient (BF16, ReLU-masked) with the transposed,
+// tap-mirrored weights, and its epilogue makes of it what the next one down
+// the chain reads (dn::TcFuse::grad): the masked BF16 gradient of the tensor's
+// producer, through the pooling, the concatenation and the upsampling, and
+// the producer's bias sums. So the chain is 18 convolutions and nothing
+// between them. Every output gradient has a buffer of its own; the weight
+// gradients follow the chain.
+cudaError_t Denoiser::backward_tc(const float *target, cudaStream_t st) {
+    const size_t px0 = (size_t)h_ * w_dim_, px = px0 * n_;
+    cudaError_t e = cudaSuccess;
+    auto chk = [&](cudaError_t x) { if (x != cudaSuccess && e == cudaSuccess) e = x; };
+    chk(dn::l1_loss_tc(out_, target, feat_, gq_[kNumConvs - 1], l1_part_, px, px0, st));
+    // the act_ index of the tensor whose gradient convolution i passes on (its
+    // input's producer), and the level of the skip tensor it shares or adds
+    static const int kMaskOf[kNumConvs] = {0,  1,  2,  4,  5,  7,  8,  10, 11, 13,
+                                           14, 16, 17, 19, 20, 22, 23, 25, 26};
+    for (int i = kNumConvs - 1; i >= 1; i--) {
+        dn::TcFuse f;
+        f.mask = act_[kMaskOf[i]].x;
+        f.g = gq_[i - 1];
+        f.bias_part = bias_part_[i - 1];
+        if (i == 2 || i == 4 || i == 6 || i == 8) {  // the input is pooled from encoder level i / 2 - 1
+            f.grad = dn::kGradUnpool;
+            f.skip = skip_g_[i / 2 - 1];
+        } else if (i == 10 || i == 12 || i == 14 || i == 16) {  // a concatenation at level (16 - i) / 2
+            f.grad = dn::kGradCat;
+            f.skip = skip_g_[(16 - i) / 2];
+            f.low_c = act_[kMaskOf[i]].c;
+        } else {
+            f.grad = dn::kGradMask;
+        }
+        // (its prologue loads the transposed weights, packed after the last
+        // optimizer step, beside the previous kernel)
+        chk(dn::conv3x3_forward_tc(plans_bwd_[i], wtcb_ + tcb_off_[i], nullptr, nullptr, nullptr, err_, st, &f, true));
+    }
+    for (int i = kNumConvs - 1; i >= 0; i--)
+        chk(dn::conv3x3_wgrad_tc(plans_wg_[i], plans_[i], g_ + convs_[i].offset, partial_wg_, err_, st));
+    chk(dn::bias_all(bias_jobs_, kNumConvs, 128, st));
+    chk(dn::l1_finalize(l1_part_, dn::l1_blocks(px), px * 3, loss_, st));
+    return e;
+}
+
+cudaError_t Denoiser::backward_cc(const float *target, cudaStream_t st) {
     const int n = n_, h = h_, w = w_dim_;
     const size_t px = (size_t)n * h * w;
     cudaError_t e = cudaSuccess;
@@ -379,52 +467,19 @@ cudaError_t Denoiser::backward(const float *target, cudaStream_t st) {
     chk(dn::l1_loss(out_, target, feat_, gout_, loss_, loss_ + 1, px * 3, st));
     // input gradient (when need_dx) and weight / bias gradients of convolution
     // ci from its output gradient g, masked by the ReLU of its output y (NULL:
-    // no ReLU). With the tensor cores the input gradient is a forward
-    // convolution of the masked gradient (BF16) with the transposed,
-    // tap-mirrored weights, and one pass over g gives that BF16 operand and
-    // the bias gradient.
+    // no ReLU)
     auto conv_bwd = [&](int ci, Buf &in, const float *g, const __nv_bfloat16 *y, int level, bool need_dx) {
         const Conv &c = convs_[ci];
         const int hh = h >> level, ww = w >> level;
         const size_t p = (size_t)n * hh * ww;
         float *dw = g_ + c.offset, *db = dw + (size_t)c.cout * 9 * c.cin;
-        if (!tensor_cores_) {
-            const float *gpre = g;
-            if (y) {
-                chk(dn::relu_mask(y, g, gtmp_, p * c.cout, st));
-                gpre = gtmp_;
-            }
-            chk(dn::conv3x3_backward(in.x, wb_ + c.offset, gpre, need_dx ? in.g : nullptr, dw, db, n, hh, ww, c.cin,
-                                     c.cout, st));
-            return;
+        const float *gpre = g;
+        if (y) {
+            chk(dn::relu_mask(y, g, gtmp_, p * c.cout, st));
+            gpre = gtmp_;
         }
-        chk(dn::grad_prep(y, g, gb16_, bias_part_, db, p, (size_t)hh * ww, c.cout, pad16(c.cout), st));
-        if (need_dx) {
-            dn::TcConvPlan &pl = plans_bwd_[ci];
-            if (pl.x != gb16_ || pl.n != n || pl.h != hh || pl.w != ww) {
-                cudaError_t pe = dn::tc_conv_plan(pl, gb16_, n, hh, ww, pad16(c.cout), c.cin, false, sm_count_);
-                if (pe != cudaSuccess) {
-                    pl.x = nullptr;
-                    chk(pe);
-                    return;
-                }
-            }
-            // programmatic launch: its prologue loads the transposed weights
-            // (packed after the last optimizer step) while the bias
-            // gradient's final sums (the last kernel of grad_prep) run
-            chk(dn::conv3x3_forward_tc(pl, wtcb_ + tcb_off_[ci], zero_bias_, nullptr, in.g, err_, st, nullptr,
-                                       true));
-        }
-        dn::TcWgradPlan &wg = plans_wg_[ci];
-        if (wg.g != gb16_ || wg.n != n || wg.h != hh || wg.w != ww) {
-            cudaError_t pe = dn::tc_wgrad_plan(wg, gb16_, n, hh, ww, c.cin, pad16(c.cin), c.cout, sm_count_);
-            if (pe != cudaSuccess) {
-                wg.g = nullptr;
-                chk(pe);
-                return;
-            }
-        }
-        chk(dn::conv3x3_wgrad_tc(wg, plans_[ci], dw, partial_wg_, err_, st));
+        chk(dn::conv3x3_backward(in.x, wb_ + c.offset, gpre, need_dx ? in.g : nullptr, dw, db, n, hh, ww, c.cin,
+                                 c.cout, st));
     };
     // output conv: input d0 (26), no ReLU
     conv_bwd(18, act_[26], gout_, nullptr, 0, true);

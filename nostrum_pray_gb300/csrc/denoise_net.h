@@ -58,6 +58,9 @@ class Denoiser {
     template <class T>
     cudaError_t take(T *&p, size_t n);
     cudaError_t ensure(int n, int h, int w);
+    cudaError_t ensure_backward();
+    cudaError_t backward_tc(const float *target, cudaStream_t st);
+    cudaError_t backward_cc(const float *target, cudaStream_t st);
     cudaError_t conv_fwd(int ci, const Buf &in, __nv_bfloat16 *y, float *y32, cudaStream_t st,
                          const dn::TcFuse *fuse = nullptr, bool overlap = false);
     // the tensor-core plan of convolution ci on input `in` (made on first use)
@@ -80,13 +83,17 @@ class Denoiser {
     std::vector<size_t> tc_off_;
     std::vector<dn::TcConvPlan> plans_;
     int sm_count_ = 0;
-    // tensor-core backward-data: per convolution the transposed, tap-mirrored
-    // packed weights (dn::tc_pack_weights_bwd) and a plan over the output
-    // gradient in BF16 (gb16_), and a zero bias
-    __nv_bfloat16 *wtcb_ = nullptr, *gb16_ = nullptr;
+    // tensor-core backward: per convolution the transposed, tap-mirrored packed
+    // weights (dn::tc_pack_weights_bwd), its output gradient (BF16, masked,
+    // planar), a backward-data and a weight-gradient plan over it and the
+    // per-CTA sums of its bias gradient; per encoder level the skip
+    // connection's share of the gradient (FP32, planar)
+    __nv_bfloat16 *wtcb_ = nullptr, *gq_[19] = {};
     std::vector<size_t> tcb_off_;
     std::vector<dn::TcConvPlan> plans_bwd_;
-    float *zero_bias_ = nullptr;
+    float *bias_part_[19] = {}, *skip_g_[4] = {}, *l1_part_ = nullptr;
+    dn::BiasJob *bias_jobs_ = nullptr;
+    bool backward_tc_ = false, backward_cc_ = false;  // backward buffers exist
     // every forward and backward-data packing as one launch (dn::tc_pack_all)
     dn::TcPackJob *pack_jobs_ = nullptr;
     int n_pack_jobs_ = 0;
@@ -94,7 +101,6 @@ class Denoiser {
     // tensor-core weight gradients: one plan per convolution, per-group partial sums
     std::vector<dn::TcWgradPlan> plans_wg_;
     float *partial_wg_ = nullptr;
-    float *bias_part_ = nullptr;  // per-block bias-gradient sums (dn::grad_prep)
     float *out_ = nullptr, *gout_ = nullptr, *gtmp_ = nullptr;
     const __half *feat_ = nullptr;  // features of the last forward (the caller's buffer; used until the call returns)
     int *err_ = nullptr;

@@ -179,65 +179,22 @@ __global__ void k_relu_mask(const __nv_bfloat16 *y, const float *g, float *out, 
     for (size_t i = gtid(); i < n; i += gstride()) out[i] = bf(y[i]) > 0.f ? g[i] : 0.f;
 }
 
-// Threads (r, q), r < rows, q < c_pad / 8: the 8-channel chunk q of pixels p0
-// + r, p0 + r + rows, ... of the block's range. y and out are planar (images
-// of px pixels), g channels last. c = 3 or a multiple of 8.
-__global__ void k_grad_prep(const __nv_bfloat16 *y, const float *g, __nv_bfloat16 *out, float *part, size_t pixels,
-                            size_t px, size_t chunk, int c, int c_pad, int rows) {
-    __shared__ float sm[256][9];
-    const int nq = c_pad >> 3, q = (int)threadIdx.x % nq, r = (int)threadIdx.x / nq;
-    const size_t p0 = (size_t)blockIdx.x * chunk, p1 = p0 + chunk < pixels ? p0 + chunk : pixels;
-    float acc[8] = {};
-    for (size_t p = p0 + r; p < p1; p += rows) {
-        const size_t img = p / px, plane = (img * nq + q) * px + (p - img * px);
-        float v[8] = {};
-        if (c & 7) {
-            for (int k = 0; k < 8; k++)
-                if (8 * q + k < c) v[k] = g[p * c + 8 * q + k];
-        } else {
-            const float4 *s = reinterpret_cast<const float4 *>(g + p * c + 8 * q);
-            const float4 a = s[0], b = s[1];
-            v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
-        }
-        if (y) {
-            const uint4 m4 = reinterpret_cast<const uint4 *>(y)[plane];
-            const __nv_bfloat16 *m = reinterpret_cast<const __nv_bfloat16 *>(&m4);
-#pragma unroll
-            for (int k = 0; k < 8; k++)
-                if (!(bf(m[k]) > 0.f)) v[k] = 0.f;
-        }
-        __nv_bfloat16 o[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) o[k] = __float2bfloat16(v[k]), acc[k] += v[k];
-        reinterpret_cast<uint4 *>(out)[plane] = *reinterpret_cast<const uint4 *>(o);
-    }
-#pragma unroll
-    for (int k = 0; k < 8; k++) sm[threadIdx.x][k] = acc[k];
-    __syncthreads();
-    for (int k = (int)threadIdx.x; k < c; k += (int)blockDim.x) {
-        float s = 0.f;
-        for (int i = 0; i < rows; i++) s += sm[i * nq + (k >> 3)][k & 7];
-        part[(size_t)blockIdx.x * c + k] = s;
-    }
-}
-
-// One block (256 threads) per channel: thread t adds the partials of blocks
-// t, t + 256, ..., then a fixed tree adds the 256 sums (the same order on
-// every run).
-__global__ void k_bias_finalize(const float *part, float *db, int blocks, int c) {
-    // a backward-data convolution launched next may start its prologue now
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+// One block (256 threads) per channel of each job: thread t adds rows t, t +
+// 256, ..., then a fixed tree adds the 256 sums (the same order on every run).
+__global__ void k_bias_all(const BiasJob *jobs) {
     __shared__ float sm[256];
+    const BiasJob J = jobs[blockIdx.y];
     const int k = (int)blockIdx.x, t = (int)threadIdx.x;
+    if (k >= J.c) return;
     float s = 0.f;
-    for (int b = t; b < blocks; b += 256) s += part[(size_t)b * c + k];
+    for (int r = t; r < J.rows; r += 256) s += J.part[(size_t)r * J.c + k];
     sm[t] = s;
     __syncthreads();
     for (int o = 128; o > 0; o >>= 1) {
         if (t < o) sm[t] += sm[t + o];
         __syncthreads();
     }
-    if (t == 0) db[k] += sm[0];
+    if (t == 0) J.db[k] = sm[0];
 }
 
 __global__ void k_bias_grad(const float *g, float *db, size_t pixels, int c) {
@@ -361,6 +318,49 @@ __global__ void k_l1(const float *out, const float *target, const __half *feat, 
     if (threadIdx.x == 0) part[blockIdx.x] = sm[0];
 }
 
+// k_l1 for the tensor-core backward, a pixel per thread: the gradient goes
+// straight into the BF16 operand of the output convolution's backward pass.
+__global__ void __launch_bounds__(256) k_l1_tc(const float *out, const float *target, const __half *feat,
+                                               __nv_bfloat16 *g, float *part, float *bias_part, size_t pixels,
+                                               size_t px) {
+    // the first backward-data convolution may start up now
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __shared__ float sm[4][8];
+    float acc[4] = {};
+    const float inv = 1.f / (float)(3 * pixels);
+    for (size_t p = gtid(); p < pixels; p += gstride()) {
+        const size_t img = p / px;
+        __nv_bfloat16 v[8];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const size_t i = 3 * p + k;
+            const float d = out[i] - log1pf(fmaxf(target[i], 0.f) / demod(feat, i));
+            const float gk = (d > 0.f ? 1.f : (d < 0.f ? -1.f : 0.f)) * inv;
+            acc[0] += fabsf(d), acc[1 + k] += gk;
+            v[k] = __float2bfloat16(gk);
+        }
+#pragma unroll
+        for (int k = 3; k < 8; k++) v[k] = __float2bfloat16(0.f);
+        uint4 *o = reinterpret_cast<uint4 *>(g) + img * px + p;  // plane 2 img, pixel p - img px
+        o[0] = *reinterpret_cast<const uint4 *>(v);
+        o[px] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    // fixed-order sums: lanes, then warps
+    const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xFFFFFFFFu, acc[k], o);
+        if (lane == 0) sm[k][warp] = acc[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        float s = 0.f;
+        for (int w = 0; w < 8; w++) s += sm[threadIdx.x][w];
+        if (threadIdx.x == 0) part[blockIdx.x] = s;
+        else bias_part[(size_t)blockIdx.x * 3 + threadIdx.x - 1] = s;
+    }
+}
+
 __global__ void k_l1_finalize(const float *part, int blocks, float *loss, float inv) {
     __shared__ float sm[256];
     float s = 0.f;
@@ -464,16 +464,9 @@ cudaError_t bias_grad(const float *g, float *db, size_t pixels, int c, cudaStrea
     k_bias_grad<<<c, 256, 0, st>>>(g, db, pixels, c);
     return cudaGetLastError();
 }
-cudaError_t grad_prep(const __nv_bfloat16 *y, const float *g, __nv_bfloat16 *out, float *part, float *db,
-                      size_t pixels, size_t px, int c, int c_pad, cudaStream_t st) {
-    if (c_pad < c || c_pad > 256 || (c_pad & 15) || (c != 3 && (c & 7)) || pixels == 0) return cudaErrorInvalidValue;
-    const int rows = 256 / (c_pad / 8);
-    const size_t chunk = (pixels + kGradPrepBlocks - 1) / kGradPrepBlocks;
-    const int blocks = (int)((pixels + chunk - 1) / chunk);
-    k_grad_prep<<<blocks, rows * (c_pad / 8), 0, st>>>(y, g, out, part, pixels, px, chunk, c, c_pad, rows);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_bias_finalize<<<c, 256, 0, st>>>(part, db, blocks, c);
+cudaError_t bias_all(const BiasJob *jobs_dev, int njobs, int max_c, cudaStream_t st) {
+    if (njobs <= 0 || max_c <= 0) return cudaErrorInvalidValue;
+    k_bias_all<<<dim3((unsigned)max_c, (unsigned)njobs), 256, 0, st>>>(jobs_dev);
     return cudaGetLastError();
 }
 cudaError_t avgpool(const __nv_bfloat16 *x, __nv_bfloat16 *y, int n, int h, int w, int c, cudaStream_t st) {
@@ -509,6 +502,16 @@ cudaError_t l1_loss(const float *out, const float *target, const __half *feat, f
     const unsigned blocks = blocks_for(n);
     k_l1<<<blocks, 256, 0, st>>>(out, target, feat, g, part, n);
     k_l1_finalize<<<1, 256, 0, st>>>(part, (int)blocks, loss, 1.f / (float)n);
+    return cudaGetLastError();
+}
+cudaError_t l1_loss_tc(const float *out, const float *target, const __half *feat, __nv_bfloat16 *g, float *part,
+                       size_t pixels, size_t px, cudaStream_t st) {
+    k_l1_tc<<<(unsigned)l1_blocks(pixels), 256, 0, st>>>(out, target, feat, g, part, part + kL1Blocks, pixels, px);
+    return cudaGetLastError();
+}
+int l1_blocks(size_t pixels) { return (int)std::min<size_t>((pixels + 255) / 256, kL1Blocks); }
+cudaError_t l1_finalize(const float *part, int blocks, size_t n, float *loss, cudaStream_t st) {
+    k_l1_finalize<<<1, 256, 0, st>>>(part, blocks, loss, 1.f / (float)n);
     return cudaGetLastError();
 }
 cudaError_t add_input(float *out, const __nv_bfloat16 *x0, int x0_c, size_t pixels, cudaStream_t st) {

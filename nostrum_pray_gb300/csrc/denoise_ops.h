@@ -30,17 +30,18 @@ struct TcConvPlan {
     int grid, per_sm;             // persistent CTAs of each chunk, and the CTAs per SM it was planned for
     int ring, wstages;            // halo slots; weight slots of a tap each (9: all resident)
     int acc_slots, acc_stride, tmem_cols;
+    int grad;                     // planned for TcFuse::grad
     uint32_t halo_stride, w_off, bias_off, bar_off;
     size_t smem;
 };
 cudaError_t tc_conv_plan(TcConvPlan &p, const __nv_bfloat16 *x, int n, int h, int w, int cin, int cout, bool relu,
-                         int sm_count);
+                         int sm_count, bool grad = false);
 size_t tc_packed_weight_elems(int cin_pad, int cout);
 cudaError_t tc_pack_weights(const float *w, __nv_bfloat16 *packed, int cin, int cin_pad, int cout, cudaStream_t st);
 // Weights of the backward-data convolution of a forward convolution with
 // cin_f inputs and cout_f outputs (w[cout_f][9][cin_f]): a plan with
 // cin = cout_f rounded up to 16 and cout = cin_f runs it on the output
-// gradient (as BF16, grad_prep) and writes the input gradient.
+// gradient (BF16, planar) and writes the input gradient.
 cudaError_t tc_pack_weights_bwd(const float *w, __nv_bfloat16 *packed, int cin_f, int cout_f, cudaStream_t st);
 // Every packing of a network's weights in one launch: job j packs w (the
 // FP32 [cout_f][9][cin_f] weights of one convolution) into out, as
@@ -66,7 +67,19 @@ cudaError_t tc_pack_all(const TcPackJob *jobs_dev, int njobs, size_t total, cuda
 //         upsampling, at the 2 x 2 block of a 2h x 2w tensor (cat_up 1);
 //   res:  FP32 output += res[pixel * res_c + channel] (BF16);
 //   rad:  (cout 3) rad = expm1(FP32 output) * (max(albedo, 0) + kDemodFloor),
-//         the albedo from feat (7 halves per pixel).
+//         the albedo from feat (7 halves per pixel);
+//   grad: for a backward-data convolution, whose FP32 output is the gradient
+//         of the forward convolution's input tensor: what the next one down
+//         the chain reads, the gradient masked by the ReLU of that tensor
+//         (mask: its BF16 values, planar) and rounded to BF16 (g, planar), with
+//         per-CTA sums of the masked FP32 values (bias_part: grid x channels of
+//         g, for the bias gradient).
+//         kGradMask: the input is itself a convolution's output;
+//         kGradCat: it is a concatenation; of channels [0, low_c) the sums over
+//         2 x 2 blocks (mask, g: h / 2 x w / 2, low_c channels), the others as
+//         they are into skip (FP32, planar);
+//         kGradUnpool: it is the 2 x 2 average of a tensor whose other share of
+//         the gradient is skip (mask, g, skip: 2h x 2w): skip + output / 4.
 // pool and cat need cout a multiple of 16; pool comes with cat at the same
 // pixel; res (cout at most 4) goes with rad or the FP32 output, which take no
 // other store.
@@ -78,7 +91,13 @@ struct TcFuse {
     int res_c = 0;
     float *rad = nullptr;
     const __half *feat = nullptr;
+    int grad = 0;
+    const __nv_bfloat16 *mask = nullptr;
+    __nv_bfloat16 *g = nullptr;
+    float *skip = nullptr, *bias_part = nullptr;
+    int low_c = 0;
 };
+enum { kGradNone = 0, kGradMask, kGradCat, kGradUnpool };
 cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked, const float *bias,
                                __nv_bfloat16 *y, float *y32, int *err, cudaStream_t st,
                                const TcFuse *fuse = nullptr, bool overlap_prologue = false);
@@ -89,10 +108,10 @@ cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked
 // previous kernel of the stream; its input copies wait for that kernel to
 // complete. The previous kernel must not write the weights or the bias.
 // Weight gradient of a 3x3 convolution on the tensor cores:
-// dw[co][tap][ci] += sum over pixels p of g[p][co] * x[p + offset(tap)][ci],
+// dw[co][tap][ci] = sum over pixels p of g[p][co] * x[p + offset(tap)][ci],
 // a GEMM with M = output channels (padded to 128), N = input channels, K =
 // pixels. g: the output gradient as BF16 with cout_pad = cout rounded up to
-// 16 channels (grad_prep); x: the convolution's input, read through the
+// 16 channels (planar); x: the convolution's input, read through the
 // forward plan's halo tensor map (fwd: a plan over x with cin = cin_pad).
 // Each CTA accumulates the nine taps (or a group of them, as many as tensor
 // memory holds) over a group of 16 x 8 tiles and writes them to `partial`
@@ -117,15 +136,14 @@ cudaError_t conv3x3_backward(const __nv_bfloat16 *x, const __nv_bfloat16 *w, con
 cudaError_t relu_mask(const __nv_bfloat16 *y, const float *g, float *out, size_t n, cudaStream_t st);
 // db[c] += sum over pixels of g[p][c]
 cudaError_t bias_grad(const float *g, float *db, size_t pixels, int c, cudaStream_t st);
-// One pass over a convolution's output gradient g (pixels x c FP32) for the
-// tensor-core backward: the ReLU mask of the convolution's output y (NULL:
-// no mask), the masked gradient as BF16 with c_pad >= c channels (the pad
-// zero), and the bias gradient: per-block partial sums in part
-// (kGradPrepBlocks x c floats), added in block order into db. y and out are
-// planar (images of px pixels), g channels last; c is 3 or a multiple of 8.
-constexpr int kGradPrepBlocks = 1024;
-cudaError_t grad_prep(const __nv_bfloat16 *y, const float *g, __nv_bfloat16 *out, float *part, float *db,
-                      size_t pixels, size_t px, int c, int c_pad, cudaStream_t st);
+// Bias gradients: db[k] = the sum over rows of part[row * c + k], in a fixed
+// order (jobs on the device).
+struct BiasJob {
+    const float *part;
+    float *db;
+    int rows, c;
+};
+cudaError_t bias_all(const BiasJob *jobs_dev, int njobs, int max_c, cudaStream_t st);
 cudaError_t avgpool(const __nv_bfloat16 *x, __nv_bfloat16 *y, int n, int h, int w, int c, cudaStream_t st);
 cudaError_t avgpool_backward(const float *gy, float *gx, int n, int h, int w, int c, cudaStream_t st);
 cudaError_t upsample_backward(const float *gy, float *gx, int n, int h, int w, int c, int cy, cudaStream_t st);
@@ -146,6 +164,16 @@ cudaError_t upsample_concat(const __nv_bfloat16 *low, const __nv_bfloat16 *skip,
 constexpr int kL1Parts = 152 * 32;
 cudaError_t l1_loss(const float *out, const float *target, const __half *feat, float *g, float *loss, float *part,
                     size_t n, cudaStream_t st);
+// The same for the tensor-core backward: the gradient of each pixel's three
+// values as BF16, planar, padded to 16 channels (images of px pixels); per
+// block the sum of the |differences| in part[block] and of the three gradients
+// in part[kL1Blocks + 3 block + k] (part: 4 kL1Blocks floats, l1_blocks(pixels)
+// blocks). l1_finalize makes the loss of the former.
+constexpr int kL1Blocks = 608;
+int l1_blocks(size_t pixels);
+cudaError_t l1_loss_tc(const float *out, const float *target, const __half *feat, __nv_bfloat16 *g, float *part,
+                       size_t pixels, size_t px, cudaStream_t st);
+cudaError_t l1_finalize(const float *part, int blocks, size_t n, float *loss, cudaStream_t st);
 // out (3 channels) += the first 3 of x0's x0_c channels (the input's log radiance)
 cudaError_t add_input(float *out, const __nv_bfloat16 *x0, int x0_c, size_t pixels, cudaStream_t st);
 cudaError_t expm1_out(const float *out, const __half *feat, float *rad, size_t n, cudaStream_t st);

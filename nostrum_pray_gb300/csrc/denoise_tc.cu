@@ -60,7 +60,7 @@ constexpr int kTaps = 9;
 
 struct TcArgs {
     const __nv_bfloat16 *w;  // packed weights [tap][chunk][row][8]
-    const float *bias;       // NULL: none
+    const float *bias;       // forward
     __nv_bfloat16 *y;
     float *y32;
     int n, h, wd, cin, cout, npad, relu;
@@ -253,8 +253,9 @@ __device__ __forceinline__ void load_tmem(uint32_t taddr, uint32_t *r) {
 // What a convolution stores (a kernel instance each): the BF16 outputs; also
 // their 2 x 2 averages and a copy into a concatenation; also (or only) the
 // outputs upsampled into a concatenation; FP32 outputs (channels last), with
-// the residual and the output transform.
-enum EpiMode { kEpiY, kEpiPool, kEpiUp, kEpiF32 };
+// the residual and the output transform; and the three of a backward-data
+// convolution (TcFuse::grad).
+enum EpiMode { kEpiY, kEpiPool, kEpiUp, kEpiF32, kEpiGradMask, kEpiGradCat, kEpiGradUnpool };
 
 // A warp's share of a tile: one pixel per lane (tile row m = pixel (m / 8,
 // m % 8)), the planes' size and where the pixel's first stores go.
@@ -265,7 +266,146 @@ struct EpiPixel {
     uint4 *y, *cat, *pool; // the tile's chunk n0 / 8 at the lane's pixel
     size_t pix;            // channels-last pixel
     const __nv_bfloat16 *res;
+    // backward: gradient and mask (16 bytes per pixel and chunk), the FP32 share
+    // (32 bytes) at chunk n0 / 8 of the lane's pixel, block or low-resolution
+    // pixel; the warp's bias sums (npad floats)
+    uint4 *g;
+    const uint4 *mask;
+    float4 *skip;
+    float *bsum;
 };
+
+// v where the BF16 pair m is positive, else 0.
+__device__ __forceinline__ uint64_t mask2(uint64_t v, uint32_t m) {
+    const bool a = __uint_as_float(m << 16) > 0.f, b = __uint_as_float(m & 0xFFFF0000u) > 0.f;
+    return pair(a ? (uint32_t)v : 0u, b ? (uint32_t)(v >> 32) : 0u);
+}
+
+// Adds the sums over the warp's lanes of 16 values each (pairs) to
+// sums[0..16): halves are exchanged so that every step adds half as many
+// values; lane 2 c ends with channel c (in the order of its bits).
+__device__ __forceinline__ void lane_sums16(const uint64_t *p, int lane, float *sums) {
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    float v[16];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[2 * k] = __uint_as_float((uint32_t)p[k]), v[2 * k + 1] = __uint_as_float((uint32_t)(p[k] >> 32));
+#pragma unroll
+    for (int n = 8, o = 16; n >= 1; n >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (k < n) {
+                const float got = __shfl_xor_sync(kFull, up ? v[k] : v[k + n], o);
+                v[k] = (up ? v[k + n] : v[k]) + got;
+            }
+    }
+    v[0] += __shfl_xor_sync(kFull, v[0], 1);
+    const int c = (lane >> 4 & 1) * 8 + (lane >> 3 & 1) * 4 + (lane >> 2 & 1) * 2 + (lane >> 1 & 1);
+    if (!(lane & 1)) sums[c] += v[0];
+}
+
+// The backward stores (TcFuse::grad) of 16 channels; q: chunk from the CTA's
+// first, c0: channel from the CTA's first, c: channel.
+template <int kMode>
+__device__ __forceinline__ void store_grad16(const TcArgs &P, const uint32_t *r, const EpiPixel &e, int q, int c0,
+                                             int c) {
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    uint64_t v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = pair(r[2 * k], r[2 * k + 1]);
+    if (kMode == kEpiGradCat && c >= P.f.low_c) {
+        if (e.valid) {
+            float4 *o = e.skip + (size_t)q * 2 * e.px;
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    const uint64_t a = v[4 * j + 2 * k], b = v[4 * j + 2 * k + 1];
+                    o[(size_t)j * 2 * e.px + k] = make_float4(
+                        __uint_as_float((uint32_t)a), __uint_as_float((uint32_t)(a >> 32)),
+                        __uint_as_float((uint32_t)b), __uint_as_float((uint32_t)(b >> 32)));
+                }
+        }
+        return;
+    }
+    if (kMode == kEpiGradMask) {
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            uint4 m = make_uint4(0u, 0u, 0u, 0u);
+            if (e.valid) m = e.mask[(size_t)(q + j) * e.px];
+            const uint32_t mw[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+            for (int k = 0; k < 4; k++) v[4 * j + k] = mask2(v[4 * j + k], mw[k]);
+            if (e.valid)
+                e.g[(size_t)(q + j) * e.px] = make_uint4(round2(v[4 * j]), round2(v[4 * j + 1]), round2(v[4 * j + 2]),
+                                                         round2(v[4 * j + 3]));
+        }
+        lane_sums16(v, e.lane, e.bsum + c0);
+    }
+    if (kMode == kEpiGradCat) {
+        // 2 x 2 sums (row-major), as in the pooling: each lane of a block ends
+        // with two of the eight channel pairs
+        const bool odd = e.lane & 1, low = e.lane & 8;
+        uint64_t a[4], b[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint64_t got = __shfl_xor_sync(kFull, odd ? v[k] : v[4 + k], 1);
+            a[k] = odd ? got : v[k], b[k] = odd ? v[4 + k] : got;
+        }
+        uint2 m = make_uint2(0u, 0u);
+        const size_t at = (size_t)(q + (odd ? 1 : 0)) * e.pp;
+        if (e.pool_valid) m = reinterpret_cast<const uint2 *>(e.mask + at)[low ? 1 : 0];
+        uint64_t sum[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const uint64_t ga = __shfl_xor_sync(kFull, low ? a[k] : a[2 + k], 8);
+            const uint64_t gb = __shfl_xor_sync(kFull, low ? b[k] : b[2 + k], 8);
+            const uint64_t ta = low ? ga : a[k], tb = low ? gb : b[k];          // the upper row's
+            const uint64_t ba = low ? a[2 + k] : ga, bb = low ? b[2 + k] : gb;  // the lower row's
+            sum[k] = mask2(add2(add2(add2(ta, tb), ba), bb), k ? m.y : m.x);
+        }
+        if (e.pool_valid) reinterpret_cast<uint2 *>(e.g + at)[low ? 1 : 0] = make_uint2(round2(sum[0]), round2(sum[1]));
+        // over the warp's eight blocks (lane bits 1, 2 and 4)
+#pragma unroll
+        for (int o : {2, 4, 16})
+#pragma unroll
+            for (int k = 0; k < 2; k++) sum[k] = add2(sum[k], __shfl_xor_sync(kFull, sum[k], o));
+        if ((e.lane & ~9) == 0) {
+            float *d = e.bsum + c0 + (odd ? 8 : 0) + (low ? 4 : 0);
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+                d[2 * k] += __uint_as_float((uint32_t)sum[k]), d[2 * k + 1] += __uint_as_float((uint32_t)(sum[k] >> 32));
+        }
+    }
+    if (kMode == kEpiGradUnpool) {
+        const uint32_t W2 = 2 * (uint32_t)P.wd;
+        const uint64_t quarter = pair(0x3E800000u, 0x3E800000u);
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            uint64_t s[4] = {};  // the chunk's sums over the four pixels
+            uint64_t share[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(share[k]) : "l"(v[4 * j + k]), "l"(quarter));
+            if (e.valid) {
+                const size_t plane = (size_t)(q + j) * 4 * e.px;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const size_t at = plane + (i >> 1) * W2 + (i & 1);
+                    const uint4 m = e.mask[at];
+                    const ulonglong2 *sk = reinterpret_cast<const ulonglong2 *>(e.skip + 2 * at);
+                    const ulonglong2 s0 = sk[0], s1 = sk[1];
+                    const uint64_t g0 = mask2(add2(s0.x, share[0]), m.x), g1 = mask2(add2(s0.y, share[1]), m.y);
+                    const uint64_t g2 = mask2(add2(s1.x, share[2]), m.z), g3 = mask2(add2(s1.y, share[3]), m.w);
+                    e.g[at] = make_uint4(round2(g0), round2(g1), round2(g2), round2(g3));
+                    s[0] = add2(s[0], g0), s[1] = add2(s[1], g1), s[2] = add2(s[2], g2), s[3] = add2(s[3], g3);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) v[4 * j + k] = s[k];
+        }
+        lane_sums16(v, e.lane, e.bsum + c0);
+    }
+}
 
 // The stores of 16 channels (chunk q and q + 1 from the CTA's first;
 // accumulators r) of a lane's pixel: bias + ReLU as BF16 (planar: the eight
@@ -359,7 +499,8 @@ __device__ __forceinline__ void store16(const TcArgs &P, const uint32_t *r, cons
 // on, 32 columns at a time.
 template <int kMode>
 __device__ __forceinline__ void epilogue(const TcArgs &P, uint32_t tmem, int img, int y0, int x0, int quad, int n0,
-                                         const float *bias) {
+                                         const float *bias, float *bsum) {
+    constexpr bool kGrad = kMode == kEpiGradMask || kMode == kEpiGradCat || kMode == kEpiGradUnpool;
     EpiPixel e;
     e.lane = (int)(threadIdx.x & 31);
     const int m = quad * 32 + e.lane, yy = y0 + (m >> 3), xx = x0 + (m & 7);
@@ -370,7 +511,7 @@ __device__ __forceinline__ void epilogue(const TcArgs &P, uint32_t tmem, int img
     if (kMode == kEpiF32) {
         e.pix = (size_t)img * e.px + at;
         e.res = P.f.res ? P.f.res + ((size_t)img * (P.f.res_c >> 3) * e.px + at) * 8 : nullptr;
-    } else {
+    } else if (!kGrad) {
         e.y = reinterpret_cast<uint4 *>(P.y) + ((size_t)img * (P.cout >> 3) + q0) * e.px + at;
     }
     if (kMode == kEpiPool || kMode == kEpiUp) {
@@ -385,17 +526,43 @@ __device__ __forceinline__ void epilogue(const TcArgs &P, uint32_t tmem, int img
         e.pp = (uint32_t)ho * (uint32_t)wo;
         e.pool = reinterpret_cast<uint4 *>(P.f.pool) + ((size_t)img * (P.cout >> 3) + q0) * e.pp + (uint32_t)yo * wo + xo;
     }
+    if (kGrad) {
+        size_t plane, pos;  // of mask and g
+        const size_t planes = (size_t)img * (P.cout >> 3) + q0;
+        e.bsum = bsum;
+        if (kMode == kEpiGradMask) {
+            plane = planes * e.px, pos = at;
+        } else if (kMode == kEpiGradCat) {
+            e.pp = (uint32_t)(P.h >> 1) * (uint32_t)(P.wd >> 1);
+            e.pool_valid = e.valid;  // (h and w are even where a concatenation is)
+            plane = ((size_t)img * (P.f.low_c >> 3) + q0) * e.pp;
+            pos = (size_t)(yy >> 1) * (P.wd >> 1) + (xx >> 1);
+            // the chunk at or after low_c (store_grad16 uses it from there on)
+            e.skip = reinterpret_cast<float4 *>(P.f.skip) +
+                     (((size_t)img * ((P.cout - P.f.low_c) >> 3) + q0) * e.px + at) * 2 -
+                     (size_t)(P.f.low_c >> 3) * e.px * 2;
+        } else {
+            plane = planes * 4 * e.px, pos = 4 * (size_t)yy * P.wd + 2 * xx;
+            e.skip = reinterpret_cast<float4 *>(P.f.skip) + 2 * (plane + pos);
+        }
+        e.mask = reinterpret_cast<const uint4 *>(P.f.mask) + plane + pos;
+        e.g = reinterpret_cast<uint4 *>(P.f.g) + plane + pos;
+    }
+    auto store = [&](const uint32_t *v, int c0) {
+        if constexpr (kGrad) store_grad16<kMode>(P, v, e, c0 >> 3, c0, n0 + c0);
+        else store16<kMode>(P, v, e, c0 >> 3, n0 + c0, bias + c0);
+    };
     const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16);
     uint32_t r[32];
     int c0 = 0;
     for (; c0 + 32 <= P.npad; c0 += 32) {
         load_tmem<2>(taddr + c0, r);
-        store16<kMode>(P, r, e, c0 >> 3, n0 + c0, bias + c0);
-        store16<kMode>(P, r + 16, e, (c0 >> 3) + 2, n0 + c0 + 16, bias + c0 + 16);
+        store(r, c0);
+        store(r + 16, c0 + 16);
     }
     if (c0 < P.npad) {
         load_tmem<1>(taddr + c0, r);
-        store16<kMode>(P, r, e, c0 >> 3, n0 + c0, bias + c0);
+        store(r, c0);
     }
 }
 
@@ -408,7 +575,8 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 }
 
 constexpr int kEpiGroups = 3;  // groups of four epilogue warps
-constexpr int kConvThreads = 64 + 128 * kEpiGroups;
+constexpr int kEpiWarps = 4 * kEpiGroups;
+constexpr int kConvThreads = 64 + 32 * kEpiWarps;
 
 // A position in a ring of n slots and its phase (the parity of the completed
 // rounds), moved on without divisions: the roles' loops are one thread's or
@@ -553,8 +721,10 @@ __global__ void __launch_bounds__(kConvThreads, 2) k_conv_tc(const __grid_consta
         *C.abort_flag = 0, *C.h_issued = 0, *C.h_waited = 0, *C.w_issued = 0, *C.w_waited = 0;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    for (int i = tid - 64; i >= 0 && i < P.npad; i += kConvThreads - 64)
-        bias[i] = P.bias && n0 + i < P.cout ? __ldg(P.bias + n0 + i) : 0.f;
+    constexpr bool kGrad = kMode == kEpiGradMask || kMode == kEpiGradCat || kMode == kEpiGradUnpool;
+    // forward: the chunk's bias; backward: each epilogue warp's bias-gradient sums
+    for (int i = tid - 64; i >= 0 && i < (kGrad ? kEpiWarps * P.npad : P.npad); i += kConvThreads - 64)
+        bias[i] = !kGrad && n0 + i < P.cout ? __ldg(P.bias + n0 + i) : 0.f;
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -642,7 +812,8 @@ __global__ void __launch_bounds__(kConvThreads, 2) k_conv_tc(const __grid_consta
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            epilogue<kMode>(P, C.tmem + (uint32_t)(acc.slot * P.acc_stride), t.img, t.y0(), t.x0(), quad, n0, bias);
+            epilogue<kMode>(P, C.tmem + (uint32_t)(acc.slot * P.acc_stride), t.img, t.y0(), t.x0(), quad, n0, bias,
+                            bias + (warp - 2) * P.npad);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             mbar_arrive(C.bar(C.afree + acc.slot));
             for (int k = 0; k < groups; k++) acc.next();
@@ -654,6 +825,14 @@ __global__ void __launch_bounds__(kConvThreads, 2) k_conv_tc(const __grid_consta
         // copies still in flight (bounded) before the shared memory goes away
         for (int j = *C.h_waited; j < *C.h_issued; j++) mbar_wait(C.bar(C.hfull + j % H), (uint32_t)(j / H) & 1u);
         for (int j = *C.w_waited; j < *C.w_issued; j++) mbar_wait(C.bar(C.wfull + j % S), (uint32_t)(j / S) & 1u);
+    }
+    if (kGrad) {  // the warps' sums in warp order (the roles have met above)
+        const int channels = kMode == kEpiGradCat ? P.f.low_c : P.cout;
+        for (int i = tid; i < P.npad && n0 + i < channels; i += kConvThreads) {
+            float sum = 0.f;
+            for (int k = 0; k < kEpiWarps; k++) sum += bias[k * P.npad + i];
+            P.f.bias_part[(size_t)blockIdx.x * channels + n0 + i] = sum;
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -848,7 +1027,7 @@ __global__ void __launch_bounds__(128) k_wgrad_tc(const __grid_constant__ CUtens
     }
 }
 
-// dw[co][tap][ci] += sum over groups (in order) of partial[group][tap][co][ci]
+// dw[co][tap][ci] = sum over groups (in order) of partial[group][tap][co][ci]
 // Block of 256 threads: 32 consecutive gradient elements x 8 slices; slice
 // s adds groups s, s + 8, ..., and the 8 slice sums are added in slice order
 // (the same order on every run).
@@ -871,7 +1050,7 @@ __global__ void k_wgrad_finalize(const float *partial, float *dw, int groups, in
     if (slice == 0 && i < total) {
         float s = sm[0][lane];
         for (int k = 1; k < kFinSlices; k++) s += sm[k][lane];
-        dw[i] += s;
+        dw[i] = s;
     }
 }
 
@@ -1078,7 +1257,7 @@ cudaError_t conv3x3_wgrad_tc(const TcWgradPlan &p, const TcConvPlan &fwd, float 
 }
 
 cudaError_t tc_conv_plan(TcConvPlan &p, const __nv_bfloat16 *x, int n, int h, int w, int cin, int cout, bool relu,
-                         int sm_count) {
+                         int sm_count, bool grad) {
     std::memset(&p, 0, sizeof(p));
     if (n <= 0 || h <= 0 || w <= 0 || cin <= 0 || (cin & 15) || cout <= 0 ||
         !(cin <= 128 || cin == 160 || cin == 224))  // (the pair counts that issue() unrolls)
@@ -1118,7 +1297,7 @@ cudaError_t tc_conv_plan(TcConvPlan &p, const __nv_bfloat16 *x, int n, int h, in
             while (cols < acc * stride) cols <<= 1;
             if (cols * per_sm > 512) continue;
             const size_t budget = per_sm == 2 ? kSmemPerSm / 2 - 1024 : kSmemMax;
-            const size_t misc = 4 * (size_t)cw + 8 * (2 * 4 + 2 * 4 + 2 * kTaps + 1) + 64;
+            const size_t misc = 4 * (size_t)cw * (grad ? kEpiWarps : 1) + 8 * (2 * 4 + 2 * 4 + 2 * kTaps + 1) + 64;
             for (int wst = kTaps; wst >= 3; wst--) {
                 const size_t rest = misc + wst * wtap;
                 if (rest + halo > budget) continue;
@@ -1149,7 +1328,8 @@ cudaError_t tc_conv_plan(TcConvPlan &p, const __nv_bfloat16 *x, int n, int h, in
     p.halo_stride = (uint32_t)halo;
     p.w_off = (uint32_t)(p.ring * halo);
     p.bias_off = (uint32_t)(p.w_off + p.wstages * wtap);
-    p.bar_off = (p.bias_off + 4 * (uint32_t)p.npad + 15) & ~15u;
+    p.bar_off = (p.bias_off + 4 * (uint32_t)p.npad * (grad ? kEpiWarps : 1) + 15) & ~15u;
+    p.grad = grad ? 1 : 0;
     p.smem = p.bar_off + 8 * (2 * (size_t)p.ring + 2 * (size_t)p.acc_slots + 2 * (size_t)p.wstages + 1) + 32;
     // no more CTAs per SM than TMEM has columns for (tcgen05.alloc would wait)
     const size_t max_ctas = 512 / p.tmem_cols;
@@ -1162,6 +1342,7 @@ cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked
                                __nv_bfloat16 *y, float *y32, int *err, cudaStream_t st, const TcFuse *fuse,
                                bool overlap_prologue) {
     if (y && (p.cout & 15)) return cudaErrorInvalidValue;
+    if (!bias && !(fuse && fuse->grad != kGradNone)) return cudaErrorInvalidValue;
     if (fuse) {
         if ((fuse->pool || fuse->cat) && (p.cout & 15)) return cudaErrorInvalidValue;
         if (fuse->cat && (fuse->cat_c & 7 || fuse->cat_off & 7 || fuse->cat_off + p.cout > fuse->cat_c))
@@ -1169,6 +1350,13 @@ cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked
         // one of: pooling with the copy into a concatenation, upsampling, FP32
         if ((fuse->pool != nullptr) != (fuse->cat && !fuse->cat_up)) return cudaErrorInvalidValue;
         if ((y32 || fuse->rad) && (y || fuse->cat)) return cudaErrorInvalidValue;
+        if (fuse->grad != kGradNone) {
+            if (!p.grad || y || y32 || fuse->cat || fuse->rad || (p.cout & 15) || !fuse->mask || !fuse->g ||
+                !fuse->bias_part || (fuse->grad != kGradMask && !fuse->skip))
+                return cudaErrorInvalidValue;
+            if (fuse->grad == kGradCat && ((fuse->low_c & 15) || fuse->low_c > p.cout || ((p.h | p.w) & 1)))
+                return cudaErrorInvalidValue;
+        }
         if (fuse->res && (p.cout > 4 || (!y32 && !fuse->rad))) return cudaErrorInvalidValue;
         if (fuse->rad && (p.cout != 3 || !fuse->feat)) return cudaErrorInvalidValue;
     }
@@ -1179,7 +1367,8 @@ cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked
     if (e0 != cudaSuccess) return e0;
     const uint64_t bit = dev < 64 ? 1ull << dev : 0;
     if (!bit || !(attr_set.load() & bit)) {
-        for (auto k : {k_conv_tc<kEpiY>, k_conv_tc<kEpiPool>, k_conv_tc<kEpiUp>, k_conv_tc<kEpiF32>}) {
+        for (auto k : {k_conv_tc<kEpiY>, k_conv_tc<kEpiPool>, k_conv_tc<kEpiUp>, k_conv_tc<kEpiF32>,
+                       k_conv_tc<kEpiGradMask>, k_conv_tc<kEpiGradCat>, k_conv_tc<kEpiGradUnpool>}) {
             const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
             if (e != cudaSuccess) return e;
         }
@@ -1222,8 +1411,13 @@ cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked
     cfg.numAttrs = overlap_prologue ? 1 : 0;
     cfg.gridDim = dim3((unsigned)p.grid, (unsigned)p.nsplit), cfg.blockDim = dim3(kConvThreads);
     const bool f32 = y32 || (fuse && fuse->rad), pool = fuse && fuse->pool, cat = fuse && fuse->cat;
+    const int grad = fuse ? fuse->grad : kGradNone;
     const cudaError_t e = cudaLaunchKernelEx(
-        &cfg, f32 ? k_conv_tc<kEpiF32> : pool ? k_conv_tc<kEpiPool> : cat ? k_conv_tc<kEpiUp> : k_conv_tc<kEpiY>, map,
+        &cfg,
+        grad == kGradMask     ? k_conv_tc<kEpiGradMask>
+        : grad == kGradCat    ? k_conv_tc<kEpiGradCat>
+        : grad == kGradUnpool ? k_conv_tc<kEpiGradUnpool>
+        : f32 ? k_conv_tc<kEpiF32> : pool ? k_conv_tc<kEpiPool> : cat ? k_conv_tc<kEpiUp> : k_conv_tc<kEpiY>, map,
         wmap, a);
     return e == cudaSuccess ? cudaGetLastError() : e;
 }
