@@ -92,7 +92,6 @@ cudaError_t Denoiser::init(uint64_t seed) {
     }
     plans_.assign(kNumConvs, dn::TcConvPlan{});
     plans_bwd_.assign(kNumConvs, dn::TcConvPlan{});
-    plans_wg_.assign(kNumConvs, dn::TcWgradPlan{});
     cudaError_t e;
     if ((e = cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) return e;
     if ((e = take(w_, total)) != cudaSuccess || (e = take(g_, total)) != cudaSuccess ||
@@ -180,7 +179,6 @@ cudaError_t Denoiser::ensure(int n, int h, int w) {
     backward_tc_ = backward_cc_ = false;
     plans_.assign(kNumConvs, dn::TcConvPlan{});
     plans_bwd_.assign(kNumConvs, dn::TcConvPlan{});
-    plans_wg_.assign(kNumConvs, dn::TcWgradPlan{});
     for (void *p : owned_)
         if (std::find(keep.begin(), keep.end(), p) == keep.end()) cudaFree(p);
     owned_ = keep;
@@ -241,8 +239,8 @@ cudaError_t Denoiser::ensure_backward() {
     for (int l = 0; l < 4; l++)
         if ((e = take(skip_g_[l], pixels(l) * kEnc[l])) != cudaSuccess) return e;
     if ((e = take(l1_part_, (size_t)4 * dn::kL1Blocks)) != cudaSuccess) return e;
-    std::vector<dn::BiasJob> jobs;
-    size_t partial_wg = 0;
+    bias_jobs_.clear();
+    dn::TcWgradConv wg[kNumConvs];
     for (int i = kNumConvs - 1; i >= 0; i--) {
         const Conv &c = convs_[i];
         const int l = kLevel[i], h = h_ >> l, w = w_dim_ >> l;
@@ -261,18 +259,16 @@ cudaError_t Denoiser::ensure_backward() {
             if ((e = take(bias_part_[i], (size_t)j.rows * c.cout)) != cudaSuccess) return e;
             j.part = bias_part_[i];
         }
-        jobs.push_back(j);
+        bias_jobs_.push_back(j);
         if (i > 0 && (e = dn::tc_conv_plan(plans_bwd_[i], g, n_, h, w, pad16(c.cout), c.cin, false, sm_count_,
                                            true)) != cudaSuccess)
             return e;
-        if ((e = dn::tc_wgrad_plan(plans_wg_[i], g, n_, h, w, c.cin, pad16(c.cin), c.cout, sm_count_)) != cudaSuccess)
-            return e;
-        partial_wg = std::max(partial_wg, plans_wg_[i].partial_floats);
+        wg[i].g = g, wg[i].fwd = &plans_[i], wg[i].cin = c.cin, wg[i].cout = c.cout, wg[i].dw = g_ + c.offset;
     }
-    if ((e = take(partial_wg_, partial_wg)) != cudaSuccess || (e = take(bias_jobs_, jobs.size())) != cudaSuccess ||
-        (e = cudaMemcpy(bias_jobs_, jobs.data(), jobs.size() * sizeof(jobs[0]), cudaMemcpyHostToDevice)) !=
-            cudaSuccess)
+    if ((e = dn::tc_wgrad_plan(plan_wg_, wg, kNumConvs, sm_count_)) != cudaSuccess ||
+        (e = take(partial_wg_, plan_wg_.partial_floats)) != cudaSuccess)
         return e;
+    dn::tc_wgrad_place(plan_wg_, partial_wg_);
     backward_tc_ = true;
     return cudaSuccess;
 }
@@ -449,10 +445,10 @@ cudaError_t Denoiser::backward_tc(const float *target, cudaStream_t st) {
         // optimizer step, beside the previous kernel)
         chk(dn::conv3x3_forward_tc(plans_bwd_[i], wtcb_ + tcb_off_[i], nullptr, nullptr, nullptr, err_, st, &f, true));
     }
-    for (int i = kNumConvs - 1; i >= 0; i--)
-        chk(dn::conv3x3_wgrad_tc(plans_wg_[i], plans_[i], g_ + convs_[i].offset, partial_wg_, err_, st));
-    chk(dn::bias_all(bias_jobs_, kNumConvs, 128, st));
-    chk(dn::l1_finalize(l1_part_, dn::l1_blocks(px), px * 3, loss_, st));
+    if (e == cudaSuccess) chk(dn::wgrad_all_tc(plan_wg_, err_, st));
+    if (e == cudaSuccess)
+        chk(dn::grad_finish(plan_wg_, bias_jobs_.data(), (int)bias_jobs_.size(), l1_part_, dn::l1_blocks(px), loss_,
+                            1.f / (float)(px * 3), st));
     return e;
 }
 

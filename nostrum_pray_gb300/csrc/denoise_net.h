@@ -92,14 +92,14 @@ class Denoiser {
     std::vector<size_t> tcb_off_;
     std::vector<dn::TcConvPlan> plans_bwd_;
     float *bias_part_[19] = {}, *skip_g_[4] = {}, *l1_part_ = nullptr;
-    dn::BiasJob *bias_jobs_ = nullptr;
+    std::vector<dn::BiasJob> bias_jobs_;
     bool backward_tc_ = false, backward_cc_ = false;  // backward buffers exist
     // every forward and backward-data packing as one launch (dn::tc_pack_all)
     dn::TcPackJob *pack_jobs_ = nullptr;
     int n_pack_jobs_ = 0;
     size_t pack_total_ = 0;
-    // tensor-core weight gradients: one plan per convolution, per-group partial sums
-    std::vector<dn::TcWgradPlan> plans_wg_;
+    // tensor-core weight gradients: the plan of all of them, per-group partial sums
+    dn::TcWgradPlan plan_wg_{};
     float *partial_wg_ = nullptr;
     float *out_ = nullptr, *gout_ = nullptr, *gtmp_ = nullptr;
     const __half *feat_ = nullptr;  // features of the last forward (the caller's buffer; used until the call returns)

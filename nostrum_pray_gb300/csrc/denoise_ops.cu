@@ -179,24 +179,6 @@ __global__ void k_relu_mask(const __nv_bfloat16 *y, const float *g, float *out, 
     for (size_t i = gtid(); i < n; i += gstride()) out[i] = bf(y[i]) > 0.f ? g[i] : 0.f;
 }
 
-// One block (256 threads) per channel of each job: thread t adds rows t, t +
-// 256, ..., then a fixed tree adds the 256 sums (the same order on every run).
-__global__ void k_bias_all(const BiasJob *jobs) {
-    __shared__ float sm[256];
-    const BiasJob J = jobs[blockIdx.y];
-    const int k = (int)blockIdx.x, t = (int)threadIdx.x;
-    if (k >= J.c) return;
-    float s = 0.f;
-    for (int r = t; r < J.rows; r += 256) s += J.part[(size_t)r * J.c + k];
-    sm[t] = s;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (t < o) sm[t] += sm[t + o];
-        __syncthreads();
-    }
-    if (t == 0) J.db[k] = sm[0];
-}
-
 __global__ void k_bias_grad(const float *g, float *db, size_t pixels, int c) {
     // one block per channel
     __shared__ float sm[256];
@@ -464,11 +446,6 @@ cudaError_t bias_grad(const float *g, float *db, size_t pixels, int c, cudaStrea
     k_bias_grad<<<c, 256, 0, st>>>(g, db, pixels, c);
     return cudaGetLastError();
 }
-cudaError_t bias_all(const BiasJob *jobs_dev, int njobs, int max_c, cudaStream_t st) {
-    if (njobs <= 0 || max_c <= 0) return cudaErrorInvalidValue;
-    k_bias_all<<<dim3((unsigned)max_c, (unsigned)njobs), 256, 0, st>>>(jobs_dev);
-    return cudaGetLastError();
-}
 cudaError_t avgpool(const __nv_bfloat16 *x, __nv_bfloat16 *y, int n, int h, int w, int c, cudaStream_t st) {
     k_avgpool<<<blocks_for((size_t)n * h * w * c / 4), 256, 0, st>>>(x, y, n, h, w, c);
     return cudaGetLastError();
@@ -510,10 +487,6 @@ cudaError_t l1_loss_tc(const float *out, const float *target, const __half *feat
     return cudaGetLastError();
 }
 int l1_blocks(size_t pixels) { return (int)std::min<size_t>((pixels + 255) / 256, kL1Blocks); }
-cudaError_t l1_finalize(const float *part, int blocks, size_t n, float *loss, cudaStream_t st) {
-    k_l1_finalize<<<1, 256, 0, st>>>(part, blocks, loss, 1.f / (float)n);
-    return cudaGetLastError();
-}
 cudaError_t add_input(float *out, const __nv_bfloat16 *x0, int x0_c, size_t pixels, cudaStream_t st) {
     k_add_input<<<blocks_for(pixels * 3), 256, 0, st>>>(out, x0, x0_c, pixels);
     return cudaGetLastError();

@@ -107,27 +107,53 @@ cudaError_t conv3x3_forward_tc(const TcConvPlan &p, const __nv_bfloat16 *wpacked
 // kernel's prologue (barriers, tensor memory, weight copies) overlaps the
 // previous kernel of the stream; its input copies wait for that kernel to
 // complete. The previous kernel must not write the weights or the bias.
-// Weight gradient of a 3x3 convolution on the tensor cores:
+// Weight gradients of a network's 3x3 convolutions on the tensor cores:
 // dw[co][tap][ci] = sum over pixels p of g[p][co] * x[p + offset(tap)][ci],
-// a GEMM with M = output channels (padded to 128), N = input channels, K =
-// pixels. g: the output gradient as BF16 with cout_pad = cout rounded up to
-// 16 channels (planar); x: the convolution's input, read through the
-// forward plan's halo tensor map (fwd: a plan over x with cin = cin_pad).
-// Each CTA accumulates the nine taps (or a group of them, as many as tensor
-// memory holds) over a group of 16 x 8 tiles and writes them to `partial`
-// (partial_floats floats); a second kernel adds the groups in order into dw.
-struct TcWgradPlan {
+// per tap a GEMM with M = output channels (padded to 64 or 128), N = input channels,
+// K = pixels. g: the output gradient as BF16 with cout rounded up to 16
+// channels (planar); x: the convolution's input, read through a forward
+// plan's tensor map. One launch serves every convolution: its CTAs are items
+// (convolution, group of tiles, group of taps); an item's sums go to `partial`
+// per group of tiles, or, where one group holds every tile, straight to dw.
+// grad_finish adds the groups in order, sums the bias gradients' rows and
+// makes the loss, in one launch.
+constexpr int kMaxWgrad = 24;
+struct TcWgradJob {
     alignas(64) unsigned char gmap[128];  // CUtensorMap of g: (8 W, H, cout_pad / 8, N), box (64, 16, cout_pad / 8, 1)
-    const __nv_bfloat16 *g;
-    int n, h, w, cin, cin_pad, cout, cout_pad;
-    int tiles_x, tiles_y, tiles, tiles_per_cta, groups, taps_per_pass, passes, tmem_cols, stages;
-    uint32_t b_off, stage_bytes, bar_off;
+    alignas(64) unsigned char xmap[128];  // the forward plan's
+    float *dw, *out;                      // out: partial sums [group][9][cout][cin_pad], or dw (one group)
+    int n, cin, cin_pad, cout, cout_pad, rows, tiles_x, tiles_y, tiles;  // rows: M
+    int tiles_per_cta, groups, taps_per_pass, passes, stages, first_item;
+    uint32_t b_off, stage_bytes;
+    size_t partial_off;
+};
+struct TcWgradPlan {
+    TcWgradJob job[kMaxWgrad];  // in the order of their items
+    int jobs, items, tmem_cols;
+    uint32_t bar_off;
     size_t smem, partial_floats;
 };
-cudaError_t tc_wgrad_plan(TcWgradPlan &p, const __nv_bfloat16 *g, int n, int h, int w, int cin, int cin_pad, int cout,
-                          int sm_count);
-cudaError_t conv3x3_wgrad_tc(const TcWgradPlan &p, const TcConvPlan &fwd, float *dw, float *partial, int *err,
-                             cudaStream_t st);
+// One convolution of a plan to be made.
+struct TcWgradConv {
+    const __nv_bfloat16 *g;
+    const TcConvPlan *fwd;  // a plan over x with cin = cin_pad
+    int cin, cout;
+    float *dw;
+};
+cudaError_t tc_wgrad_plan(TcWgradPlan &p, const TcWgradConv *convs, int count, int sm_count);
+// Places the partial sums (partial_floats floats).
+void tc_wgrad_place(TcWgradPlan &p, float *partial);
+cudaError_t wgrad_all_tc(const TcWgradPlan &p, int *err, cudaStream_t st);
+// Bias gradient: db[k] = the sum over rows of part[row * c + k].
+struct BiasJob {
+    const float *part;
+    float *db;
+    int rows, c;
+};
+// After wgrad_all_tc: the group sums, the bias gradients, and the loss as inv
+// times the sum of l1[0..l1_n).
+cudaError_t grad_finish(const TcWgradPlan &p, const BiasJob *bias, int nbias, const float *l1, int l1_n, float *loss,
+                        float inv, cudaStream_t st);
 cudaError_t conv3x3_forward(const __nv_bfloat16 *x, const __nv_bfloat16 *w, const float *b, __nv_bfloat16 *y,
                             float *y32, int n, int h, int wd, int cin, int cout, bool relu, cudaStream_t st);
 // gpre: output gradient after the ReLU mask (FP32, n*h*w*cout); dx may be NULL
@@ -136,14 +162,6 @@ cudaError_t conv3x3_backward(const __nv_bfloat16 *x, const __nv_bfloat16 *w, con
 cudaError_t relu_mask(const __nv_bfloat16 *y, const float *g, float *out, size_t n, cudaStream_t st);
 // db[c] += sum over pixels of g[p][c]
 cudaError_t bias_grad(const float *g, float *db, size_t pixels, int c, cudaStream_t st);
-// Bias gradients: db[k] = the sum over rows of part[row * c + k], in a fixed
-// order (jobs on the device).
-struct BiasJob {
-    const float *part;
-    float *db;
-    int rows, c;
-};
-cudaError_t bias_all(const BiasJob *jobs_dev, int njobs, int max_c, cudaStream_t st);
 cudaError_t avgpool(const __nv_bfloat16 *x, __nv_bfloat16 *y, int n, int h, int w, int c, cudaStream_t st);
 cudaError_t avgpool_backward(const float *gy, float *gx, int n, int h, int w, int c, cudaStream_t st);
 cudaError_t upsample_backward(const float *gy, float *gx, int n, int h, int w, int c, int cy, cudaStream_t st);
@@ -168,12 +186,11 @@ cudaError_t l1_loss(const float *out, const float *target, const __half *feat, f
 // values as BF16, planar, padded to 16 channels (images of px pixels); per
 // block the sum of the |differences| in part[block] and of the three gradients
 // in part[kL1Blocks + 3 block + k] (part: 4 kL1Blocks floats, l1_blocks(pixels)
-// blocks). l1_finalize makes the loss of the former.
+// blocks); grad_finish adds them.
 constexpr int kL1Blocks = 608;
 int l1_blocks(size_t pixels);
 cudaError_t l1_loss_tc(const float *out, const float *target, const __half *feat, __nv_bfloat16 *g, float *part,
                        size_t pixels, size_t px, cudaStream_t st);
-cudaError_t l1_finalize(const float *part, int blocks, size_t n, float *loss, cudaStream_t st);
 // out (3 channels) += the first 3 of x0's x0_c channels (the input's log radiance)
 cudaError_t add_input(float *out, const __nv_bfloat16 *x0, int x0_c, size_t pixels, cudaStream_t st);
 cudaError_t expm1_out(const float *out, const __half *feat, float *rad, size_t n, cudaStream_t st);

@@ -846,7 +846,7 @@ __global__ void __launch_bounds__(kConvThreads, 2) k_conv_tc(const __grid_consta
 // ---- weight gradient ---------------------------------------------------------
 //
 // dw[co][tap][ci] = sum_p g[p][co] x[p + offset(tap)][ci]: per tap a GEMM with
-// M = co (128 rows: the output-gradient channels, zero rows above cout),
+// M = co (64 or 128 rows: the output-gradient channels, zero rows above cout),
 // N = ci (cin_pad), K = pixels. Both operands come straight from the
 // channel-planar tiles TMA writes ([8-channel plane][pixel][8 channels], 16
 // bytes per pixel), read as MN-major matrices (the 8 channels of a pixel
@@ -859,57 +859,56 @@ __global__ void __launch_bounds__(kConvThreads, 2) k_conv_tc(const __grid_consta
 //      halo pixel (2k + dy, dx), core matrices one halo row (160 bytes) apart
 //      along K and one plane apart along N.
 // So every tap reads the same halo, shifted by whole 16-byte pixels, as in
-// the forward pass. Each CTA owns a group of tiles and a group of taps
-// (tensor memory holds taps_per_pass x cin_pad FP32 columns). One thread
-// loads the tiles into two shared-memory stages, the next tile's planes
-// while the tensor cores work on this one's (one stage where two do not
-// fit), and issues the MMAs. The accumulators of the output channels below
-// cout go to partial[group][tap][co][ci]; k_wgrad_finalize adds the groups in
-// order into dw. Every wait is bounded (error flag, drain, TMEM freed).
+// the forward pass. An item is a group of tiles and of taps of one
+// convolution (tensor memory holds taps_per_pass x cin_pad FP32 columns, half
+// of it, so that two CTAs share an SM and one's epilogue runs beside the
+// other's MMAs); all convolutions' items are one grid, the longest first, so
+// that the deep levels' few tiles fill the SMs that the wide levels leave (one
+// launch per convolution: 8 to 34 us each, 340 us and 130 us of finalizing
+// for a batch of 8 x 128^2). One thread loads the
+// tiles through up to four shared-memory stages and issues the MMAs. The sums
+// of the output channels below cout go to out[group][tap][co][ci]. Every wait
+// is bounded (error flag, drain, TMEM freed).
 constexpr uint32_t kGradPlaneBytes = kTileW * kTileH * 16;  // 2,048
-constexpr int kGradPlanes = 16;                             // 128 rows of A
 
 struct WgArgs {
-    float *partial;  // [group][9][cout][cin_pad]
-    int n, h, wd, cin_pad, cout, cout_pad;
-    int tiles_x, tiles_y, tiles, tiles_per_cta, taps_per_pass, tmem_cols, stages;
-    uint32_t b_off, stage_bytes, bar_off;
+    TcWgradPlan p;
     int *err;
 };
 
 // MN-major A and B: transpose bits of the kind::f16 instruction descriptor
 __host__ __device__ constexpr uint32_t inst_desc_mn(int m, int n) { return inst_desc(m, n) | (1u << 15) | (1u << 16); }
 
-__global__ void __launch_bounds__(128) k_wgrad_tc(const __grid_constant__ CUtensorMap gmap,
-                                                  const __grid_constant__ CUtensorMap xmap, WgArgs P) {
+__global__ void __launch_bounds__(128, 2) k_wgrad_tc(const __grid_constant__ WgArgs A) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const int tid = threadIdx.x, warp = tid >> 5;
+    int ji = 0;
+    while (ji + 1 < A.p.jobs && A.p.job[ji + 1].first_item <= (int)blockIdx.x) ji++;
+    const TcWgradJob &P = A.p.job[ji];
     const int S = P.stages;
     const uint32_t base = smem_u32(smem);
-    // bars[s] stage s loaded, bars[2 + s] MMAs reading stage s done, bars[4] drain
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + P.bar_off);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 5);
+    // bars[s] stage s loaded, bars[4 + s] MMAs reading stage s done, bars[8] drain
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + A.p.bar_off);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 9);
     int *okflag = reinterpret_cast<int *>(tmem_slot + 1);
     const int gplanes = P.cout_pad >> 3, xplanes = P.cin_pad >> 3;
-    const int group = blockIdx.x, pass = blockIdx.y;
+    const int item = (int)blockIdx.x - P.first_item, group = item / P.passes, pass = item - group * P.passes;
     const int tap0 = pass * P.taps_per_pass, ntaps = min(9 - tap0, P.taps_per_pass);
-    const int t_begin = group * P.tiles_per_cta, t_end = min(P.tiles, t_begin + P.tiles_per_cta);
-    auto abase = [&](int st) { return base + (uint32_t)st * P.stage_bytes; };
+    const int t_begin = group * P.tiles_per_cta, n = min(P.tiles, t_begin + P.tiles_per_cta) - t_begin;
     auto bar = [&](int i) { return smem_u32(&bars[i]); };
 
     // the rows of A above cout_pad stay zero, in every stage
     for (int st = 0; st < S; st++)
-        for (uint32_t i = (uint32_t)gplanes * kGradPlaneBytes / 16 + tid; i < kGradPlanes * kGradPlaneBytes / 16;
-             i += 128)
+        for (uint32_t i = (uint32_t)gplanes * kGradPlaneBytes / 16 + tid; i < P.b_off / 16; i += 128)
             reinterpret_cast<uint4 *>(smem + (size_t)st * P.stage_bytes)[i] = make_uint4(0u, 0u, 0u, 0u);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(P.tmem_cols)
+                     "r"(A.p.tmem_cols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        for (int i = 0; i < 5; i++) mbar_init(bar(i));
+        for (int i = 0; i < 9; i++) mbar_init(bar(i));
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the zero rows, for the tensor cores
@@ -919,138 +918,170 @@ __global__ void __launch_bounds__(128) k_wgrad_tc(const __grid_constant__ CUtens
     const uint32_t tmem = *tmem_slot;
 
     if (tid == 0) {
-        bool ok = true;
-        const uint32_t idesc = inst_desc_mn(128, P.cin_pad);
+        grid_dependency_wait();
+        const CUtensorMap *gmap = reinterpret_cast<const CUtensorMap *>(P.gmap);
+        const CUtensorMap *xmap = reinterpret_cast<const CUtensorMap *>(P.xmap);
+        const uint32_t idesc = inst_desc_mn(P.rows, P.cin_pad);
         const uint32_t bytes = (uint32_t)gplanes * kGradPlaneBytes + (uint32_t)xplanes * kPlaneBytes;
-        const int per_img = P.tiles_x * P.tiles_y;
-        const int n = t_end > t_begin ? t_end - t_begin : 0;
-        // tile i of the group goes to stage i % S; issue() starts its loads
-        auto issue = [&](int i) {
-            const int t = t_begin + i, st = i % S;
-            const int img = t / per_img, rem = t - img * per_img;
-            const int y0 = (rem / P.tiles_x) * kTileH, x0 = (rem % P.tiles_x) * kTileW;
-            const uint32_t a = abase(st), b = a + P.b_off;
-            mbar_expect_tx(bar(st), bytes);
-            tma_tile(a, &gmap, bar(st), x0, y0, img);
-            tma_tile(b, &xmap, bar(st), x0 - 1, y0 - 1, img);
+        TileWalk t(t_begin, 1, P.tiles_x, P.tiles_y);
+        Ring in(S), out(S);  // stages loaded, stages consumed
+        int issued = 0, waited = 0;
+        auto load = [&]() {
+            const uint32_t a = base + (uint32_t)in.slot * P.stage_bytes, b = bar(in.slot);
+            mbar_expect_tx(b, bytes);
+            tma_tile(a, gmap, b, t.x0(), t.y0(), t.img);
+            tma_tile(a + P.b_off, xmap, b, t.x0() - 1, t.y0() - 1, t.img);
+            in.next(), t.next();
+            issued++;
         };
-        int issued = 0, consumed = 0, committed = 0;
-        if (n > 0) issue(issued++);
-        for (int i = 0; i < n && ok; i++) {
-            const int st = i % S;
-            // with two stages, load tile i + 1 into the other stage as soon as
-            // the MMAs of tile i - 1, which read it, are done
-            if (S == 2 && i + 1 < n) {
-                if (i >= 1 && !mbar_wait(bar(2 + (st ^ 1)), (uint32_t)((i - 1) / 2) & 1u)) {
-                    ok = false;
-                    break;
-                }
-                issue(issued++);
-            }
-            if (!mbar_wait(bar(st), (uint32_t)(i / S) & 1u)) {
-                ok = false;
-                break;
-            }
-            consumed = i + 1;
+        bool ok = true;
+        while (issued < S && issued < n) load();
+        for (int i = 0; i < n; i++) {
+            if (!(ok = mbar_wait(bar(out.slot), out.phase))) break;
+            waited = i + 1;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t a = abase(st), b = a + P.b_off;
+            const uint32_t a = base + (uint32_t)out.slot * P.stage_bytes, b = a + P.b_off;
+            const uint64_t ad = smem_desc(a, 128u, kGradPlaneBytes);
             for (int q = 0; q < ntaps; q++) {
-                const int tap = tap0 + q, dy = tap / 3, dx = tap - 3 * (tap / 3);
+                const int tap = tap0 + q, dy = tap / 3, dx = tap - 3 * dy;
                 const uint32_t d = tmem + (uint32_t)(q * P.cin_pad);
-                const uint64_t ad = smem_desc(a, 128u, kGradPlaneBytes);
                 const uint64_t bd = smem_desc(b + (uint32_t)(dy * kHaloW + dx) * 16u, kRowBytes, kPlaneBytes);
 #pragma unroll
                 for (int k = 0; k < kTileH / 2; k++)  // two tile rows per step
                     mma(d, ad + k * (256u >> 4), bd + k * (2 * kRowBytes >> 4), idesc, (i == 0 && k == 0) ? 0u : 1u);
             }
-            commit(bar(2 + st));
-            committed = i + 1;
-            if (S == 1) {
-                // one stage: the next load waits for this tile's MMAs
-                if (!mbar_wait(bar(2), (uint32_t)i & 1u)) {
-                    ok = false;
-                    break;
-                }
-                if (i + 1 < n) issue(issued++);
+            commit(bar(4 + out.slot));
+            // refill the stage of the tile before this one, whose MMAs end
+            // while this one's run (one stage: this one's own)
+            const int prev = S == 1 ? i : i - 1;
+            if (prev >= 0 && issued < n) {
+                const int slot = S == 1 ? out.slot : (out.slot ? out.slot : S) - 1;
+                const uint32_t phase = S == 1 || out.slot ? out.phase : out.phase ^ 1u;
+                if (!(ok = mbar_wait(bar(4 + slot), phase))) break;
+                load();
             }
+            out.next();
         }
-        if (ok && n > 0 && S == 2 && !mbar_wait(bar(2 + (n - 1) % 2), (uint32_t)((n - 1) / 2) & 1u)) ok = false;
-        *okflag = !ok ? 0 : (n == 0 ? 2 : 1);  // 2: no tile in this group
+        // everything issued completes before the epilogue reads and TMEM is freed
+        commit(bar(8));
+        ok = mbar_wait(bar(8), 0) && ok;
+        *okflag = ok ? 1 : 0;
         if (!ok) {
-            // bounded drain: copies still in flight, then every MMA issued
-            for (int j = consumed; j < issued; j++) mbar_wait(bar(j % S), (uint32_t)(j / S) & 1u);
-            if (committed > 0) {
-                commit(bar(4));
-                mbar_wait(bar(4), 0);
-            }
+            // copies still in flight (bounded)
+            Ring r(S);
+            for (int i = 0; i < issued; i++, r.next())
+                if (i >= waited) mbar_wait(bar(r.slot), r.phase);
         }
     }
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int flag = *okflag;
-    if (flag == 0 && tid == 0) atomicExch(P.err, 1);
-    // epilogue: warp q reads TMEM lanes 32q..32q+31 (rows co), all columns;
-    // rows from cout on are zero padding and are not stored
-    const int co = warp * 32 + (tid & 31);
-    for (int q = 0; q < ntaps && warp * 32 < P.cout; q++) {
-        float *dst = P.partial + (((size_t)group * 9 + tap0 + q) * P.cout + co) * P.cin_pad;
+    const bool ok = *okflag != 0;
+    if (!ok && tid == 0) atomicExch(A.err, 1);
+    // epilogue: warp q reads TMEM lanes 32q..32q+31, all columns. With M = 128
+    // these are rows (co) 32q..32q+31, with M = 64 the first 16 lanes are rows
+    // 16q..16q+15; rows from cout on are zero padding and are not stored
+    const int lane = tid & 31, co = P.rows == 64 ? (lane < 16 ? warp * 16 + lane : P.cout) : warp * 32 + lane;
+    const bool direct = P.out == P.dw;  // [co][tap][ci]
+    for (int q = 0; ok && q < ntaps && warp * (P.rows >> 2) < P.cout; q++) {
+        float *dst = direct ? P.out + ((size_t)co * 9 + tap0 + q) * P.cin_pad
+                            : P.out + (((size_t)group * 9 + tap0 + q) * P.cout + co) * P.cin_pad;
+        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(q * P.cin_pad);
         for (int c0 = 0; c0 < P.cin_pad; c0 += 16) {
             uint32_t r[16];
-            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(q * P.cin_pad + c0);
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
-                "[%16];"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                  "=r"(r[15])
-                : "r"(taddr)
-                : "memory");
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            load_tmem<1>(taddr + c0, r);
             if (co >= P.cout) continue;
             float4 *o = reinterpret_cast<float4 *>(dst + c0);
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const float v0 = flag == 1 ? __uint_as_float(r[4 * k]) : 0.f;
-                const float v1 = flag == 1 ? __uint_as_float(r[4 * k + 1]) : 0.f;
-                const float v2 = flag == 1 ? __uint_as_float(r[4 * k + 2]) : 0.f;
-                const float v3 = flag == 1 ? __uint_as_float(r[4 * k + 3]) : 0.f;
-                o[k] = make_float4(v0, v1, v2, v3);
-            }
+            for (int k = 0; k < 4; k++)
+                o[k] = make_float4(__uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1]),
+                                   __uint_as_float(r[4 * k + 2]), __uint_as_float(r[4 * k + 3]));
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(P.tmem_cols)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(A.p.tmem_cols)
                      : "memory");
     }
 }
 
-// dw[co][tap][ci] = sum over groups (in order) of partial[group][tap][co][ci]
-// Block of 256 threads: 32 consecutive gradient elements x 8 slices; slice
-// s adds groups s, s + 8, ..., and the 8 slice sums are added in slice order
-// (the same order on every run).
+// The end of a backward pass, one grid of 256-thread blocks:
+//   weight gradients: four consecutive input channels per thread; of more
+//     than kFinSlices groups, a warp's 32 such elements x 8 slices (slice s
+//     adds groups s, s + 8, ..., and the slice sums are added in order), else
+//     256 elements, each thread all groups;
+//   bias gradients: a block per channel, thread t adds rows t, t + 256, ...,
+//     then a fixed tree;
+//   the loss (the last block): the same over the loss kernel's block sums.
+// The same order on every run.
 constexpr int kFinSlices = 8;
-__global__ void k_wgrad_finalize(const float *partial, float *dw, int groups, int cout, int cin, int cin_pad) {
-    __shared__ float sm[kFinSlices][32];
-    const size_t total = (size_t)cout * 9 * cin;
-    const int lane = (int)threadIdx.x & 31, slice = (int)threadIdx.x >> 5;
-    const size_t i = (size_t)blockIdx.x * 32 + lane;
-    float v = 0.f;
-    if (i < total) {
-        const int ci = (int)(i % cin);
-        const size_t rest = i / cin;
-        const int tap = (int)(rest % 9), co = (int)(rest / 9);
-        for (int g = slice; g < groups; g += kFinSlices)
-            v += partial[(((size_t)g * 9 + tap) * cout + co) * cin_pad + ci];
+struct FinishArgs {
+    struct Weights {
+        const float *partial;
+        float *dw;
+        int groups, cout, cin, cin_pad, sliced, first_block;
+    } w[kMaxWgrad];
+    BiasJob bias[kMaxWgrad];
+    int bias_first[kMaxWgrad];
+    int nw, nbias;
+    const float *l1;
+    float *loss;
+    float inv;
+    int l1_n;
+};
+
+__global__ void __launch_bounds__(256) k_grad_finish(const __grid_constant__ FinishArgs A) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __shared__ float sm[256];
+    __shared__ float4 sm4[kFinSlices][32];
+    const int tid = (int)threadIdx.x, b = (int)blockIdx.x;
+    if (b >= A.bias_first[0]) {
+        int j = 0;
+        while (j + 1 < A.nbias && A.bias_first[j + 1] <= b) j++;
+        const int k = b - A.bias_first[j];
+        const bool loss = k >= A.bias[j].c;  // (past the last bias job)
+        const int rows = loss ? A.l1_n : A.bias[j].rows;
+        float s = 0.f;
+        for (int r = tid; r < rows; r += 256) s += loss ? A.l1[r] : A.bias[j].part[(size_t)r * A.bias[j].c + k];
+        sm[tid] = s;
+        __syncthreads();
+        for (int o = 128; o > 0; o >>= 1) {
+            if (tid < o) sm[tid] += sm[tid + o];
+            __syncthreads();
+        }
+        if (tid == 0) {
+            if (loss) A.loss[0] = sm[0] * A.inv;
+            else A.bias[j].db[k] = sm[0];
+        }
+        return;
     }
-    sm[slice][lane] = v;
-    __syncthreads();
-    if (slice == 0 && i < total) {
-        float s = sm[0][lane];
-        for (int k = 1; k < kFinSlices; k++) s += sm[k][lane];
-        dw[i] = s;
+    int j = 0;
+    while (j + 1 < A.nw && A.w[j + 1].first_block <= b) j++;
+    const FinishArgs::Weights &W = A.w[j];
+    const int lane = tid & 31, slice = W.sliced ? tid >> 5 : 0, step = W.sliced ? kFinSlices : 1;
+    const int i = (b - W.first_block) * (W.sliced ? 32 : 256) + (W.sliced ? lane : tid);
+    const int quads = W.cin_pad >> 2, total = W.cout * 9 * quads;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto add = [](float4 &a, const float4 &x) { a.x += x.x, a.y += x.y, a.z += x.z, a.w += x.w; };
+    const int ci = 4 * (i % quads), rest = i / quads, co = rest % W.cout, tap = rest / W.cout;
+    if (i < total) {
+        // [group][tap][co][ci]
+        const float4 *src = reinterpret_cast<const float4 *>(W.partial) + i;
+        for (int g = slice; g < W.groups; g += step) add(v, src[(size_t)g * total]);
+    }
+    if (W.sliced) {
+        sm4[slice][lane] = v;
+        __syncthreads();
+        if (slice) return;
+        for (int k = 1; k < kFinSlices; k++) add(v, sm4[k][lane]);
+    }
+    if (i < total) {
+        float *d = W.dw + ((size_t)co * 9 + tap) * W.cin + ci;
+        const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (ci + k < W.cin) d[k] = f[k];
     }
 }
 
@@ -1179,55 +1210,123 @@ cudaError_t tc_pack_weights_bwd(const float *w, __nv_bfloat16 *packed, int cin_f
     return cudaGetLastError();
 }
 
-cudaError_t tc_wgrad_plan(TcWgradPlan &p, const __nv_bfloat16 *g, int n, int h, int w, int cin, int cin_pad, int cout,
-                          int sm_count) {
+cudaError_t tc_wgrad_plan(TcWgradPlan &p, const TcWgradConv *convs, int count, int sm_count) {
     std::memset(&p, 0, sizeof(p));
-    if (n <= 0 || h <= 0 || w <= 0 || cin <= 0 || cin > cin_pad || (cin_pad & 15) || cin_pad > 256 || cout <= 0 ||
-        cout > 128)
-        return cudaErrorInvalidValue;
-    p.g = g, p.n = n, p.h = h, p.w = w, p.cin = cin, p.cin_pad = cin_pad, p.cout = cout;
-    p.cout_pad = (cout + 15) / 16 * 16;
-    p.tiles_x = (w + kTileW - 1) / kTileW;
-    p.tiles_y = (h + kTileH - 1) / kTileH;
-    const long long tiles = (long long)n * p.tiles_x * p.tiles_y;
-    if (tiles > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
-    p.tiles = (int)tiles;
-    // taps per pass: as many accumulators of cin_pad columns as 512 TMEM columns hold
-    p.taps_per_pass = 512 / cin_pad < 9 ? 512 / cin_pad : 9;
-    p.passes = (9 + p.taps_per_pass - 1) / p.taps_per_pass;
-    int cols = 32;
-    while (cols < p.taps_per_pass * cin_pad) cols <<= 1;
-    p.tmem_cols = cols;
-    // about one CTA per SM over all groups and passes (a CTA overlaps its
-    // loads with its MMAs; fewer groups also mean fewer partial sums)
-    const long long want = sm_count;
-    long long per = (tiles * p.passes + want - 1) / want;
-    if (per < 1) per = 1;
-    p.tiles_per_cta = (int)per;
-    p.groups = (int)((tiles + per - 1) / per);
-    // a stage: 128 rows of A (16 planes), then the halo planes of B; two
-    // stages (loads of the next tile beside the MMAs of this one) where they fit
-    p.b_off = kGradPlanes * kGradPlaneBytes;
-    p.stage_bytes = (p.b_off + (uint32_t)(cin_pad / 8) * kPlaneBytes + 1023) & ~1023u;
-    p.stages = 2 * (size_t)p.stage_bytes + 64 <= kSmemMax ? 2 : 1;
-    p.bar_off = (uint32_t)p.stages * p.stage_bytes;
-    p.smem = p.bar_off + 5 * 8 + 16;
-    if (p.smem > kSmemMax) return cudaErrorInvalidValue;
-    // no more CTAs per SM than TMEM has columns for (tcgen05.alloc would wait):
-    // ask for enough shared memory to keep the others off the SM
-    const size_t max_ctas = 512 / cols;
-    if (kSmemPerSm / (p.smem + 1024) > max_ctas) {
-        p.smem = kSmemPerSm / max_ctas - 1024 + 16;
-        if (p.smem > kSmemMax) p.smem = kSmemMax;
+    if (count <= 0 || count > kMaxWgrad) return cudaErrorInvalidValue;
+    // two CTAs per SM: half of the shared memory and of the tensor memory each
+    constexpr int kCols = 256;
+    const size_t budget = kSmemPerSm / 2 - 1024 - 128;
+    // clocks of a tile's MMAs of one tap (operands at 128 bytes per clock)
+    auto tap_clk = [](const TcWgradJob &j) { return 8.0 * (32 * j.rows + 32 * j.cin_pad) / 128; };
+    double total = 0;
+    for (int i = 0; i < count; i++) {
+        TcWgradJob &j = p.job[i];
+        const TcWgradConv &c = convs[i];
+        const TcConvPlan &f = *c.fwd;
+        j.n = f.n, j.cin = c.cin, j.cin_pad = f.cin, j.cout = c.cout, j.cout_pad = (c.cout + 15) / 16 * 16;
+        if (!c.g || !c.dw || c.cin <= 0 || c.cin > j.cin_pad || (j.cin_pad & 15) || j.cin_pad > kCols || c.cout <= 0 ||
+            c.cout > 128)
+            return cudaErrorInvalidValue;
+        j.dw = c.dw;
+        j.tiles_x = f.tiles_x, j.tiles_y = f.tiles_y, j.tiles = f.tiles;
+        // 64 rows where they suffice: half the operand bytes of A, which bound
+        // the MMAs of few input channels
+        j.rows = j.cout <= 64 ? 64 : 128;
+        // a stage: the rows of A (8 per plane), then the halo planes of B
+        j.b_off = (uint32_t)j.rows / 8 * kGradPlaneBytes;
+        j.stage_bytes = (j.b_off + (uint32_t)(j.cin_pad / 8) * kPlaneBytes + 1023) & ~1023u;
+        if (j.stage_bytes > budget) return cudaErrorInvalidValue;
+        j.stages = (int)std::min<size_t>(4, budget / j.stage_bytes);
+        std::memcpy(j.xmap, f.tmap, sizeof(j.xmap));
+        const cudaError_t e = tile_map(j.gmap, c.g, f.n, f.h, f.w, j.cout_pad, kTileW, kTileH);
+        if (e != cudaSuccess) return e;
+        total += j.tiles * 9.0 * tap_clk(j);
     }
-    p.partial_floats = (size_t)p.groups * 9 * cout * cin_pad;
-    return tile_map(p.gmap, g, n, h, w, p.cout_pad, kTileW, kTileH);
+    // Each convolution's groups of tiles and of taps: the cheapest split, an
+    // item costing its MMAs, its copies (64 bytes per clock and 2,600 clocks of
+    // latency, beside the MMAs where there is more than one stage), its stores
+    // (32 bytes per clock) and about 3,000 clocks to start up and end; items
+    // longer than about an SM's share of all MMAs are penalised (the longest
+    // one ends the launch). A group has at most seven tiles, or, of more than
+    // seven per SM, the tiles that one SM of a launch of its own would get with
+    // all of tensor memory: the FP32 sums run over its pixels one after
+    // another, and longer chains round worse (257 tiles per group moved the
+    // gradients of 8 x 128^2 by 6e-5, relative).
+    const double cap = std::max(0.6 * total / sm_count + 4000, 9000.0);
+    double cost[kMaxWgrad];
+    for (int i = 0; i < count; i++) {
+        TcWgradJob &j = p.job[i];
+        const double tile_load = (j.cout_pad / 8 * (double)kGradPlaneBytes + j.cin_pad / 8 * (double)kPlaneBytes) / 64;
+        double best = -1;
+        const int taps512 = std::min(9, 512 / j.cin_pad), passes512 = (9 + taps512 - 1) / taps512;
+        const long long chain = std::max(7LL, ((long long)j.tiles * passes512 + sm_count - 1) / sm_count);
+        for (int t = 1; t <= 9 && t * j.cin_pad <= kCols; t++)
+            for (long long q = 1; q <= chain && q <= j.tiles; q = q < 16 ? q + 1 : q + q / 8) {
+                const double m = t * tap_clk(j);
+                const double tile =
+                    j.stages > 1 ? std::max({m, tile_load, 2600.0 / j.stages}) : m + tile_load + 1600;
+                const double item = q * tile + 4.0 * t * j.cin_pad * j.cout / 32 + 3000;
+                const int passes = (9 + t - 1) / t, groups = (int)((j.tiles + q - 1) / q);
+                // (too long an item counts as if it alone kept its SM)
+                const double c = (double)passes * groups * item + std::max(0.0, item - cap) * sm_count +
+                                 (groups > 1 ? groups * 9.0 * j.cout * j.cin_pad / 128 : 0.0);
+                if (best < 0 || c < best) {
+                    best = c, cost[i] = item;
+                    j.taps_per_pass = t, j.passes = passes, j.tiles_per_cta = (int)q, j.groups = groups;
+                }
+            }
+    }
+    // the longest items first
+    for (int i = 1; i < count; i++)
+        for (int k = i; k > 0 && cost[k] > cost[k - 1]; k--)
+            std::swap(cost[k], cost[k - 1]), std::swap(p.job[k], p.job[k - 1]);
+    p.jobs = count;
+    int cols = 32;
+    for (int i = 0; i < count; i++) {
+        TcWgradJob &j = p.job[i];
+        j.first_item = p.items;
+        p.items += j.passes * j.groups;
+        p.bar_off = std::max(p.bar_off, (uint32_t)j.stages * j.stage_bytes);
+        while (cols < j.taps_per_pass * j.cin_pad) cols <<= 1;
+        j.partial_off = p.partial_floats;
+        if (j.groups > 1 || j.cin != j.cin_pad) p.partial_floats += (size_t)j.groups * 9 * j.cout * j.cin_pad;
+    }
+    p.tmem_cols = cols;
+    p.smem = p.bar_off + 9 * 8 + 16;
+    // (no more CTAs per SM than TMEM has columns for)
+    const size_t max_ctas = 512 / cols;
+    if (kSmemPerSm / (p.smem + 1024) > max_ctas) p.smem = kSmemPerSm / max_ctas - 1024 + 16;
+    if (p.smem > kSmemMax) p.smem = kSmemMax;
+    return cudaSuccess;
 }
 
-cudaError_t conv3x3_wgrad_tc(const TcWgradPlan &p, const TcConvPlan &fwd, float *dw, float *partial, int *err,
-                             cudaStream_t st) {
-    if (!partial || !dw || fwd.cin != p.cin_pad || fwd.n != p.n || fwd.h != p.h || fwd.w != p.w)
-        return cudaErrorInvalidValue;
+void tc_wgrad_place(TcWgradPlan &p, float *partial) {
+    for (int i = 0; i < p.jobs; i++) {
+        TcWgradJob &j = p.job[i];
+        j.out = j.groups > 1 || j.cin != j.cin_pad ? partial + j.partial_off : j.dw;
+    }
+}
+
+namespace {
+
+// Launches with programmatic stream serialisation: the kernel's prologue may
+// overlap the previous kernel, which it waits for itself.
+template <class Kernel, class Args>
+cudaError_t launch_overlapped(Kernel kernel, unsigned grid, unsigned block, size_t smem, cudaStream_t st, const Args &a) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3(grid), cfg.blockDim = dim3(block), cfg.dynamicSmemBytes = smem, cfg.stream = st;
+    cfg.attrs = attr, cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a);
+    return e == cudaSuccess ? cudaGetLastError() : e;
+}
+
+}  // namespace
+
+cudaError_t wgrad_all_tc(const TcWgradPlan &p, int *err, cudaStream_t st) {
+    if (p.jobs <= 0 || !p.job[0].out) return cudaErrorInvalidValue;
     static std::atomic<uint64_t> attr_set{0};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -1239,21 +1338,36 @@ cudaError_t conv3x3_wgrad_tc(const TcWgradPlan &p, const TcConvPlan &fwd, float 
         attr_set.fetch_or(bit);
     }
     WgArgs a;
-    a.partial = partial;
-    a.n = p.n, a.h = p.h, a.wd = p.w, a.cin_pad = p.cin_pad, a.cout = p.cout, a.cout_pad = p.cout_pad;
-    a.tiles_x = p.tiles_x, a.tiles_y = p.tiles_y, a.tiles = p.tiles, a.tiles_per_cta = p.tiles_per_cta;
-    a.taps_per_pass = p.taps_per_pass, a.tmem_cols = p.tmem_cols, a.stages = p.stages;
-    a.b_off = p.b_off, a.stage_bytes = p.stage_bytes, a.bar_off = p.bar_off;
+    a.p = p;
     a.err = err;
-    CUtensorMap gm, xm;
-    std::memcpy(&gm, p.gmap, sizeof(gm));
-    std::memcpy(&xm, fwd.tmap, sizeof(xm));
-    k_wgrad_tc<<<dim3((unsigned)p.groups, (unsigned)p.passes), 128, p.smem, st>>>(gm, xm, a);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    const size_t elems = (size_t)p.cout * 9 * p.cin;
-    k_wgrad_finalize<<<(unsigned)((elems + 31) / 32), 32 * kFinSlices, 0, st>>>(partial, dw, p.groups, p.cout, p.cin,
-                                                                             p.cin_pad);
-    return cudaGetLastError();
+    return launch_overlapped(k_wgrad_tc, (unsigned)p.items, 128, p.smem, st, a);
+}
+
+cudaError_t grad_finish(const TcWgradPlan &p, const BiasJob *bias, int nbias, const float *l1, int l1_n, float *loss,
+                        float inv, cudaStream_t st) {
+    if (nbias <= 0 || nbias > kMaxWgrad) return cudaErrorInvalidValue;
+    FinishArgs a;
+    std::memset(&a, 0, sizeof(a));
+    int blocks = 0;
+    for (int i = 0; i < p.jobs; i++) {
+        const TcWgradJob &j = p.job[i];
+        if (j.out == j.dw) continue;
+        FinishArgs::Weights &w = a.w[a.nw++];
+        w.partial = j.out, w.dw = j.dw;
+        w.groups = j.groups, w.cout = j.cout, w.cin = j.cin, w.cin_pad = j.cin_pad;
+        w.sliced = j.groups > kFinSlices ? 1 : 0;
+        w.first_block = blocks;
+        const int per_block = w.sliced ? 32 : 256;
+        blocks += (j.cout * 9 * (j.cin_pad / 4) + per_block - 1) / per_block;
+    }
+    for (int i = 0; i < nbias; i++) {
+        a.bias[i] = bias[i];
+        a.bias_first[i] = blocks;
+        blocks += bias[i].c;
+    }
+    a.nbias = nbias;
+    a.l1 = l1, a.l1_n = l1_n, a.loss = loss, a.inv = inv;
+    return launch_overlapped(k_grad_finish, (unsigned)blocks + 1, 256, 0, st, a);
 }
 
 cudaError_t tc_conv_plan(TcConvPlan &p, const __nv_bfloat16 *x, int n, int h, int w, int cin, int cout, bool relu,
