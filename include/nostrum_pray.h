@@ -52,8 +52,9 @@ typedef struct {
     float sah_traversal_cost;      /* traversalCost (5) */
     float sah_intersection_cost;   /* triangleIntersectionCost (1.5) */
     int32_t build_threads;         /* host threads for the build, 0 = all */
-    int32_t leaf_refine;           /* device layout only: leaves with more references than this get a
-                                      conservative sub-hierarchy (8; 0 = off). Results are unchanged. */
+    int32_t leaf_refine;           /* device layout only: most triangles per leaf (at most 4) of the conservative
+                                      hierarchy that the kernels cull with (8; 0 = off, they walk the reference's
+                                      tree itself). Results are unchanged. */
 } pray_tree_options;
 
 /* Ray-tracing frame parameters: the scene JSON's camera, lights and
@@ -136,8 +137,9 @@ pray_status pray_host_tree_dump(const pray_host_tree *t, float *boxes, float *sp
 pray_status pray_host_tree_precompute(const pray_host_tree *t, float *out18);
 
 /* The device layout this tree would be uploaded as (no device work):
- * out[4] = node records, triangle references, refined leaves, nodes added by
- * the refinement. Fails if the layout would not pass the upload checks. */
+ * out[4] = node records (the tree's and the culling hierarchy's), triangle
+ * references of the tree, triangles and node records of the culling
+ * hierarchy. Fails if the layout would not pass the upload checks. */
 pray_status pray_host_tree_device_layout(const pray_host_tree *t, int32_t leaf_refine, uint64_t *out);
 
 /* Camera constants the kernels use: inverse view matrix rows 0-2 (columns

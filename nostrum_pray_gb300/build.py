@@ -22,7 +22,8 @@ CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 ARCH = "-gencode=arch=compute_103a,code=sm_103a"
 
 CU_SOURCES = ["trace.cu", "pt.cu", "wavefront.cu", "wavefront_noalloc.cu", "batch.cu", "denoise_ops.cu", "denoise_tc.cu"]
-CPP_SOURCES = ["capi.cpp", "host/kdtree.cpp", "host/camera.cpp", "host/flatten.cpp", "denoise_net.cpp"]
+CPP_SOURCES = ["capi.cpp", "host/kdtree.cpp", "host/camera.cpp", "host/flatten.cpp", "host/cull_bvh.cpp",
+               "denoise_net.cpp"]
 CLI_SOURCES = ["cli/pray_main.cpp", "cli/scene_io.cpp"]
 DUMP_SOURCES = ["cli/scene_dump.cpp"]
 DUMP = os.path.join(BUILD, "pray_scene_dump")
@@ -34,7 +35,7 @@ CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-pthread", "-ffp-contract=off", "-Wa
 
 
 def _headers() -> List[str]:
-    hs = glob.glob(os.path.join(CSRC, "**", "*.h"), recursive=True)
+    hs = [h for e in ("*.h", "*.cuh") for h in glob.glob(os.path.join(CSRC, "**", e), recursive=True)]
     hs += glob.glob(os.path.join(ROOT, "include", "*.h"))
     return hs
 

@@ -8,6 +8,8 @@
 #include <atomic>
 #include <cstring>
 #include <exception>
+#include <functional>
+#include <future>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -94,12 +96,12 @@ struct pray_scene {
     GNode *d_nodes = nullptr;
     GTri *d_tris = nullptr;
     GShade *d_shade = nullptr;
+    GOwner *d_owners = nullptr;
     GTri *d_emit = nullptr;
     float *d_emit_cdf = nullptr;
     uint32_t n_emit = 0;
     float emit_area = 0.f;
     uint32_t n_gnodes = 0;
-    uint64_t refined_leaves = 0;
     int device_depth = 0;  // deepest node of the device hierarchy
     float tol = 0.f;
     float cull_c[3] = {0.f, 0.f, 0.f}, cull_r2 = -1.f;
@@ -136,6 +138,7 @@ struct pray_scene {
         v.nodes = d_nodes;
         v.tris = d_tris;
         v.shade = d_shade;
+        v.owners = d_owners;
         v.n_nodes = n_gnodes;
         v.n_refs = (uint32_t)tree.refs.size();
         v.n_tris = (uint32_t)n_tris;
@@ -153,6 +156,8 @@ struct pray_scene {
         cudaFree(d_nodes);
         cudaFree(d_tris);
         cudaFree(d_shade);
+        cudaFree(d_owners);
+        d_owners = nullptr;
         cudaFree(d_rgb);
         cudaFree(d_counters);
         cudaFree(d_emit);
@@ -489,13 +494,15 @@ pray_status pray_host_tree_device_layout(const pray_host_tree *t, int32_t leaf_r
     if (leaf_refine < 0) return set_error(PRAY_ERR_INVALID_ARGUMENT, "leaf_refine must be >= 0");
     PRAY_TRY({
         DeviceImage img;
-        flatten_for_device(t->tree, t->tris, leaf_refine, img);
+        CullBvh bvh;
+        if (leaf_refine > 0) bvh = build_cull_bvh(t->tris, leaf_refine, 0);
+        flatten_for_device(t->tree, t->tris, leaf_refine > 0 ? &bvh : nullptr, img);
         std::string bad;
         if (!validate_device_image(img, bad)) return set_error(PRAY_ERR_UNSUPPORTED, "device layout: " + bad);
-        out[0] = img.nodes.size();
-        out[1] = img.tris.size();
-        out[2] = img.refined_leaves;
-        out[3] = img.sub_nodes;
+        out[0] = img.nodes.size() + img.cull.size();
+        out[1] = img.refs;
+        out[2] = img.tris.size() - img.refs;
+        out[3] = img.cull.size();
         return PRAY_OK;
     })
 }
@@ -525,6 +532,7 @@ pray_status pray_scene_create(const float *verts, const float *colors, const uin
     std::vector<TriPre> pre;
     std::vector<GNode> gnodes;
     std::vector<GTri> gtris;
+    std::vector<GOwner> gowners;
     std::vector<GShade> gshade;
     std::vector<GTri> gemit;
     std::vector<float> gcdf;
@@ -533,20 +541,27 @@ pray_status pray_scene_create(const float *verts, const float *colors, const uin
         s->device = device;
         s->n_tris = n;
         pre = precompute_triangles(verts, n, opt->build_threads);
+        // the culling hierarchy beside the reference's tree
+        std::future<CullBvh> cull;
+        if (opt->leaf_refine > 0)
+            cull = std::async(std::launch::async, build_cull_bvh, std::cref(pre), opt->leaf_refine, opt->build_threads);
         s->tree = build_tree(pre, to_options(opt));
+        CullBvh bvh;
+        if (cull.valid()) bvh = cull.get();
         if (s->tree.refs.size() >= (1ull << 31))
             return set_error(PRAY_ERR_UNSUPPORTED, "more than 2^31-1 leaf references");
         DeviceImage img;
-        flatten_for_device(s->tree, pre, opt->leaf_refine, img);
+        flatten_for_device(s->tree, pre, opt->leaf_refine > 0 ? &bvh : nullptr, img);
         std::string bad;
         if (!validate_device_image(img, bad, &s->device_depth))
             return set_error(PRAY_ERR_UNSUPPORTED, "device layout: " + bad);
         gnodes.swap(img.nodes);
-        gnodes.insert(gnodes.end(), img.nodes_tight.begin(), img.nodes_tight.end());  // both copies, one buffer
+        s->n_gnodes = (uint32_t)gnodes.size();
+        gnodes.insert(gnodes.end(), img.cull.begin(), img.cull.end());  // both copies, one buffer
+        gowners.swap(img.owners);
         for (int k = 0; k < 3; k++) s->cull_c[k] = img.cull_center[k];
         s->cull_r2 = img.cull_radius2;
         gtris.swap(img.tris);
-        s->refined_leaves = img.refined_leaves;
         gshade.resize(n);
         for (uint64_t i = 0; i < n; i++) {
             GShade &g = gshade[i];
@@ -605,6 +620,13 @@ pray_status pray_scene_create(const float *verts, const float *colors, const uin
         s->release();
         return cuda_error(e, "cudaMemcpy (scene upload)");
     }
+    if (!gowners.empty() &&
+        ((e = cudaMalloc(&s->d_owners, gowners.size() * sizeof(GOwner))) != cudaSuccess ||
+         (e = cudaMemcpy(s->d_owners, gowners.data(), gowners.size() * sizeof(GOwner), cudaMemcpyHostToDevice)) !=
+             cudaSuccess)) {
+        s->release();
+        return cuda_error(e, "cudaMemcpy (owner lists)");
+    }
     if (!gemit.empty()) {
         if ((e = cudaMalloc(&s->d_emit, gemit.size() * sizeof(GTri))) != cudaSuccess ||
             (e = cudaMalloc(&s->d_emit_cdf, gcdf.size() * sizeof(float))) != cudaSuccess ||
@@ -617,8 +639,7 @@ pray_status pray_scene_create(const float *verts, const float *colors, const uin
         }
         s->n_emit = (uint32_t)gemit.size();
     }
-    s->n_gnodes = (uint32_t)(gnodes.size() / 2);
-    s->device_bytes = nb + tb + sb + gemit.size() * (sizeof(GTri) + sizeof(float));
+    s->device_bytes = nb + tb + sb + gowners.size() * sizeof(GOwner) + gemit.size() * (sizeof(GTri) + sizeof(float));
     *out = s.release();
     return PRAY_OK;
 }

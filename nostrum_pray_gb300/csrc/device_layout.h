@@ -13,7 +13,12 @@
 // order (a triangle referenced by two SAH leaves is stored twice). The
 // position of a reference in this array is the reference's depth-first visit
 // order, which breaks distance ties.
-//   v0 = (a.xyz, triangle id as bits), e1 = (b - a, 0), e2 = (c - a, 0)
+//   v0 = (a.xyz, triangle id as bits), e1 = (b - a, key), e2 = (c - a, owner)
+// key: the position; owner: kNoOwner. After the references come the culling
+// copy's triangles, each once, in its leaf order: with one owner (a leaf of
+// the exact copy) owner is that leaf's node and key its position, with more
+// owner is kOwnerList | their number and key the first one's index in the
+// owner lists.
 // Shading records: per triangle id, normal (w: 1 for emitters) and colour.
 #pragma once
 
@@ -22,8 +27,9 @@
 namespace pray_gpu {
 
 constexpr uint32_t kLeafFlag = 0x80000000u;
+constexpr uint32_t kOwnerList = 0x80000000u, kNoOwner = 0x7FFFFFFFu;
 constexpr int kMaxTreeDepth = 30;        // deepest reference tree the API accepts
-constexpr int kMaxTraversalDepth = 62;   // deepest device hierarchy (reference tree + leaf refinement)
+constexpr int kMaxTraversalDepth = 62;   // deepest device hierarchy (reference tree or culling copy)
 
 struct alignas(32) GNode {  // 32-byte aligned: one 256-bit load per node (traverse.cuh ldg_node)
     float lo[3];
@@ -40,6 +46,10 @@ struct alignas(16) GTri {
 };
 static_assert(sizeof(GTri) == 48, "GTri must be 48 bytes");
 
+struct alignas(8) GOwner {
+    uint32_t leaf, key;  // node of the exact copy, position of the reference
+};
+
 struct alignas(16) GShade {
     float n[4];
     float c[4];
@@ -47,10 +57,10 @@ struct alignas(16) GShade {
 
 // Launch-time view of a device scene.
 struct DevScene {
-    const GNode *nodes;  // n_nodes nodes with the reference's boxes and linear leaves, then the culling
-                         // copy (same topology, refined leaves, interior boxes bounding their triangles;
-                         // for finite-direction rays whose origin is within cull_r2 of cull_c)
+    const GNode *nodes;  // n_nodes nodes of the exact copy (the reference's tree), then the culling copy
+                         // (for finite-direction rays whose origin is within cull_r2 of cull_c)
     const GTri *tris;
+    const GOwner *owners;
     const GShade *shade;
     uint32_t n_nodes, n_refs, n_tris;
     float tol;  // absolute distance tolerance for culling boxes behind the origin

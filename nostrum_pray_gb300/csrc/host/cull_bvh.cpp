@@ -1,0 +1,204 @@
+#include "cull_bvh.h"
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <thread>
+
+namespace pray_gpu {
+
+namespace {
+
+constexpr int kBins = 16;
+// Costs of one node visit (two boxes) and of one triangle test, relative. A
+// visit outweighs a test: a warp walks its lanes' nodes one by one, but
+// tests their leaves together.
+constexpr double kVisit = 2.0, kTest = 1.0;
+constexpr size_t kParallel = 1024;  // subtrees from this size on may get a thread of their own
+
+struct Box {
+    float lo[3], hi[3];
+    void clear() {
+        for (int k = 0; k < 3; k++) lo[k] = INFINITY, hi[k] = -INFINITY;
+    }
+    void add(const Box &b) {
+        for (int k = 0; k < 3; k++) lo[k] = std::min(lo[k], b.lo[k]), hi[k] = std::max(hi[k], b.hi[k]);
+    }
+    double half_area() const {
+        const double x = (double)hi[0] - lo[0], y = (double)hi[1] - lo[1], z = (double)hi[2] - lo[2];
+        return x * y + y * z + z * x;
+    }
+};
+
+struct Prim {
+    Box box;
+    float c[3];  // twice the centre; 0 where the bounds are not finite (such
+                 // triangles still get a box that every ray enters)
+    uint32_t id;
+};
+
+struct Builder {
+    std::vector<Prim> prims;
+    int leaf_max;
+    // node pairs by the position of their split: the subtree over [lo, hi)
+    // uses pairs lo .. hi - 2, so parallel subtrees share nothing
+    struct Node {
+        Box box;
+        uint32_t pair, lo, count;  // interior: pair index; leaf: count > 0
+    };
+    std::vector<Node> root, pairs;
+
+    static int levels(size_t n, int leaf) {  // halvings until at most `leaf` are left
+        int d = 0;
+        while (n > (size_t)leaf) n = (n + 1) / 2, d++;
+        return d;
+    }
+
+    void build(Node &node, size_t lo, size_t hi, int depth, int threads) {
+        const size_t n = hi - lo;
+        Box bounds, centres;
+        bounds.clear(), centres.clear();
+        for (size_t i = lo; i < hi; i++) {
+            const Prim &p = prims[i];
+            bounds.add(p.box);
+            for (int k = 0; k < 3; k++) {
+                const float c = p.c[k];
+                centres.lo[k] = std::min(centres.lo[k], c), centres.hi[k] = std::max(centres.hi[k], c);
+            }
+        }
+        node.box = bounds;
+        node.pair = 0, node.lo = (uint32_t)lo, node.count = (uint32_t)n;
+        if (n <= 1) return;
+        int best_axis = -1, best_bin = 0;
+        double best = INFINITY;
+        float scale[3];
+        for (int k = 0; k < 3; k++) {
+            const float e = centres.hi[k] - centres.lo[k];
+            scale[k] = e > 0.f && std::isfinite(e) ? kBins * 0.9999f / e : 0.f;
+        }
+        auto bin_of = [&](const Prim &p, int k) {
+            const int b = (int)((p.c[k] - centres.lo[k]) * scale[k]);
+            return b < 0 ? 0 : (b >= kBins ? kBins - 1 : b);
+        };
+        const bool halve = depth + levels(n, leaf_max) >= kCullDepth;
+        if (!halve) {
+            Box box[3][kBins];
+            uint32_t count[3][kBins] = {};
+            for (auto &axis : box)
+                for (Box &b : axis) b.clear();
+            for (size_t i = lo; i < hi; i++)
+                for (int k = 0; k < 3; k++) {
+                    const int b = bin_of(prims[i], k);
+                    box[k][b].add(prims[i].box);
+                    count[k][b]++;
+                }
+            for (int k = 0; k < 3; k++) {
+                if (scale[k] == 0.f) continue;
+                double right[kBins];
+                uint32_t right_n[kBins], c = 0;
+                Box acc;
+                acc.clear();
+                for (int b = kBins - 1; b > 0; b--) {
+                    acc.add(box[k][b]);
+                    c += count[k][b];
+                    right[b] = c ? acc.half_area() : 0.0, right_n[b] = c;
+                }
+                acc.clear();
+                c = 0;
+                for (int b = 0; b + 1 < kBins; b++) {
+                    acc.add(box[k][b]);
+                    c += count[k][b];
+                    if (!c || !right_n[b + 1]) continue;
+                    const double cost = acc.half_area() * c + right[b + 1] * right_n[b + 1];
+                    if (cost < best) best = cost, best_axis = k, best_bin = b;
+                }
+            }
+        }
+        if (n <= (size_t)leaf_max) {
+            const double area = bounds.half_area();
+            if (best_axis < 0 || !(kVisit * area + kTest * best < kTest * (double)n * area)) return;  // leaf
+        }
+        size_t mid = lo + n / 2;
+        if (best_axis >= 0) {
+            mid = std::partition(prims.begin() + lo, prims.begin() + hi,
+                                 [&](const Prim &p) { return bin_of(p, best_axis) <= best_bin; }) -
+                  prims.begin();
+        } else {
+            // equal centres, or no levels to spare: halves along the longest axis
+            int axis = 0;
+            for (int k = 1; k < 3; k++)
+                if (centres.hi[k] - centres.lo[k] > centres.hi[axis] - centres.lo[axis]) axis = k;
+            std::nth_element(prims.begin() + lo, prims.begin() + mid, prims.begin() + hi,
+                             [&](const Prim &x, const Prim &y) {
+                                 const float a = x.c[axis], b = y.c[axis];
+                                 return a < b || (a == b && x.id < y.id);
+                             });
+        }
+        const size_t pair = mid - 1;  // one split position each: unique in [lo, hi - 2]
+        node.count = 0, node.pair = (uint32_t)pair;
+        Node &l = pairs[2 * pair], &r = pairs[2 * pair + 1];
+        if (threads > 1 && n >= kParallel) {
+            const int lt = threads / 2;
+            std::thread other([&] { build(l, lo, mid, depth + 1, lt); });
+            build(r, mid, hi, depth + 1, threads - lt);
+            other.join();
+        } else {
+            build(l, lo, mid, depth + 1, 1);
+            build(r, mid, hi, depth + 1, 1);
+        }
+    }
+
+    void emit(const Node &n, uint32_t slot, std::vector<GNode> &out) const {
+        GNode g;
+        for (int k = 0; k < 3; k++) g.lo[k] = n.box.lo[k], g.hi[k] = n.box.hi[k];
+        if (n.count) {
+            g.a = n.lo, g.b = kLeafFlag | n.count;
+            out[slot] = g;
+            return;
+        }
+        const uint32_t at = (uint32_t)out.size();
+        g.a = at, g.b = 0;
+        out[slot] = g;
+        out.resize(out.size() + 2);
+        emit(pairs[2 * (size_t)n.pair], at, out);
+        emit(pairs[2 * (size_t)n.pair + 1], at + 1, out);
+    }
+};
+
+}  // namespace
+
+CullBvh build_cull_bvh(const std::vector<TriPre> &tris, int leaf_max, int threads) {
+    CullBvh out;
+    out.nodes.assign(2, GNode{});
+    const size_t n = tris.size();
+    if (n == 0) {
+        for (int k = 0; k < 3; k++) out.nodes[0].lo[k] = INFINITY, out.nodes[0].hi[k] = -INFINITY;
+        out.nodes[0].b = kLeafFlag;
+        return out;
+    }
+    if (threads <= 0) threads = std::max(1, (int)std::thread::hardware_concurrency());
+    Builder b;
+    b.leaf_max = std::min(std::max(1, leaf_max), kCullLeaf);
+    b.prims.resize(n);
+    for (size_t i = 0; i < n; i++) {
+        Prim &p = b.prims[i];
+        const Aabb &t = tris[i].box;
+        p.id = (uint32_t)i;
+        for (int k = 0; k < 3; k++) {
+            const bool ok = std::isfinite(t.lo[k]) && std::isfinite(t.hi[k]);
+            p.box.lo[k] = ok ? t.lo[k] : -INFINITY, p.box.hi[k] = ok ? t.hi[k] : INFINITY;
+            const float c = t.lo[k] + t.hi[k];
+            p.c[k] = std::isfinite(c) ? c : 0.f;
+        }
+    }
+    b.root.resize(1);
+    b.pairs.resize(2 * std::max<size_t>(n - 1, 1));
+    b.build(b.root[0], 0, n, 0, threads);
+    out.nodes.reserve(2 * n + 2);
+    b.emit(b.root[0], 0, out.nodes);
+    out.order.resize(n);
+    for (size_t i = 0; i < n; i++) out.order[i] = b.prims[i].id;
+    return out;
+}
+
+}  // namespace pray_gpu

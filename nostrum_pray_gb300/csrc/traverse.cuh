@@ -150,6 +150,14 @@ __device__ __forceinline__ bool intersect_tri(const float4 &v0, const float4 &e1
 
 __device__ __forceinline__ float4 ldg4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
 
+// Whether the reference reports hits of a triangle record of the culling copy
+// on this ray, and with which key: it holds the triangle in the leaves that
+// own it, in depth-first order, and reaches one of them exactly when its own
+// box passes the reference's slab test (host/flatten.h). References of the
+// exact copy have no owner: the walk came through their leaf. e1w, e2w: the
+// record's key and owner words.
+__device__ __forceinline__ bool owned(const DevScene &s, const RayF &r, float e1w, float e2w, uint32_t &key);
+
 // One node (box lo + payload a, box hi + payload b) in one 256-bit read-only
 // load: nodes are 32-byte aligned, so a lane's node is one 32-byte sector and
 // one load instruction instead of two 16-byte ones (half the L1 wavefronts
@@ -159,6 +167,26 @@ __device__ __forceinline__ void ldg_node(const GNode *n, float4 &lo, float4 &hi)
     asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=f"(lo.x), "=f"(lo.y), "=f"(lo.z), "=f"(lo.w), "=f"(hi.x), "=f"(hi.y), "=f"(hi.z), "=f"(hi.w)
         : "l"(n));
+}
+
+__device__ __forceinline__ bool owned(const DevScene &s, const RayF &r, float e1w, float e2w, uint32_t &key) {
+    key = __float_as_uint(e1w);
+    const uint32_t owner = __float_as_uint(e2w);
+    if (owner == kNoOwner) return true;
+    const bool list = owner & kOwnerList;
+    const uint32_t n = list ? owner & ~kOwnerList : 1u, first = key;
+    for (uint32_t i = 0; i < n; i++) {
+        uint32_t leaf = owner;
+        if (list) {
+            const uint2 o = __ldg(reinterpret_cast<const uint2 *>(s.owners + first + i));
+            leaf = o.x, key = o.y;
+        }
+        float4 lo, hi;
+        ldg_node(s.nodes + leaf, lo, hi);
+        float tn, tf;
+        if (slab(lo, hi, r, true, tn, tf)) return true;
+    }
+    return false;
 }
 
 // Closest hit (kAny = false): returns the reference position of the winning
@@ -323,17 +351,17 @@ __device__ __forceinline__ void trav_round(const DevScene &s, const RayF &r, flo
                     const float4 v0 = ldg4(Tr->v0), e1 = ldg4(Tr->e1), e2 = ldg4(Tr->e2);
                     float t;
                     if (intersect_tri(v0, e1, e2, r, eps, t) && t > 0) {
+                        uint32_t key;
                         if (any_hit) {
-                            if (d2 > t * t) {
+                            if (d2 > t * t && owned(s, r, e1.w, e2.w, key)) {
                                 T.best = (int)i;
                                 T.have_node = T.have_leaf = false;
                                 T.sp = 0;
                                 break;
                             }
-                        } else {
-                            // depth-first position in the reference's leaf order
-                            const uint32_t key = __float_as_uint(e1.w);
-                            if (t < T.best_t || (T.best >= 0 && t == T.best_t && key < T.best_key)) {
+                        } else if (t < T.best_t || (T.best >= 0 && t == T.best_t)) {
+                            // key: depth-first position in the reference's leaf order
+                            if (owned(s, r, e1.w, e2.w, key) && (t < T.best_t || key < T.best_key)) {
                                 T.best_t = t;
                                 T.best = (int)i;
                                 T.best_key = key;
@@ -442,14 +470,14 @@ __device__ __forceinline__ int traverse_packet(const DevScene &s, const RayF &r,
                     if (kCount) fc->tris++;
                     float t;
                     if (intersect_tri(v0, e1, e2, r, eps, t) && t > 0) {
+                        uint32_t key;
                         if (kAny) {
-                            if (d2 > t * t) {
+                            if (d2 > t * t && owned(s, r, e1.w, e2.w, key)) {
                                 best = (int)i;
                                 open = false;
                             }
-                        } else {
-                            const uint32_t key = __float_as_uint(e1.w);
-                            if (t < best_t || (best >= 0 && t == best_t && key < best_key)) {
+                        } else if (t < best_t || (best >= 0 && t == best_t)) {
+                            if (owned(s, r, e1.w, e2.w, key) && (t < best_t || key < best_key)) {
                                 best_t = t;
                                 best = (int)i;
                                 best_key = key;

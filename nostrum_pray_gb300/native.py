@@ -243,7 +243,8 @@ class HostTree:
         return out
 
     def device_layout(self, leaf_refine: int = 4) -> np.ndarray:
-        """[node records, triangle references, refined leaves, added nodes]."""
+        """[node records, triangle references, triangles and node records of
+        the culling hierarchy]."""
         out = np.zeros(4, np.uint64)
         check(lib().pray_host_tree_device_layout(self._h, leaf_refine, out.ctypes.data))
         return out

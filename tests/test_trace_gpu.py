@@ -349,3 +349,117 @@ def test_host_rays_from_many_threads(oracle):
     ids, ts = sc.trace_closest_host(rays[:0], st.det_eps)
     assert ids.size == 0
     sc.close()
+
+
+def _hard_rays(mesh, seed, n):
+    """Rays that culling gets wrong first: at vertices, edge midpoints and
+    interior points of triangles (ties at shared edges) from around and inside
+    the scene, near-axis and axis-parallel directions, and random ones."""
+    rng = np.random.default_rng(seed)
+    v = mesh.verts.reshape(-1, 3, 3).astype(np.float64)
+    lo, hi = v.min((0, 1)), v.max((0, 1))
+    size = max(float(np.linalg.norm(hi - lo)), 1e-3)
+    t = v[rng.integers(0, len(v), n)]
+    w = rng.dirichlet((1, 1, 1), n)
+    kind = rng.integers(0, 4, n)
+    w[kind == 0] = np.eye(3)[rng.integers(0, 3, (kind == 0).sum())]
+    w[kind == 1] = (0.5, 0.5, 0.0)
+    p = np.einsum("nk,nkc->nc", w, t)
+    o = rng.uniform(lo - size, hi + size, (n, 3))
+    d = p - o
+    d[kind == 3] = rng.normal(size=((kind == 3).sum(), 3))
+    axis = rng.integers(0, 8, n) == 0  # nearly or exactly parallel to an axis
+    d[axis] = np.eye(3)[rng.integers(0, 3, axis.sum())] * size
+    d[axis] += rng.normal(size=(axis.sum(), 3)) * rng.choice([0.0, 1e-7, 1e-3], (axis.sum(), 1)) * size
+    o[axis] = p[axis] - 1.5 * d[axis]
+    d32 = (d / np.maximum(np.linalg.norm(d, axis=1, keepdims=True), 1e-30)).astype(np.float32)
+    with np.errstate(divide="ignore"):
+        return np.concatenate([o.astype(np.float32), d32, np.float32(1.0) / d32], 1)
+
+
+def _well_posed(mesh, rays):
+    """Rays within the culling pad's bound (host/flatten.cpp): sin a sin b of at
+    least 1/50 (a the smallest angle, b the ray's angle to the plane) for
+    every triangle that the ray's line passes through or within a hundredth
+    of its size, and no zero-area triangle within that of the line. Outside it
+    a reported distance can lie anywhere, and any walk that skips boxes beyond
+    the best hit may miss the reference's choice."""
+    v = mesh.verts.reshape(-1, 3, 3).astype(np.float64)
+    a, e1, e2 = v[:, 0], v[:, 1] - v[:, 0], v[:, 2] - v[:, 0]
+    n = np.cross(e1, e2)
+    area = np.linalg.norm(n, axis=1)
+    e = np.sort(np.stack([np.linalg.norm(x, axis=1) for x in (e1, e2, e2 - e1)]), 0)
+    sin_a = area / np.maximum(e[1] * e[2], 1e-300)
+    ok = np.ones(len(rays), bool)
+    for i in range(0, len(rays), 500):
+        o, d = rays[i:i + 500, 0:3].astype(np.float64), rays[i:i + 500, 3:6].astype(np.float64)
+        sin_b = np.abs(d @ n.T) / np.maximum(area, 1e-300)
+        # distance of the line to the triangle's plane section: barycentrics of the line's closest approach
+        p = np.cross(d[:, None], e2[None])
+        det = np.einsum("rtc,tc->rt", p, e1)
+        t = o[:, None] - a[None]
+        u = np.einsum("rtc,rtc->rt", t, p)
+        w = np.einsum("rc,rtc->rt", d, np.cross(t, e1[None]))
+        # the line's distance to the triangle's centroid against its size
+        c = v.mean(1)[None] - o[:, None]
+        dist = np.linalg.norm(c - np.einsum("rtc,rc->rt", c, d)[..., None] * d[:, None], axis=2)
+        near = dist <= e[2] * (2 / 3) * 1.01
+        with np.errstate(divide="ignore", invalid="ignore"):
+            u, w = u / det, w / det
+            inside = (u > -0.01) & (w > -0.01) & (u + w < 1.01)
+        posed = sin_a * sin_b >= 1 / 50
+        ok[i:i + 500] = ~(near & ~posed & (inside | (sin_b < 1 / 50) | (sin_a[None] < 1 / 50))).any(1)
+    return ok
+
+
+def _hard_mesh(name):
+    rng = np.random.default_rng(5)
+    if name == "one":
+        v = rng.uniform(-1, 1, (1, 9))
+    elif name == "copies":  # one triangle 40 times (equal centres), a few others
+        v = np.concatenate([np.repeat(rng.uniform(-1, 1, (1, 9)), 40, 0), rng.uniform(-1, 1, (9, 9))])
+    elif name == "layers":  # a quad grid twice in the same plane: every hit is a tie
+        g = scenes._quad_grid((-1, -1, 0), (2, 0, 0), (0, 2, 0), 9)
+        v = np.concatenate([g, g[::-1]])
+    elif name == "flat":  # zero-area triangles among others
+        v = rng.uniform(-1, 1, (60, 9))
+        v[::3, 6:9] = v[::3, 3:6]
+    elif name == "offset":
+        v = scenes.icosphere(3).verts + np.tile([300.0, -200.0, 100.0], 3)
+    elif name == "room":
+        return scenes.room(grid=3)
+    else:
+        return scenes.soup(700, 2)
+    v = np.asarray(v, np.float32)
+    return scenes.Mesh(v, np.full((len(v), 3), 0.5, np.float32), np.zeros(len(v), np.uint8))
+
+
+@pytest.mark.parametrize("tree", ["median", "sah"])
+@pytest.mark.parametrize("name", ["one", "copies", "layers", "flat", "offset", "room", "soup"])
+def test_culling_hierarchy_matches_reference_walk(oracle, name, tree):
+    """The culling hierarchy (triangles once each, hits checked against the
+    reference's leaves that own them) gives the oracle's ids and distances bit
+    for bit, and its occlusion answers, for every leaf size and both trees, on
+    the rays that use it (finite inverse directions) within the error bound
+    that it rests on."""
+    m = _hard_mesh(name)
+    st = scenes.soup_setup()
+    st.det_eps = 0.0
+    st.tree, st.leaf_size, st.sah_ct = tree, 4, 1.0
+    rays = _hard_rays(m, 3, 6000)
+    rays = np.ascontiguousarray(rays[_well_posed(m, rays) & np.isfinite(rays[:, 6:9]).all(1)])
+    assert len(rays) > 1000
+    want, want_t = oracle.OracleScene.from_setup(m, st).trace(rays, st.det_eps)
+    rng = np.random.default_rng(9)
+    d2 = np.where(rng.random(len(rays)) < 0.5, np.minimum(want_t, 1e3) ** 2, 1.0) * rng.choice([0.9, 1.0, 1.1], len(rays))
+    d2 = d2.astype(np.float32)
+    with np.errstate(over="ignore"):
+        want_occ = (want >= 0) & (want_t * want_t < d2)
+    for refine in (8, 3, 1):
+        sc = native.Scene.from_setup(m, st, leaf_refine=refine)
+        ids, ts = trace(sc, rays, st.det_eps)
+        np.testing.assert_array_equal(ids, want.astype(np.int32))
+        np.testing.assert_array_equal(ts.view(np.uint32), want_t.view(np.uint32))
+        occ = torch.empty(len(rays), dtype=torch.uint8, device="cuda")
+        sc.trace_occluded(torch.from_numpy(rays).cuda(), torch.from_numpy(d2).cuda(), st.det_eps, occ)
+        np.testing.assert_array_equal(occ.cpu().numpy(), want_occ.astype(np.uint8))
