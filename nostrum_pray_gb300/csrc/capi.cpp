@@ -557,7 +557,11 @@ pray_status pray_scene_create(const float *verts, const float *colors, const uin
             return set_error(PRAY_ERR_UNSUPPORTED, "device layout: " + bad);
         gnodes.swap(img.nodes);
         s->n_gnodes = (uint32_t)gnodes.size();
-        gnodes.insert(gnodes.end(), img.cull.begin(), img.cull.end());  // both copies, one buffer
+        for (GNode g : img.cull) {  // both copies, one buffer
+            if ((g.b & kLeafFlag) && (g.b & ~kLeafFlag))
+                g.a |= kLeafFlag | ((g.b & ~kLeafFlag) - 1) << kCullCountShift;
+            gnodes.push_back(g);
+        }
         gowners.swap(img.owners);
         for (int k = 0; k < 3; k++) s->cull_c[k] = img.cull_center[k];
         s->cull_r2 = img.cull_radius2;

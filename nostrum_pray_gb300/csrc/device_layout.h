@@ -5,6 +5,8 @@
 // boxes and tests them before descending (root at index 0, slot 1 unused).
 //   interior: a = index of the first child of its pair, b = 0
 //   leaf:     a = first triangle reference, b = kLeafFlag | reference count
+// In the culling copy on the device, a leaf's a is one word that holds both
+// (kCullCountShift), so that a traversal keeps one word per node.
 // Every node keeps its own box (tight triangle bounds for the median tree,
 // the voxel for the SAH tree) so the kernels apply the reference's slab test
 // to exactly the boxes the reference tests.
@@ -27,6 +29,9 @@
 namespace pray_gpu {
 
 constexpr uint32_t kLeafFlag = 0x80000000u;
+// Device word of a culling leaf: kLeafFlag | (count - 1) << kCullCountShift |
+// first record (counts up to 4, records below 2^kCullCountShift).
+constexpr int kCullCountShift = 29;
 constexpr uint32_t kOwnerList = 0x80000000u, kNoOwner = 0x7FFFFFFFu;
 constexpr int kMaxTreeDepth = 30;        // deepest reference tree the API accepts
 constexpr int kMaxTraversalDepth = 62;   // deepest device hierarchy (reference tree or culling copy)

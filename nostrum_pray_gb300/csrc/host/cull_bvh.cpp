@@ -13,7 +13,7 @@ constexpr int kBins = 16;
 // Costs of one node visit (two boxes) and of one triangle test, relative. A
 // visit outweighs a test: a warp walks its lanes' nodes one by one, but
 // tests their leaves together.
-constexpr double kVisit = 2.0, kTest = 1.0;
+constexpr double kVisit = 1.5, kTest = 1.0;
 constexpr size_t kParallel = 1024;  // subtrees from this size on may get a thread of their own
 
 struct Box {

@@ -99,7 +99,8 @@ void flatten_for_device(const BuiltTree &t, const std::vector<TriPre> &pre, cons
     std::vector<uint32_t> leaf_of(t.refs.size());
     f.put(0, 0, leaf_of);
     out.refs = out.tris.size();
-    if (!bvh || !sized) return;
+    // (no culling copy where its leaves' words could not hold the records' numbers)
+    if (!bvh || !sized || out.refs + pre.size() >= (1ull << kCullCountShift)) return;
     for (int k = 0; k < 3; k++) out.cull_center[k] = 0.5f * (root.lo[k] + root.hi[k]);
     out.cull_radius2 = (kCullReach * diag) * (kCullReach * diag);
     // each triangle's references, in depth-first order

@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(kShadowPacket ? kPacketThreads : 128, kShadowP
     uint32_t shadows = 0;
     FetchCount fc;
     // one traversal stack per warp (the tile's rays are coherent)
-    __shared__ uint32_t stacks[4][3 * kStackN];
+    __shared__ uint32_t stacks[4][2 * kStackN];
     uint32_t *stk = stacks[threadIdx.x >> 5];
     const RayF r = primary_ray(L.cam, active ? px : 0, active ? py : 0);
     float dist = FLT_MAX;

@@ -198,21 +198,6 @@ struct FetchCount {
     uint32_t pairs = 0, tris = 0;
 };
 
-// Pops the next stacked node that can still hold a closer hit.
-__device__ __forceinline__ bool pop_node(const uint32_t *stk_a, const uint32_t *stk_b, const float *stk_t, int &sp,
-                                         float limit, uint32_t &a, uint32_t &b, float &tn) {
-    while (sp > 0) {
-        sp--;
-        if (stk_t[sp] <= limit) {
-            a = stk_a[sp];
-            b = stk_b[sp];
-            tn = stk_t[sp];
-            return true;
-        }
-    }
-    return false;
-}
-
 // Warp-collective traversal: every lane of the warp must call it together
 // (inactive lanes pass valid = false). Structure after Aila & Laine,
 // "Understanding the Efficiency of Ray Traversal on GPUs" (HPG 2009): the
@@ -236,22 +221,54 @@ __device__ __forceinline__ bool pop_node(const uint32_t *stk_a, const uint32_t *
 enum TravMode { kClosest = 0, kAnyHit = 1, kPerLane = 2 };
 
 struct Trav {
-    uint32_t a, b, la, lb;
+    // the current node and the postponed leaf, one word each: an interior
+    // node's first child, or a leaf (kLeafFlag; culling copy: count and first
+    // record, exact copy: its node)
+    uint32_t w, lw;
     uint32_t node_off;  // 0: the exact copy; n_nodes: the culling copy (finite inverse direction, near origin)
     float cur_tn, leaf_tn, limit, back, best_t;
+    float nox, noy, noz;  // culling copy: -origin / direction (slab_fma)
     int best, sp;
     uint32_t best_key;
     bool have_node, have_leaf, finite, any;
     __device__ __forceinline__ bool active() const { return have_node || have_leaf; }
+    __device__ __forceinline__ bool on_leaf() const { return have_node && (w & kLeafFlag); }
 };
 
 // The traversal stack of one lane (kept apart from Trav so that the scalar
-// state stays in registers).
+// state stays in registers): a node's word and its entry distance, one 8-byte
+// local access per push or pop.
 template <int kStackN>
 struct TravStack {
-    uint32_t a[kStackN], b[kStackN];
-    float t[kStackN];
+    uint2 e[kStackN];
 };
+
+// The next stacked node that can still hold a closer hit.
+template <int kStackN>
+__device__ __forceinline__ void pop_node(Trav &T, const TravStack<kStackN> &S) {
+    while (T.sp > 0) {
+        const uint2 e = S.e[--T.sp];
+        T.cur_tn = __uint_as_float(e.y);
+        if (T.cur_tn <= T.limit) {
+            T.w = e.x;
+            return;
+        }
+    }
+    T.have_node = false;
+}
+
+// Triangle records of a leaf word.
+__device__ __forceinline__ void leaf_range(const DevScene &s, uint32_t node_off, uint32_t w, uint32_t &first,
+                                           uint32_t &end) {
+    if (node_off) {
+        first = w & ((1u << kCullCountShift) - 1u);
+        end = first + ((w >> kCullCountShift) & 3u) + 1u;
+    } else {
+        const GNode *n = s.nodes + (w & ~kLeafFlag);
+        first = __ldg(&n->a);
+        end = first + (__ldg(&n->b) & ~kLeafFlag);
+    }
+}
 
 // `any` (kPerLane only): this lane's ray looks for any occluder.
 template <int kMode>
@@ -263,21 +280,22 @@ __device__ __forceinline__ void trav_start(const DevScene &s, const RayF &r, flo
     T.best_key = 0xFFFFFFFFu;
     T.limit = T.any ? sqrtf(d2) * kPruneRel : FLT_MAX;
     T.back = -s.tol;
-    T.a = T.b = T.la = T.lb = 0;
+    T.w = T.lw = 0;
     T.cur_tn = T.leaf_tn = 0.f;
     T.have_node = T.have_leaf = false;
     T.sp = 0;
     T.finite = isfinite(r.ix) && isfinite(r.iy) && isfinite(r.iz);
+    T.nox = -(r.ox * r.ix), T.noy = -(r.oy * r.iy), T.noz = -(r.oz * r.iz);
     const float cx = r.ox - s.cull_c[0], cy = r.oy - s.cull_c[1], cz = r.oz - s.cull_c[2];
-    T.node_off = (T.finite && cx * cx + cy * cy + cz * cz <= s.cull_r2) ? s.n_nodes : 0u;
+    T.node_off = (T.finite && isfinite(T.nox) && isfinite(T.noy) && isfinite(T.noz) && cx * cx + cy * cy + cz * cz <= s.cull_r2) ? s.n_nodes : 0u;
     if (valid) {
         float tn, tf;
         const GNode *root = s.nodes + T.node_off;
         float4 rlo, rhi;
         ldg_node(root, rlo, rhi);
         if (slab(rlo, rhi, r, tn, tf)) {
-            T.a = __float_as_uint(rlo.w);
-            T.b = __float_as_uint(rhi.w);
+            T.w = __float_as_uint(rlo.w);
+            if (!T.node_off && (__float_as_uint(rhi.w) & kLeafFlag)) T.w = kLeafFlag;  // (node 0)
             T.cur_tn = tn;
             T.have_node = true;
         }
@@ -292,59 +310,65 @@ __device__ __forceinline__ void trav_round(const DevScene &s, const RayF &r, flo
     const bool any_hit = kMode == kAnyHit || (kMode == kPerLane && T.any);
     // 1. interior nodes, until every lane has found a leaf
     while (true) {
-        const bool interior = T.have_node && !(T.b & kLeafFlag);
+        const bool interior = T.have_node && !(T.w & kLeafFlag);
         if (!__any_sync(kFull, interior && !T.have_leaf)) break;
         if (interior) {
             if (kCount) fc->pairs++;
-            // culling copy: boxes around the triangles (same topology; the
-            // reference's leaf boxes decide which leaves count)
-            const GNode *c = s.nodes + (T.a + T.node_off);
+            const GNode *c = s.nodes + (T.w + T.node_off);
             float4 l0, h0, l1, h1;
             ldg_node(c, l0, h0);
             ldg_node(c + 1, l1, h1);
+            uint32_t w0 = __float_as_uint(l0.w), w1 = __float_as_uint(l1.w);
             float tn0, tf0, tn1, tf1;
-            const bool v0 = slab(l0, h0, r, T.finite, tn0, tf0) && tn0 <= T.limit && tf0 >= T.back;
-            const bool v1 = slab(l1, h1, r, T.finite, tn1, tf1) && tn1 <= T.limit && tf1 >= T.back;
+            bool v0, v1;
+            // entered: tn <= tf, not beyond the best hit, not behind the origin
+            if (T.node_off) {
+                slab_fma(l0, h0, r, T.nox, T.noy, T.noz, tn0, tf0);
+                slab_fma(l1, h1, r, T.nox, T.noy, T.noz, tn1, tf1);
+                tn0 = fmaxf(tn0, T.back), tn1 = fmaxf(tn1, T.back);
+                v0 = tn0 <= fminf(tf0, T.limit), v1 = tn1 <= fminf(tf1, T.limit);
+            } else {
+                v0 = slab(l0, h0, r, T.finite, tn0, tf0) && tn0 <= T.limit && tf0 >= T.back;
+                v1 = slab(l1, h1, r, T.finite, tn1, tf1) && tn1 <= T.limit && tf1 >= T.back;
+                if (__float_as_uint(h0.w) & kLeafFlag) w0 = kLeafFlag | T.w;
+                if (__float_as_uint(h1.w) & kLeafFlag) w1 = kLeafFlag | (T.w + 1);
+            }
             if (v0 && v1) {
                 const bool first0 = tn0 <= tn1;
-                S.a[T.sp] = __float_as_uint(first0 ? l1.w : l0.w);
-                S.b[T.sp] = __float_as_uint(first0 ? h1.w : h0.w);
-                S.t[T.sp] = first0 ? tn1 : tn0;
-                T.sp++;
-                T.a = __float_as_uint(first0 ? l0.w : l1.w);
-                T.b = __float_as_uint(first0 ? h0.w : h1.w);
+                S.e[T.sp++] = make_uint2(first0 ? w1 : w0, __float_as_uint(first0 ? tn1 : tn0));
+                T.w = first0 ? w0 : w1;
                 T.cur_tn = first0 ? tn0 : tn1;
             } else if (v0 || v1) {
-                T.a = __float_as_uint(v0 ? l0.w : l1.w);
-                T.b = __float_as_uint(v0 ? h0.w : h1.w);
+                T.w = v0 ? w0 : w1;
                 T.cur_tn = v0 ? tn0 : tn1;
             } else {
-                T.have_node = pop_node(S.a, S.b, S.t, T.sp, T.limit, T.a, T.b, T.cur_tn);
+                pop_node(T, S);
             }
-            if (T.have_node && (T.b & kLeafFlag) && !T.have_leaf) {
+            if (T.on_leaf() && !T.have_leaf) {
                 // first leaf: postpone it and keep walking
-                T.la = T.a, T.lb = T.b, T.leaf_tn = T.cur_tn;
+                T.lw = T.w, T.leaf_tn = T.cur_tn;
                 T.have_leaf = true;
-                T.have_node = pop_node(S.a, S.b, S.t, T.sp, T.limit, T.a, T.b, T.cur_tn);
+                pop_node(T, S);
             }
         }
     }
     // 2. leaves: the postponed one, then any leaf the walk stopped on
     while (true) {
-        const bool work = T.have_leaf || (T.have_node && (T.b & kLeafFlag));
+        const bool work = T.have_leaf || T.on_leaf();
         if (!__any_sync(kFull, work)) break;
         if (work) {
-            uint32_t fa, fb;
+            uint32_t fw;
             float ftn;
             if (T.have_leaf) {
-                fa = T.la, fb = T.lb, ftn = T.leaf_tn;
+                fw = T.lw, ftn = T.leaf_tn;
                 T.have_leaf = false;
             } else {
-                fa = T.a, fb = T.b, ftn = T.cur_tn;
-                T.have_node = pop_node(S.a, S.b, S.t, T.sp, T.limit, T.a, T.b, T.cur_tn);
+                fw = T.w, ftn = T.cur_tn;
+                pop_node(T, S);
             }
             if (ftn <= T.limit) {
-                const uint32_t end = fa + (fb & ~kLeafFlag);
+                uint32_t fa, end;
+                leaf_range(s, T.node_off, fw, fa, end);
                 for (uint32_t i = fa; i < end; i++) {
                     if (kCount) fc->tris++;
                     const GTri *Tr = s.tris + i;
@@ -392,8 +416,8 @@ __device__ __forceinline__ int traverse(const DevScene &s, const RayF &r, float 
 // Garanzha & Loop (2010): the warp walks one node sequence of the culling
 // copy with a mask of the lanes whose own box tests passed, so node and
 // triangle loads are warp-uniform (one broadcast each) and the traversal
-// stack is one shared stack per warp (`stk`: 3 x kStackN words of shared
-// memory: node payload, lane mask) instead of one per lane. Every lane still
+// stack is one shared stack per warp (`stk`: 2 x kStackN words of shared
+// memory: node word, lane mask) instead of one per lane. Every lane still
 // applies its own slab test (with its own pruning bound) to every box on its
 // way and its own triangle test to every reference of the leaves it reaches,
 // so it returns the same lexicographic minimum as traverse(); only the order
@@ -415,28 +439,29 @@ __device__ __forceinline__ int traverse_packet(const DevScene &s, const RayF &r,
     best_t = FLT_MAX;
     int best = -1;
     uint32_t best_key = 0xFFFFFFFFu;
-    uint32_t a, b;
+    uint32_t w;
     unsigned mask;
     {
         float4 lo, hi;
         ldg_node(nodes, lo, hi);
         float tn, tf;
         mask = __ballot_sync(kFull, valid && slab_fma(lo, hi, r, nox, noy, noz, tn, tf));
-        a = __float_as_uint(lo.w);
-        b = __float_as_uint(hi.w);
+        w = __float_as_uint(lo.w);
     }
     int sp = 0;
     while (mask) {
         const bool in = (mask >> lane) & 1u;
-        if (!(b & kLeafFlag)) {
-            const GNode *c = nodes + a;
+        if (!(w & kLeafFlag)) {
+            const GNode *c = nodes + w;
             float4 l0, h0, l1, h1;
             ldg_node(c, l0, h0);
             ldg_node(c + 1, l1, h1);
             if (kCount && in) fc->pairs++;
             float tn0, tf0, tn1, tf1;
-            const bool v0 = in && slab_fma(l0, h0, r, nox, noy, noz, tn0, tf0) && tn0 <= limit && tf0 >= back;
-            const bool v1 = in && slab_fma(l1, h1, r, nox, noy, noz, tn1, tf1) && tn1 <= limit && tf1 >= back;
+            slab_fma(l0, h0, r, nox, noy, noz, tn0, tf0);
+            slab_fma(l1, h1, r, nox, noy, noz, tn1, tf1);
+            const bool v0 = in && fmaxf(tn0, back) <= fminf(tf0, limit);
+            const bool v1 = in && fmaxf(tn1, back) <= fminf(tf1, limit);
             const unsigned m0 = __ballot_sync(kFull, v0), m1 = __ballot_sync(kFull, v1);
             if (m0 && m1) {
                 const unsigned both = m0 & m1;
@@ -444,26 +469,24 @@ __device__ __forceinline__ int traverse_packet(const DevScene &s, const RayF &r,
                 const bool go0 = both ? 2 * __popc(near0) >= __popc(both) : __popc(m0) >= __popc(m1);
                 if (lane == 0) {
                     stk[sp] = __float_as_uint(go0 ? l1.w : l0.w);
-                    stk[kStackN + sp] = __float_as_uint(go0 ? h1.w : h0.w);
-                    stk[2 * kStackN + sp] = go0 ? m1 : m0;
+                    stk[kStackN + sp] = go0 ? m1 : m0;
                 }
                 sp++;
-                a = __float_as_uint(go0 ? l0.w : l1.w);
-                b = __float_as_uint(go0 ? h0.w : h1.w);
+                w = __float_as_uint(go0 ? l0.w : l1.w);
                 mask = go0 ? m0 : m1;
                 continue;
             }
             if (m0 | m1) {
-                a = __float_as_uint(m0 ? l0.w : l1.w);
-                b = __float_as_uint(m0 ? h0.w : h1.w);
+                w = __float_as_uint(m0 ? l0.w : l1.w);
                 mask = m0 | m1;
                 continue;
             }
         } else {
             // the lanes in the mask test the leaf's references
             bool open = in;
-            const uint32_t end = a + (b & ~kLeafFlag);
-            for (uint32_t i = a; i < end; i++) {
+            uint32_t first, end;
+            leaf_range(s, s.n_nodes, w, first, end);
+            for (uint32_t i = first; i < end; i++) {
                 const GTri *Tr = s.tris + i;
                 const float4 v0 = ldg4(Tr->v0), e1 = ldg4(Tr->e1), e2 = ldg4(Tr->e2);
                 if (open) {
@@ -495,9 +518,8 @@ __device__ __forceinline__ int traverse_packet(const DevScene &s, const RayF &r,
         __syncwarp();
         while (sp > 0 && !mask) {
             sp--;
-            a = stk[sp];
-            b = stk[kStackN + sp];
-            mask = stk[2 * kStackN + sp] & ~done;
+            w = stk[sp];
+            mask = stk[kStackN + sp] & ~done;
         }
         __syncwarp();
     }
