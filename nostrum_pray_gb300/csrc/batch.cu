@@ -88,7 +88,7 @@ struct TileSrc {
 // refilled across the scene's tiles; otherwise each tile runs pt_pixel_sync
 // (modes 0 and 1).
 template <int kStackN, bool kLanes>
-__global__ void __launch_bounds__(256, 4) k_batch_pt(BatchLaunch B) {
+__global__ void __launch_bounds__(256, 3) k_batch_pt(BatchLaunch B) {
     constexpr unsigned kFull = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31u;
     if (kLanes) {

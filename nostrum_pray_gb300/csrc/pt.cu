@@ -55,13 +55,13 @@ __global__ void __launch_bounds__(128, kBlocks) k_render_pt(DevScene s, PtLaunch
     uint32_t segments = 0, pixels = 0;
     if (kRefill) {
         FrameSrc src{L.next_pixel, warp_tiles(L.cam.width, L.cam.height) * 32, L.cam.width, L.cam.height, false};
-        pt_sync<kStack>(s, L, src, segments, pixels);
+        pt_sync<kStack, 1>(s, L, src, segments, pixels);
     } else {
         const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
         uint32_t px, py;
         const bool active = pixel_of(i, L.cam.width, L.cam.height, px, py);
         OnePixel src{active, px, py, false};
-        pt_sync<kStack>(s, L, src, segments, pixels);
+        pt_sync<kStack, 0>(s, L, src, segments, pixels);
     }
     if (L.counters) {
         unsigned long long paths = (unsigned long long)pixels * L.num_samples, segs = segments;
@@ -107,6 +107,8 @@ cudaError_t launch_render_pt(const DevScene &s, const PtLaunch &L, int sm_count,
             const uint64_t resident = sms * 10;
             k_render_pt<true, 10><<<(unsigned)(blocks < resident ? blocks : resident), bs, 0, stream>>>(s, L);
         }
+    } else if (blocks <= (uint64_t)(sm_count > 0 ? sm_count : 1) * 8) {
+        k_render_pt<false, 8><<<(unsigned)blocks, bs, 0, stream>>>(s, L);
     } else {
         k_render_pt<false, 10><<<(unsigned)blocks, bs, 0, stream>>>(s, L);
     }

@@ -69,6 +69,15 @@ struct OnePixel {
     }
 };
 
+// The first hit of a lane's pixel. The camera ray of a pixel is the same for
+// all of its samples, so only the first sample traces it: when it ends the
+// path there (background, emitter, depth limit) every sample has its value,
+// else the others start at the hit.
+struct FirstHit {
+    float x, y, z;  // the hit point
+    int id;         // its triangle
+};
+
 // Modes 0 and 1 bounce by bounce: all lanes of a warp call pt_sync together
 // and run each bounce's extension rays, then its next-event occlusion rays,
 // as two warp-collective traversals. Each lane works through its pixel's
@@ -79,12 +88,16 @@ struct OnePixel {
 // pixels counts the pixels a lane finished. The per-pixel kernel runs it for
 // modes 0 and 1, the batch kernel for mode 1 (next-event occlusion rays, all
 // aimed at the emitters, keep the warp more coherent traced together than
-// mixed with bounce rays).
-template <int kStackN, class Src>
+// mixed with bounce rays). In mode 0 the first hit of a pixel is traced
+// once (FirstHit) and later samples start with their first bounce ray; in
+// mode 1, where they would start with an occlusion ray and sit out the warp's
+// extension rays, keeping it costs more than it saves.
+template <int kStackN, int kMode, class Src>
 __device__ __forceinline__ void pt_sync(const DevScene &s, const PtLaunch &L, Src &src, uint32_t &segments,
                                         uint32_t &pixels) {
     constexpr unsigned kFull = 0xFFFFFFFFu;
-    float alb_r[kMaxPtDepth], alb_g[kMaxPtDepth], alb_b[kMaxPtDepth];
+    constexpr int kAlb = kMode == 0 ? kMaxPtDepth : 1;
+    float alb_r[kAlb], alb_g[kAlb], alb_b[kAlb];
     const bool any_geometry = s.n_refs > 0;
     // the lane's pixel
     bool have = false;
@@ -100,13 +113,27 @@ __device__ __forceinline__ void pt_sync(const DevScene &s, const PtLaunch &L, Sr
     float tr = 1.f, tg = 1.f, tb = 1.f;
     uint32_t depth = 0;
     bool alive = false;
+    FirstHit first;
+    auto bounce = [&](float hx, float hy, float hz, const float4 &nrm) {
+        const float u1 = pray_uniform(&rng), u2 = pray_uniform(&rng);
+        const float n3[3] = {nrm.x, nrm.y, nrm.z};
+        float d[3];
+        pray_sample_hemisphere(n3, u1, u2, d);
+        r = make_ray(hx, hy, hz, d[0], d[1], d[2]);
+        depth++;
+    };
     auto start = [&]() {
         rng = pray_pcg32_stream(L.seed, pixel(), L.sample_offset + smp);
-        r = primary_ray(L.cam, px, py);
         lr = lg = lb = 0.f;
         tr = tg = tb = 1.f;
         depth = 0;
         alive = true;
+        if (kMode != 0 || smp == 0) {
+            r = primary_ray(L.cam, px, py);
+        } else {
+            segments++;  // the camera ray
+            bounce(first.x, first.y, first.z, shade_n(s, first.id));
+        }
     };
     auto finish_pixel = [&]() {
         const uint64_t pix = pixel();
@@ -157,22 +184,23 @@ __device__ __forceinline__ void pt_sync(const DevScene &s, const PtLaunch &L, Sr
         if (alive) {
             segments++;
             if (pos < 0) {
-                if (L.mode == 0) lr = L.bg[0], lg = L.bg[1], lb = L.bg[2];
+                if (kMode == 0) lr = L.bg[0], lg = L.bg[1], lb = L.bg[2];
                 else lr = lr + tr * L.bg[0], lg = lg + tg * L.bg[1], lb = lb + tb * L.bg[2];
                 alive = false;
             } else {
                 const int id = (int)__float_as_uint(__ldg(&s.tris[pos].v0[3]));
                 nrm = shade_n(s, id), col = shade_c(s, id);
                 if (nrm.w != 0.f) {
-                    if (L.mode == 0) lr = col.x, lg = col.y, lb = col.z;
+                    if (kMode == 0) lr = col.x, lg = col.y, lb = col.z;
                     else if (depth == 0) lr = lr + tr * col.x, lg = lg + tg * col.y, lb = lb + tb * col.z;
                     alive = false;
                 } else if (depth >= L.max_depth) {
-                    if (L.mode == 0) lr = 0.f, lg = 0.f, lb = 0.f;
+                    if (kMode == 0) lr = 0.f, lg = 0.f, lb = 0.f;
                     alive = false;
                 } else {
                     hx = r.ox + r.dx * t, hy = r.oy + r.dy * t, hz = r.oz + r.dz * t;
-                    if (L.mode != 0 && s.n_emit > 0) {
+                    if (kMode == 0 && depth == 0) first.x = hx, first.y = hy, first.z = hz, first.id = id;
+                    if (kMode != 0 && s.n_emit > 0) {
                         const float ue = pray_uniform(&rng), ua = pray_uniform(&rng), ub = pray_uniform(&rng);
                         const GTri *E = s.emit_tris + pick_emitter(s, ue);
                         const float4 ev0 = __ldg(reinterpret_cast<const float4 *>(E->v0));
@@ -206,53 +234,58 @@ __device__ __forceinline__ void pt_sync(const DevScene &s, const PtLaunch &L, Sr
                 }
             }
         }
-        float dummy;
-        const bool occluded = traverse<true, false, kStackN>(s, sray, L.eps, sd2, need, dummy) >= 0;
-        if (need) {
-            segments++;
-            if (!occluded) lr = lr + cxr, lg = lg + cxg, lb = lb + cxb;
+        if (kMode != 0) {
+            float dummy;
+            const bool occluded = traverse<true, false, kStackN>(s, sray, L.eps, sd2, need, dummy) >= 0;
+            if (need) {
+                segments++;
+                if (!occluded) lr = lr + cxr, lg = lg + cxg, lb = lb + cxb;
+            }
         }
+        const bool at_camera = depth == 0 && !alive;  // the path ended at its first hit
         if (alive) {
             // cosine bounce (and, in mode 1, Russian roulette)
-            if (L.mode == 0) alb_r[depth] = col.x, alb_g[depth] = col.y, alb_b[depth] = col.z;
-            const float u1 = pray_uniform(&rng), u2 = pray_uniform(&rng);
-            const float n3[3] = {nrm.x, nrm.y, nrm.z};
-            float d[3];
-            pray_sample_hemisphere(n3, u1, u2, d);
-            r = make_ray(hx, hy, hz, d[0], d[1], d[2]);
-            if (L.mode != 0) {
+            if (kMode == 0) alb_r[depth] = col.x, alb_g[depth] = col.y, alb_b[depth] = col.z;
+            bounce(hx, hy, hz, nrm);
+            if (kMode != 0) {
                 tr = tr * col.x, tg = tg * col.y, tb = tb * col.z;
-                if (depth >= L.rr_depth) {
+                if (depth > L.rr_depth) {
                     const float q = smin(smax(smax(tr, tg), tb), 0.95f);
                     if (!(pray_uniform(&rng) < q)) alive = false;
                     else tr = tr / q, tg = tg / q, tb = tb / q;
                 }
             }
-            depth++;
         }
         if (was_alive && !alive) {
             // the path ended: its value joins the pixel's sums in sample order
-            if (L.mode == 0) {
+            if (kMode == 0) {
                 while (depth > 0) {
                     depth--;
                     lr = lr * alb_r[depth], lg = lg * alb_g[depth], lb = lb * alb_b[depth];
                 }
             }
-            sr = sr + lr, sg = sg + lg, sb = sb + lb;
-            if (L.sum64) ax = ax + (double)lr, ay = ay + (double)lg, az = az + (double)lb;
-            if (++smp < L.num_samples) start();
+            auto add = [&]() {
+                sr = sr + lr, sg = sg + lg, sb = sb + lb;
+                if (L.sum64) ax = ax + (double)lr, ay = ay + (double)lg, az = az + (double)lb;
+                smp++;
+            };
+            add();
+            if (kMode == 0 && at_camera)  // every sample has this value
+                while (smp < L.num_samples) segments++, add();
+            if (smp < L.num_samples) start();
             else finish_pixel();
         }
     }
 }
 
-// One fixed pixel per lane (active lanes).
+// One fixed pixel per lane (active lanes), in the launch's mode.
 template <int kStackN>
 __device__ __forceinline__ void pt_pixel_sync(const DevScene &s, const PtLaunch &L, bool active, uint32_t px,
                                          uint32_t py, uint32_t &segments) {
     OnePixel src{active, px, py, false};
     uint32_t pixels = 0;
-    pt_sync<kStackN>(s, L, src, segments, pixels);
+    if (L.mode == 0) pt_sync<kStackN, 0>(s, L, src, segments, pixels);
+    else pt_sync<kStackN, 1>(s, L, src, segments, pixels);
 }
 
 // Mode 0 as a per-lane state machine (the batch kernel's: 355 against 296
@@ -286,31 +319,49 @@ __device__ __forceinline__ void pt_lanes(const DevScene &s, const PtLaunch &L, S
     TravStack<kStackN> S;
     T.have_node = T.have_leaf = false;
     T.best = -1;
+    FirstHit first;  // of the pixel, traced by its first sample only
 
     auto extend = [&](const RayF &ray) {
         r = ray;
         job = true;
         trav_start<kClosest>(s, r, 0.f, any_geometry, T);
     };
+    auto bounce = [&](float hx, float hy, float hz, const float4 &nrm) {
+        const float u1 = pray_uniform(&rng), u2 = pray_uniform(&rng);
+        const float n3[3] = {nrm.x, nrm.y, nrm.z};
+        float d[3];
+        pray_sample_hemisphere(n3, u1, u2, d);
+        depth++;
+        extend(make_ray(hx, hy, hz, d[0], d[1], d[2]));
+    };
     auto start_sample = [&]() {
         rng = pray_pcg32_stream(L.seed, pixel(), L.sample_offset + smp);
         depth = 0;
-        extend(primary_ray(L.cam, px, py));
+        if (smp == 0) {
+            extend(primary_ray(L.cam, px, py));
+        } else {
+            segments++;  // the camera ray
+            bounce(first.x, first.y, first.z, shade_n(s, first.id));
+        }
     };
     // the path ended with value l: the albedos of its bounces are applied
     // deepest first, and it joins the pixel's sums in sample order
     auto end_path = [&](float lr, float lg, float lb) {
         job = false;
+        uint32_t last = smp + 1;  // at the camera ray's end, all samples at once
+        if (depth == 0) last = L.num_samples, segments += last - smp - 1;
         while (depth > 0) {
             depth--;
             lr = lr * alb_r[depth], lg = lg * alb_g[depth], lb = lb * alb_b[depth];
         }
-        sr = sr + lr, sg = sg + lg, sb = sb + lb;
-        if (L.sum64) {
-            double *a = L.sum64 + 3 * pixel();
-            a[0] = a[0] + (double)lr, a[1] = a[1] + (double)lg, a[2] = a[2] + (double)lb;
+        for (; smp < last; smp++) {
+            sr = sr + lr, sg = sg + lg, sb = sb + lb;
+            if (L.sum64) {
+                double *a = L.sum64 + 3 * pixel();
+                a[0] = a[0] + (double)lr, a[1] = a[1] + (double)lg, a[2] = a[2] + (double)lb;
+            }
         }
-        if (++smp < L.num_samples) {
+        if (smp < L.num_samples) {
             start_sample();
             return;
         }
@@ -350,12 +401,8 @@ __device__ __forceinline__ void pt_lanes(const DevScene &s, const PtLaunch &L, S
         const float t = T.best_t;
         const float hx = r.ox + r.dx * t, hy = r.oy + r.dy * t, hz = r.oz + r.dz * t;
         alb_r[depth] = col.x, alb_g[depth] = col.y, alb_b[depth] = col.z;
-        const float u1 = pray_uniform(&rng), u2 = pray_uniform(&rng);
-        const float n3[3] = {nrm.x, nrm.y, nrm.z};
-        float d[3];
-        pray_sample_hemisphere(n3, u1, u2, d);
-        depth++;
-        extend(make_ray(hx, hy, hz, d[0], d[1], d[2]));
+        if (depth == 0) first.x = hx, first.y = hy, first.z = hz, first.id = id;
+        bounce(hx, hy, hz, nrm);
     };
 
     while (true) {
