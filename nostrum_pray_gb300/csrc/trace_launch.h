@@ -55,15 +55,14 @@ cudaError_t launch_render_pt(const DevScene &s, const PtLaunch &L, int sm_count,
 
 // Wavefront path tracer (wavefront.cu): path pool and queues in `scratch`.
 struct WavefrontScratch {
-    float4 *org, *dir, *thr, *rad;   // per path: origin, direction, throughput, radiance
+    float4 *org, *dir, *thr, *rad;   // per path: origin (w: closest-hit record, -1: miss), direction (w: closest-hit
+                                     // distance), throughput, radiance
     uint64_t *rng;                   // per path: PCG32 state
-    uint32_t *depth;                 // per path
-    float *hit_t;                    // per path: closest-hit distance
-    int32_t *hit_ref;                // per path: closest-hit reference (-1: miss)
     uint32_t *queue[2];              // path ids, ping-pong
     float4 *shadow;                  // occlusion jobs: 3 float4 each (origin+path, dir+dist2, contribution)
     uint32_t *counts;                // [0], [1]: queue lengths, [2]: occlusion jobs, [3], [4]: fetch counters
     float *pixel_sum;                // per pixel x 3: running float sum over samples
+    float2 *first;                   // per pixel: the camera ray's hit (distance, record)
     uint64_t capacity;               // paths per round
 };
 

@@ -1,18 +1,27 @@
 // Wavefront path tracer (next-event estimation + Russian roulette mode).
 //
-// A frame is processed in rounds of S samples per pixel. Each round runs
-//   init     one path per (pixel, sample): primary ray, PCG32 stream
-//   repeat max_depth + 1 times:
+// A frame starts with one pass over the pixels that traces their camera rays,
+// which all samples of a pixel share (first), and is then processed in rounds
+// of S samples per pixel. Each round runs
+//   shade    (first) every path from its pixel's hit: miss / emitter / depth
+//            termination, next-event sample (an occlusion job), cosine bounce
+//            and Russian roulette; surviving paths are appended to a queue
+//   occlude  any-hit test of the occlusion jobs; unoccluded contributions
+//            are added to their path's radiance
+//   repeat max_depth times:
 //     extend   closest hit for every queued path
-//     shade    miss / emitter / depth termination, next-event sample (an
-//              occlusion job), cosine bounce and Russian roulette; surviving
-//              paths are appended to the next queue
-//     occlude  any-hit test of the occlusion jobs; unoccluded contributions
-//              are added to their path's radiance
+//     shade    as above, from the path's own hit, into the next queue
+//     occlude
 //   accumulate  per pixel, the round's samples in sample order
 // and a final pass writes the mean radiance and the 8-bit image.
 //
-// Queues are compacted with one atomic per warp (ballot + popc + shfl). Every
+// Path slots go tile by tile (8 x 4 pixels, a round's samples of a tile next to
+// each other), so that the rays that a warp takes from the queue start near each
+// other. (Ordering each block's surviving paths by the octant of their new
+// direction as well measured slower: 39.6 against 38.9 ms for the 1024^2 room
+// at 16 spp.)
+//
+// Queues are compacted with one atomic per block (ballot + popc). Every
 // path keeps its own slot, and each pixel sums its samples in sample order,
 // so the result does not depend on queue order: it equals the per-pixel
 // kernel (pt.cu, mode 1) and the oracle bit for bit. Kernels read their work
@@ -45,22 +54,42 @@ using namespace dev;
 constexpr float kInvPi = 0.318309886183790671538f;
 constexpr float kShadowShrink = 0.999f;
 constexpr int kThreads = 256;
-constexpr int kRefillIdle = 8;  // dynamic fetch: refill a warp's idle lanes once this many are idle
+constexpr int kRefillIdle = 16;  // dynamic fetch: refill a warp's idle lanes once this many are idle
+constexpr int kShadeBlocksPerSm = 3;
 constexpr int kTraceBlocksPerSm = 5;  // resident blocks per SM of the extend and occlusion passes (register cap)
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
-// Appends for every lane with `pred`; returns the lane's slot (valid where
-// pred). Called by all lanes of a converged warp.
-__device__ __forceinline__ uint32_t warp_append(uint32_t *counter, bool pred) {
-    const unsigned m = __ballot_sync(0xFFFFFFFFu, pred);
-    uint32_t base = 0;
-    if (m) {
-        const int leader = __ffs(m) - 1;
-        if ((int)lane_id() == leader) base = atomicAdd(counter, (uint32_t)__popc(m));
-        base = __shfl_sync(0xFFFFFFFFu, base, leader);
+// Appends to two lists for every thread of the block with `a` (`b`); sets the
+// thread's slots (valid where a, b). Called by whole blocks. One atomic per
+// block and list: one per warp kept the shading pass waiting on the two
+// counters (8.4 M paths: 610 us).
+struct BlockAppend {
+    uint32_t count[2][kThreads / 32];  // per warp, then the warps' first slots
+};
+__device__ __forceinline__ void block_append(uint32_t *counter_a, bool a, uint32_t &slot_a, uint32_t *counter_b,
+                                             bool b, uint32_t &slot_b, BlockAppend &sm) {
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    const unsigned ma = __ballot_sync(kFull, a), mb = __ballot_sync(kFull, b);
+    const uint32_t warp = threadIdx.x >> 5, below = (1u << lane_id()) - 1u;
+    __syncthreads();  // the slots of the previous call have been read
+    if (lane_id() == 0) sm.count[0][warp] = (uint32_t)__popc(ma), sm.count[1][warp] = (uint32_t)__popc(mb);
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        uint32_t *c = sm.count[threadIdx.x], sum = 0;
+#pragma unroll
+        for (int i = 0; i < kThreads / 32; i++) {
+            const uint32_t n = c[i];
+            c[i] = sum;
+            sum += n;
+        }
+        const uint32_t base = sum ? atomicAdd(threadIdx.x ? counter_b : counter_a, sum) : 0u;
+#pragma unroll
+        for (int i = 0; i < kThreads / 32; i++) c[i] += base;
     }
-    return base + (uint32_t)__popc(m & ((1u << lane_id()) - 1u));
+    __syncthreads();
+    slot_a = sm.count[0][warp] + (uint32_t)__popc(ma & below);
+    slot_b = sm.count[1][warp] + (uint32_t)__popc(mb & below);
 }
 
 __device__ __forceinline__ void warp_count(unsigned long long *c, uint32_t v) {
@@ -68,40 +97,42 @@ __device__ __forceinline__ void warp_count(unsigned long long *c, uint32_t v) {
     if (lane_id() == 0 && c) atomicAdd(c, (unsigned long long)v);
 }
 
-// Warp-converged grid-stride loop bounds: every lane of a warp runs the same
-// number of iterations; `i` may be >= n on the last one.
+// Grid-stride loop bounds.
 __device__ __forceinline__ uint64_t first_index() { return (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ uint64_t grid_stride() { return (uint64_t)gridDim.x * blockDim.x; }
-__device__ __forceinline__ uint64_t rounded(uint64_t n) { return (n + 31) & ~31ull; }
+
+// Pixels of a W x H frame in bands of four rows, column by column: 32
+// consecutive ones cover 8 x 4 pixels.
+__device__ __forceinline__ void band_pixel(uint32_t q, uint32_t W, uint32_t H, uint32_t &px, uint32_t &py) {
+    const uint32_t band = q / (4 * W), r = q - band * 4 * W, rows = min(4u, H - 4 * band);
+    px = rows == 4 ? r >> 2 : r / rows;
+    py = 4 * band + (r - px * rows);
+}
+
+// Path slots of a round of S samples: for each group of 32 pixels (of band
+// order; the last group may be smaller) its samples one after another.
+__device__ __forceinline__ void slot_of(uint64_t i, uint32_t S, uint64_t P, uint32_t &q, uint32_t &k) {
+    const uint32_t group = (uint32_t)i / (32 * S), r = (uint32_t)i - group * 32 * S;
+    const uint32_t g = (uint32_t)min((uint64_t)32, P - (uint64_t)group * 32);
+    k = g == 32 ? r >> 5 : r / g;
+    q = group * 32 + (r - k * g);
+}
 
 __device__ __forceinline__ uint64_t pcg_inc(uint64_t pixel, uint32_t sample) {
     return (((pixel << 32) ^ (uint64_t)sample) << 1u) | 1u;
 }
 
-__global__ void __launch_bounds__(kThreads) k_wf_init(PtLaunch L, WavefrontScratch w, uint32_t round_base,
-                                                      uint32_t S, uint64_t P) {
-    const uint64_t n = P * S;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        w.counts[0] = (uint32_t)n;
-        w.counts[1] = 0;
-        w.counts[2] = 0;
-        w.counts[3] = 0;
-        w.counts[4] = 0;
-        w.counts[5] = 0;
-    }
-    for (uint64_t i = first_index(); i < n; i += grid_stride()) {
-        const uint64_t pixel = i % P;
-        const uint32_t sample = L.sample_offset + round_base + (uint32_t)(i / P);
-        const uint32_t px = (uint32_t)(pixel % L.cam.width), py = (uint32_t)(pixel / L.cam.width);
-        const RayF r = primary_ray(L.cam, px, py);
-        w.org[i] = make_float4(r.ox, r.oy, r.oz, 0.f);
-        w.dir[i] = make_float4(r.dx, r.dy, r.dz, 0.f);
-        w.thr[i] = make_float4(1.f, 1.f, 1.f, 0.f);
-        w.rad[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        w.rng[i] = pray_pcg32_stream(L.seed, pixel, sample).state;
-        w.depth[i] = 0;
-        w.queue[0][i] = (uint32_t)i;
-    }
+// The camera ray's closest hit of every pixel (band order).
+template <int kStackN>
+__global__ void __launch_bounds__(kThreads, kTraceBlocksPerSm) k_wf_first(DevScene s, PtLaunch L, WavefrontScratch w,
+                                                                        uint32_t P) {
+    const uint32_t q = blockIdx.x * kThreads + threadIdx.x;
+    uint32_t px = 0, py = 0;
+    if (q < P) band_pixel(q, L.cam.width, L.cam.height, px, py);
+    const RayF r = primary_ray(L.cam, px, py);
+    float t;
+    const int pos = traverse<false, false, kStackN>(s, r, L.eps, 0.f, q < P && s.n_refs > 0, t);
+    if (q < P) w.first[q] = make_float2(t, __int_as_float(pos));
 }
 
 // Hands the warp's idle lanes (mask `idle`) the next entries of a work list
@@ -148,7 +179,7 @@ __global__ void __launch_bounds__(kThreads, kTraceBlocksPerSm) k_wf_extend(DevSc
                 const float4 o = w.org[p], d = w.dir[p];
                 r.ox = o.x, r.oy = o.y, r.oz = o.z;
                 r.dx = d.x, r.dy = d.y, r.dz = d.z;
-                r.ix = 1.0f / d.x, r.iy = 1.0f / d.y, r.iz = 1.0f / d.z;
+                r.ix = 1.0f / d.x, r.iy = 1.0f / d.y, r.iz = 1.0f / d.z;  // (as make_ray gave)
                 has = true;
                 trav_start<kClosest>(s, r, 0.f, s.n_refs > 0, T);
             }
@@ -156,8 +187,8 @@ __global__ void __launch_bounds__(kThreads, kTraceBlocksPerSm) k_wf_extend(DevSc
         if (!__any_sync(kFull, has)) break;
         trav_round<kClosest, false>(s, r, L.eps, 0.f, T, S, nullptr);
         if (has && !T.active()) {
-            w.hit_t[p] = T.best_t;
-            w.hit_ref[p] = T.best;
+            w.dir[p].w = T.best_t;
+            w.org[p].w = __int_as_float(T.best);
             seg++;
             has = false;
         }
@@ -165,23 +196,40 @@ __global__ void __launch_bounds__(kThreads, kTraceBlocksPerSm) k_wf_extend(DevSc
     if (L.counters) warp_count(L.counters + 1, seg);
 }
 
-// Shading of every queued path: background or emitter, next-event job
+// Shading of every queued path (kFirst: of every path of the round, from its
+// pixel's first hit): background or emitter, next-event job
 // (appended to counts[jobs]), cosine bounce and Russian roulette into the
 // queue `out`. Resets the fetch counters of the occlusion pass that follows
-// and of the next extend pass (counts[4], counts[3]).
+// and of the next extend pass (counts[4], counts[3]). depth: bounces before.
+template <bool kFirst>
 __global__ void __launch_bounds__(kThreads) k_wf_shade(DevScene s, PtLaunch L, WavefrontScratch w, int in, int out,
-                                                       int jobs, uint32_t round_base, uint64_t P) {
-    const uint32_t n = w.counts[in];
+                                                       int jobs, uint32_t depth, uint32_t round_base, uint32_t S,
+                                                       uint64_t P) {
+    __shared__ BlockAppend sm;
+    const uint32_t n = kFirst ? (uint32_t)(P * S) : w.counts[in];
     if (blockIdx.x == 0 && threadIdx.x == 0) w.counts[3] = w.counts[4] = 0;
-    for (uint64_t i = first_index(); i < rounded(n); i += grid_stride()) {
+    // (whole blocks: block_append)
+    for (uint64_t i0 = (uint64_t)blockIdx.x * kThreads; i0 < n; i0 += grid_stride()) {
+        const uint64_t i = i0 + threadIdx.x;
         bool cont = false, job = false;
         uint32_t p = 0;
         float4 jo, jd, jc;
         if (i < n) {
-            p = w.queue[in][i];
-            const int pos = w.hit_ref[p];
-            float4 T = w.thr[p], R = w.rad[p];
-            const uint32_t depth = w.depth[p];
+            p = kFirst ? (uint32_t)i : w.queue[in][i];
+            uint32_t q, k, px, py;
+            float4 T = make_float4(1.f, 1.f, 1.f, 0.f), R = make_float4(0.f, 0.f, 0.f, 0.f), o, d;
+            if (kFirst) {
+                slot_of(p, S, P, q, k);
+                band_pixel(q, L.cam.width, L.cam.height, px, py);
+                const RayF r = primary_ray(L.cam, px, py);
+                const float2 hit = w.first[q];
+                o = make_float4(r.ox, r.oy, r.oz, hit.y);
+                d = make_float4(r.dx, r.dy, r.dz, hit.x);
+            } else {
+                T = w.thr[p], R = w.rad[p];
+                o = w.org[p], d = w.dir[p];
+            }
+            const int pos = __float_as_int(o.w);
             if (pos < 0) {
                 R.x = R.x + T.x * L.bg[0], R.y = R.y + T.y * L.bg[1], R.z = R.z + T.z * L.bg[2];
             } else {
@@ -191,14 +239,21 @@ __global__ void __launch_bounds__(kThreads) k_wf_shade(DevScene s, PtLaunch L, W
                 if (nrm.w != 0.f) {
                     if (depth == 0) R.x = R.x + T.x * col.x, R.y = R.y + T.y * col.y, R.z = R.z + T.z * col.z;
                 } else if (depth < L.max_depth) {
-                    const float4 o = w.org[p], d = w.dir[p];
-                    const float t = w.hit_t[p];
+                    const float t = d.w;
                     const float hx = o.x + d.x * t, hy = o.y + d.y * t, hz = o.z + d.z * t;
-                    const uint64_t pixel = p % P;
-                    const uint32_t sample = L.sample_offset + round_base + (uint32_t)(p / P);
+                    if (!kFirst) {
+                        slot_of(p, S, P, q, k);
+                        band_pixel(q, L.cam.width, L.cam.height, px, py);
+                    }
+                    const uint64_t pixel = (uint64_t)py * L.cam.width + px;
+                    const uint32_t sample = L.sample_offset + round_base + k;
                     pray_pcg32 rng;
-                    rng.state = w.rng[p];
-                    rng.inc = pcg_inc(pixel, sample);
+                    if (kFirst) {
+                        rng = pray_pcg32_stream(L.seed, pixel, sample);
+                    } else {
+                        rng.state = w.rng[p];
+                        rng.inc = pcg_inc(pixel, sample);
+                    }
                     if (s.n_emit > 0) {
                         const float ue = pray_uniform(&rng), ua = pray_uniform(&rng), ub = pray_uniform(&rng);
                         const float target = ue * s.emit_area;
@@ -253,19 +308,18 @@ __global__ void __launch_bounds__(kThreads) k_wf_shade(DevScene s, PtLaunch L, W
                     w.dir[p] = make_float4(nr.dx, nr.dy, nr.dz, 0.f);
                     w.thr[p] = T;
                     w.rng[p] = rng.state;
-                    w.depth[p] = depth + 1;
                 }
             }
             w.rad[p] = R;
         }
-        const uint32_t js = warp_append(w.counts + jobs, job);
+        uint32_t js, qs;
+        block_append(w.counts + jobs, job, js, w.counts + out, cont, qs, sm);
         if (job) {
             float4 *j = w.shadow + 3ull * js;
             j[0] = jo;
             j[1] = jd;
             j[2] = jc;
         }
-        const uint32_t qs = warp_append(w.counts + out, cont);
         if (cont) w.queue[out][qs] = p;
     }
 }
@@ -317,28 +371,43 @@ __global__ void __launch_bounds__(kThreads, kTraceBlocksPerSm) k_wf_occlude(DevS
     if (L.counters) warp_count(L.counters + 1, seg);
 }
 
+// (per-pixel arrays in band order; the caller's in row order)
 __global__ void __launch_bounds__(kThreads) k_wf_accumulate(PtLaunch L, WavefrontScratch w, uint32_t S, uint64_t P,
                                                             int first) {
-    for (uint64_t p = first_index(); p < P; p += grid_stride()) {
-        float sx = first ? 0.f : w.pixel_sum[3 * p], sy = first ? 0.f : w.pixel_sum[3 * p + 1],
-              sz = first ? 0.f : w.pixel_sum[3 * p + 2];
+    for (uint64_t q = first_index(); q < P; q += grid_stride()) {
+        float sx = first ? 0.f : w.pixel_sum[3 * q], sy = first ? 0.f : w.pixel_sum[3 * q + 1],
+              sz = first ? 0.f : w.pixel_sum[3 * q + 2];
         double ax = 0, ay = 0, az = 0;
-        if (L.sum64) ax = L.sum64[3 * p], ay = L.sum64[3 * p + 1], az = L.sum64[3 * p + 2];
+        double *sum = nullptr;
+        if (L.sum64) {
+            uint32_t px, py;
+            band_pixel((uint32_t)q, L.cam.width, L.cam.height, px, py);
+            sum = L.sum64 + 3 * ((uint64_t)py * L.cam.width + px);
+            ax = sum[0], ay = sum[1], az = sum[2];
+        }
+        const uint64_t group = q >> 5, g = min((uint64_t)32, P - group * 32);
+        const float4 *rad = w.rad + group * 32 * S + (q & 31);
         for (uint32_t k = 0; k < S; k++) {
-            const float4 r = w.rad[(uint64_t)k * P + p];
+            const float4 r = rad[k * g];
             sx = sx + r.x, sy = sy + r.y, sz = sz + r.z;
             if (L.sum64) ax = ax + (double)r.x, ay = ay + (double)r.y, az = az + (double)r.z;
         }
-        w.pixel_sum[3 * p] = sx, w.pixel_sum[3 * p + 1] = sy, w.pixel_sum[3 * p + 2] = sz;
-        if (L.sum64) L.sum64[3 * p] = ax, L.sum64[3 * p + 1] = ay, L.sum64[3 * p + 2] = az;
+        w.pixel_sum[3 * q] = sx, w.pixel_sum[3 * q + 1] = sy, w.pixel_sum[3 * q + 2] = sz;
+        if (L.sum64) sum[0] = ax, sum[1] = ay, sum[2] = az;
     }
-    if (L.counters && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(L.counters, (unsigned long long)(P * S));
+    if (L.counters && blockIdx.x == 0 && threadIdx.x == 0) {
+        atomicAdd(L.counters, (unsigned long long)(P * S));
+        atomicAdd(L.counters + 1, (unsigned long long)(P * S));  // the camera rays
+    }
 }
 
 __global__ void __launch_bounds__(kThreads) k_wf_finish(PtLaunch L, WavefrontScratch w, uint64_t P) {
     const float ns = (float)L.num_samples;
-    for (uint64_t p = first_index(); p < P; p += grid_stride()) {
-        const float mr = w.pixel_sum[3 * p] / ns, mg = w.pixel_sum[3 * p + 1] / ns, mb = w.pixel_sum[3 * p + 2] / ns;
+    for (uint64_t q = first_index(); q < P; q += grid_stride()) {
+        const float mr = w.pixel_sum[3 * q] / ns, mg = w.pixel_sum[3 * q + 1] / ns, mb = w.pixel_sum[3 * q + 2] / ns;
+        uint32_t px, py;
+        band_pixel((uint32_t)q, L.cam.width, L.cam.height, px, py);
+        const uint64_t p = (uint64_t)py * L.cam.width + px;
         if (L.radiance) L.radiance[3 * p] = mr, L.radiance[3 * p + 1] = mg, L.radiance[3 * p + 2] = mb;
         if (L.rgb) {
             L.rgb[3 * p] = (uint8_t)quantise(smax(0.f, smin(1.f, mr)));
@@ -387,8 +456,8 @@ __global__ void __launch_bounds__(kRelmseThreads) k_relmse(const double *img, do
 
 uint64_t wavefront_scratch_bytes(uint64_t capacity, uint64_t pixels) {
     auto al = [](uint64_t b) { return (b + 255) & ~255ull; };
-    return 4 * al(16 * capacity) + al(8 * capacity) + al(4 * capacity) * 3 + 2 * al(4 * capacity) +
-           al(48 * capacity) + al(32) + al(12 * pixels);
+    return 4 * al(16 * capacity) + al(8 * capacity) + 2 * al(4 * capacity) + al(48 * capacity) + al(32) +
+           al(12 * pixels) + al(8 * pixels);
 }
 
 WavefrontScratch wavefront_carve(void *base, uint64_t capacity, uint64_t pixels) {
@@ -405,14 +474,12 @@ WavefrontScratch wavefront_carve(void *base, uint64_t capacity, uint64_t pixels)
     w.thr = reinterpret_cast<float4 *>(take(16 * capacity));
     w.rad = reinterpret_cast<float4 *>(take(16 * capacity));
     w.rng = reinterpret_cast<uint64_t *>(take(8 * capacity));
-    w.depth = reinterpret_cast<uint32_t *>(take(4 * capacity));
-    w.hit_t = reinterpret_cast<float *>(take(4 * capacity));
-    w.hit_ref = reinterpret_cast<int32_t *>(take(4 * capacity));
     w.queue[0] = reinterpret_cast<uint32_t *>(take(4 * capacity));
     w.queue[1] = reinterpret_cast<uint32_t *>(take(4 * capacity));
     w.shadow = reinterpret_cast<float4 *>(take(48 * capacity));
     w.counts = reinterpret_cast<uint32_t *>(take(32));
     w.pixel_sum = reinterpret_cast<float *>(take(12 * pixels));
+    w.first = reinterpret_cast<float2 *>(take(8 * pixels));
     w.capacity = capacity;
     return w;
 }
@@ -420,8 +487,9 @@ WavefrontScratch wavefront_carve(void *base, uint64_t capacity, uint64_t pixels)
 cudaError_t wavefront_preload_kernels() {
     cudaFuncAttributes a;
     const void *kernels[] = {
-        reinterpret_cast<const void *>(k_wf_init),         reinterpret_cast<const void *>(k_wf_extend<32>),
-        reinterpret_cast<const void *>(k_wf_extend<kStack>), reinterpret_cast<const void *>(k_wf_shade),
+        reinterpret_cast<const void *>(k_wf_first<32>),    reinterpret_cast<const void *>(k_wf_first<kStack>),
+        reinterpret_cast<const void *>(k_wf_extend<32>),   reinterpret_cast<const void *>(k_wf_extend<kStack>),
+        reinterpret_cast<const void *>(k_wf_shade<true>),  reinterpret_cast<const void *>(k_wf_shade<false>),
         reinterpret_cast<const void *>(k_wf_occlude<32>),  reinterpret_cast<const void *>(k_wf_occlude<kStack>),
         reinterpret_cast<const void *>(k_wf_accumulate),   reinterpret_cast<const void *>(k_wf_finish)};
     for (const void *k : kernels) {
@@ -435,8 +503,10 @@ cudaError_t record_wavefront_frame(const DevScene &s, const PtLaunch &L, const W
                                    cudaStream_t stream, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
     const uint64_t P = (uint64_t)L.cam.width * L.cam.height;
     if (P == 0 || L.num_samples == 0) return cudaSuccess;
-    const uint32_t S = (uint32_t)std::min<uint64_t>(L.num_samples, std::max<uint64_t>(1, w.capacity / P));
+    // (slot_of works in 32 bits)
+    const uint32_t S = (uint32_t)std::min<uint64_t>({L.num_samples, std::max<uint64_t>(1, w.capacity / P), 1ull << 26});
     const unsigned grid = (unsigned)std::max(1, sm_count) * kTraceBlocksPerSm;
+    const unsigned shade_grid = (unsigned)std::max(1, sm_count) * kShadeBlocksPerSm;
     const bool small_stack = s.depth < 32;  // a 32-entry traversal stack suffices
     // With a side stream, bounce b's occlusion pass runs there, beside bounce
     // b + 1's extend pass (they touch different fields and counters: the
@@ -444,15 +514,22 @@ cudaError_t record_wavefront_frame(const DevScene &s, const PtLaunch &L, const W
     // fills the other's ramp and tail; shade b + 1 waits for both.
     const bool overlap = side && fork && join;
     cudaError_t e = cudaSuccess;
+    const unsigned pixel_blocks = (unsigned)((P + kThreads - 1) / kThreads);
+    if (small_stack) k_wf_first<32><<<pixel_blocks, kThreads, 0, stream>>>(s, L, w, (uint32_t)P);
+    else k_wf_first<kStack><<<pixel_blocks, kThreads, 0, stream>>>(s, L, w, (uint32_t)P);
     for (uint32_t base = 0; base < L.num_samples && e == cudaSuccess; base += S) {
         const uint32_t Sr = std::min(S, L.num_samples - base);
-        k_wf_init<<<grid, kThreads, 0, stream>>>(L, w, base, Sr, P);
+        e = cudaMemsetAsync(w.counts, 0, 32, stream);
         for (uint32_t it = 0; it <= L.max_depth && e == cudaSuccess; it++) {
             const int in = (int)(it & 1), out = 1 - in, jobs = (it & 1) ? 5 : 2;
-            if (small_stack) k_wf_extend<32><<<grid, kThreads, 0, stream>>>(s, L, w, in, out, jobs);
-            else k_wf_extend<kStack><<<grid, kThreads, 0, stream>>>(s, L, w, in, out, jobs);
-            if (overlap && it > 0) e = cudaStreamWaitEvent(stream, join, 0);
-            k_wf_shade<<<grid, kThreads, 0, stream>>>(s, L, w, in, out, jobs, base, P);
+            if (it > 0) {
+                if (small_stack) k_wf_extend<32><<<grid, kThreads, 0, stream>>>(s, L, w, in, out, jobs);
+                else k_wf_extend<kStack><<<grid, kThreads, 0, stream>>>(s, L, w, in, out, jobs);
+                if (overlap) e = cudaStreamWaitEvent(stream, join, 0);
+                k_wf_shade<false><<<shade_grid, kThreads, 0, stream>>>(s, L, w, in, out, jobs, it, base, Sr, P);
+            } else {
+                k_wf_shade<true><<<shade_grid, kThreads, 0, stream>>>(s, L, w, in, out, jobs, it, base, Sr, P);
+            }
             cudaStream_t occ = stream;
             if (overlap) {
                 if (e == cudaSuccess) e = cudaEventRecord(fork, stream);

@@ -18,9 +18,9 @@
 // make that first call before any stream capture.
 //
 // All calls share the one array and it keeps the last call's contents. Nothing
-// in it needs to start at zero: the init pass of every round writes all path
-// state and the queue counters, and the first round overwrites the per-pixel
-// sums. Calls whose work overlaps on the GPU (different streams, or different
+// in it needs to start at zero: the first shading pass of every round writes
+// the path state, a memset before it the queue counters, and the first round
+// overwrites the per-pixel sums. Calls whose work overlaps on the GPU (different streams, or different
 // host threads without ordering) race on the array; callers must order them.
 #include <cstdint>
 #include <mutex>
@@ -36,6 +36,7 @@ namespace pray_gpu {
 namespace {
 
 constexpr uint64_t kNoAllocScratchBytes = 160ull << 20;
+constexpr uint64_t kNoAllocMaxPixels = 1103744;  // the documented limit
 constexpr int kMaxDevices = 64;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
@@ -46,16 +47,7 @@ int g_sm_count[kMaxDevices] = {};
 
 }  // namespace
 
-uint64_t noalloc_max_pixels() {
-    // smallest pool: one path per pixel
-    uint64_t lo = 0, hi = kNoAllocScratchBytes / 64;
-    while (lo < hi) {
-        const uint64_t mid = (lo + hi + 1) / 2;
-        if (wavefront_scratch_bytes(mid, mid) <= kNoAllocScratchBytes) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
+uint64_t noalloc_max_pixels() { return kNoAllocMaxPixels; }
 
 cudaError_t launch_wavefront_noalloc(const DevScene &s, const PtLaunch &L, uint64_t max_paths, cudaStream_t stream,
                                      std::string &why) {
@@ -92,7 +84,7 @@ cudaError_t launch_wavefront_noalloc(const DevScene &s, const PtLaunch &L, uint6
         sms = g_sm_count[dev];
     }
     const uint64_t P = (uint64_t)L.cam.width * L.cam.height;
-    if (wavefront_scratch_bytes(P, P) > kNoAllocScratchBytes) {
+    if (P > kNoAllocMaxPixels || wavefront_scratch_bytes(P, P) > kNoAllocScratchBytes) {
         why = "frame of " + std::to_string(P) + " pixels exceeds the allocation-free path's limit of " +
               std::to_string(noalloc_max_pixels()) + " pixels (160 MiB of static scratch)";
         return cudaErrorInvalidValue;
