@@ -247,7 +247,7 @@ cudaError_t render_rt(pray_scene *s, RtLaunch L, cudaStream_t stream) {
             for (int m = 0; m < kModes && e == cudaSuccess; m++) {
                 C.packets = modes[m];
                 if (rep == 1) e = cudaEventRecord(ev[2 * m], stream);
-                if (e == cudaSuccess) e = launch_render_rt(s->view(), C, stream);
+                if (e == cudaSuccess) e = launch_render_rt(s->view(), C, s->sm_count, stream);
                 if (rep == 1 && e == cudaSuccess) e = cudaEventRecord(ev[2 * m + 1], stream);
             }
         if (e == cudaSuccess) e = cudaEventSynchronize(ev[2 * kModes - 1]);
@@ -264,7 +264,7 @@ cudaError_t render_rt(pray_scene *s, RtLaunch L, cudaStream_t stream) {
         s->rt_packets.store(modes[best]);
     }
     L.packets = s->rt_packets.load();
-    return launch_render_rt(s->view(), L, stream);
+    return launch_render_rt(s->view(), L, s->sm_count, stream);
 }
 
 pray_status check_pt_params(const pray_pt_params *p) {
@@ -300,6 +300,7 @@ PtLaunch make_pt_launch(const pray_pt_params *p) {
     L.seed = p->seed;
     L.eps = p->det_epsilon;
     L.sample_offset = p->sample_offset;
+    L.lanes = 32;
     return L;
 }
 
@@ -360,9 +361,6 @@ pray_status run_pt(pray_scene *s, const PtLaunch &L, int scheduler, uint32_t wav
             (e = cudaEventCreateWithFlags(&s->wf_fork, cudaEventDisableTiming)) != cudaSuccess ||
             (e = cudaEventCreateWithFlags(&s->wf_join, cudaEventDisableTiming)) != cudaSuccess)
             return cuda_error(e, "path-tracer stream set-up");
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, dev);
     }
     if (scheduler == PRAY_SCHED_PIXEL) {
         if (!s->d_pt_next && (e = cudaMalloc(&s->d_pt_next, sizeof(unsigned long long))) != cudaSuccess)
@@ -608,6 +606,8 @@ pray_status pray_scene_create(const float *verts, const float *colors, const uin
     })
     cudaError_t e = cudaSetDevice(device);
     if (e != cudaSuccess) return cuda_error(e, "cudaSetDevice");
+    if ((e = cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess)
+        return cuda_error(e, "cudaDeviceGetAttribute");
     const size_t nb = gnodes.size() * sizeof(GNode), tb = std::max<size_t>(gtris.size(), 1) * sizeof(GTri),
                  sb = std::max<size_t>(gshade.size(), 1) * sizeof(GShade);
     if ((e = cudaMalloc(&s->d_nodes, nb)) != cudaSuccess || (e = cudaMalloc(&s->d_tris, tb)) != cudaSuccess ||
@@ -686,7 +686,7 @@ pray_status pray_trace_closest(pray_scene *s, const float *rays, uint64_t n, flo
     if (n >= (1ull << 40)) return set_error(PRAY_ERR_INVALID_ARGUMENT, "too many rays");
     cudaError_t e = cudaSetDevice(s->device);
     if (e != cudaSuccess) return cuda_error(e, "cudaSetDevice");
-    e = launch_trace_closest(s->view(), rays, n, eps, ids, ts, (cudaStream_t)stream);
+    e = launch_trace_closest(s->view(), rays, n, eps, ids, ts, s->sm_count, (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_error(e, "trace_closest launch");
     return PRAY_OK;
 }
@@ -697,7 +697,7 @@ pray_status pray_trace_occluded(pray_scene *s, const float *rays, const float *d
     if (n >= (1ull << 40)) return set_error(PRAY_ERR_INVALID_ARGUMENT, "too many rays");
     cudaError_t e = cudaSetDevice(s->device);
     if (e != cudaSuccess) return cuda_error(e, "cudaSetDevice");
-    e = launch_trace_occluded(s->view(), rays, dist2, n, eps, occluded, (cudaStream_t)stream);
+    e = launch_trace_occluded(s->view(), rays, dist2, n, eps, occluded, s->sm_count, (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_error(e, "trace_occluded launch");
     return PRAY_OK;
 }
@@ -725,7 +725,7 @@ pray_status pray_trace_closest_host(pray_scene *s, const float *rays_host, uint6
     float *d_t = reinterpret_cast<float *>(d_ids + s->trace_cap);
     if ((e = cudaMemcpy(d_rays, rays_host, n * 9 * sizeof(float), cudaMemcpyHostToDevice)) != cudaSuccess)
         return cuda_error(e, "cudaMemcpy (rays)");
-    if ((e = launch_trace_closest(s->view(), d_rays, n, eps, d_ids, d_t, 0)) != cudaSuccess)
+    if ((e = launch_trace_closest(s->view(), d_rays, n, eps, d_ids, d_t, s->sm_count, 0)) != cudaSuccess)
         return cuda_error(e, "trace_closest launch");
     if ((e = cudaMemcpy(ids_host, d_ids, n * sizeof(int32_t), cudaMemcpyDeviceToHost)) != cudaSuccess)
         return cuda_error(e, "cudaMemcpy (ids)");
@@ -1113,7 +1113,8 @@ pray_status pray_render_features(pray_scene *s, const pray_pt_params *p, uint16_
     cudaError_t e = cudaSetDevice(s->device);
     if (e != cudaSuccess) return cuda_error(e, "cudaSetDevice");
     const CameraConsts cam = make_camera(p->width, p->height, p->fov, p->camera_position, p->camera_look);
-    e = launch_features(s->view(), cam, p->det_epsilon, reinterpret_cast<__half *>(features), (cudaStream_t)stream);
+    e = launch_features(s->view(), cam, p->det_epsilon, reinterpret_cast<__half *>(features), s->sm_count,
+                        (cudaStream_t)stream);
     return e == cudaSuccess ? PRAY_OK : cuda_error(e, "features launch");
 }
 

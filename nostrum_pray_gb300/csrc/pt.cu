@@ -57,9 +57,9 @@ __global__ void __launch_bounds__(128, kBlocks) k_render_pt(DevScene s, PtLaunch
         FrameSrc src{L.next_pixel, warp_tiles(L.cam.width, L.cam.height) * 32, L.cam.width, L.cam.height, false};
         pt_sync<kStack, 1>(s, L, src, segments, pixels);
     } else {
-        const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+        const uint64_t warp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
         uint32_t px, py;
-        const bool active = pixel_of(i, L.cam.width, L.cam.height, px, py);
+        const bool active = pixel_of(warp * L.lanes + (threadIdx.x & 31u), L.cam.width, L.cam.height, px, py);
         OnePixel src{active, px, py, false};
         pt_sync<kStack, 0>(s, L, src, segments, pixels);
     }
@@ -87,18 +87,20 @@ __global__ void __launch_bounds__(128) k_render_pt_diffuse(DevScene s, PtLaunch 
 
 }  // namespace
 
-cudaError_t launch_render_pt(const DevScene &s, const PtLaunch &L, int sm_count, cudaStream_t stream) {
-    const uint64_t tiles = warp_tiles(L.cam.width, L.cam.height);
-    const uint64_t threads = tiles * 32;
-    if (threads == 0) return cudaSuccess;
-    const unsigned bs = 128;
-    const uint64_t blocks = (threads + bs - 1) / bs;
+cudaError_t launch_render_pt(const DevScene &s, const PtLaunch &launch, int sm_count, cudaStream_t stream) {
+    PtLaunch L = launch;
+    const uint64_t slots = warp_tiles(L.cam.width, L.cam.height) * 32;
+    if (slots == 0) return cudaSuccess;
+    constexpr unsigned bs = 128, kWarps = bs / 32;
+    const uint64_t sms = (uint64_t)(sm_count > 0 ? sm_count : 1);
+    // (a frame small enough for fewer lanes runs 8 blocks per SM below)
+    L.lanes = lanes_for(slots, sms * 8 * kWarps);
+    const uint64_t blocks = (slots + kWarps * L.lanes - 1) / (kWarps * L.lanes);
     if (L.mode == 2) {
-        k_render_pt_diffuse<<<(unsigned)blocks, bs, 0, stream>>>(s, L);
+        k_render_pt_diffuse<<<(unsigned)((slots + bs - 1) / bs), bs, 0, stream>>>(s, L);
     } else if (L.mode == 1) {
         if (!L.next_pixel) return cudaErrorInvalidValue;
         // persistent: as many blocks as stay resident, or fewer
-        const uint64_t sms = (uint64_t)(sm_count > 0 ? sm_count : 1);
         const uint64_t paths = (uint64_t)L.cam.width * L.cam.height * L.num_samples;
         if (paths < 2 * sms * 10 * bs) {
             const uint64_t resident = sms * 8;
@@ -107,7 +109,7 @@ cudaError_t launch_render_pt(const DevScene &s, const PtLaunch &L, int sm_count,
             const uint64_t resident = sms * 10;
             k_render_pt<true, 10><<<(unsigned)(blocks < resident ? blocks : resident), bs, 0, stream>>>(s, L);
         }
-    } else if (blocks <= (uint64_t)(sm_count > 0 ? sm_count : 1) * 8) {
+    } else if (blocks <= sms * 8) {
         k_render_pt<false, 8><<<(unsigned)blocks, bs, 0, stream>>>(s, L);
     } else {
         k_render_pt<false, 10><<<(unsigned)blocks, bs, 0, stream>>>(s, L);

@@ -99,8 +99,8 @@ __device__ __forceinline__ void pt_sync(const DevScene &s, const PtLaunch &L, Sr
     constexpr int kAlb = kMode == 0 ? kMaxPtDepth : 1;
     float alb_r[kAlb], alb_g[kAlb], alb_b[kAlb];
     const bool any_geometry = s.n_refs > 0;
-    // the lane's pixel
-    bool have = false;
+    // the lane's pixel (lanes beyond L.lanes take none)
+    bool have = (threadIdx.x & 31u) >= L.lanes;
     uint32_t px = 0, py = 0;
     auto pixel = [&]() { return (uint64_t)py * L.cam.width + px; };
     float sr = 0.f, sg = 0.f, sb = 0.f;

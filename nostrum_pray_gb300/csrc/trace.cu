@@ -18,16 +18,30 @@ namespace {
 
 using namespace dev;
 
+// The item of this thread when each warp takes `lanes` of them; idle: none.
+__device__ __forceinline__ uint64_t warp_item(uint32_t lanes, bool &idle) {
+    const uint32_t lane = threadIdx.x & 31u;
+    idle = lane >= lanes;
+    return ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * lanes + lane;
+}
+
+// Blocks of `threads` threads for n items, `lanes` per warp.
+unsigned blocks_for(uint64_t n, uint32_t lanes, unsigned threads) {
+    const uint64_t per = (uint64_t)(threads / 32) * lanes;
+    return (unsigned)((n + per - 1) / per);
+}
+
 // Occlusion of caller-given rays: 1 iff some triangle is hit at t > 0 with
 // t^2 < dist2 (the any-hit walk stops at the first such triangle). The
 // reference asks for the closest hit and tests lightDistSq > dst * dst
 // (src/pray.cpp:39-43); the closest t satisfies it iff some t does.
 template <int kStackN>
 __global__ void __launch_bounds__(128) k_trace_occluded(DevScene s, const float *__restrict__ rays,
-                                                        const float *__restrict__ dist2, uint64_t n, float eps,
-                                                        uint8_t *__restrict__ occluded) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = i < n;
+                                                        const float *__restrict__ dist2, uint64_t n, uint32_t lanes,
+                                                        float eps, uint8_t *__restrict__ occluded) {
+    bool idle;
+    const uint64_t i = warp_item(lanes, idle);
+    const bool valid = !idle && i < n;
     RayF r{};
     float d2 = 0.f;
     if (valid) {
@@ -44,10 +58,11 @@ __global__ void __launch_bounds__(128) k_trace_occluded(DevScene s, const float 
 
 template <int kStackN>
 __global__ void __launch_bounds__(128) k_trace_closest(DevScene s, const float *__restrict__ rays, uint64_t n,
-                                                       float eps, int32_t *__restrict__ ids,
+                                                       uint32_t lanes, float eps, int32_t *__restrict__ ids,
                                                        float *__restrict__ ts) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = i < n;
+    bool idle;
+    const uint64_t i = warp_item(lanes, idle);
+    const bool valid = !idle && i < n;
     RayF r{};
     if (valid) {
         const float *p = rays + 9 * i;
@@ -82,9 +97,10 @@ constexpr int kPacketBlocks = 10, kPacketThreads = 128;
 template <bool kCount, int kStackN, bool kPrimPacket, bool kShadowPacket>
 __global__ void __launch_bounds__(kShadowPacket ? kPacketThreads : 128, kShadowPacket ? kPacketBlocks : 8)
     k_render_rt(DevScene s, RtLaunch L) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    bool idle;
+    const uint64_t i = warp_item(L.lanes, idle);
     uint32_t px, py;
-    const bool active = pixel_of(i, L.cam.width, L.cam.height, px, py);
+    const bool active = pixel_of(i, L.cam.width, L.cam.height, px, py) && !idle;
     uint32_t shadows = 0;
     FetchCount fc;
     // one traversal stack per warp (the tile's rays are coherent)
@@ -179,10 +195,12 @@ __global__ void __launch_bounds__(kShadowPacket ? kPacketThreads : 128, kShadowP
 
 // First-hit features of each pixel for the denoiser: albedo (or emitted
 // colour) 3, geometric normal 3, hit distance 1, as FP16; zeros on a miss.
-__global__ void __launch_bounds__(128) k_features(DevScene s, CameraConsts cam, float eps, __half *out) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(128) k_features(DevScene s, CameraConsts cam, float eps, uint32_t lanes,
+                                                  __half *out) {
+    bool idle;
+    const uint64_t i = warp_item(lanes, idle);
     uint32_t px, py;
-    const bool active = pixel_of(i, cam.width, cam.height, px, py);
+    const bool active = pixel_of(i, cam.width, cam.height, px, py) && !idle;
     const RayF r = primary_ray(cam, active ? px : 0, active ? py : 0);
     float t = FLT_MAX;
     const int pos = traverse<false>(s, r, eps, 0.f, active && s.n_refs > 0, t);
@@ -200,42 +218,48 @@ __global__ void __launch_bounds__(128) k_features(DevScene s, CameraConsts cam, 
 
 }  // namespace
 
-cudaError_t launch_features(const DevScene &s, const CameraConsts &cam, float eps, __half *out, cudaStream_t stream) {
-    const uint64_t threads = warp_tiles(cam.width, cam.height) * 32;
-    k_features<<<(unsigned)((threads + 127) / 128), 128, 0, stream>>>(s, cam, eps, out);
+namespace {
+// warps per SM that the register counts of these kernels keep resident
+constexpr uint64_t kTraceWarpsPerSm = 36, kFrameWarpsPerSm = 32;
+uint64_t resident(int sm_count, uint64_t per_sm) { return (uint64_t)(sm_count > 0 ? sm_count : 1) * per_sm; }
+}  // namespace
+
+cudaError_t launch_features(const DevScene &s, const CameraConsts &cam, float eps, __half *out, int sm_count,
+                            cudaStream_t stream) {
+    const uint64_t slots = warp_tiles(cam.width, cam.height) * 32;
+    const uint32_t lanes = lanes_for(slots, resident(sm_count, kTraceWarpsPerSm));
+    k_features<<<blocks_for(slots, lanes, 128), 128, 0, stream>>>(s, cam, eps, lanes, out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_trace_occluded(const DevScene &s, const float *rays, const float *dist2, uint64_t n, float eps,
-                                  uint8_t *occluded, cudaStream_t stream) {
+                                  uint8_t *occluded, int sm_count, cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
-    const unsigned threads = 128;
-    const uint64_t blocks = (n + threads - 1) / threads;
+    const uint32_t lanes = lanes_for(n, resident(sm_count, kTraceWarpsPerSm));
+    const unsigned blocks = blocks_for(n, lanes, 128);
     // a 32-entry stack (half the per-thread local memory) when the hierarchy is shallow enough
-    if (s.depth < 32)
-        k_trace_occluded<32><<<(unsigned)blocks, threads, 0, stream>>>(s, rays, dist2, n, eps, occluded);
-    else
-        k_trace_occluded<kStack><<<(unsigned)blocks, threads, 0, stream>>>(s, rays, dist2, n, eps, occluded);
+    if (s.depth < 32) k_trace_occluded<32><<<blocks, 128, 0, stream>>>(s, rays, dist2, n, lanes, eps, occluded);
+    else k_trace_occluded<kStack><<<blocks, 128, 0, stream>>>(s, rays, dist2, n, lanes, eps, occluded);
     return cudaGetLastError();
 }
 
 cudaError_t launch_trace_closest(const DevScene &s, const float *rays, uint64_t n, float eps, int32_t *ids,
-                                 float *ts, cudaStream_t stream) {
+                                 float *ts, int sm_count, cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
-    const unsigned threads = 128;
-    const uint64_t blocks = (n + threads - 1) / threads;
-    if (s.depth < 32)
-        k_trace_closest<32><<<(unsigned)blocks, threads, 0, stream>>>(s, rays, n, eps, ids, ts);
-    else
-        k_trace_closest<kStack><<<(unsigned)blocks, threads, 0, stream>>>(s, rays, n, eps, ids, ts);
+    const uint32_t lanes = lanes_for(n, resident(sm_count, kTraceWarpsPerSm));
+    const unsigned blocks = blocks_for(n, lanes, 128);
+    if (s.depth < 32) k_trace_closest<32><<<blocks, 128, 0, stream>>>(s, rays, n, lanes, eps, ids, ts);
+    else k_trace_closest<kStack><<<blocks, 128, 0, stream>>>(s, rays, n, lanes, eps, ids, ts);
     return cudaGetLastError();
 }
 
-cudaError_t launch_render_rt(const DevScene &s, const RtLaunch &L, cudaStream_t stream) {
-    const uint64_t tiles = warp_tiles(L.cam.width, L.cam.height);
-    const uint64_t threads = tiles * 32;
-    if (threads == 0) return cudaSuccess;
-    const unsigned bs = L.packets == 1 ? kPacketThreads : 128, grid = (unsigned)((threads + bs - 1) / bs);
+cudaError_t launch_render_rt(const DevScene &s, const RtLaunch &launch, int sm_count, cudaStream_t stream) {
+    RtLaunch L = launch;
+    const uint64_t slots = warp_tiles(L.cam.width, L.cam.height) * 32;
+    if (slots == 0) return cudaSuccess;
+    constexpr uint64_t kPacketWarpsPerSm = kPacketBlocks * kPacketThreads / 32;
+    L.lanes = lanes_for(slots, resident(sm_count, L.packets == 1 ? kPacketWarpsPerSm : kFrameWarpsPerSm));
+    const unsigned bs = L.packets == 1 ? kPacketThreads : 128, grid = blocks_for(slots, L.lanes, bs);
     // a 32-entry stack (half the per-thread local memory) when the hierarchy is shallow enough
     const bool small = s.depth < 32;
     auto go = [&](auto kernel) { kernel<<<grid, bs, 0, stream>>>(s, L); };

@@ -16,6 +16,26 @@ namespace pray_gpu {
 
 constexpr int kMaxLights = 64;
 
+// Lanes of each warp that a launch over n rays or pixels puts to work on a GPU
+// that holds `warps` warps of the kernel at once. A warp walks the union of
+// its lanes' nodes and waits for its longest ray, so a launch that is too
+// small to fill the GPU ends sooner with fewer rays in each of more warps
+// (152 SMs, us, 32 lanes against this rule: closest hits of 1,000 rays 88 to
+// 56 in a soup and 54 to 38 on a sphere, 20,000 rays 105 to 84 and 64 to 60;
+// paths of 64 x 48 pixels 651 to 321, of 160 x 120 697 to 521). The power of
+// two that still leaves half of the resident warps' places free: filling
+// them costs more than the wider union (160 x 120 paths: 613 with 4 lanes in
+// every place). kFewLanes may fill them all (40,000 rays in a room 70 to 66),
+// but 10 lanes in more places than there are do not pay (256 x 192 paths 770
+// to 795, frame of a room 73 to 87): beyond that, all 32.
+constexpr uint32_t kLeastLanes = 1, kFewLanes = 8;
+inline uint32_t lanes_for(uint64_t n, uint64_t warps) {
+    if (n > warps * kFewLanes) return 32;
+    uint32_t k = kLeastLanes;
+    while (k < kFewLanes && n > warps * k / 2) k *= 2;
+    return k;
+}
+
 struct RtLaunch {
     CameraConsts cam;
     float lights[kMaxLights][6];  // position, colour
@@ -27,6 +47,7 @@ struct RtLaunch {
     float *ts;                       // optional out: primary hit distance per pixel (FLT_MAX: miss)
     unsigned long long *counters;    // optional out (accumulated): [0] primary rays, [1] occlusion rays
     int count_fetches;               // also accumulate [2] node-pair fetches, [3] triangle fetches, [4] shaded hits
+    uint32_t lanes;                  // pixels per warp (lanes_for)
     int packets;                     // pray_traversal: warp packets (traverse_packet) for primary and occlusion
                                      // rays (1), primary rays only (2), none (0)
 };
@@ -46,6 +67,7 @@ struct PtLaunch {
     float *radiance;                 // optional out: height x width x 3 mean radiance
     double *sum64;                   // optional in/out: height x width x 3 FP64 sums, samples added in order
     unsigned long long *counters;    // optional out (accumulated): [0] paths, [1] ray segments
+    uint32_t lanes;                  // per-pixel kernel: pixels per warp at a time (lanes_for)
     unsigned long long *next_pixel;  // per-pixel kernel: work counter of the frame (zero at launch)
 };
 
@@ -92,13 +114,14 @@ uint64_t noalloc_max_pixels();
 cudaError_t launch_relmse(const double *img, double img_scale, const double *ref, double ref_scale, uint64_t n,
                           double *out, cudaStream_t stream);
 
-cudaError_t launch_features(const DevScene &s, const CameraConsts &cam, float eps, __half *out, cudaStream_t stream);
+cudaError_t launch_features(const DevScene &s, const CameraConsts &cam, float eps, __half *out, int sm_count,
+                            cudaStream_t stream);
 
 cudaError_t launch_trace_occluded(const DevScene &s, const float *rays, const float *dist2, uint64_t n, float eps,
-                                  uint8_t *occluded, cudaStream_t stream);
+                                  uint8_t *occluded, int sm_count, cudaStream_t stream);
 cudaError_t launch_trace_closest(const DevScene &s, const float *rays, uint64_t n, float eps, int32_t *ids,
-                                 float *ts, cudaStream_t stream);
+                                 float *ts, int sm_count, cudaStream_t stream);
 
-cudaError_t launch_render_rt(const DevScene &s, const RtLaunch &L, cudaStream_t stream);
+cudaError_t launch_render_rt(const DevScene &s, const RtLaunch &L, int sm_count, cudaStream_t stream);
 
 }  // namespace pray_gpu

@@ -104,6 +104,47 @@ def test_wavefront_matches_oracle_and_pixel_scheduler(oracle):
     np.testing.assert_array_equal(got[(96, 1000)], got[(96, 0)])
 
 
+@pytest.mark.parametrize("edge", [0.5, 1, 2, 8])
+@pytest.mark.parametrize("mode", [native.PT_KAJIYA, native.PT_NEE])
+def test_pixels_per_warp(oracle, mode, edge):
+    """Ragged frames just below and above the pixel counts at which the
+    per-pixel kernel changes its lanes per warp (`edge` times 32 warps per SM)."""
+    m = scenes.room(grid=3)
+    n = int(edge * 32 * torch.cuda.get_device_properties(0).multi_processor_count)
+    for h in (n // 61 - 2, n // 61 + 3):
+        st = scenes.room_setup(61, h)
+        compare(oracle, m, st, spp=2, depth=3, seed=6, mode=mode, rr=2)
+
+
+@pytest.mark.parametrize("visible_light", [False, True])
+@pytest.mark.parametrize("spp,depth", [(1, 1), (2, 1), (5, 2), (3, 0)])
+def test_camera_ray_is_shared_by_samples(oracle, spp, depth, visible_light):
+    """A pixel's camera ray is traced once for all samples of a call: first
+    hits on nothing, an emitter, a wall; paths that end at the first hit; sums
+    over calls of few samples."""
+    m = scenes.room(grid=4)
+    if visible_light:
+        m.emit[::5] = 1
+    st = scenes.room_setup(29, 19)
+    st.fov = 100
+    sc = native.Scene.from_setup(m, st)
+    for mode, sched in ((native.PT_KAJIYA, native.SCHED_PIXEL), (native.PT_NEE, native.SCHED_PIXEL),
+                        (native.PT_NEE, native.SCHED_WAVEFRONT)):
+        kw = dict(max_depth=depth, seed=21, mode=mode, rr_depth=2)
+        _, rad, cnt = sc.render_pt_host(native.pt_params(st, spp=spp, scheduler=sched, **kw))
+        orc = oracle.OracleScene.from_setup(m, st)
+        _, orad, osegs = orc.render_pt(st, spp=spp, **kw)
+        np.testing.assert_allclose(rad, orad, rtol=RTOL, atol=ATOL)
+        assert (int(cnt[0]), int(cnt[1])) == (29 * 19 * spp, osegs)
+        acc = torch.zeros((19, 29, 3), dtype=torch.float64, device="cuda")
+        for off, k in ((0, spp), (spp, 1), (spp + 1, 2)):
+            sc.accumulate_pt(native.pt_params(st, spp=k, scheduler=sched, sample_offset=off, **kw), acc)
+        torch.cuda.synchronize()
+        want = np.zeros((19, 29, 3), np.float64)
+        orc.render_pt(st, spp=spp + 3, sum64=want, **kw)
+        np.testing.assert_array_equal(acc.cpu().numpy(), want)
+
+
 def test_wavefront_rejects_kajiya_mode():
     m = scenes.room(grid=4)
     st = scenes.room_setup(8, 8)

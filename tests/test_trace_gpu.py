@@ -463,3 +463,51 @@ def test_culling_hierarchy_matches_reference_walk(oracle, name, tree):
         occ = torch.empty(len(rays), dtype=torch.uint8, device="cuda")
         sc.trace_occluded(torch.from_numpy(rays).cuda(), torch.from_numpy(d2).cuda(), st.det_eps, occ)
         np.testing.assert_array_equal(occ.cpu().numpy(), want_occ.astype(np.uint8))
+
+
+def _edges(warps_per_sm):
+    """Item counts at which a launch over few rays or pixels changes its lanes
+    per warp: half of the resident warps times 1, 2, 4; all of them times 8."""
+    w = torch.cuda.get_device_properties(0).multi_processor_count * warps_per_sm
+    return [w // 2, w, 2 * w, 8 * w]
+
+
+@pytest.mark.parametrize("edge", [-1, 0, 1, 2, 3])
+def test_rays_per_warp(oracle, edge):
+    """Closest hits and occlusion of ray counts on both sides of each edge (and
+    of 1, 3, 33 rays): every ray is answered, none beyond the last is written."""
+    m, st = scenes.soup(2_000, 8), scenes.soup_setup()
+    sc = native.Scene.from_setup(m, st)
+    orc = oracle.OracleScene.from_setup(m, st)
+    counts = [1, 3, 33] if edge < 0 else [_edges(36)[edge] + k for k in (-1, 0, 1)]
+    rng = np.random.default_rng(edge + 9)
+    n = max(counts)
+    o = rng.uniform(-0.2, 1.2, (n, 3)).astype(np.float32)
+    d = rng.normal(size=(n, 3)).astype(np.float32)
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    rays = np.concatenate([o, d, (1.0 / d).astype(np.float32)], 1)
+    wid, wt = orc.trace(rays, 1e-4)
+    d2 = rng.uniform(0.0, 1.0, n).astype(np.float32)
+    want = (wid >= 0) & (d2 > (wt * wt).astype(np.float32))
+    r, dd = torch.from_numpy(rays).cuda(), torch.from_numpy(d2).cuda()
+    for k in counts:
+        ids = torch.full((n + 40,), -7, dtype=torch.int32, device="cuda")
+        ts = torch.full((n + 40,), -7.0, dtype=torch.float32, device="cuda")
+        occ = torch.full((n + 40,), 9, dtype=torch.uint8, device="cuda")
+        sc.trace_closest(r[:k], 1e-4, ids[:k], ts[:k])
+        sc.trace_occluded(r[:k], dd[:k], 1e-4, occ[:k])
+        torch.cuda.synchronize()
+        assert (ids[k:] == -7).all() and (ts[k:] == -7).all() and (occ[k:] == 9).all()
+        np.testing.assert_array_equal(ids[:k].cpu().numpy(), wid[:k].astype(np.int32))
+        np.testing.assert_array_equal(ts[:k].cpu().numpy().view(np.uint32), wt[:k].view(np.uint32))
+        np.testing.assert_array_equal(occ[:k].cpu().numpy(), want[:k].astype(np.uint8))
+
+
+@pytest.mark.parametrize("traversal", [native.TRAVERSAL_LANES, native.TRAVERSAL_PACKETS,
+                                       native.TRAVERSAL_PRIMARY_PACKETS])
+@pytest.mark.parametrize("warps", [32, 40])
+def test_pixels_per_warp(oracle, traversal, warps):
+    """Frames of ragged sizes on both sides of each edge."""
+    m = scenes.soup(2_000, 9)
+    for w, h in [(1, 1), (9, 5)] + [(97, e // 97 + k) for e in _edges(warps) for k in (-2, 3)]:
+        check_frame(oracle, m, scenes.soup_setup(w, h), traversal)
