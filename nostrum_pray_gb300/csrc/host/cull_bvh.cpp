@@ -16,14 +16,19 @@ constexpr int kBins = 16;
 constexpr double kVisit = 1.5, kTest = 1.0;
 constexpr size_t kParallel = 1024;  // subtrees from this size on may get a thread of their own
 
+// x, y, z and an unused lane: one vector register on either host
+typedef float V4 __attribute__((vector_size(16)));
+typedef int I4 __attribute__((vector_size(16)));
+inline V4 vmin(V4 a, V4 b) { return a < b ? a : b; }
+inline V4 vmax(V4 a, V4 b) { return a > b ? a : b; }
+
 struct Box {
-    float lo[3], hi[3];
+    V4 lo, hi;
     void clear() {
-        for (int k = 0; k < 3; k++) lo[k] = INFINITY, hi[k] = -INFINITY;
+        lo = V4{INFINITY, INFINITY, INFINITY, INFINITY};
+        hi = -lo;
     }
-    void add(const Box &b) {
-        for (int k = 0; k < 3; k++) lo[k] = std::min(lo[k], b.lo[k]), hi[k] = std::max(hi[k], b.hi[k]);
-    }
+    void add(const Box &b) { lo = vmin(lo, b.lo), hi = vmax(hi, b.hi); }
     double half_area() const {
         const double x = (double)hi[0] - lo[0], y = (double)hi[1] - lo[1], z = (double)hi[2] - lo[2];
         return x * y + y * z + z * x;
@@ -32,8 +37,9 @@ struct Box {
 
 struct Prim {
     Box box;
-    float c[3];  // twice the centre; 0 where the bounds are not finite (such
-                 // triangles still get a box that every ray enters)
+    // twice the centre; 0 where the bounds are not finite (such triangles
+    // still get a box that every ray enters)
+    V4 c;
     uint32_t id;
 };
 
@@ -61,56 +67,57 @@ struct Builder {
         for (size_t i = lo; i < hi; i++) {
             const Prim &p = prims[i];
             bounds.add(p.box);
-            for (int k = 0; k < 3; k++) {
-                const float c = p.c[k];
-                centres.lo[k] = std::min(centres.lo[k], c), centres.hi[k] = std::max(centres.hi[k], c);
-            }
+            centres.lo = vmin(centres.lo, p.c), centres.hi = vmax(centres.hi, p.c);
         }
         node.box = bounds;
         node.pair = 0, node.lo = (uint32_t)lo, node.count = (uint32_t)n;
         if (n <= 1) return;
         int best_axis = -1, best_bin = 0;
         double best = INFINITY;
-        float scale[3];
+        V4 scale = {0.f, 0.f, 0.f, 0.f};
         for (int k = 0; k < 3; k++) {
             const float e = centres.hi[k] - centres.lo[k];
             scale[k] = e > 0.f && std::isfinite(e) ? kBins * 0.9999f / e : 0.f;
         }
-        auto bin_of = [&](const Prim &p, int k) {
-            const int b = (int)((p.c[k] - centres.lo[k]) * scale[k]);
-            return b < 0 ? 0 : (b >= kBins ? kBins - 1 : b);
-        };
+        const V4 from = centres.lo, last = V4{1.f, 1.f, 1.f, 1.f} * (float)(kBins - 1);
+        auto bins_of = [&](const Prim &p) { return __builtin_convertvector(vmin((p.c - from) * scale, last), I4); };
         const bool halve = depth + levels(n, leaf_max) >= kCullDepth;
         if (!halve) {
+            // bins without a triangle are skipped: they change no box and no cost
             Box box[3][kBins];
-            uint32_t count[3][kBins] = {};
-            for (auto &axis : box)
-                for (Box &b : axis) b.clear();
-            for (size_t i = lo; i < hi; i++)
+            uint32_t count[3][kBins], used[3] = {0, 0, 0};
+            for (size_t i = lo; i < hi; i++) {
+                const Prim &p = prims[i];
+                const I4 at = bins_of(p);
                 for (int k = 0; k < 3; k++) {
-                    const int b = bin_of(prims[i], k);
-                    box[k][b].add(prims[i].box);
-                    count[k][b]++;
+                    const int b = at[k];
+                    if (used[k] >> b & 1u) {
+                        box[k][b].add(p.box);
+                        count[k][b]++;
+                    } else {
+                        used[k] |= 1u << b;
+                        box[k][b] = p.box;
+                        count[k][b] = 1;
+                    }
                 }
+            }
             for (int k = 0; k < 3; k++) {
-                if (scale[k] == 0.f) continue;
+                int bins[kBins], m = 0;
+                for (uint32_t u = used[k]; u; u &= u - 1) bins[m++] = __builtin_ctz(u);
+                if (m < 2 || scale[k] == 0.f) continue;
                 double right[kBins];
-                uint32_t right_n[kBins], c = 0;
-                Box acc;
-                acc.clear();
-                for (int b = kBins - 1; b > 0; b--) {
-                    acc.add(box[k][b]);
-                    c += count[k][b];
-                    right[b] = c ? acc.half_area() : 0.0, right_n[b] = c;
+                Box acc = box[k][bins[m - 1]];
+                for (int q = m - 1; q > 0; q--) {
+                    if (q < m - 1) acc.add(box[k][bins[q]]);
+                    right[q] = acc.half_area();
                 }
-                acc.clear();
-                c = 0;
-                for (int b = 0; b + 1 < kBins; b++) {
-                    acc.add(box[k][b]);
-                    c += count[k][b];
-                    if (!c || !right_n[b + 1]) continue;
-                    const double cost = acc.half_area() * c + right[b + 1] * right_n[b + 1];
-                    if (cost < best) best = cost, best_axis = k, best_bin = b;
+                acc = box[k][bins[0]];
+                uint32_t c = 0;
+                for (int q = 0; q + 1 < m; q++) {
+                    if (q) acc.add(box[k][bins[q]]);
+                    c += count[k][bins[q]];
+                    const double cost = acc.half_area() * c + right[q + 1] * (double)(n - c);
+                    if (cost < best) best = cost, best_axis = k, best_bin = bins[q];
                 }
             }
         }
@@ -121,7 +128,7 @@ struct Builder {
         size_t mid = lo + n / 2;
         if (best_axis >= 0) {
             mid = std::partition(prims.begin() + lo, prims.begin() + hi,
-                                 [&](const Prim &p) { return bin_of(p, best_axis) <= best_bin; }) -
+                                 [&](const Prim &p) { return bins_of(p)[best_axis] <= best_bin; }) -
                   prims.begin();
         } else {
             // equal centres, or no levels to spare: halves along the longest axis
