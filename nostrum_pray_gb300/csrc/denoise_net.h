@@ -84,7 +84,7 @@ class Denoiser {
     std::vector<dn::TcConvPlan> plans_;
     int sm_count_ = 0;
     // tensor-core backward: per convolution the transposed, tap-mirrored packed
-    // weights (dn::tc_pack_weights_bwd), its output gradient (BF16, masked,
+    // weights, its output gradient (BF16, masked,
     // planar), a backward-data and a weight-gradient plan over it and the
     // per-CTA sums of its bias gradient; per encoder level the skip
     // connection's share of the gradient (FP32, planar)

@@ -18,7 +18,7 @@ namespace dn {
 // 8-channel chunks: [image][channel / 8][y][x][8] (the CUDA-core kernels'
 // tensors are channels last). A plan holds the input's TMA tensor map (the
 // input buffer is fixed) and the launch shape; Cin must be a multiple of 16
-// (pack_input pads the network input), the weights packed by tc_pack_weights
+// (pack_input pads the network input), the weights packed by tc_pack_all
 // (cin_pad = Cin of the plan). *err is set to 1 if one of the kernel's bounded
 // mbarrier waits ran out.
 struct TcConvPlan {
@@ -37,18 +37,14 @@ struct TcConvPlan {
 cudaError_t tc_conv_plan(TcConvPlan &p, const __nv_bfloat16 *x, int n, int h, int w, int cin, int cout, bool relu,
                          int sm_count, bool grad = false);
 size_t tc_packed_weight_elems(int cin_pad, int cout);
-cudaError_t tc_pack_weights(const float *w, __nv_bfloat16 *packed, int cin, int cin_pad, int cout, cudaStream_t st);
-// Weights of the backward-data convolution of a forward convolution with
-// cin_f inputs and cout_f outputs (w[cout_f][9][cin_f]): a plan with
-// cin = cout_f rounded up to 16 and cout = cin_f runs it on the output
-// gradient (BF16, planar) and writes the input gradient.
-cudaError_t tc_pack_weights_bwd(const float *w, __nv_bfloat16 *packed, int cin_f, int cout_f, cudaStream_t st);
 // Every packing of a network's weights in one launch: job j packs w (the
-// FP32 [cout_f][9][cin_f] weights of one convolution) into out, as
-// tc_pack_weights (bwd 0: cin_pad = cin_f rounded up to 16, npad = cout_f
-// rounded up) or tc_pack_weights_bwd (bwd 1: cin_pad = cout_f rounded up,
-// npad = cin_f rounded up) does; its 9 x cin_pad x npad elements start at
-// `begin` of the concatenated range, jobs in increasing begin (at most 64).
+// FP32 [cout_f][9][cin_f] weights of one convolution) into out, for the
+// forward convolution (bwd 0: cin_pad = cin_f rounded up to 16, npad = cout_f
+// rounded up) or for its backward-data convolution (bwd 1: cin_pad = cout_f
+// rounded up, npad = cin_f rounded up): a plan with cin = cout_f rounded up to
+// 16 and cout = cin_f that runs on the output gradient (BF16, planar) and
+// gives the input gradient. Its 9 x cin_pad x npad elements start at `begin`
+// of the concatenated range, jobs in increasing begin (at most 64).
 struct TcPackJob {
     const float *w;
     __nv_bfloat16 *out;

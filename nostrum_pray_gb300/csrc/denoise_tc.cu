@@ -18,7 +18,7 @@
 // groups (stride 160 bytes = one halo row), the two 8-channel chunks are the
 // K-direction core matrices (stride = one plane), and the start address moves
 // by (dy * 10 + dx) * 16 bytes. So all nine taps read the same halo and the
-// threads gather nothing. The weights are packed once (tc_pack_weights) as
+// threads gather nothing. The weights are packed once (tc_pack_all) as
 // [tap][8-channel chunk][row][8] BF16 - exactly the no-swizzle K-major
 // core-matrix layout - and a CTA copies the rows of its channels tap by tap.
 // One thread issues the kind::f16 MMAs (M 128, N Npad, K 16) and commits them
@@ -1085,43 +1085,11 @@ __global__ void __launch_bounds__(256) k_grad_finish(const __grid_constant__ Fin
     }
 }
 
-// out[tap][chunk][row][8] from w[cout][9][cin] (zero rows and channels pad).
-__global__ void k_pack_weights(const float *w, __nv_bfloat16 *out, int cin, int cin_pad, int cout, int npad) {
-    const int nchunk = cin_pad >> 3;
-    const size_t total = (size_t)9 * cin_pad * npad;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int e = (int)(i & 7);
-        const size_t rowi = i >> 3;
-        const int r = (int)(rowi % npad);
-        const size_t ct = rowi / npad;
-        const int chunk = (int)(ct % nchunk), tap = (int)(ct / nchunk);
-        const int ci = chunk * 8 + e;
-        const float v = (r < cout && ci < cin) ? w[((size_t)r * 9 + tap) * cin + ci] : 0.f;
-        out[i] = __float2bfloat16(v);
-    }
-}
-
-// The backward-data convolution's weights, packed like k_pack_weights: the
+// Forward weights: out[tap][chunk][row][8] from w[cout][9][cin] (zero rows and
+// channels pad). The backward-data convolution's (bwd), in the same order: the
 // input gradient of a 3x3 convolution is a 3x3 convolution of the output
-// gradient (cout_f channels, padded to cin_pad) with the weights transposed
-// (output channel ci, input channel co) and the taps mirrored (tap 8 - t):
-// out[tap][chunk][ci][8] = w[co][8 - tap][ci], w[cout_f][9][cin_f].
-__global__ void k_pack_weights_bwd(const float *w, __nv_bfloat16 *out, int cin_f, int cout_f, int cin_pad,
-                                   int npad) {
-    const int nchunk = cin_pad >> 3;
-    const size_t total = (size_t)9 * cin_pad * npad;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int e = (int)(i & 7);
-        const size_t rowi = i >> 3;
-        const int r = (int)(rowi % npad);  // ci
-        const size_t ct = rowi / npad;
-        const int chunk = (int)(ct % nchunk), tap = (int)(ct / nchunk);
-        const int co = chunk * 8 + e;
-        const float v = (r < cin_f && co < cout_f) ? w[((size_t)co * 9 + (8 - tap)) * cin_f + r] : 0.f;
-        out[i] = __float2bfloat16(v);
-    }
-}
-
+// gradient with the weights transposed (output channel ci, input channel co)
+// and the taps mirrored: out[tap][chunk][ci][8] = w[co][8 - tap][ci].
 __global__ void k_pack_all(const TcPackJob *jobs, int njobs, size_t total) {
     __shared__ TcPackJob sj[64];
     for (int i = (int)threadIdx.x; i < njobs; i += (int)blockDim.x) sj[i] = jobs[i];
@@ -1190,23 +1158,9 @@ cudaError_t tile_map(void *out, const __nv_bfloat16 *x, int n, int h, int w, int
 
 size_t tc_packed_weight_elems(int cin_pad, int cout) { return (size_t)9 * cin_pad * ((cout + 15) / 16 * 16); }
 
-cudaError_t tc_pack_weights(const float *w, __nv_bfloat16 *packed, int cin, int cin_pad, int cout, cudaStream_t st) {
-    const int npad = (cout + 15) / 16 * 16;
-    k_pack_weights<<<grid_for(tc_packed_weight_elems(cin_pad, cout)), 256, 0, st>>>(w, packed, cin, cin_pad, cout,
-                                                                                   npad);
-    return cudaGetLastError();
-}
-
 cudaError_t tc_pack_all(const TcPackJob *jobs_dev, int njobs, size_t total, cudaStream_t st) {
     if (njobs <= 0 || njobs > 64) return cudaErrorInvalidValue;
     k_pack_all<<<grid_for(total), 256, 0, st>>>(jobs_dev, njobs, total);
-    return cudaGetLastError();
-}
-
-cudaError_t tc_pack_weights_bwd(const float *w, __nv_bfloat16 *packed, int cin_f, int cout_f, cudaStream_t st) {
-    const int cin_pad = (cout_f + 15) / 16 * 16, npad = (cin_f + 15) / 16 * 16;
-    k_pack_weights_bwd<<<grid_for(tc_packed_weight_elems(cin_pad, cin_f)), 256, 0, st>>>(w, packed, cin_f, cout_f,
-                                                                                        cin_pad, npad);
     return cudaGetLastError();
 }
 

@@ -215,10 +215,8 @@ struct FetchCount {
 // Closest hit: best = index of the winning triangle record or -1, its
 // distance in best_t. Any hit: best >= 0 once a triangle with t > 0 and
 // t * t < d2 is found (the occlusion test of src/pray.cpp:42). A traversal
-// looks for one or the other for the whole warp (kClosest, kAnyHit), or per
-// lane as Trav::any says (kPerLane: a warp mixing extension and occlusion
-// rays).
-enum TravMode { kClosest = 0, kAnyHit = 1, kPerLane = 2 };
+// looks for one or the other for the whole warp.
+enum TravMode { kClosest = 0, kAnyHit = 1 };
 
 struct Trav {
     // the current node and the postponed leaf, one word each: an interior
@@ -230,7 +228,7 @@ struct Trav {
     float nox, noy, noz;  // culling copy: -origin / direction (slab_fma)
     int best, sp;
     uint32_t best_key;
-    bool have_node, have_leaf, finite, any;
+    bool have_node, have_leaf, finite;
     __device__ __forceinline__ bool active() const { return have_node || have_leaf; }
     __device__ __forceinline__ bool on_leaf() const { return have_node && (w & kLeafFlag); }
 };
@@ -270,15 +268,12 @@ __device__ __forceinline__ void leaf_range(const DevScene &s, uint32_t node_off,
     }
 }
 
-// `any` (kPerLane only): this lane's ray looks for any occluder.
 template <int kMode>
-__device__ __forceinline__ void trav_start(const DevScene &s, const RayF &r, float d2, bool valid, Trav &T,
-                                           bool any = false) {
-    T.any = kMode == kAnyHit || (kMode == kPerLane && any);
+__device__ __forceinline__ void trav_start(const DevScene &s, const RayF &r, float d2, bool valid, Trav &T) {
     T.best_t = FLT_MAX;
     T.best = -1;
     T.best_key = 0xFFFFFFFFu;
-    T.limit = T.any ? sqrtf(d2) * kPruneRel : FLT_MAX;
+    T.limit = kMode == kAnyHit ? sqrtf(d2) * kPruneRel : FLT_MAX;
     T.back = -s.tol;
     T.w = T.lw = 0;
     T.cur_tn = T.leaf_tn = 0.f;
@@ -307,7 +302,6 @@ __device__ __forceinline__ void trav_round(const DevScene &s, const RayF &r, flo
                                            TravStack<kStackN> &S, FetchCount *fc) {
     static_assert(kStackN >= 2 && kStackN <= kStack, "stack entries");
     constexpr unsigned kFull = 0xFFFFFFFFu;
-    const bool any_hit = kMode == kAnyHit || (kMode == kPerLane && T.any);
     // 1. interior nodes, until every lane has found a leaf
     while (true) {
         const bool interior = T.have_node && !(T.w & kLeafFlag);
@@ -376,7 +370,7 @@ __device__ __forceinline__ void trav_round(const DevScene &s, const RayF &r, flo
                     float t;
                     if (intersect_tri(v0, e1, e2, r, eps, t) && t > 0) {
                         uint32_t key;
-                        if (any_hit) {
+                        if (kMode == kAnyHit) {
                             if (d2 > t * t && owned(s, r, e1.w, e2.w, key)) {
                                 T.best = (int)i;
                                 T.have_node = T.have_leaf = false;

@@ -79,7 +79,9 @@ def forward_bytes(h: int, w: int, n: int = 1) -> int:
     output), the second convolutions of levels 4-1 their output upsampled
     into the next concatenation (4 pixels each), the output convolution the
     log-space and the final radiance (FP32) after reading 3 channels of the
-    input and the albedo; the others their output."""
+    input and the albedo; the others their output. (Inference does not store
+    the log-space radiance: its 12 bytes per pixel, 1 % of the sum, are counted
+    all the same.)"""
     px0 = n * h * w
     total = px0 * (12 + 14 + 32)
     for i, (ci, co, l) in enumerate(CONVS):
@@ -99,16 +101,14 @@ def forward_bytes(h: int, w: int, n: int = 1) -> int:
 
 
 def denoise_launches(h: int, w: int, n: int = 1, sm_count: int = 152, tensor_cores: bool = True) -> int:
-    """Kernels one pray_denoise call launches. On the CUDA cores: input
-    packing, 4 poolings, 4 upsample-concatenations, the 19 convolutions, the
-    residual add and the output transform. On the tensor cores the poolings,
-    concatenations, residual and output transform are stores of the
-    convolutions' epilogues: input packing and the 19 convolutions. There a
-    convolution with fewer than two 16x8-pixel tiles per SM splits its output
-    channels over CTAs, or, with a single 16-channel chunk, its taps, which
-    adds a finalize kernel (the rule of tc_conv_plan in
-    csrc/denoise_tc.cu); the output convolution split so keeps the residual
-    and output kernels."""
+    """Kernels one pray_denoise call launches, at most. On the CUDA cores:
+    input packing, 4 poolings, 4 upsample-concatenations, the 19 convolutions,
+    the residual add and the output transform. On the tensor cores the
+    poolings, concatenations, residual and output transform are stores of the
+    convolutions' epilogues: input packing and the 19 convolutions, 20 launches
+    at every size. The bound is larger where the output convolution has fewer
+    than two 16x8-pixel tiles per SM (it allows that one a finalize kernel and
+    separate residual and output kernels)."""
     convs, split = 0, False
     for _, co, l in CONVS:
         tiles = n * -(-(w >> l) // 8) * -(-(h >> l) // 16)
