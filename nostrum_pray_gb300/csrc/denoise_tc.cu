@@ -1090,34 +1090,40 @@ __global__ void __launch_bounds__(256) k_grad_finish(const __grid_constant__ Fin
 // input gradient of a 3x3 convolution is a 3x3 convolution of the output
 // gradient with the weights transposed (output channel ci, input channel co)
 // and the taps mirrored: out[tap][chunk][ci][8] = w[co][8 - tap][ci].
-__global__ void k_pack_all(const TcPackJob *jobs, int njobs, size_t total) {
+// A thread packs one row of 8 channels (16 bytes) with 32-bit index
+// arithmetic. Bound by latency (12 MB at 1,016,419 weights, both ways): one
+// element per thread with 64-bit divisions took 22.7 us, this 10.6 us.
+__global__ void __launch_bounds__(256) k_pack_all(const TcPackJob *jobs, int njobs, uint32_t rows) {
     __shared__ TcPackJob sj[64];
     for (int i = (int)threadIdx.x; i < njobs; i += (int)blockDim.x) sj[i] = jobs[i];
     __syncthreads();
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        int j = 0;
-        while (j + 1 < njobs && sj[j + 1].begin <= i) j++;
-        const TcPackJob &J = sj[j];
-        const size_t li = i - J.begin;
-        const int e = (int)(li & 7);
-        const size_t rowi = li >> 3;
-        const int r = (int)(rowi % J.npad);
-        const size_t ct = rowi / J.npad;
-        const int nchunk = J.cin_pad >> 3;
-        const int chunk = (int)(ct % nchunk), tap = (int)(ct / nchunk);
-        const int c = chunk * 8 + e;
-        float v;
-        if (!J.bwd)  // row r = output channel, c = input channel
-            v = (r < J.cout_f && c < J.cin_f) ? J.w[((size_t)r * 9 + tap) * J.cin_f + c] : 0.f;
-        else  // transposed, taps mirrored: row r = input channel, c = output channel
-            v = (r < J.cin_f && c < J.cout_f) ? J.w[((size_t)c * 9 + (8 - tap)) * J.cin_f + r] : 0.f;
-        J.out[li] = __float2bfloat16(v);
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= rows) return;
+    int lo = 0, hi = njobs - 1;  // the last job that begins at or before row i
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if ((uint32_t)(sj[mid].begin / 8) <= i) lo = mid;
+        else hi = mid - 1;
     }
-}
-
-unsigned grid_for(size_t n) {
-    const size_t b = (n + 255) / 256;
-    return (unsigned)(b < 4096 ? (b ? b : 1) : 4096);
+    const TcPackJob &J = sj[lo];
+    const uint32_t row = i - (uint32_t)(J.begin / 8), npad = (uint32_t)J.npad, nchunk = (uint32_t)J.cin_pad / 8;
+    const uint32_t ct = row / npad, tap = ct / nchunk;
+    const int r = (int)(row - ct * npad), c0 = (int)(ct - tap * nchunk) * 8;
+    __nv_bfloat162 v[4];
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+        const int c = c0 + e;
+        float f;
+        if (!J.bwd)  // row r = output channel, c = input channel
+            f = (r < J.cout_f && c < J.cin_f) ? J.w[((size_t)r * 9 + tap) * J.cin_f + c] : 0.f;
+        else  // transposed, taps mirrored: row r = input channel, c = output channel
+            f = (r < J.cin_f && c < J.cout_f) ? J.w[((size_t)c * 9 + (8 - tap)) * J.cin_f + r] : 0.f;
+        if (e & 1) v[e >> 1].y = __float2bfloat16(f);
+        else v[e >> 1].x = __float2bfloat16(f);
+    }
+    uint4 q;
+    memcpy(&q, v, 16);
+    *reinterpret_cast<uint4 *>(J.out + (size_t)row * 8) = q;
 }
 
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -1159,8 +1165,9 @@ cudaError_t tile_map(void *out, const __nv_bfloat16 *x, int n, int h, int w, int
 size_t tc_packed_weight_elems(int cin_pad, int cout) { return (size_t)9 * cin_pad * ((cout + 15) / 16 * 16); }
 
 cudaError_t tc_pack_all(const TcPackJob *jobs_dev, int njobs, size_t total, cudaStream_t st) {
-    if (njobs <= 0 || njobs > 64) return cudaErrorInvalidValue;
-    k_pack_all<<<grid_for(total), 256, 0, st>>>(jobs_dev, njobs, total);
+    if (njobs <= 0 || njobs > 64 || total % 8 || total / 8 > 0xFFFFFFFFull - 255) return cudaErrorInvalidValue;
+    const uint32_t rows = (uint32_t)(total / 8);
+    k_pack_all<<<(rows + 255) / 256, 256, 0, st>>>(jobs_dev, njobs, rows);
     return cudaGetLastError();
 }
 
