@@ -105,6 +105,8 @@ struct pray_scene {
     int device_depth = 0;  // deepest node of the device hierarchy
     float tol = 0.f;
     float cull_c[3] = {0.f, 0.f, 0.f}, cull_r2 = -1.f;
+    uint32_t grid_base = 0;
+    float grid_org[3] = {0.f, 0.f, 0.f}, grid_scale = 1.f;
     std::atomic<int> rt_packets{PRAY_TRAVERSAL_AUTO};  // pray_traversal of the ray-traced frames
     uint64_t device_bytes = 0;
     // wavefront path tracer: scratch (path pool, queues), private stream,
@@ -146,6 +148,9 @@ struct pray_scene {
         v.depth = (uint32_t)device_depth;
         for (int k = 0; k < 3; k++) v.cull_c[k] = cull_c[k];
         v.cull_r2 = cull_r2;
+        v.grid_base = grid_base;
+        for (int k = 0; k < 3; k++) v.grid_org[k] = grid_org[k];
+        v.grid_scale = grid_scale;
         v.emit_tris = d_emit;
         v.emit_cdf = d_emit_cdf;
         v.n_emit = n_emit;
@@ -555,11 +560,27 @@ pray_status pray_scene_create(const float *verts, const float *colors, const uin
             return set_error(PRAY_ERR_UNSUPPORTED, "device layout: " + bad);
         gnodes.swap(img.nodes);
         s->n_gnodes = (uint32_t)gnodes.size();
-        for (GNode g : img.cull) {  // both copies, one buffer
-            if ((g.b & kLeafFlag) && (g.b & ~kLeafFlag))
-                g.a |= kLeafFlag | ((g.b & ~kLeafFlag) - 1) << kCullCountShift;
+        // both copies and the grid pairs, one buffer
+        const auto leaf_word = [](const GNode &g) {
+            const uint32_t n = g.b & ~kLeafFlag;
+            return n ? g.a | kLeafFlag | (n - 1) << kCullCountShift : g.a;
+        };
+        GridImage grid;
+        if (!img.cull.empty() && !grid_for_device(img.cull, leaf_word, grid) && img.cull.size() > 2)
+            img.cull.clear(), img.cull_radius2 = -1.f;
+        gnodes.reserve(gnodes.size() + img.cull.size() + grid.pairs.size());
+        for (GNode g : img.cull) {
+            if (g.b & kLeafFlag) g.a = leaf_word(g);
             gnodes.push_back(g);
         }
+        s->grid_base = (uint32_t)gnodes.size();
+        s->grid_scale = grid.scale;
+        for (int k = 0; k < 3; k++) s->grid_org[k] = grid.org[k];
+        static_assert(sizeof(GPair) == sizeof(GNode), "pairs share the nodes' buffer");
+        gnodes.resize(gnodes.size() + grid.pairs.size());
+        if (!grid.pairs.empty())
+            std::memcpy(static_cast<void *>(gnodes.data() + s->grid_base), grid.pairs.data(),
+                        grid.pairs.size() * sizeof(GPair));
         gowners.swap(img.owners);
         for (int k = 0; k < 3; k++) s->cull_c[k] = img.cull_center[k];
         s->cull_r2 = img.cull_radius2;

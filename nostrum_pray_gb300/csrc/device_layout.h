@@ -60,10 +60,20 @@ struct alignas(16) GShade {
     float c[4];
 };
 
+// The two children of an interior node of the culling copy with their boxes on
+// a scene-wide grid of 16-bit steps: planes x0 y0 z0 x1 y1 z1 (box min, max),
+// two per word, low half first. The per-lane walks read these, half the bytes
+// of two GNodes. Words as in the culling copy, but an interior child's is the
+// index of its own pair.
+struct alignas(32) GPair {
+    uint32_t q0[3], w0, q1[3], w1;
+};
+
 // Launch-time view of a device scene.
 struct DevScene {
     const GNode *nodes;  // n_nodes nodes of the exact copy (the reference's tree), then the culling copy
-                         // (for finite-direction rays whose origin is within cull_r2 of cull_c)
+                         // (for finite-direction rays whose origin is within cull_r2 of cull_c), then, from
+                         // grid_base on, its child pairs on the grid (GPair)
     const GTri *tris;
     const GOwner *owners;
     const GShade *shade;
@@ -71,6 +81,8 @@ struct DevScene {
     float tol;  // absolute distance tolerance for culling boxes behind the origin
     uint32_t depth;  // deepest node level of the hierarchy (root 0): a traversal pushes at most this many nodes
     float cull_c[3], cull_r2;  // centre and squared radius of the region of origins served by the culling copy
+    uint32_t grid_base;
+    float grid_org[3], grid_scale;  // grid origin, 1 / cell (a power of two)
     // emitting triangles (for next-event estimation): geometry as GTri (v0.w
     // = triangle id) and the inclusive prefix sums of their areas
     const GTri *emit_tris;

@@ -154,6 +154,55 @@ void flatten_for_device(const BuiltTree &t, const std::vector<TriPre> &pre, cons
     }
 }
 
+bool grid_for_device(const std::vector<GNode> &cull, uint32_t (*leaf_word)(const GNode &), GridImage &out) {
+    out = GridImage{};
+    if (cull.size() < 4) return false;  // no interior node
+    double lo[3], hi[3], ext = 0.0;
+    for (int k = 0; k < 3; k++) lo[k] = cull[0].lo[k], hi[k] = cull[0].hi[k];
+    for (size_t i = 2; i < cull.size(); i++)
+        for (int k = 0; k < 3; k++)
+            lo[k] = std::min(lo[k], (double)cull[i].lo[k]), hi[k] = std::max(hi[k], (double)cull[i].hi[k]);
+    for (int k = 0; k < 3; k++) {
+        if (!std::isfinite(lo[k]) || !std::isfinite(hi[k])) return false;
+        ext = std::max(ext, hi[k] - lo[k]);
+    }
+    // the smallest power-of-two cell whose 65,536 steps hold every box and two
+    // cells around it from a float origin
+    int e = 0;
+    std::frexp(ext / 65528.0, &e);
+    if (!(ext > 0.0)) return false;
+    for (;; e++) {
+        if (e < -90 || e > 90) return false;
+        const double cell = std::ldexp(1.0, e);
+        bool fits = true;
+        for (int k = 0; k < 3; k++) {
+            float o = (float)(lo[k] - 3.0 * cell);
+            if ((double)o > lo[k] - 3.0 * cell) o = std::nextafter(o, -INFINITY);
+            out.org[k] = o;
+            fits = fits && (hi[k] - o) / cell <= 65532.0;
+        }
+        if (fits) break;
+    }
+    const double scale = std::ldexp(1.0, -e);
+    out.scale = (float)scale;
+    out.pairs.resize(cull.size() / 2);
+    for (size_t p = 1; p < out.pairs.size(); p++) {
+        GPair &g = out.pairs[p];
+        for (int c = 0; c < 2; c++) {
+            const GNode &n = cull[2 * p + c];
+            uint32_t q[6];
+            for (int k = 0; k < 3; k++) {
+                q[k] = (uint32_t)(std::floor(((double)n.lo[k] - out.org[k]) * scale) - 1.0);
+                q[3 + k] = (uint32_t)(std::ceil(((double)n.hi[k] - out.org[k]) * scale) + 1.0);
+            }
+            uint32_t *w = c ? g.q1 : g.q0;
+            for (int k = 0; k < 3; k++) w[k] = q[2 * k] | q[2 * k + 1] << 16;
+            (c ? g.w1 : g.w0) = (n.b & kLeafFlag) ? leaf_word(n) : n.a / 2;
+        }
+    }
+    return true;
+}
+
 namespace {
 
 // nodes' leaves hold triangle records [begin, end).

@@ -47,6 +47,17 @@ struct DeviceImage {
     std::vector<GOwner> owners; // owner lists of triangles with more than one
 };
 
+// The child pairs of a culling copy on a 16-bit grid (GPair; pair p holds nodes
+// 2p and 2p + 1; pair 0 is unused). Every box is rounded outwards by one to
+// two cells: one cell more than the grid needs, for the rounding of the
+// distances that the kernels compute from grid steps (slab_grid). leaf_word:
+// the device's word of a leaf node. False: the boxes do not fit a grid.
+struct GridImage {
+    std::vector<GPair> pairs;
+    float org[3] = {0.f, 0.f, 0.f}, scale = 1.f;
+};
+bool grid_for_device(const std::vector<GNode> &cull, uint32_t (*leaf_word)(const GNode &), GridImage &out);
+
 // bvh: the hierarchy of the culling copy (build_cull_bvh over pre); NULL: none.
 void flatten_for_device(const BuiltTree &t, const std::vector<TriPre> &pre, const CullBvh *bvh, DeviceImage &out);
 

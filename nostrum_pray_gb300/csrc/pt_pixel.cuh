@@ -324,7 +324,7 @@ __device__ __forceinline__ void pt_lanes(const DevScene &s, const PtLaunch &L, S
     auto extend = [&](const RayF &ray) {
         r = ray;
         job = true;
-        trav_start<kClosest>(s, r, 0.f, any_geometry, T);
+        trav_start<kClosest, false>(s, r, 0.f, any_geometry, T);
     };
     auto bounce = [&](float hx, float hy, float hz, const float4 &nrm) {
         const float u1 = pray_uniform(&rng), u2 = pray_uniform(&rng);
@@ -419,7 +419,7 @@ __device__ __forceinline__ void pt_lanes(const DevScene &s, const PtLaunch &L, S
         }
         // (a source may hand out slots outside the image: go on until it is drained)
         if (!__any_sync(kFull, job) && src.drained()) break;
-        trav_round<kClosest, false>(s, r, L.eps, 0.f, T, S, nullptr);
+        trav_round<kClosest, false, false>(s, r, L.eps, 0.f, T, S, nullptr);
         if (job && !T.active()) {
             segments++;
             shade();

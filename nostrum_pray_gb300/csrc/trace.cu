@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(128) k_trace_occluded(DevScene s, const float 
         d2 = dist2[i];
     }
     float t;
-    const int pos = traverse<true, false, kStackN>(s, r, eps, d2, valid && s.n_refs > 0 && d2 > 0.f, t);
+    const int pos = traverse<true, false, kStackN, true>(s, r, eps, d2, valid && s.n_refs > 0 && d2 > 0.f, t);
     if (valid) occluded[i] = pos >= 0 ? 1 : 0;
 }
 
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(128) k_trace_closest(DevScene s, const float *
         r.ix = p[6], r.iy = p[7], r.iz = p[8];
     }
     float t;
-    const int pos = traverse<false, false, kStackN>(s, r, eps, 0.f, valid && s.n_refs > 0, t);
+    const int pos = traverse<false, false, kStackN, true>(s, r, eps, 0.f, valid && s.n_refs > 0, t);
     if (valid) {
         ids[i] = pos >= 0 ? (int32_t)__float_as_uint(__ldg(&s.tris[pos].v0[3])) : -1;
         ts[i] = t;

@@ -120,6 +120,26 @@ __device__ __forceinline__ bool slab_fma(const float4 &lo, const float4 &hi, con
     return tn <= tf;
 }
 
+// The same on a grid box (GPair), in units of the grid's cell: a 16-bit step q
+// becomes the float 2^23 + q by a byte permute, and the distance of its plane
+// is (2^23 + q) * inv + no with no = (org - o) / cell * inv - 2^23 * inv, so a
+// plane costs a permute and an FMA. Error, in cells: 0.5 from the rounding of
+// no (magnitude about 2^23 inv), 0.15 from (org - o) / cell * inv and the
+// FMA's own rounding (origins lie within 10 extents of the grid's origin, an
+// extent is at most 2^16 cells): below the one cell that each box was widened
+// for it (host/flatten.h).
+__device__ __forceinline__ float grid_lo(uint32_t w) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7610)); }
+__device__ __forceinline__ float grid_hi(uint32_t w) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7632)); }
+__device__ __forceinline__ void slab_grid(float q0, float q1, float q2, const RayF &r, float nox, float noy, float noz,
+                                          float &tn, float &tf) {
+    const uint32_t a = __float_as_uint(q0), b = __float_as_uint(q1), c = __float_as_uint(q2);
+    const float t1x = fmaf(grid_lo(a), r.ix, nox), t1y = fmaf(grid_hi(a), r.iy, noy);
+    const float t1z = fmaf(grid_lo(b), r.iz, noz), t2x = fmaf(grid_hi(b), r.ix, nox);
+    const float t2y = fmaf(grid_lo(c), r.iy, noy), t2z = fmaf(grid_hi(c), r.iz, noz);
+    tn = max3f(fminf(t1x, t2x), fminf(t1y, t2y), fminf(t1z, t2z));
+    tf = min3f(fmaxf(t1x, t2x), fmaxf(t1y, t2y), fmaxf(t1z, t2z));
+}
+
 // One-sided Moeller-Trumbore, include/geometry.h:242-262, with the det
 // threshold as a parameter (the reference's EPSILON is 1e-4).
 __device__ __forceinline__ bool intersect_tri(const float4 &v0, const float4 &e1, const float4 &e2, const RayF &r,
@@ -223,9 +243,11 @@ struct Trav {
     // node's first child, or a leaf (kLeafFlag; culling copy: count and first
     // record, exact copy: its node)
     uint32_t w, lw;
-    uint32_t node_off;  // 0: the exact copy; n_nodes: the culling copy (finite inverse direction, near origin)
-    float cur_tn, leaf_tn, limit, back, best_t;
-    float nox, noy, noz;  // culling copy: -origin / direction (slab_fma)
+    uint32_t node_off;  // 0: the exact copy, else the culling copy's nodes or grid pairs (finite inverse
+                        // direction, near origin)
+    float cur_tn, leaf_tn, limit, back;  // grid pairs: in cells
+    float best_t;
+    float nox, noy, noz;  // culling copy: -origin / direction (slab_fma), or slab_grid's
     int best, sp;
     uint32_t best_key;
     bool have_node, have_leaf, finite;
@@ -268,7 +290,15 @@ __device__ __forceinline__ void leaf_range(const DevScene &s, uint32_t node_off,
     }
 }
 
-template <int kMode>
+// kGrid: the culling copy's boxes come from its grid pairs: one 32-byte load
+// per pair instead of two, for twelve byte permutes more. The divergent walks
+// of ray queries and of the wavefront's extension and occlusion passes, which
+// L1 throughput bounds (83 to 89 % of its peak under ncu), gain: room 1024^2
+// at 16 spp 37.43 -> 34.00 ms, 300k closest hits 178 -> 168 us, 100k occlusion
+// rays 105 -> 98 us. The others are bound by instruction issue or registers
+// and lose (per-pixel paths of 512^2 at 1 spp 832 -> 950 us, 12 scenes 6.18 ->
+// 6.44 ms) and keep whole nodes.
+template <int kMode, bool kGrid>
 __device__ __forceinline__ void trav_start(const DevScene &s, const RayF &r, float d2, bool valid, Trav &T) {
     T.best_t = FLT_MAX;
     T.best = -1;
@@ -279,13 +309,27 @@ __device__ __forceinline__ void trav_start(const DevScene &s, const RayF &r, flo
     T.cur_tn = T.leaf_tn = 0.f;
     T.have_node = T.have_leaf = false;
     T.sp = 0;
-    T.finite = isfinite(r.ix) && isfinite(r.iy) && isfinite(r.iz);
-    T.nox = -(r.ox * r.ix), T.noy = -(r.oy * r.iy), T.noz = -(r.oz * r.iz);
+    if (!kGrid) {
+        T.finite = isfinite(r.ix) && isfinite(r.iy) && isfinite(r.iz);
+        T.nox = -(r.ox * r.ix), T.noy = -(r.oy * r.iy), T.noz = -(r.oz * r.iz);
+    }
     const float cx = r.ox - s.cull_c[0], cy = r.oy - s.cull_c[1], cz = r.oz - s.cull_c[2];
-    T.node_off = (T.finite && isfinite(T.nox) && isfinite(T.noy) && isfinite(T.noz) && cx * cx + cy * cy + cz * cz <= s.cull_r2) ? s.n_nodes : 0u;
+    if (kGrid) {
+        // (2^23 inverses, and 2^20 cells of inverses, stay finite)
+        constexpr float kMaxInv = 1e30f;
+        const bool cull = fabsf(r.ix) < kMaxInv && fabsf(r.iy) < kMaxInv && fabsf(r.iz) < kMaxInv &&
+                          cx * cx + cy * cy + cz * cz <= s.cull_r2;
+        T.node_off = cull ? s.grid_base : 0u;
+        T.finite = cull || (isfinite(r.ix) && isfinite(r.iy) && isfinite(r.iz));
+    } else {
+        T.node_off = (T.finite && isfinite(T.nox) && isfinite(T.noy) && isfinite(T.noz) &&
+                      cx * cx + cy * cy + cz * cz <= s.cull_r2)
+                         ? s.n_nodes
+                         : 0u;
+    }
     if (valid) {
         float tn, tf;
-        const GNode *root = s.nodes + T.node_off;
+        const GNode *root = s.nodes + (kGrid ? (T.node_off ? s.n_nodes : 0u) : T.node_off);
         float4 rlo, rhi;
         ldg_node(root, rlo, rhi);
         if (slab(rlo, rhi, r, tn, tf)) {
@@ -293,11 +337,19 @@ __device__ __forceinline__ void trav_start(const DevScene &s, const RayF &r, flo
             if (!T.node_off && (__float_as_uint(rhi.w) & kLeafFlag)) T.w = kLeafFlag;  // (node 0)
             T.cur_tn = tn;
             T.have_node = true;
+            if (kGrid && T.node_off) {
+                if (!(T.w & kLeafFlag)) T.w /= 2;
+                T.cur_tn *= s.grid_scale, T.limit *= s.grid_scale, T.back *= s.grid_scale;
+                constexpr float kBias = 8388608.f;
+                T.nox = fmaf(-kBias, r.ix, (s.grid_org[0] - r.ox) * s.grid_scale * r.ix);
+                T.noy = fmaf(-kBias, r.iy, (s.grid_org[1] - r.oy) * s.grid_scale * r.iy);
+                T.noz = fmaf(-kBias, r.iz, (s.grid_org[2] - r.oz) * s.grid_scale * r.iz);
+            }
         }
     }
 }
 
-template <int kMode, bool kCount, int kStackN>
+template <int kMode, bool kGrid, bool kCount, int kStackN>
 __device__ __forceinline__ void trav_round(const DevScene &s, const RayF &r, float eps, float d2, Trav &T,
                                            TravStack<kStackN> &S, FetchCount *fc) {
     static_assert(kStackN >= 2 && kStackN <= kStack, "stack entries");
@@ -311,17 +363,26 @@ __device__ __forceinline__ void trav_round(const DevScene &s, const RayF &r, flo
             const GNode *c = s.nodes + (T.w + T.node_off);
             float4 l0, h0, l1, h1;
             ldg_node(c, l0, h0);
-            ldg_node(c + 1, l1, h1);
-            uint32_t w0 = __float_as_uint(l0.w), w1 = __float_as_uint(l1.w);
+            if (!kGrid) ldg_node(c + 1, l1, h1);
+            uint32_t w0 = __float_as_uint(l0.w), w1 = __float_as_uint(kGrid ? h0.w : l1.w);
             float tn0, tf0, tn1, tf1;
             bool v0, v1;
             // entered: tn <= tf, not beyond the best hit, not behind the origin
             if (T.node_off) {
-                slab_fma(l0, h0, r, T.nox, T.noy, T.noz, tn0, tf0);
-                slab_fma(l1, h1, r, T.nox, T.noy, T.noz, tn1, tf1);
+                if (kGrid) {
+                    slab_grid(l0.x, l0.y, l0.z, r, T.nox, T.noy, T.noz, tn0, tf0);
+                    slab_grid(h0.x, h0.y, h0.z, r, T.nox, T.noy, T.noz, tn1, tf1);
+                } else {
+                    slab_fma(l0, h0, r, T.nox, T.noy, T.noz, tn0, tf0);
+                    slab_fma(l1, h1, r, T.nox, T.noy, T.noz, tn1, tf1);
+                }
                 tn0 = fmaxf(tn0, T.back), tn1 = fmaxf(tn1, T.back);
                 v0 = tn0 <= fminf(tf0, T.limit), v1 = tn1 <= fminf(tf1, T.limit);
             } else {
+                if (kGrid) {
+                    ldg_node(c + 1, l1, h1);
+                    w1 = __float_as_uint(l1.w);
+                }
                 v0 = slab(l0, h0, r, T.finite, tn0, tf0) && tn0 <= T.limit && tf0 >= T.back;
                 v1 = slab(l1, h1, r, T.finite, tn1, tf1) && tn1 <= T.limit && tf1 >= T.back;
                 if (__float_as_uint(h0.w) & kLeafFlag) w0 = kLeafFlag | T.w;
@@ -384,6 +445,7 @@ __device__ __forceinline__ void trav_round(const DevScene &s, const RayF &r, flo
                                 T.best = (int)i;
                                 T.best_key = key;
                                 T.limit = t * kPruneRel;
+                                if (kGrid && T.node_off) T.limit *= s.grid_scale;
                             }
                         }
                     }
@@ -393,14 +455,14 @@ __device__ __forceinline__ void trav_round(const DevScene &s, const RayF &r, flo
     }
 }
 
-template <bool kAny, bool kCount = false, int kStackN = kStack>
+template <bool kAny, bool kCount = false, int kStackN = kStack, bool kGrid = false>
 __device__ __forceinline__ int traverse(const DevScene &s, const RayF &r, float eps, float d2, bool valid,
                                         float &best_t, FetchCount *fc = nullptr) {
     constexpr int kMode = kAny ? kAnyHit : kClosest;
     Trav T;
     TravStack<kStackN> S;
-    trav_start<kMode>(s, r, d2, valid, T);
-    while (__any_sync(0xFFFFFFFFu, T.active())) trav_round<kMode, kCount>(s, r, eps, d2, T, S, fc);
+    trav_start<kMode, kGrid>(s, r, d2, valid, T);
+    while (__any_sync(0xFFFFFFFFu, T.active())) trav_round<kMode, kGrid, kCount>(s, r, eps, d2, T, S, fc);
     best_t = T.best_t;
     return T.best;
 }

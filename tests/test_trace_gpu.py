@@ -511,3 +511,27 @@ def test_pixels_per_warp(oracle, traversal, warps):
     m = scenes.soup(2_000, 9)
     for w, h in [(1, 1), (9, 5)] + [(97, e // 97 + k) for e in _edges(warps) for k in (-2, 3)]:
         check_frame(oracle, m, scenes.soup_setup(w, h), traversal)
+
+
+@pytest.mark.parametrize("scale,squash", [(1.0, 1.0), (1e-6, 1.0), (1e6, 1.0), (1.0, 1e-3), (37.0, 30.0)])
+def test_grid_boxes_match_reference_walk(oracle, scale, squash):
+    """Ray queries, which test boxes on a scene-wide grid, over scenes of
+    different sizes and proportions: ids and distances are the oracle's, also
+    for directions so close to an axis that an inverse is up to 1e37 (the grid
+    serves those up to 1e30)."""
+    m = scenes.soup(700, 4)
+    m.verts[:] = (m.verts.reshape(-1, 3, 3) * np.float32([scale, scale, scale * squash])).reshape(m.verts.shape)
+    st = scenes.soup_setup()
+    st.det_eps = 0.0
+    rays = _hard_rays(m, 6, 6000)
+    rng = np.random.default_rng(7)
+    k = len(rays) // 3
+    d = (10.0 ** rng.uniform(-37, -20, (k, 3)) * rng.choice([-1, 1], (k, 3))).astype(np.float32)
+    d[np.arange(k), rng.integers(0, 3, k)] = rng.choice([-1, 1], k)
+    rays[:k, 3:6], rays[:k, 6:9] = d, 1.0 / d
+    rays = np.ascontiguousarray(rays[_well_posed(m, rays) & np.isfinite(rays[:, 6:9]).all(1)])
+    assert len(rays) > 1000
+    ids, ts = trace(native.Scene.from_setup(m, st), rays, 0.0)
+    want, want_t = oracle.OracleScene.from_setup(m, st).trace(rays, 0.0)
+    np.testing.assert_array_equal(ids, want.astype(np.int32))
+    np.testing.assert_array_equal(ts.view(np.uint32), want_t.view(np.uint32))
