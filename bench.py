@@ -66,7 +66,7 @@ def parse():
     ap.add_argument("--no-secondary", action="store_true",
                     help="default workload: skip the path-tracing room and the 64-scene batch")
     ap.add_argument("--leaf-refine", type=int, default=8,
-                    help="device layout: sub-hierarchy inside reference leaves larger than this (0 = off)")
+                    help="device layout: most triangles per leaf of the culling hierarchy, at most 4 (0 = none)")
     ap.add_argument("--cpu-seconds", type=float, default=12.0, help="CPU baseline sample budget")
     return ap.parse_args()
 
