@@ -326,8 +326,11 @@ __global__ void __launch_bounds__(kThreads) k_wf_shade(DevScene s, PtLaunch L, W
 
 // Any-hit test of every occlusion job (counts[jobs] of them), with the same
 // dynamic fetch (counts[4]); an unoccluded job adds its contribution to its
-// path.
-template <int kStackN>
+// path. The rays of the first bounce start on neighbouring pixels' hits and aim
+// at the light, so their walks share nodes in L1 and instruction issue binds
+// them: whole nodes; later bounces take grid pairs (4 spp of the 1024^2 room,
+// first / later bounces, us under ncu: whole nodes 677 / 904, grid 790 / 824).
+template <int kStackN, bool kGrid>
 __global__ void __launch_bounds__(kThreads, kTraceBlocksPerSm) k_wf_occlude(DevScene s, PtLaunch L,
                                                                           WavefrontScratch w, int jobs) {
     constexpr unsigned kFull = 0xFFFFFFFFu;
@@ -352,11 +355,11 @@ __global__ void __launch_bounds__(kThreads, kTraceBlocksPerSm) k_wf_occlude(DevS
                 r = make_ray(jo.x, jo.y, jo.z, jd.x, jd.y, jd.z);
                 d2 = jd.w;
                 has = true;
-                trav_start<kAnyHit, true>(s, r, d2, s.n_refs > 0, T);
+                trav_start<kAnyHit, kGrid>(s, r, d2, s.n_refs > 0, T);
             }
         }
         if (!__any_sync(kFull, has)) break;
-        trav_round<kAnyHit, true, false>(s, r, L.eps, d2, T, S, nullptr);
+        trav_round<kAnyHit, kGrid, false>(s, r, L.eps, d2, T, S, nullptr);
         if (has && !T.active()) {
             seg++;
             if (T.best < 0) {
@@ -490,7 +493,10 @@ cudaError_t wavefront_preload_kernels() {
         reinterpret_cast<const void *>(k_wf_first<32>),    reinterpret_cast<const void *>(k_wf_first<kStack>),
         reinterpret_cast<const void *>(k_wf_extend<32>),   reinterpret_cast<const void *>(k_wf_extend<kStack>),
         reinterpret_cast<const void *>(k_wf_shade<true>),  reinterpret_cast<const void *>(k_wf_shade<false>),
-        reinterpret_cast<const void *>(k_wf_occlude<32>),  reinterpret_cast<const void *>(k_wf_occlude<kStack>),
+        reinterpret_cast<const void *>(k_wf_occlude<32, false>),
+        reinterpret_cast<const void *>(k_wf_occlude<kStack, false>),
+        reinterpret_cast<const void *>(k_wf_occlude<32, true>),
+        reinterpret_cast<const void *>(k_wf_occlude<kStack, true>),
         reinterpret_cast<const void *>(k_wf_accumulate),   reinterpret_cast<const void *>(k_wf_finish)};
     for (const void *k : kernels) {
         cudaError_t e = cudaFuncGetAttributes(&a, k);
@@ -536,8 +542,9 @@ cudaError_t record_wavefront_frame(const DevScene &s, const PtLaunch &L, const W
                 if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
                 occ = side;
             }
-            if (small_stack) k_wf_occlude<32><<<grid, kThreads, 0, occ>>>(s, L, w, jobs);
-            else k_wf_occlude<kStack><<<grid, kThreads, 0, occ>>>(s, L, w, jobs);
+            const auto occlude = it == 0 ? (small_stack ? k_wf_occlude<32, false> : k_wf_occlude<kStack, false>)
+                                         : (small_stack ? k_wf_occlude<32, true> : k_wf_occlude<kStack, true>);
+            occlude<<<grid, kThreads, 0, occ>>>(s, L, w, jobs);
             if (overlap && e == cudaSuccess) e = cudaEventRecord(join, side);
         }
         if (overlap && e == cudaSuccess) e = cudaStreamWaitEvent(stream, join, 0);
