@@ -3,7 +3,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <thread>
 
 namespace pray_gpu {
 
@@ -46,6 +45,7 @@ struct Prim {
 struct Builder {
     std::vector<Prim> prims;
     int leaf_max;
+    Threads &threads;
     // node pairs by the position of their split: the subtree over [lo, hi)
     // uses pairs lo .. hi - 2, so parallel subtrees share nothing
     struct Node {
@@ -60,7 +60,7 @@ struct Builder {
         return d;
     }
 
-    void build(Node &node, size_t lo, size_t hi, int depth, int threads) {
+    void build(Node &node, size_t lo, size_t hi, int depth) {
         const size_t n = hi - lo;
         Box bounds, centres;
         bounds.clear(), centres.clear();
@@ -144,15 +144,11 @@ struct Builder {
         const size_t pair = mid - 1;  // one split position each: unique in [lo, hi - 2]
         node.count = 0, node.pair = (uint32_t)pair;
         Node &l = pairs[2 * pair], &r = pairs[2 * pair + 1];
-        if (threads > 1 && n >= kParallel) {
-            const int lt = threads / 2;
-            std::thread other([&] { build(l, lo, mid, depth + 1, lt); });
-            build(r, mid, hi, depth + 1, threads - lt);
-            other.join();
-        } else {
-            build(l, lo, mid, depth + 1, 1);
-            build(r, mid, hi, depth + 1, 1);
-        }
+        std::future<void> other;
+        if (n >= kParallel) other = threads.start([&, mid] { build(l, lo, mid, depth + 1); });
+        if (!other.valid()) build(l, lo, mid, depth + 1);
+        build(r, mid, hi, depth + 1);
+        if (other.valid()) other.get();
     }
 
     void emit(const Node &n, uint32_t slot, std::vector<GNode> &out) const {
@@ -175,6 +171,7 @@ struct Builder {
 }  // namespace
 
 CullBvh build_cull_bvh(const std::vector<TriPre> &tris, int leaf_max, int threads) {
+    Threads budget(threads);
     CullBvh out;
     out.nodes.assign(2, GNode{});
     const size_t n = tris.size();
@@ -183,9 +180,7 @@ CullBvh build_cull_bvh(const std::vector<TriPre> &tris, int leaf_max, int thread
         out.nodes[0].b = kLeafFlag;
         return out;
     }
-    if (threads <= 0) threads = std::max(1, (int)std::thread::hardware_concurrency());
-    Builder b;
-    b.leaf_max = std::min(std::max(1, leaf_max), kCullLeaf);
+    Builder b{{}, std::min(std::max(1, leaf_max), kCullLeaf), budget, {}, {}};
     b.prims.resize(n);
     for (size_t i = 0; i < n; i++) {
         Prim &p = b.prims[i];
@@ -200,7 +195,7 @@ CullBvh build_cull_bvh(const std::vector<TriPre> &tris, int leaf_max, int thread
     }
     b.root.resize(1);
     b.pairs.resize(2 * std::max<size_t>(n - 1, 1));
-    b.build(b.root[0], 0, n, 0, threads);
+    b.build(b.root[0], 0, n, 0);
     out.nodes.reserve(2 * n + 2);
     b.emit(b.root[0], 0, out.nodes);
     out.order.resize(n);

@@ -9,6 +9,7 @@
 
 #include "../device_layout.h"
 #include "geom.h"
+#include "threads.h"
 
 namespace pray_gpu {
 

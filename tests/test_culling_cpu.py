@@ -1,0 +1,31 @@
+"""Host side of the culling hierarchy (host/cull_bvh.cpp, host/flatten.cpp),
+checked by a small C++ program built from the same sources."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+HOST = os.path.join(ROOT, "nostrum_pray_gb300", "csrc", "host")
+
+
+@pytest.fixture(scope="session")
+def cull_check(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("cull") / "cull_check")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-pthread", "-I", HOST, "-o", exe,
+                    os.path.join(ROOT, "tests", "native", "cull_check.cpp"), os.path.join(HOST, "cull_bvh.cpp"),
+                    os.path.join(HOST, "flatten.cpp"), os.path.join(HOST, "kdtree.cpp"), "-ldl"], check=True)
+
+    def run(*args):
+        return subprocess.run([exe, *map(str, args)], capture_output=True, text=True, timeout=300)
+
+    return run
+
+
+@pytest.mark.parametrize("limit", [0, 1, 3])
+def test_build_survives_a_thread_limit(cull_check, limit):
+    """A system that gives fewer threads than were asked for costs time, not the
+    process: the hierarchy is the same."""
+    r = cull_check("threads", limit)
+    assert r.returncode == 0, (r.returncode, r.stderr)
+    assert r.stdout.split() == ["same", "1"]
