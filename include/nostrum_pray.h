@@ -51,7 +51,8 @@ typedef struct {
     int32_t max_depth;             /* MAX_DEPTH: leaf at this depth (20); at most 30 */
     float sah_traversal_cost;      /* traversalCost (5) */
     float sah_intersection_cost;   /* triangleIntersectionCost (1.5) */
-    int32_t build_threads;         /* host threads for the build, 0 = all */
+    int32_t build_threads;         /* most host threads that the build runs at once, the caller's
+                                      included; 0 = all */
     int32_t leaf_refine;           /* device layout only: most triangles per leaf (at most 4) of the conservative
                                       hierarchy that the kernels cull with (8; 0 = off, they walk the reference's
                                       tree itself). Results are unchanged. */

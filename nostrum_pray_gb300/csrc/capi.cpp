@@ -8,8 +8,6 @@
 #include <atomic>
 #include <cstring>
 #include <exception>
-#include <functional>
-#include <future>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -543,14 +541,16 @@ pray_status pray_scene_create(const float *verts, const float *colors, const uin
         s = std::make_unique<pray_scene>();
         s->device = device;
         s->n_tris = n;
-        pre = precompute_triangles(verts, n, opt->build_threads);
+        Threads threads(opt->build_threads);
+        pre = precompute_triangles(verts, n, threads);
         // the culling hierarchy beside the reference's tree
-        std::future<CullBvh> cull;
-        if (opt->leaf_refine > 0)
-            cull = std::async(std::launch::async, build_cull_bvh, std::cref(pre), opt->leaf_refine, opt->build_threads);
-        s->tree = build_tree(pre, to_options(opt));
         CullBvh bvh;
-        if (cull.valid()) bvh = cull.get();
+        std::future<void> cull;
+        auto build_cull = [&] { bvh = build_cull_bvh(pre, opt->leaf_refine, threads); };
+        if (opt->leaf_refine > 0) cull = threads.start(build_cull);
+        s->tree = build_tree(pre, to_options(opt), threads);
+        if (cull.valid()) cull.get();
+        else if (opt->leaf_refine > 0) build_cull();
         if (s->tree.refs.size() >= (1ull << 31))
             return set_error(PRAY_ERR_UNSUPPORTED, "more than 2^31-1 leaf references");
         DeviceImage img;

@@ -170,8 +170,7 @@ struct Builder {
 
 }  // namespace
 
-CullBvh build_cull_bvh(const std::vector<TriPre> &tris, int leaf_max, int threads) {
-    Threads budget(threads);
+CullBvh build_cull_bvh(const std::vector<TriPre> &tris, int leaf_max, Threads &threads) {
     CullBvh out;
     out.nodes.assign(2, GNode{});
     const size_t n = tris.size();
@@ -180,7 +179,7 @@ CullBvh build_cull_bvh(const std::vector<TriPre> &tris, int leaf_max, int thread
         out.nodes[0].b = kLeafFlag;
         return out;
     }
-    Builder b{{}, std::min(std::max(1, leaf_max), kCullLeaf), budget, {}, {}};
+    Builder b{{}, std::min(std::max(1, leaf_max), kCullLeaf), threads, {}, {}};
     b.prims.resize(n);
     for (size_t i = 0; i < n; i++) {
         Prim &p = b.prims[i];

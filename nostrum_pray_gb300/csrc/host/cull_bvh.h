@@ -25,8 +25,12 @@ struct CullBvh {
 // at most `leaf_max` triangles (1 to kCullLeaf), at most kCullDepth levels
 // below the root as long as halving can reach that: the kernels need their
 // larger traversal stack from there on. The same result for any number of
-// threads.
+// threads (0: every hardware thread).
 constexpr int kCullLeaf = 4, kCullDepth = 31;
-CullBvh build_cull_bvh(const std::vector<TriPre> &tris, int leaf_max, int threads);
+CullBvh build_cull_bvh(const std::vector<TriPre> &tris, int leaf_max, Threads &threads);
+inline CullBvh build_cull_bvh(const std::vector<TriPre> &tris, int leaf_max, int threads) {
+    Threads budget(threads);
+    return build_cull_bvh(tris, leaf_max, budget);
+}
 
 }  // namespace pray_gpu

@@ -6,7 +6,6 @@
 #include <algorithm>
 #include <future>
 #include <memory>
-#include <thread>
 
 namespace pray_gpu {
 
@@ -21,25 +20,17 @@ struct BNode {
     bool leaf() const { return !tris.empty() || (!left && !right); }
 };
 
-int hw_threads(int requested) {
-    if (requested > 0) return requested;
-    unsigned h = std::thread::hardware_concurrency();
-    return h ? (int)h : 1;
-}
-
-// Depth up to which the two subtrees of a node are built concurrently.
-int parallel_depth(int threads) {
-    int d = 0;
-    while ((1 << d) < 2 * threads && d < 8) d++;
-    return d;
-}
+// Nodes whose two subtrees may be built concurrently: near the root, and large
+// enough to be worth a thread's start.
+constexpr int kParallelDepth = 8;
+constexpr size_t kParallelSize = 1024;
 
 // ---------------------------------------------------------------- median
 
 struct MedianBuilder {
     const std::vector<TriPre> &tris;
     const TreeOptions &opt;
-    int par_depth;
+    Threads &threads;
 
     std::unique_ptr<BNode> build(std::vector<uint32_t> &idx, int depth) {
         auto node = std::make_unique<BNode>();
@@ -57,14 +48,12 @@ struct MedianBuilder {
         std::nth_element(idx.begin(), idx.begin() + half, idx.end(),
                          [&](uint32_t l, uint32_t r) { return tris[l].mid[axis] < tris[r].mid[axis]; });
         std::vector<uint32_t> li(idx.begin(), idx.begin() + half), ri(idx.begin() + half, idx.end());
-        if (depth < par_depth) {
-            auto fut = std::async(std::launch::async, [&] { return build(li, depth + 1); });
-            node->right = build(ri, depth + 1);
-            node->left = fut.get();
-        } else {
-            node->left = build(li, depth + 1);
-            node->right = build(ri, depth + 1);
-        }
+        std::future<std::unique_ptr<BNode>> left;
+        if (depth < kParallelDepth && idx.size() >= kParallelSize)
+            left = threads.start([&] { return build(li, depth + 1); });
+        if (!left.valid()) node->left = build(li, depth + 1);
+        node->right = build(ri, depth + 1);
+        if (left.valid()) node->left = left.get();
         node->axis = axis;
         node->split = tris[idx[half]].mid[axis];
         return node;
@@ -86,37 +75,29 @@ inline bool ev_less(const Ev &a, const Ev &b) {
     return (a.d < b.d) || (a.d == b.d && a.axis < b.axis) || (a.d == b.d && a.axis == b.axis && a.type < b.type);
 }
 
-// Sorts events by ev_less on up to `threads` threads: a power-of-two number
-// of chunks sorted concurrently, then merged pairwise. Events that compare
-// equal are interchangeable, so the tree does not depend on their order.
-void sort_events(std::vector<Ev> &ev, int threads) {
+// Sorts events by ev_less: a power-of-two number of chunks (at most 64, as
+// many as there are hardware threads) sorted concurrently, then merged
+// pairwise. Events that compare equal are interchangeable, so the tree does
+// not depend on their order.
+void sort_events(std::vector<Ev> &ev, Threads &threads) {
     const size_t n = ev.size();
     int parts = 1;
-    while (2 * parts <= threads && n / (2 * (size_t)parts) >= ((size_t)1 << 16)) parts *= 2;
+    while (2 * parts <= std::min(64, threads.total()) && n / (2 * (size_t)parts) >= ((size_t)1 << 16)) parts *= 2;
     if (parts == 1) {
         std::sort(ev.begin(), ev.end(), ev_less);
         return;
     }
     std::vector<size_t> cut(parts + 1);
     for (int i = 0; i <= parts; i++) cut[i] = n * (size_t)i / (size_t)parts;
-    {
-        std::vector<std::thread> pool;
-        for (int i = 0; i < parts; i++)
-            pool.emplace_back([&, i] { std::sort(ev.begin() + cut[i], ev.begin() + cut[i + 1], ev_less); });
-        for (auto &t : pool) t.join();
-    }
+    threads.each(parts, [&](int i) { std::sort(ev.begin() + cut[i], ev.begin() + cut[i + 1], ev_less); });
     std::vector<Ev> tmp(n);
     std::vector<Ev> *src = &ev, *dst = &tmp;
     for (int w = 1; w < parts; w *= 2) {
-        std::vector<std::thread> pool;
-        for (int i = 0; i < parts; i += 2 * w) {
-            const size_t a = cut[i], m = cut[i + w], b = cut[i + 2 * w];
-            pool.emplace_back([=] {
-                std::merge(src->begin() + a, src->begin() + m, src->begin() + m, src->begin() + b, dst->begin() + a,
-                           ev_less);
-            });
-        }
-        for (auto &t : pool) t.join();
+        threads.each(parts / (2 * w), [&](int k) {
+            const size_t a = cut[2 * w * k], m = cut[2 * w * k + w], b = cut[2 * w * (k + 1)];
+            std::merge(src->begin() + a, src->begin() + m, src->begin() + m, src->begin() + b, dst->begin() + a,
+                       ev_less);
+        });
         std::swap(src, dst);
     }
     if (src != &ev) ev.swap(tmp);
@@ -127,7 +108,7 @@ enum : int8_t { kLeftOnly = -1, kBoth = 0, kRightOnly = 1 };
 struct SahBuilder {
     const std::vector<TriPre> &tris;
     const TreeOptions &opt;
-    int par_depth;
+    Threads &threads;
     size_t ntris;
 
     void events_of(uint32_t t, const Aabb &vox, std::vector<Ev> &ev) const {
@@ -273,17 +254,15 @@ struct SahBuilder {
         }
         std::vector<Ev>().swap(bl);
         std::vector<Ev>().swap(br);
-        if (depth < par_depth) {
-            auto fut = std::async(std::launch::async, [&] {
+        std::future<std::unique_ptr<BNode>> left;
+        if (depth < kParallelDepth && idx.size() >= kParallelSize)
+            left = threads.start([&] {
                 std::vector<int8_t> own(ntris, kBoth);
                 return build(tl, vl, std::move(le), axis, d, depth + 1, own);
             });
-            node->right = build(tr, vr, std::move(re), axis, d, depth + 1, side);
-            node->left = fut.get();
-        } else {
-            node->left = build(tl, vl, std::move(le), axis, d, depth + 1, side);
-            node->right = build(tr, vr, std::move(re), axis, d, depth + 1, side);
-        }
+        if (!left.valid()) node->left = build(tl, vl, std::move(le), axis, d, depth + 1, side);
+        node->right = build(tr, vr, std::move(re), axis, d, depth + 1, side);
+        if (left.valid()) node->left = left.get();
         node->axis = axis;
         node->split = d;
         return node;
@@ -326,35 +305,31 @@ Stats flatten(const BNode *n, BuiltTree &out) {
 
 }  // namespace
 
-std::vector<TriPre> precompute_triangles(const float *verts, uint64_t n, int threads) {
+std::vector<TriPre> precompute_triangles(const float *verts, uint64_t n, Threads &threads) {
     std::vector<TriPre> out(n);
-    const int nt = std::max(1, std::min<int>(hw_threads(threads), (int)(n / 65536) + 1));
-    std::vector<std::thread> pool;
-    for (int w = 0; w < nt; w++)
-        pool.emplace_back([&, w] {
-            for (uint64_t i = w; i < n; i += nt) out[i] = precompute_triangle(verts + 9 * i);
-        });
-    for (auto &t : pool) t.join();
+    const int parts = std::min<int>(threads.total(), (int)(n / 65536) + 1);
+    threads.each(parts, [&](int w) {
+        for (uint64_t i = w; i < n; i += parts) out[i] = precompute_triangle(verts + 9 * i);
+    });
     return out;
 }
 
-BuiltTree build_tree(const std::vector<TriPre> &tris, const TreeOptions &opt) {
+BuiltTree build_tree(const std::vector<TriPre> &tris, const TreeOptions &opt, Threads &threads) {
     BuiltTree out;
     if (tris.empty()) {
         out.nodes.emplace_back();  // empty root leaf (src/kd_tree.cpp:26-29)
         return out;
     }
-    const int threads = hw_threads(opt.threads);
     std::vector<uint32_t> idx(tris.size());
     for (size_t i = 0; i < idx.size(); i++) idx[i] = (uint32_t)i;
     std::unique_ptr<BNode> root;
     if (opt.kind == kTreeMedian) {
-        MedianBuilder mb{tris, opt, parallel_depth(threads)};
+        MedianBuilder mb{tris, opt, threads};
         root = mb.build(idx, 0);
     } else {
         Aabb rb = tris[0].box;
         for (size_t i = 0; i < tris.size(); i++) rb = rb.grown(tris[i].box);
-        SahBuilder sb{tris, opt, parallel_depth(threads), tris.size()};
+        SahBuilder sb{tris, opt, threads, tris.size()};
         std::vector<Ev> ev;
         ev.reserve(tris.size() * 6);
         for (uint32_t t : idx) sb.events_of(t, rb, ev);

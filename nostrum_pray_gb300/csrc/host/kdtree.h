@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "geom.h"
+#include "threads.h"
 
 namespace pray_gpu {
 
@@ -44,8 +45,17 @@ struct BuiltTree {
     uint64_t maxdepth = 0, leaf_nodes = 0, empty_leaves = 0;
 };
 
-std::vector<TriPre> precompute_triangles(const float *verts, uint64_t n, int threads);
+std::vector<TriPre> precompute_triangles(const float *verts, uint64_t n, Threads &threads);
+BuiltTree build_tree(const std::vector<TriPre> &tris, const TreeOptions &opt, Threads &threads);
 
-BuiltTree build_tree(const std::vector<TriPre> &tris, const TreeOptions &opt);
+// On `threads` threads (0: every hardware thread) of their own.
+inline std::vector<TriPre> precompute_triangles(const float *verts, uint64_t n, int threads) {
+    Threads budget(threads);
+    return precompute_triangles(verts, n, budget);
+}
+inline BuiltTree build_tree(const std::vector<TriPre> &tris, const TreeOptions &opt) {
+    Threads budget(opt.threads);
+    return build_tree(tris, opt, budget);
+}
 
 }  // namespace pray_gpu

@@ -14,11 +14,13 @@
 namespace pray_gpu {
 
 class Threads {
+    const int total_;
     std::atomic<int> free_;
 
   public:
     // total <= 0: every hardware thread
-    explicit Threads(int total) : free_((total > 0 ? total : hardware()) - 1) {}
+    explicit Threads(int total) : total_(total > 0 ? total : hardware()), free_(total_ - 1) {}
+    int total() const { return total_; }
     static int hardware() {
         const unsigned h = std::thread::hardware_concurrency();
         return h ? (int)h : 1;

@@ -18,13 +18,29 @@
 using namespace pray_gpu;
 
 // Thread creation as this program's libraries see it: fails once `g_left`
-// threads have been made.
-static std::atomic<int> g_left{1 << 30};
+// threads have been made; counts the threads at work.
+static std::atomic<int> g_left{1 << 30}, g_running{0}, g_most{0};
+struct Started {
+    void *(*f)(void *);
+    void *arg;
+};
+static void *counted(void *p) {
+    const Started s = *static_cast<Started *>(p);
+    delete static_cast<Started *>(p);
+    const int n = ++g_running;
+    for (int m = g_most; m < n && !g_most.compare_exchange_weak(m, n);) {}
+    void *r = s.f(s.arg);
+    g_running--;
+    return r;
+}
 extern "C" int pthread_create(pthread_t *t, const pthread_attr_t *a, void *(*f)(void *), void *arg) {
     using Fn = int (*)(pthread_t *, const pthread_attr_t *, void *(*)(void *), void *);
     static Fn real = reinterpret_cast<Fn>(dlsym(RTLD_NEXT, "pthread_create"));
     if (g_left.fetch_sub(1) <= 0) return EAGAIN;
-    return real(t, a, f, arg);
+    auto *s = new Started{f, arg};
+    const int e = real(t, a, counted, s);
+    if (e) delete s;
+    return e;
 }
 
 static std::vector<float> soup(size_t n, double spread, unsigned seed) {
@@ -52,8 +68,26 @@ static int threads_mode(int limit) {
     return same ? 0 : 1;
 }
 
+// budget <n>: most threads that ran at once, the caller included, while a tree
+// and its hierarchy were built on a budget of n as a scene's creation does.
+static int budget_mode(int n) {
+    const auto verts = soup(200000, 0.01, 2);
+    Threads threads(n);
+    const auto pre = precompute_triangles(verts.data(), verts.size() / 9, threads);
+    TreeOptions opt;
+    opt.kind = kTreeSah;
+    CullBvh bvh;
+    auto cull = threads.start([&] { bvh = build_cull_bvh(pre, 4, threads); });
+    const BuiltTree tree = build_tree(pre, opt, threads);
+    if (cull.valid()) cull.get();
+    else bvh = build_cull_bvh(pre, 4, threads);
+    std::printf("most %d nodes %zu %zu\n", 1 + g_most.load(), tree.nodes.size(), bvh.nodes.size());
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string mode = argc > 1 ? argv[1] : "";
     if (mode == "threads") return threads_mode(std::atoi(argv[2]));
+    if (mode == "budget") return budget_mode(std::atoi(argv[2]));
     return 2;
 }

@@ -29,3 +29,15 @@ def test_build_survives_a_thread_limit(cull_check, limit):
     r = cull_check("threads", limit)
     assert r.returncode == 0, (r.returncode, r.stderr)
     assert r.stdout.split() == ["same", "1"]
+
+
+@pytest.mark.parametrize("n", [1, 2, 5])
+def test_build_threads_bounds_the_whole_build(cull_check, n):
+    """build_threads counts everything a scene's creation runs at once: the
+    reference's tree, the culling hierarchy beside it and the caller. (A
+    thread that has given its place back may still be ending when the next
+    starts: room for that where there is more than one.)"""
+    r = cull_check("budget", n)
+    assert r.returncode == 0, r.stderr
+    most = int(r.stdout.split()[1])
+    assert most <= 2 * n - 1
