@@ -263,7 +263,7 @@ __global__ void k_pack_input(const float *rad, const __half *feat, __nv_bfloat16
     // kernel; it waits for this kernel's completion before reading x16)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     for (size_t p = gtid(); p < pixels; p += gstride()) {
-        __nv_bfloat16 v[16];
+        alignas(16) __nv_bfloat16 v[16];
         for (int k = 0; k < 3; k++) v[k] = __float2bfloat16(log1pf(fmaxf(rad[3 * p + k], 0.f) / demod(feat, 3 * p + k)));
         for (int k = 0; k < 7; k++) v[3 + k] = __float2bfloat16(__half2float(feat[7 * p + k]));
         for (int k = 10; k < 16; k++) v[k] = __float2bfloat16(0.f);
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(256) k_l1_tc(const float *out, const float *ta
     const float inv = 1.f / (float)(3 * pixels);
     for (size_t p = gtid(); p < pixels; p += gstride()) {
         const size_t img = p / px;
-        __nv_bfloat16 v[8];
+        alignas(16) __nv_bfloat16 v[8];
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             const size_t i = 3 * p + k;
