@@ -220,12 +220,20 @@ cudaError_t Denoiser::ensure(int n, int h, int w) {
 }
 
 // Buffers and plans of the backward pass, made by the first one after a
-// change of size (inference needs none).
+// change of size (inference needs none). A failure leaves none behind.
 cudaError_t Denoiser::ensure_backward() {
+    if (tensor_cores_ ? backward_tc_ : backward_cc_) return cudaSuccess;
+    const size_t before = owned_.size();
+    const cudaError_t e = make_backward();
+    if (e != cudaSuccess)
+        for (; owned_.size() > before; owned_.pop_back()) cudaFree(owned_.back());
+    return e;
+}
+
+cudaError_t Denoiser::make_backward() {
     const size_t px = (size_t)n_ * h_ * w_dim_;
     cudaError_t e = cudaSuccess;
     if (!tensor_cores_) {
-        if (backward_cc_) return cudaSuccess;
         for (size_t i = 1; i < act_.size(); i++)
             if ((e = take(act_[i].g, (size_t)n_ * (h_ >> act_[i].level) * (w_dim_ >> act_[i].level) * act_[i].c)) !=
                 cudaSuccess)
@@ -234,7 +242,6 @@ cudaError_t Denoiser::ensure_backward() {
         backward_cc_ = true;
         return cudaSuccess;
     }
-    if (backward_tc_) return cudaSuccess;
     auto pixels = [&](int level) { return (size_t)n_ * (h_ >> level) * (w_dim_ >> level); };
     for (int l = 0; l < 4; l++)
         if ((e = take(skip_g_[l], pixels(l) * kEnc[l])) != cudaSuccess) return e;

@@ -59,6 +59,7 @@ class Denoiser {
     cudaError_t take(T *&p, size_t n);
     cudaError_t ensure(int n, int h, int w);
     cudaError_t ensure_backward();
+    cudaError_t make_backward();
     cudaError_t backward_tc(const float *target, cudaStream_t st);
     cudaError_t backward_cc(const float *target, cudaStream_t st);
     cudaError_t conv_fwd(int ci, const Buf &in, __nv_bfloat16 *y, float *y32, cudaStream_t st,
