@@ -185,6 +185,7 @@ cudaError_t Denoiser::ensure(int n, int h, int w) {
     generation_++;
     act_.clear();
     grad_.clear();
+    cap_pixels_ = 0;  // until every buffer below is there
     n_ = n, h_ = h, w_dim_ = w;
     cudaError_t e;
     auto act = [&](int level, int c) -> cudaError_t {

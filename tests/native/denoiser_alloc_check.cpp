@@ -16,7 +16,7 @@ static std::map<void *, size_t> g_live;
 extern "C" {
 cudaError_t cudaMalloc(void **p, size_t n) {
     *p = nullptr;
-    if (n > g_limit - g_used) return cudaErrorMemoryAllocation;
+    if (g_used > g_limit || n > g_limit - g_used) return cudaErrorMemoryAllocation;
     // (a device pointer: nothing reads or writes through it but cudaMemcpy)
     *p = std::malloc(n < (1u << 23) ? n : 16);
     g_live[*p] = n;
@@ -126,8 +126,25 @@ static int backward_mode(bool tc, size_t left) {
     return 0;
 }
 
+// resize: a pass of 2 x 64 x 64, then one of 1 x 64 x 64 without memory for it,
+// twice: it has to fail both times.
+static int resize_mode() {
+    Denoiser d;
+    if (d.init(1) != cudaSuccess) return 3;
+    float rad;
+    __half feat;
+    std::printf("%d", (int)d.forward(&rad, &feat, 2, 64, 64, nullptr));
+    g_limit = 1 << 20;
+    if (g_used < g_limit) return 4;
+    for (int i = 0; i < 2; i++) std::printf(" %d", (int)d.forward(&rad, &feat, 1, 64, 64, nullptr));
+    g_limit = SIZE_MAX;
+    std::printf(" %d\n", (int)d.forward(&rad, &feat, 1, 64, 64, nullptr));
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string mode = argc > 1 ? argv[1] : "";
     if (mode == "backward") return backward_mode(std::atoi(argv[2]) != 0, (size_t)std::atoll(argv[3]));
+    if (mode == "resize") return resize_mode();
     return 2;
 }

@@ -37,3 +37,9 @@ def test_failed_backward_gives_its_buffers_back(alloc_check, tensor_cores, left)
     assert codes == (OUT_OF_MEMORY,) * 3 + ("0",)
     assert used[:3] == (forward,) * 3
     assert int(used[3]) > int(forward)
+
+
+def test_failed_resize_fails_again(alloc_check):
+    """A pass of another size that finds no memory is not taken for a made one
+    by the next call of that size, which would run without buffers."""
+    assert alloc_check("resize") == ["0", OUT_OF_MEMORY, OUT_OF_MEMORY, "0"]
