@@ -19,8 +19,8 @@
 // key: the position; owner: kNoOwner. After the references come the culling
 // copy's triangles, each once, in its leaf order: with one owner (a leaf of
 // the exact copy) owner is that leaf's node and key its position, with more
-// owner is kOwnerList | their number and key the first one's index in the
-// owner lists.
+// owner is kOwnerList | the entries of its list (GOwner) and key the first
+// entry's index.
 // Shading records: per triangle id, normal (w: 1 for emitters) and colour.
 #pragma once
 
@@ -51,8 +51,13 @@ struct alignas(16) GTri {
 };
 static_assert(sizeof(GTri) == 48, "GTri must be 48 bytes");
 
+// An entry of a triangle's owner list. A leaf of the exact copy: its node and
+// the reference's position there. Or an ancestor of the entries that follow:
+// its node, and kOwnerGroup | the number in the list of the first entry that is
+// not below it, to go on from where its box misses.
+constexpr uint32_t kOwnerGroup = 0x80000000u;
 struct alignas(8) GOwner {
-    uint32_t leaf, key;  // node of the exact copy, position of the reference
+    uint32_t node, key;
 };
 
 struct alignas(16) GShade {

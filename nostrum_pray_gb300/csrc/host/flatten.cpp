@@ -29,6 +29,8 @@ constexpr float kCullReach = 4.0f;
 // error bound (below): their reported hits can lie anywhere on the rays that
 // reach their leaves.
 constexpr double kSliver = 1.0 / 50.0;
+// Most leaves of an owner list that stand without an ancestor before them.
+constexpr size_t kOwnerRun = 4;
 
 bool sliver(const TriPre &p) {
     const F3 &a = p.ab, &b = p.ac;
@@ -46,6 +48,7 @@ struct Flattener {
     const BuiltTree &t;
     const std::vector<TriPre> &pre;
     DeviceImage &out;
+    std::vector<uint32_t> first_pos{};  // of each node of the exact copy: its first reference's position
 
     void put_tri(uint32_t tri, uint32_t key, uint32_t owner) {
         const TriPre &p = pre[tri];
@@ -61,6 +64,8 @@ struct Flattener {
     // order. leaf_of[i] receives the node of the leaf that holds reference i.
     void put(int32_t p, uint32_t slot, std::vector<uint32_t> &leaf_of) {
         const FlatNode &n = t.nodes[p];
+        first_pos.resize(out.nodes.size());
+        first_pos[slot] = (uint32_t)out.tris.size();
         GNode g;
         for (int k = 0; k < 3; k++) g.lo[k] = n.box.lo[k], g.hi[k] = n.box.hi[k];
         g.a = 0;
@@ -81,6 +86,33 @@ struct Flattener {
         out.nodes[slot] = g;
         put(n.left, pair, leaf_of);
         put(n.right, pair + 1, leaf_of);
+    }
+
+    // The owner list of a triangle with the references at pos[0, n), all below
+    // `node` of the exact copy; its entries are numbered from `list`. Above
+    // kOwnerRun leaves their nearest common ancestor stands before them (but
+    // for the whole list's, whose box a ray that hits the triangle hardly
+    // misses), so that a ray tests the ancestors that it meets instead of every
+    // leaf: a large triangle over a fine mesh has thousands.
+    void put_owners(const uint32_t *pos, size_t n, uint32_t node, size_t list, const std::vector<uint32_t> &leaf_of,
+                    bool whole) {
+        size_t left = 0;
+        while (n > kOwnerRun && !(out.nodes[node].b & kLeafFlag)) {
+            const uint32_t pair = out.nodes[node].a;
+            left = std::lower_bound(pos, pos + n, first_pos[pair + 1]) - pos;
+            if (left && left < n) break;
+            node = left ? pair : pair + 1;
+        }
+        if (!left || left == n) {
+            for (size_t i = 0; i < n; i++) out.owners.push_back(GOwner{leaf_of[pos[i]], pos[i]});
+            return;
+        }
+        const size_t at = out.owners.size();
+        if (!whole) out.owners.push_back(GOwner{node, 0});
+        const uint32_t pair = out.nodes[node].a;
+        put_owners(pos, left, pair, list, leaf_of, false);
+        put_owners(pos + left, n - left, pair + 1, list, leaf_of, false);
+        if (!whole) out.owners[at].key = kOwnerGroup | (uint32_t)(out.owners.size() - list);
     }
 };
 
@@ -115,8 +147,9 @@ void flatten_for_device(const BuiltTree &t, const std::vector<TriPre> &pre, cons
             f.put_tri(tri, of[a], leaf_of[of[a]]);
             continue;
         }
-        f.put_tri(tri, (uint32_t)out.owners.size(), kOwnerList | n);
-        for (uint32_t k = 0; k < n; k++) out.owners.push_back(GOwner{leaf_of[of[a + k]], of[a + k]});
+        const size_t list = out.owners.size();
+        f.put_owners(of.data() + a, n, 0, list, leaf_of, true);
+        f.put_tri(tri, (uint32_t)list, kOwnerList | (uint32_t)(out.owners.size() - list));
     }
     out.cull = bvh->nodes;
     // a sliver's box is that of the leaves that hold it; children come after
@@ -268,16 +301,17 @@ bool validate_device_image(const DeviceImage &img, std::string &why, int *max_de
             std::memcpy(&key, &img.tris[i].e1[3], 4);
             std::memcpy(&owner, &img.tris[i].e2[3], 4);
             const uint64_t n = owner & kOwnerList ? owner & ~kOwnerList : 0;
-            if (owner & kOwnerList ? key + n > img.owners.size() : owner >= img.nodes.size()) {
+            bool ok = owner & kOwnerList ? key + n <= img.owners.size() : owner < img.nodes.size();
+            for (uint64_t k = 0; ok && k < n; k++) {
+                const GOwner &o = img.owners[key + k];
+                const uint64_t next = o.key & ~kOwnerGroup;
+                ok = o.node < img.nodes.size() && (!(o.key & kOwnerGroup) || (next > k && next <= n));
+            }
+            if (!ok) {
                 why = "owner out of bounds";
                 return false;
             }
         }
-        for (const GOwner &o : img.owners)
-            if (o.leaf >= img.nodes.size()) {
-                why = "owner out of bounds";
-                return false;
-            }
     }
     if (max_depth) *max_depth = deepest;
     return true;

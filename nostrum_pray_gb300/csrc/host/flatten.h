@@ -22,7 +22,10 @@
 // nested, so it reaches a leaf exactly when the leaf's own box passes. Each
 // triangle record of the culling copy therefore names its owners, the leaves
 // that hold it, in depth-first order; the first one whose box passes the
-// reference's test gives the hit's key, and a hit without one is dropped.
+// reference's test gives the hit's key, and a hit without one is dropped. Long
+// lists are trees (Flattener::put_owners): leaf after leaf, a two-triangle
+// floor under 64 spheres of 82k triangles (1,737 leaves own it) cost 265 boxes
+// per hit and 1,569 in the worst ray.
 // Other rays use the exact copy.
 #pragma once
 

@@ -173,9 +173,10 @@ __device__ __forceinline__ float4 ldg4(const float *p) { return __ldg(reinterpre
 // Whether the reference reports hits of a triangle record of the culling copy
 // on this ray, and with which key: it holds the triangle in the leaves that
 // own it, in depth-first order, and reaches one of them exactly when its own
-// box passes the reference's slab test (host/flatten.h). References of the
-// exact copy have no owner: the walk came through their leaf. e1w, e2w: the
-// record's key and owner words.
+// box passes the reference's slab test (host/flatten.h). In a list the leaves
+// below an ancestor whose box misses are passed over (boxes are nested).
+// References of the exact copy have no owner: the walk came through their
+// leaf. e1w, e2w: the record's key and owner words.
 __device__ __forceinline__ bool owned(const DevScene &s, const RayF &r, float e1w, float e2w, uint32_t &key);
 
 // One node (box lo + payload a, box hi + payload b) in one 256-bit read-only
@@ -195,16 +196,18 @@ __device__ __forceinline__ bool owned(const DevScene &s, const RayF &r, float e1
     if (owner == kNoOwner) return true;
     const bool list = owner & kOwnerList;
     const uint32_t n = list ? owner & ~kOwnerList : 1u, first = key;
-    for (uint32_t i = 0; i < n; i++) {
-        uint32_t leaf = owner;
+    for (uint32_t i = 0; i < n;) {
+        uint32_t node = owner;
         if (list) {
             const uint2 o = __ldg(reinterpret_cast<const uint2 *>(s.owners + first + i));
-            leaf = o.x, key = o.y;
+            node = o.x, key = o.y;
         }
         float4 lo, hi;
-        ldg_node(s.nodes + leaf, lo, hi);
+        ldg_node(s.nodes + node, lo, hi);
         float tn, tf;
-        if (slab(lo, hi, r, true, tn, tf)) return true;
+        const bool pass = slab(lo, hi, r, true, tn, tf), group = key & kOwnerGroup;
+        if (pass && !group) return true;
+        i = group && !pass ? key & ~kOwnerGroup : i + 1;
     }
     return false;
 }

@@ -4,15 +4,20 @@
 #include <pthread.h>
 #include <dlfcn.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cerrno>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <random>
 #include <string>
+#include <utility>
+#include <vector>
 
 #include "cull_bvh.h"
+#include "flatten.h"
 #include "kdtree.h"
 
 using namespace pray_gpu;
@@ -85,9 +90,103 @@ static int budget_mode(int n) {
     return 0;
 }
 
+struct Ray {
+    float o[3], d[3], inv[3];
+};
+static Ray ray_to(const double o[3], const double p[3]) {
+    Ray r;
+    double d[3], l = 0;
+    for (int k = 0; k < 3; k++) d[k] = p[k] - o[k], l += d[k] * d[k];
+    for (int k = 0; k < 3; k++) r.o[k] = (float)o[k], r.d[k] = (float)(d[k] / std::sqrt(l)), r.inv[k] = 1.0f / r.d[k];
+    return r;
+}
+// the reference's slab test for finite inverses
+static bool slab(const GNode &n, const Ray &r) {
+    float tn = -3.4e38f, tf = 3.4e38f;
+    for (int k = 0; k < 3; k++) {
+        const float a = (n.lo[k] - r.o[k]) * r.inv[k], b = (n.hi[k] - r.o[k]) * r.inv[k];
+        tn = std::max(tn, std::min(a, b)), tf = std::min(tf, std::max(a, b));
+    }
+    return tn <= tf;
+}
+static uint32_t word(float f) {
+    uint32_t w;
+    std::memcpy(&w, &f, 4);
+    return w;
+}
+
+// A two-triangle floor of half-width 10 under `n` small triangles in a thin
+// layer, the SAH tree at its deepest.
+static std::vector<float> floor_scene(size_t n) {
+    auto v = soup(n, 0.004, 3);
+    for (size_t i = 0; i < v.size(); i++) v[i] = i % 3 == 1 ? v[i] + 0.3f : 20.f * (v[i] - 0.5f);
+    const float q[18] = {-10, 0, -10, -10, 0, 10, 10, 0, 10, -10, 0, -10, 10, 0, 10, 10, 0, -10};
+    v.insert(v.end(), q, q + 18);
+    return v;
+}
+
+// owners <n>: over rays from above at the floor, the first owner whose box
+// passes, as the kernels walk a record's list, against every leaf that holds
+// the triangle; the leaves of the floor's lists, and the boxes tested per ray
+// on the average and at most.
+static int owners_mode(size_t n) {
+    const auto verts = floor_scene(n);
+    const auto pre = precompute_triangles(verts.data(), verts.size() / 9, 0);
+    TreeOptions opt;
+    opt.kind = kTreeSah, opt.sah_ct = 1.f;
+    const BuiltTree tree = build_tree(pre, opt);
+    const CullBvh bvh = build_cull_bvh(pre, 4, 0);
+    DeviceImage img;
+    flatten_for_device(tree, pre, &bvh, img);
+    std::string why;
+    if (!validate_device_image(img, why)) return std::printf("%s\n", why.c_str()), 1;
+    std::mt19937 g(5);
+    std::uniform_real_distribution<double> u(-10, 10);
+    size_t leaves = 0, tests = 0, most = 0, hits = 0, wrong = 0;
+    const int kRays = 20000;
+    for (uint32_t tri = (uint32_t)n; tri < n + 2; tri++) {
+        size_t at = img.refs;
+        while (word(img.tris[at].v0[3]) != tri) at++;
+        const uint32_t first = word(img.tris[at].e1[3]), owner = word(img.tris[at].e2[3]), count = owner & 0x7FFFFFFFu;
+        if (!(owner & kOwnerList)) return std::printf("no list\n"), 1;
+        std::vector<std::pair<uint32_t, uint32_t>> all;  // (position, leaf)
+        for (uint32_t i = 0; i < img.nodes.size(); i++) {
+            const GNode &l = img.nodes[i];
+            if (i == 1 || !(l.b & kLeafFlag)) continue;
+            for (uint32_t k = l.a; k < l.a + (l.b & ~kLeafFlag); k++)
+                if (word(img.tris[k].v0[3]) == tri) all.push_back({k, i});
+        }
+        std::sort(all.begin(), all.end());
+        leaves += all.size();
+        for (int q = 0; q < kRays; q++) {
+            const double o[3] = {u(g), 4.0 + 0.3 * u(g), u(g)}, p[3] = {u(g), 0, u(g)};
+            const Ray r = ray_to(o, p);
+            uint32_t want = ~0u, got = ~0u;
+            for (const auto &[pos, leaf] : all)
+                if (slab(img.nodes[leaf], r)) {
+                    want = pos;
+                    break;
+                }
+            size_t t = 0;
+            for (uint32_t i = 0; i < count && got == ~0u;) {
+                uint32_t e[2];
+                std::memcpy(e, &img.owners[first + i], 8);
+                const bool pass = slab(img.nodes[e[0]], r), group = e[1] >> 31;
+                t++;
+                if (pass && !group) got = e[1];
+                i = !pass && group ? e[1] & 0x7FFFFFFFu : i + 1;
+            }
+            wrong += got != want, hits += want != ~0u, tests += t, most = std::max(most, t);
+        }
+    }
+    std::printf("leaves %zu wrong %zu hits %zu mean %.1f most %zu\n", leaves, wrong, hits, tests / (2.0 * kRays), most);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string mode = argc > 1 ? argv[1] : "";
     if (mode == "threads") return threads_mode(std::atoi(argv[2]));
     if (mode == "budget") return budget_mode(std::atoi(argv[2]));
+    if (mode == "owners") return owners_mode((size_t)std::atoll(argv[2]));
     return 2;
 }

@@ -41,3 +41,16 @@ def test_build_threads_bounds_the_whole_build(cull_check, n):
     assert r.returncode == 0, r.stderr
     most = int(r.stdout.split()[1])
     assert most <= 2 * n - 1
+
+
+@pytest.mark.parametrize("n", [40, 200, 100_000])
+def test_owners_of_a_large_triangle(cull_check, n):
+    """A hit on a floor that thousands of leaves hold finds the first leaf whose
+    box the ray passes, with the box tests of a walk down a tree and not of
+    all the leaves."""
+    r = cull_check("owners", n)
+    assert r.returncode == 0, r.stdout + r.stderr
+    v = dict(zip(r.stdout.split()[::2], map(float, r.stdout.split()[1::2])))
+    assert v["wrong"] == 0 and v["hits"] > 0
+    assert v["leaves"] > 0 if n < 100_000 else v["leaves"] > 1000
+    assert v["mean"] < 40 and v["most"] < 160

@@ -1,0 +1,65 @@
+"""Scenes whose triangles differ much in size, position or soundness: ray
+queries, occlusion and frames against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+from nostrum_pray_gb300 import native, scenes
+from test_trace_gpu import _well_posed, check_frame, trace
+
+pytestmark = pytest.mark.gpu
+
+
+def _mesh(v):
+    v = np.asarray(v, np.float32).reshape(-1, 9)
+    return scenes.Mesh(v, np.full((len(v), 3), 0.5, np.float32), np.zeros(len(v), np.uint8))
+
+
+def _floor(half):
+    h = float(half)
+    return np.array([[-h, 0, -h, -h, 0, h, h, 0, h], [-h, 0, -h, h, 0, h, h, 0, -h]])
+
+
+def _rays(o, p):
+    d = p - o
+    d = (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)
+    with np.errstate(divide="ignore", over="ignore"):
+        return np.concatenate([o.astype(np.float32), d, (np.float32(1) / d).astype(np.float32)], 1)
+
+
+def _setup(tree, **kw):
+    st = scenes.soup_setup(**kw)
+    st.tree, st.leaf_size, st.sah_ct, st.max_depth, st.det_eps = tree, 8, 1.0, 20, 0.0
+    return st
+
+
+def _check_queries(oracle, m, st, rays, seed=9):
+    rays = np.ascontiguousarray(rays[_well_posed(m, rays) & np.isfinite(rays[:, 6:9]).all(1)])
+    assert len(rays) > 1000
+    sc = native.Scene.from_setup(m, st)
+    want, want_t = oracle.OracleScene.from_setup(m, st).trace(rays, st.det_eps)
+    ids, ts = trace(sc, rays, st.det_eps)
+    np.testing.assert_array_equal(ids, want.astype(np.int32))
+    np.testing.assert_array_equal(ts.view(np.uint32), want_t.view(np.uint32))
+    rng = np.random.default_rng(seed)
+    with np.errstate(over="ignore"):
+        d2 = (np.minimum(want_t, 1e3) ** 2 * rng.choice([0.9, 1.0, 1.1], len(rays))).astype(np.float32)
+        want_occ = (want >= 0) & (want_t * want_t < d2)
+    occ = torch.empty(len(rays), dtype=torch.uint8, device="cuda")
+    sc.trace_occluded(torch.from_numpy(rays).cuda(), torch.from_numpy(d2).cuda(), st.det_eps, occ)
+    np.testing.assert_array_equal(occ.cpu().numpy(), want_occ.astype(np.uint8))
+    return sc, want
+
+
+@pytest.mark.parametrize("tree", ["median", "sah"])
+@pytest.mark.parametrize("n", [6, 400, 4000])
+def test_large_triangles_over_a_fine_mesh(oracle, n, tree):
+    """A floor of two triangles that many leaves of the SAH tree hold: its owner
+    lists run from a few leaves to trees of them."""
+    rng = np.random.default_rng(n)
+    small = rng.uniform(-10, 10, (n, 1, 3)) * [1, 0, 1] + [0, 0.5, 0] + rng.uniform(-0.08, 0.08, (n, 3, 3))
+    m = _mesh(np.concatenate([small.reshape(-1, 9), _floor(10)]))
+    u = lambda lo, hi: rng.uniform(lo, hi, (4000, 3))  # noqa: E731
+    rays = _rays(u([-10, 3, -10], [10, 6, 10]), u([-10, 0, -10], [10, 0, 10]))
+    _, want = _check_queries(oracle, m, _setup(tree), rays)
+    assert (want >= n).sum() > 1000
