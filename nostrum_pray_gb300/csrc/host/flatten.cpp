@@ -25,6 +25,19 @@ constexpr float kPadRel = 1.0f / 65536.0f;
 // test (p * inv - o * inv) adds at most 1/25 of the pad.
 constexpr float kPadScene = 1.0f / 65536.0f;
 constexpr float kCullReach = 4.0f;
+// Where such pads are large against the triangles, the culling copy serves a
+// smaller ball of origins: growth is the mean factor by which the pads grow the
+// area of the leaves' boxes inside it. Walks of 300k rays near an 81,920-triangle
+// sphere of radius 1 on a two-triangle floor, node pairs / triangles per ray:
+// growth 1.04 (half-width 3) 21 / 5, 2.2 (100) 25 / 10, 3.9 (2,000, a ball of
+// 2,828) 30 / 16, 8.6 (400, all origins) 41 / 33, 64 (2,000, all origins) 221 /
+// 394, where the reference's tree, which the origins outside take, costs 26 /
+// 92. Up to kRegionGrowth the wider ball is kept, and always where the
+// reference's tree has large leaves (kRegionLeaf: the mean size of the leaf that
+// a reference is in), which origins outside the ball would scan.
+constexpr double kRegionGrowth = 4.0, kRegionLeaf = 64.0;
+constexpr int kRegionSteps = 8;
+constexpr size_t kRegionSample = 4096;  // leaves looked at
 // Triangles with a smaller sine of their smallest angle are outside the pad's
 // error bound (below): their reported hits can lie anywhere on the rays that
 // reach their leaves.
@@ -42,6 +55,90 @@ bool sliver(const TriPre &p) {
                    len((double)b[0] - a[0], (double)b[1] - a[1], (double)b[2] - a[2])};
     std::sort(e, e + 3);  // the smallest angle lies between the two longest edges
     return !(area > kSliver * e[1] * e[2]);
+}
+
+double half_area(const GNode &g) {
+    const double x = (double)g.hi[0] - g.lo[0], y = (double)g.hi[1] - g.lo[1], z = (double)g.hi[2] - g.lo[2];
+    return x * y + y * z + z * x;
+}
+
+// The origins that the culling copy serves (a ball) and the pads it needs for
+// them.
+struct Region {
+    float c[3], radius;
+    float pad_all;  // > 0: the absolute part of every box's pad; else it depends on the box's distance
+    // b = a, padded
+    void pad(const GNode &a, GNode &b) const {
+        float all = pad_all;
+        if (!(all > 0.f)) {
+            double far2 = 0.0;  // from c to the box's farthest corner
+            for (int k = 0; k < 3; k++) {
+                const double d = std::max(std::fabs((double)a.lo[k] - c[k]), std::fabs((double)a.hi[k] - c[k]));
+                far2 += d * d;
+            }
+            all = (float)((radius + std::sqrt(far2)) * (kPadScene / (kCullReach + 1.0f)));
+        }
+        for (int k = 0; k < 3; k++) {
+            const float p = (std::fabs(a.lo[k]) + std::fabs(a.hi[k]) + (a.hi[k] - a.lo[k])) * kPadRel + all + 1e-30f;
+            b.lo[k] = a.lo[k] - p;
+            b.hi[k] = a.hi[k] + p;
+        }
+    }
+};
+
+// The widest region whose pads leave the leaves' boxes near their own size: the
+// reach of kCullReach diagonals around the scene, or, where the scene holds
+// something fine and small (a mesh on a floor a thousand times its size),
+// balls an eighth of that and so on around the middle of its leaves. cull:
+// unpadded boxes. shrink: smaller balls are allowed.
+Region choose_region(const std::vector<GNode> &cull, const Aabb &root, float diag, bool shrink) {
+    Region wide;
+    for (int k = 0; k < 3; k++) wide.c[k] = 0.5f * (root.lo[k] + root.hi[k]);
+    wide.radius = kCullReach * diag;
+    wide.pad_all = diag * kPadScene;
+    if (!shrink) return wide;
+    std::vector<uint32_t> leaves;  // a sample
+    for (size_t i = 0; i < cull.size(); i++)
+        if (i != 1 && (cull[i].b & kLeafFlag) && half_area(cull[i]) > 0.0 && std::isfinite(half_area(cull[i])))
+            leaves.push_back((uint32_t)i);
+    if (leaves.empty()) return wide;
+    if (leaves.size() > kRegionSample) {
+        const size_t step = leaves.size() / kRegionSample;
+        for (size_t i = 0; i < kRegionSample; i++) leaves[i] = leaves[i * step];
+        leaves.resize(kRegionSample);
+    }
+    // mean growth of the area of the leaves whose centre lies in the region
+    auto growth = [&](const Region &r) {
+        double sum = 0.0;
+        size_t n = 0;
+        for (uint32_t i : leaves) {
+            const GNode &g = cull[i];
+            double d2 = 0.0;
+            for (int k = 0; k < 3; k++) {
+                const double d = 0.5 * ((double)g.lo[k] + g.hi[k]) - r.c[k];
+                d2 += d * d;
+            }
+            if (d2 > (double)r.radius * r.radius) continue;
+            GNode p = g;
+            r.pad(g, p);
+            sum += std::min(half_area(p) / half_area(g), 64.0), n++;
+        }
+        return n ? sum / n : 0.0;
+    };
+    if (growth(wide) <= kRegionGrowth) return wide;
+    Region r = wide;
+    r.pad_all = 0.f;
+    for (int k = 0; k < 3; k++) {
+        std::vector<float> at;
+        for (uint32_t i : leaves) at.push_back(0.5f * (cull[i].lo[k] + cull[i].hi[k]));
+        std::nth_element(at.begin(), at.begin() + at.size() / 2, at.end());
+        r.c[k] = at[at.size() / 2];
+    }
+    for (int step = 0; step < kRegionSteps; step++) {
+        r.radius /= 8.f;
+        if (growth(r) <= kRegionGrowth) break;
+    }
+    return r;
 }
 
 struct Flattener {
@@ -133,8 +230,6 @@ void flatten_for_device(const BuiltTree &t, const std::vector<TriPre> &pre, cons
     out.refs = out.tris.size();
     // (no culling copy where its leaves' words could not hold the records' numbers)
     if (!bvh || !sized || out.refs + pre.size() >= (1ull << kCullCountShift)) return;
-    for (int k = 0; k < 3; k++) out.cull_center[k] = 0.5f * (root.lo[k] + root.hi[k]);
-    out.cull_radius2 = (kCullReach * diag) * (kCullReach * diag);
     // each triangle's references, in depth-first order
     std::vector<uint32_t> first(pre.size() + 1, 0);
     for (uint32_t tri : t.refs) first[tri + 1]++;
@@ -175,15 +270,15 @@ void flatten_for_device(const BuiltTree &t, const std::vector<TriPre> &pre, cons
             }
         }
     }
-    const float pad_scene = diag * kPadScene;
+    double scanned = 0.0;
+    for (const FlatNode &n : t.nodes)
+        if (n.left < 0) scanned += (double)n.count * n.count;
+    const Region region = choose_region(out.cull, root, diag, scanned <= kRegionLeaf * out.refs);
+    for (int k = 0; k < 3; k++) out.cull_center[k] = region.c[k];
+    out.cull_radius2 = region.radius * region.radius;
     for (GNode &g : out.cull) {
         if (g.b & kLeafFlag) g.a += (uint32_t)out.refs;
-        for (int k = 0; k < 3; k++) {
-            const float pad =
-                (std::fabs(g.lo[k]) + std::fabs(g.hi[k]) + (g.hi[k] - g.lo[k])) * kPadRel + pad_scene + 1e-30f;
-            g.lo[k] -= pad;
-            g.hi[k] += pad;
-        }
+        region.pad(g, g);
     }
 }
 

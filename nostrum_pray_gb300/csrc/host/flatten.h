@@ -10,7 +10,10 @@
 // with the origin) is finite and whose origin lies within cull_radius2 of
 // cull_center. It is a hierarchy of its own (cull_bvh.h) over the triangles
 // that the reference's tree holds, each once, whose boxes are the triangles'
-// bounds padded by a relative 2^-16 and by 2^-16 of the scene's diagonal: a ray
+// bounds padded by a relative 2^-16 and by a share of the way that a ray from
+// within that ball can have come (2^-16 of the scene's diagonal where the ball
+// reaches four diagonals around the scene; less in a smaller one, which scenes
+// with fine detail in a large extent get: flatten.cpp choose_region): a ray
 // skips a box only if it cannot come within that pad of any triangle inside,
 // and for such origins the pad exceeds the float error of the slab test and
 // the distance by which a hit that the one-sided Moeller-Trumbore test reports
@@ -44,7 +47,7 @@ struct DeviceImage {
     std::vector<GNode> nodes;   // the exact copy
     std::vector<GNode> cull;    // the culling copy (child indices from its own start); empty: none
     float cull_center[3] = {0.f, 0.f, 0.f};
-    float cull_radius2 = -1.f;  // origins within sqrt of this of cull_center may use the culling copy
+    float cull_radius2 = -1.f;  // origins within sqrt of this of cull_center use the culling copy
     std::vector<GTri> tris;     // leaf references of the exact copy, then the triangles of the culling copy
     uint64_t refs = 0;          // the former
     std::vector<GOwner> owners; // owner lists of triangles with more than one

@@ -183,10 +183,48 @@ static int owners_mode(size_t n) {
     return 0;
 }
 
+// mixed <half-width>: 30,000 small triangles in a unit cube on a two-triangle
+// floor of that half-width, median tree; leaf triangles per ray whose boxes the ray's line
+// passes in the culling copy, for rays between points near the cube, and
+// whether their origins are the culling copy's to serve.
+static int mixed_mode(float half) {
+    auto verts = soup(30000, 0.01, 4);
+    const float h = half, q[18] = {-h, 0, -h, -h, 0, h, h, 0, h, -h, 0, -h, h, 0, h, h, 0, -h};
+    verts.insert(verts.end(), q, q + 18);
+    const auto pre = precompute_triangles(verts.data(), verts.size() / 9, 0);
+    TreeOptions opt;
+    const BuiltTree tree = build_tree(pre, opt);
+    const CullBvh bvh = build_cull_bvh(pre, 4, 0);
+    DeviceImage img;
+    flatten_for_device(tree, pre, &bvh, img);
+    std::mt19937 g(5);
+    std::uniform_real_distribution<double> u(-1, 2);
+    const int kRays = 2000;
+    size_t tris = 0, served = 0;
+    for (int i = 0; i < kRays; i++) {
+        const double o[3] = {u(g), u(g), u(g)}, p[3] = {u(g), u(g), u(g)};
+        const Ray r = ray_to(o, p);
+        float d2 = 0;
+        for (int k = 0; k < 3; k++) d2 += (r.o[k] - img.cull_center[k]) * (r.o[k] - img.cull_center[k]);
+        served += d2 <= img.cull_radius2;
+        std::vector<uint32_t> todo{0};
+        while (!todo.empty()) {
+            const GNode &n = img.cull[todo.back()];
+            todo.pop_back();
+            if (!slab(n, r)) continue;
+            if (n.b & kLeafFlag) tris += n.b & ~kLeafFlag;
+            else todo.push_back(n.a), todo.push_back(n.a + 1);
+        }
+    }
+    std::printf("tris %.2f served %.3f\n", (double)tris / kRays, (double)served / kRays);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string mode = argc > 1 ? argv[1] : "";
     if (mode == "threads") return threads_mode(std::atoi(argv[2]));
     if (mode == "budget") return budget_mode(std::atoi(argv[2]));
     if (mode == "owners") return owners_mode((size_t)std::atoll(argv[2]));
+    if (mode == "mixed") return mixed_mode((float)std::atof(argv[2]));
     return 2;
 }

@@ -54,3 +54,16 @@ def test_owners_of_a_large_triangle(cull_check, n):
     assert v["wrong"] == 0 and v["hits"] > 0
     assert v["leaves"] > 0 if n < 100_000 else v["leaves"] > 1000
     assert v["mean"] < 40 and v["most"] < 160
+
+
+@pytest.mark.parametrize("half", [50, 1000, 30_000])
+def test_fine_detail_in_a_large_scene(cull_check, half):
+    """The pads of the culling boxes follow the origins served: rays near a fine
+    object test hardly more triangles on a large floor than on a small one."""
+    def run(h):
+        r = cull_check("mixed", h)
+        assert r.returncode == 0, r.stderr
+        return dict(zip(r.stdout.split()[::2], map(float, r.stdout.split()[1::2])))
+    small, large = run(2), run(half)
+    assert large["served"] == 1.0
+    assert large["tris"] < 4 * small["tris"]

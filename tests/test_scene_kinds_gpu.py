@@ -63,3 +63,20 @@ def test_large_triangles_over_a_fine_mesh(oracle, n, tree):
     rays = _rays(u([-10, 3, -10], [10, 6, 10]), u([-10, 0, -10], [10, 0, 10]))
     _, want = _check_queries(oracle, m, _setup(tree), rays)
     assert (want >= n).sum() > 1000
+
+
+@pytest.mark.parametrize("tree", ["median", "sah"])
+@pytest.mark.parametrize("half", [30.0, 1000.0, 20_000.0])
+def test_fine_detail_in_a_large_scene(oracle, half, tree):
+    """A fine object on a large floor: rays from near the object, from far across
+    the floor and from beyond it (culling boxes, and the reference's tree for
+    the origins they do not serve)."""
+    rng = np.random.default_rng(int(half))
+    small = rng.uniform(-1, 1, (3000, 1, 3)) + [0, 1.2, 0] + rng.uniform(-0.05, 0.05, (3000, 3, 3))
+    m = _mesh(np.concatenate([small.reshape(-1, 9), _floor(half)]))
+    at = small.reshape(-1, 3)[rng.integers(0, 9000, 4000)]
+    span = 10.0 ** rng.uniform(0.3, np.log10(2 * half), (4000, 1))
+    o = rng.normal(size=(4000, 3))
+    o = o / np.linalg.norm(o, axis=1, keepdims=True) * span
+    o[:, 1] = np.abs(o[:, 1]) + 0.5
+    _check_queries(oracle, m, _setup(tree), _rays(o, at + rng.uniform(-0.02, 0.02, (4000, 3))))
