@@ -38,23 +38,23 @@ constexpr float kCullReach = 4.0f;
 constexpr double kRegionGrowth = 4.0, kRegionLeaf = 64.0;
 constexpr int kRegionSteps = 8;
 constexpr size_t kRegionSample = 4096;  // leaves looked at
-// Triangles with a smaller sine of their smallest angle are outside the pad's
-// error bound (below): their reported hits can lie anywhere on the rays that
-// reach their leaves.
-constexpr double kSliver = 1.0 / 50.0;
+// Moeller-Trumbore's error in u and v is u(R + D) over the sine of the angle
+// between the two edges it works with (ab, ac) and of b, along those edges.
+// Where that angle's sine is below kSliver the pad does not cover it: such a
+// triangle's bounds grow along its edges by the error at sin b = 1/2, or its
+// box is that of the leaves that hold it (hits of one without area can lie
+// anywhere on the rays that reach them), whichever is smaller. Triangles per
+// ray at 60 cylinders of 64 strips: 2.0, with every sliver boxed as its leaves
+// 460 (median tree), 62 (SAH), all of them (one leaf). 200k rays at 3,000 slivers
+// of any sine from 1e-9 up: the distances of the reference's tree.
+constexpr double kSliver = 1.0 / 50.0, kSliverGrazing = 1.0 / 2.0;
+// References of a leaf up to which it stands for the slivers it holds.
+constexpr uint32_t kSliverLeaf = 64;
 // Most leaves of an owner list that stand without an ancestor before them.
 constexpr size_t kOwnerRun = 4;
 
-bool sliver(const TriPre &p) {
-    const F3 &a = p.ab, &b = p.ac;
-    const double c[3] = {(double)a[1] * b[2] - (double)a[2] * b[1], (double)a[2] * b[0] - (double)a[0] * b[2],
-                         (double)a[0] * b[1] - (double)a[1] * b[0]};
-    auto len = [](double x, double y, double z) { return std::sqrt(x * x + y * y + z * z); };
-    const double area = len(c[0], c[1], c[2]);
-    double e[3] = {len(a[0], a[1], a[2]), len(b[0], b[1], b[2]),
-                   len((double)b[0] - a[0], (double)b[1] - a[1], (double)b[2] - a[2])};
-    std::sort(e, e + 3);  // the smallest angle lies between the two longest edges
-    return !(area > kSliver * e[1] * e[2]);
+void grow(GNode &g, const GNode &b) {
+    for (int k = 0; k < 3; k++) g.lo[k] = std::min(g.lo[k], b.lo[k]), g.hi[k] = std::max(g.hi[k], b.hi[k]);
 }
 
 double half_area(const GNode &g) {
@@ -67,17 +67,19 @@ double half_area(const GNode &g) {
 struct Region {
     float c[3], radius;
     float pad_all;  // > 0: the absolute part of every box's pad; else it depends on the box's distance
+    // the absolute part of a box's pad
+    float absolute(const GNode &a) const {
+        if (pad_all > 0.f) return pad_all;
+        double far2 = 0.0;  // from c to the box's farthest corner
+        for (int k = 0; k < 3; k++) {
+            const double d = std::max(std::fabs((double)a.lo[k] - c[k]), std::fabs((double)a.hi[k] - c[k]));
+            far2 += d * d;
+        }
+        return (float)((radius + std::sqrt(far2)) * (kPadScene / (kCullReach + 1.0f)));
+    }
     // b = a, padded
     void pad(const GNode &a, GNode &b) const {
-        float all = pad_all;
-        if (!(all > 0.f)) {
-            double far2 = 0.0;  // from c to the box's farthest corner
-            for (int k = 0; k < 3; k++) {
-                const double d = std::max(std::fabs((double)a.lo[k] - c[k]), std::fabs((double)a.hi[k] - c[k]));
-                far2 += d * d;
-            }
-            all = (float)((radius + std::sqrt(far2)) * (kPadScene / (kCullReach + 1.0f)));
-        }
+        const float all = absolute(a);
         for (int k = 0; k < 3; k++) {
             const float p = (std::fabs(a.lo[k]) + std::fabs(a.hi[k]) + (a.hi[k] - a.lo[k])) * kPadRel + all + 1e-30f;
             b.lo[k] = a.lo[k] - p;
@@ -185,6 +187,40 @@ struct Flattener {
         put(n.right, pair + 1, leaf_of);
     }
 
+    // The box of triangle tri, held by the leaves of the n references at pos, if
+    // it is a sliver.
+    bool sliver_box(uint32_t tri, const Region &region, const uint32_t *pos, size_t n,
+                    const std::vector<uint32_t> &leaf_of, GNode &box) const {
+        const TriPre &p = pre[tri];
+        const F3 &a = p.ab, &b = p.ac;
+        const double c[3] = {(double)a[1] * b[2] - (double)a[2] * b[1], (double)a[2] * b[0] - (double)a[0] * b[2],
+                             (double)a[0] * b[1] - (double)a[1] * b[0]};
+        auto len = [](double x, double y, double z) { return std::sqrt(x * x + y * y + z * z); };
+        const double area = len(c[0], c[1], c[2]), la = len(a[0], a[1], a[2]), lb = len(b[0], b[1], b[2]);
+        // (an edge of no length: the determinant is zero for every ray; not
+        // finite: every ray enters its box)
+        if (!(area <= kSliver * la * lb) || la == 0.0 || lb == 0.0 || !std::isfinite(la + lb)) return false;
+        for (int k = 0; k < 3; k++) box.lo[k] = p.box.lo[k], box.hi[k] = p.box.hi[k];
+        const double sine = area / (la * lb);
+        double by = region.absolute(box) * kSliver / (kSliverGrazing * sine);
+        GNode held;
+        for (int k = 0; k < 3; k++) held.lo[k] = INFINITY, held.hi[k] = -INFINITY;
+        bool small = n > 0;
+        for (size_t i = 0; i < n && small; i++) {
+            const GNode &leaf = out.nodes[leaf_of[pos[i]]];
+            small = (leaf.b & ~kLeafFlag) <= kSliverLeaf;
+            grow(held, leaf);
+        }
+        if (!small) by = std::min(by, std::max(la, lb));
+        for (int k = 0; k < 3; k++) {
+            const float e = (float)(by * (std::fabs(a[k]) / la + std::fabs(b[k]) / lb));
+            box.lo[k] -= e;
+            box.hi[k] += e;
+        }
+        if (small && !(half_area(box) < half_area(held))) box = held;
+        return true;
+    }
+
     // The owner list of a triangle with the references at pos[0, n), all below
     // `node` of the exact copy; its entries are numbered from `list`. Above
     // kOwnerRun leaves their nearest common ancestor stands before them (but
@@ -247,15 +283,21 @@ void flatten_for_device(const BuiltTree &t, const std::vector<TriPre> &pre, cons
         f.put_tri(tri, (uint32_t)list, kOwnerList | (uint32_t)(out.owners.size() - list));
     }
     out.cull = bvh->nodes;
-    // a sliver's box is that of the leaves that hold it; children come after
-    // their parents
-    std::vector<uint32_t> thin;  // positions in bvh->order
-    for (uint32_t i = 0; i < (uint32_t)bvh->order.size(); i++)
-        if (sliver(pre[bvh->order[i]])) thin.push_back(i);
+    double scanned = 0.0;
+    for (const FlatNode &n : t.nodes)
+        if (n.left < 0) scanned += (double)n.count * n.count;
+    const Region region = choose_region(out.cull, root, diag, scanned <= kRegionLeaf * out.refs);
+    for (int k = 0; k < 3; k++) out.cull_center[k] = region.c[k];
+    out.cull_radius2 = region.radius * region.radius;
+    // the slivers' boxes; children come after their parents
+    std::vector<std::pair<uint32_t, GNode>> thin;  // positions in bvh->order
+    for (uint32_t i = 0; i < (uint32_t)bvh->order.size(); i++) {
+        const uint32_t tri = bvh->order[i];
+        GNode box;
+        if (!f.sliver_box(tri, region, of.data() + first[tri], first[tri + 1] - first[tri], leaf_of, box)) continue;
+        thin.push_back({i, box});
+    }
     if (!thin.empty()) {
-        auto grow = [](GNode &g, const GNode &b) {
-            for (int k = 0; k < 3; k++) g.lo[k] = std::min(g.lo[k], b.lo[k]), g.hi[k] = std::max(g.hi[k], b.hi[k]);
-        };
         for (size_t slot = out.cull.size(); slot-- > 0;) {
             GNode &g = out.cull[slot];
             if (slot == 1) continue;
@@ -264,18 +306,12 @@ void flatten_for_device(const BuiltTree &t, const std::vector<TriPre> &pre, cons
                 continue;
             }
             const uint32_t end = g.a + (g.b & ~kLeafFlag);
-            for (auto it = std::lower_bound(thin.begin(), thin.end(), g.a); it != thin.end() && *it < end; ++it) {
-                const uint32_t tri = bvh->order[*it];
-                for (uint32_t k = first[tri]; k < first[tri + 1]; k++) grow(g, out.nodes[leaf_of[of[k]]]);
-            }
+            for (auto it = std::lower_bound(thin.begin(), thin.end(), g.a,
+                                            [](const auto &t, uint32_t at) { return t.first < at; });
+                 it != thin.end() && it->first < end; ++it)
+                grow(g, it->second);
         }
     }
-    double scanned = 0.0;
-    for (const FlatNode &n : t.nodes)
-        if (n.left < 0) scanned += (double)n.count * n.count;
-    const Region region = choose_region(out.cull, root, diag, scanned <= kRegionLeaf * out.refs);
-    for (int k = 0; k < 3; k++) out.cull_center[k] = region.c[k];
-    out.cull_radius2 = region.radius * region.radius;
     for (GNode &g : out.cull) {
         if (g.b & kLeafFlag) g.a += (uint32_t)out.refs;
         region.pad(g, g);

@@ -183,6 +183,54 @@ static int owners_mode(size_t n) {
     return 0;
 }
 
+// Triangles of the culling copy's leaves whose boxes the ray's line passes.
+static size_t line_triangles(const DeviceImage &img, const Ray &r) {
+    size_t tris = 0;
+    std::vector<uint32_t> todo{0};
+    while (!todo.empty()) {
+        const GNode &n = img.cull[todo.back()];
+        todo.pop_back();
+        if (!slab(n, r)) continue;
+        if (n.b & kLeafFlag) tris += n.b & ~kLeafFlag;
+        else todo.push_back(n.a), todo.push_back(n.a + 1);
+    }
+    return tris;
+}
+
+// slivers <strips> <leaf size>: 30 cylinders of thin strips (two triangles
+// each); triangles per ray as above.
+static int slivers_mode(int strips, int leaf_size) {
+    std::mt19937 g(1);
+    std::uniform_real_distribution<double> u(-1, 1);
+    std::vector<float> verts;
+    for (int c = 0; c < 30; c++) {
+        const double o[3] = {3 * u(g), 3 * u(g), 3 * u(g)}, radius = 0.3 + 0.2 * u(g), height = 2.5 + 1.5 * u(g);
+        for (int i = 0; i < strips; i++) {
+            const double a = 2 * M_PI * i / strips, b = 2 * M_PI * (i + 1) / strips;
+            auto put = [&](double at, double y) {
+                for (double x : {o[0] + radius * std::cos(at), o[1] + y, o[2] + radius * std::sin(at)})
+                    verts.push_back((float)x);
+            };
+            put(a, 0), put(a, height), put(b, 0), put(b, 0), put(a, height), put(b, height);
+        }
+    }
+    const auto pre = precompute_triangles(verts.data(), verts.size() / 9, 0);
+    TreeOptions opt;
+    opt.leaf_size = leaf_size;
+    const BuiltTree tree = build_tree(pre, opt);
+    const CullBvh bvh = build_cull_bvh(pre, 4, 0);
+    DeviceImage img;
+    flatten_for_device(tree, pre, &bvh, img);
+    const int kRays = 2000;
+    size_t tris = 0;
+    for (int i = 0; i < kRays; i++) {
+        const double o[3] = {6 * u(g), 6 * u(g), 6 * u(g)}, p[3] = {3 * u(g), 3 * u(g), 3 * u(g)};
+        tris += line_triangles(img, ray_to(o, p));
+    }
+    std::printf("tris %.2f\n", (double)tris / kRays);
+    return 0;
+}
+
 // mixed <half-width>: 30,000 small triangles in a unit cube on a two-triangle
 // floor of that half-width, median tree; leaf triangles per ray whose boxes the ray's line
 // passes in the culling copy, for rays between points near the cube, and
@@ -207,14 +255,7 @@ static int mixed_mode(float half) {
         float d2 = 0;
         for (int k = 0; k < 3; k++) d2 += (r.o[k] - img.cull_center[k]) * (r.o[k] - img.cull_center[k]);
         served += d2 <= img.cull_radius2;
-        std::vector<uint32_t> todo{0};
-        while (!todo.empty()) {
-            const GNode &n = img.cull[todo.back()];
-            todo.pop_back();
-            if (!slab(n, r)) continue;
-            if (n.b & kLeafFlag) tris += n.b & ~kLeafFlag;
-            else todo.push_back(n.a), todo.push_back(n.a + 1);
-        }
+        tris += line_triangles(img, r);
     }
     std::printf("tris %.2f served %.3f\n", (double)tris / kRays, (double)served / kRays);
     return 0;
@@ -226,5 +267,6 @@ int main(int argc, char **argv) {
     if (mode == "budget") return budget_mode(std::atoi(argv[2]));
     if (mode == "owners") return owners_mode((size_t)std::atoll(argv[2]));
     if (mode == "mixed") return mixed_mode((float)std::atof(argv[2]));
+    if (mode == "slivers") return slivers_mode(std::atoi(argv[2]), std::atoi(argv[3]));
     return 2;
 }

@@ -67,3 +67,14 @@ def test_fine_detail_in_a_large_scene(cull_check, half):
     small, large = run(2), run(half)
     assert large["served"] == 1.0
     assert large["tris"] < 4 * small["tris"]
+
+
+@pytest.mark.parametrize("leaf", [8, 32, 10 ** 6])
+@pytest.mark.parametrize("strips", [40, 300, 2000])
+def test_thin_triangles(cull_check, strips, leaf):
+    """A thin triangle's box is its own, grown by the error of its hits, and not
+    that of the leaves that hold it: a line through cylinders of strips meets a
+    few strips on each wall it crosses, whatever the leaf size."""
+    r = cull_check("slivers", strips, leaf)
+    assert r.returncode == 0, r.stderr
+    assert float(r.stdout.split()[1]) < 40

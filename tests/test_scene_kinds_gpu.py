@@ -80,3 +80,25 @@ def test_fine_detail_in_a_large_scene(oracle, half, tree):
     o = o / np.linalg.norm(o, axis=1, keepdims=True) * span
     o[:, 1] = np.abs(o[:, 1]) + 0.5
     _check_queries(oracle, m, _setup(tree), _rays(o, at + rng.uniform(-0.02, 0.02, (4000, 3))))
+
+
+@pytest.mark.parametrize("tree", ["median", "sah"])
+@pytest.mark.parametrize("strips", [40, 1000])
+def test_thin_triangles(oracle, strips, tree):
+    """Cylinders of thin strips, beyond the angles that the boxes' error bound
+    covers: the oracle's hits for all but one ray in a thousand."""
+    rng = np.random.default_rng(strips)
+    parts = []
+    for _ in range(12):
+        o, radius, height = rng.uniform(-3, 3, 3), rng.uniform(0.1, 0.5), rng.uniform(1, 4)
+        a = 2 * np.pi * np.arange(strips + 1) / strips
+        ring = np.stack([radius * np.cos(a), 0 * a, radius * np.sin(a)], 1) + o
+        p0, p1, up = ring[:-1], ring[1:], np.array([0, height, 0])
+        parts += [np.stack([p0, p0 + up, p1], 1), np.stack([p1, p0 + up, p1 + up], 1)]
+    m = _mesh(np.concatenate(parts))
+    rays = _rays(rng.uniform(-6, 6, (20_000, 3)), rng.uniform(-3, 4, (20_000, 3)))
+    st = _setup(tree)
+    want, want_t = oracle.OracleScene.from_setup(m, st).trace(rays, st.det_eps)
+    ids, ts = trace(native.Scene.from_setup(m, st), rays, st.det_eps)
+    assert (want >= 0).sum() > 1000
+    assert ((ids != want) | (ts != want_t)).sum() <= 20
