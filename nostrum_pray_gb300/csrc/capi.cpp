@@ -566,21 +566,21 @@ pray_status pray_scene_create(const float *verts, const float *colors, const uin
             return n ? g.a | kLeafFlag | (n - 1) << kCullCountShift : g.a;
         };
         GridImage grid;
-        if (!img.cull.empty() && !grid_for_device(img.cull, leaf_word, grid) && img.cull.size() > 2)
-            img.cull.clear(), img.cull_radius2 = -1.f;
+        const bool on_grid = grid_for_device(img.cull, leaf_word, grid);
         gnodes.reserve(gnodes.size() + img.cull.size() + grid.pairs.size());
         for (GNode g : img.cull) {
             if (g.b & kLeafFlag) g.a = leaf_word(g);
             gnodes.push_back(g);
         }
-        s->grid_base = (uint32_t)gnodes.size();
+        s->grid_base = on_grid ? (uint32_t)gnodes.size() : 0u;
         s->grid_scale = grid.scale;
         for (int k = 0; k < 3; k++) s->grid_org[k] = grid.org[k];
-        static_assert(sizeof(GPair) == sizeof(GNode), "pairs share the nodes' buffer");
-        gnodes.resize(gnodes.size() + grid.pairs.size());
-        if (!grid.pairs.empty())
+        if (on_grid) {
+            static_assert(sizeof(GPair) == sizeof(GNode), "pairs share the nodes' buffer");
+            gnodes.resize(gnodes.size() + grid.pairs.size());
             std::memcpy(static_cast<void *>(gnodes.data() + s->grid_base), grid.pairs.data(),
                         grid.pairs.size() * sizeof(GPair));
+        }
         gowners.swap(img.owners);
         for (int k = 0; k < 3; k++) s->cull_c[k] = img.cull_center[k];
         s->cull_r2 = img.cull_radius2;

@@ -67,8 +67,8 @@ struct alignas(16) GShade {
 
 // The two children of an interior node of the culling copy with their boxes on
 // a scene-wide grid of 16-bit steps: planes x0 y0 z0 x1 y1 z1 (box min, max),
-// two per word, low half first. The per-lane walks read these, half the bytes
-// of two GNodes. Words as in the culling copy, but an interior child's is the
+// two per word, low half first. Ray queries and the wavefront's passes read
+// these, half the bytes of two GNodes, where a scene has them. Words as in the culling copy, but an interior child's is the
 // index of its own pair.
 struct alignas(32) GPair {
     uint32_t q0[3], w0, q1[3], w1;
@@ -86,7 +86,7 @@ struct DevScene {
     float tol;  // absolute distance tolerance for culling boxes behind the origin
     uint32_t depth;  // deepest node level of the hierarchy (root 0): a traversal pushes at most this many nodes
     float cull_c[3], cull_r2;  // centre and squared radius of the region of origins served by the culling copy
-    uint32_t grid_base;
+    uint32_t grid_base;  // 0: no grid pairs
     float grid_org[3], grid_scale;  // grid origin, 1 / cell (a power of two)
     // emitting triangles (for next-event estimation): geometry as GTri (v0.w
     // = triangle id) and the inclusive prefix sums of their areas

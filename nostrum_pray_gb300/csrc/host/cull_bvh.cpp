@@ -181,9 +181,18 @@ CullBvh build_cull_bvh(const std::vector<TriPre> &tris, int leaf_max, Threads &t
     }
     Builder b{{}, std::min(std::max(1, leaf_max), kCullLeaf), threads, {}, {}};
     b.prims.resize(n);
+    auto has_nan = [](const Aabb &t) {
+        bool nan = false;
+        for (int k = 0; k < 3; k++) nan = nan || std::isnan(t.lo[k]) || std::isnan(t.hi[k]);
+        return nan;
+    };
+    // a triangle with a NaN is hit by no ray (its distance is NaN): it gets a
+    // box that is in the way of nothing, another triangle's
+    size_t sound = 0;
+    while (sound + 1 < n && has_nan(tris[sound].box)) sound++;
     for (size_t i = 0; i < n; i++) {
         Prim &p = b.prims[i];
-        const Aabb &t = tris[i].box;
+        const Aabb &t = tris[has_nan(tris[i].box) ? sound : i].box;
         p.id = (uint32_t)i;
         for (int k = 0; k < 3; k++) {
             const bool ok = std::isfinite(t.lo[k]) && std::isfinite(t.hi[k]);

@@ -259,8 +259,8 @@ void flatten_for_device(const BuiltTree &t, const std::vector<TriPre> &pre, cons
     const Aabb &root = t.nodes[0].box;
     double d2 = 0.0;
     for (int k = 0; k < 3; k++) d2 += ((double)root.hi[k] - root.lo[k]) * ((double)root.hi[k] - root.lo[k]);
-    const bool sized = !t.refs.empty() && std::isfinite(d2);
-    const float diag = sized ? (float)std::sqrt(d2) : 0.f;
+    const float diag = (float)std::sqrt(d2);
+    const bool sized = !t.refs.empty() && std::isfinite(diag);
     std::vector<uint32_t> leaf_of(t.refs.size());
     f.put(0, 0, leaf_of);
     out.refs = out.tris.size();

@@ -35,7 +35,7 @@ unsigned blocks_for(uint64_t n, uint32_t lanes, unsigned threads) {
 // t^2 < dist2 (the any-hit walk stops at the first such triangle). The
 // reference asks for the closest hit and tests lightDistSq > dst * dst
 // (src/pray.cpp:39-43); the closest t satisfies it iff some t does.
-template <int kStackN>
+template <int kStackN, bool kGrid>
 __global__ void __launch_bounds__(128) k_trace_occluded(DevScene s, const float *__restrict__ rays,
                                                         const float *__restrict__ dist2, uint64_t n, uint32_t lanes,
                                                         float eps, uint8_t *__restrict__ occluded) {
@@ -52,11 +52,11 @@ __global__ void __launch_bounds__(128) k_trace_occluded(DevScene s, const float 
         d2 = dist2[i];
     }
     float t;
-    const int pos = traverse<true, false, kStackN, true>(s, r, eps, d2, valid && s.n_refs > 0 && d2 > 0.f, t);
+    const int pos = traverse<true, false, kStackN, kGrid>(s, r, eps, d2, valid && s.n_refs > 0 && d2 > 0.f, t);
     if (valid) occluded[i] = pos >= 0 ? 1 : 0;
 }
 
-template <int kStackN>
+template <int kStackN, bool kGrid>
 __global__ void __launch_bounds__(128) k_trace_closest(DevScene s, const float *__restrict__ rays, uint64_t n,
                                                        uint32_t lanes, float eps, int32_t *__restrict__ ids,
                                                        float *__restrict__ ts) {
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(128) k_trace_closest(DevScene s, const float *
         r.ix = p[6], r.iy = p[7], r.iz = p[8];
     }
     float t;
-    const int pos = traverse<false, false, kStackN, true>(s, r, eps, 0.f, valid && s.n_refs > 0, t);
+    const int pos = traverse<false, false, kStackN, kGrid>(s, r, eps, 0.f, valid && s.n_refs > 0, t);
     if (valid) {
         ids[i] = pos >= 0 ? (int32_t)__float_as_uint(__ldg(&s.tris[pos].v0[3])) : -1;
         ts[i] = t;
@@ -238,8 +238,10 @@ cudaError_t launch_trace_occluded(const DevScene &s, const float *rays, const fl
     const uint32_t lanes = lanes_for(n, resident(sm_count, kTraceWarpsPerSm));
     const unsigned blocks = blocks_for(n, lanes, 128);
     // a 32-entry stack (half the per-thread local memory) when the hierarchy is shallow enough
-    if (s.depth < 32) k_trace_occluded<32><<<blocks, 128, 0, stream>>>(s, rays, dist2, n, lanes, eps, occluded);
-    else k_trace_occluded<kStack><<<blocks, 128, 0, stream>>>(s, rays, dist2, n, lanes, eps, occluded);
+    const bool small = s.depth < 32, grid = s.grid_base != 0;
+    const auto kernel = small ? (grid ? k_trace_occluded<32, true> : k_trace_occluded<32, false>)
+                              : (grid ? k_trace_occluded<kStack, true> : k_trace_occluded<kStack, false>);
+    kernel<<<blocks, 128, 0, stream>>>(s, rays, dist2, n, lanes, eps, occluded);
     return cudaGetLastError();
 }
 
@@ -248,8 +250,10 @@ cudaError_t launch_trace_closest(const DevScene &s, const float *rays, uint64_t 
     if (n == 0) return cudaSuccess;
     const uint32_t lanes = lanes_for(n, resident(sm_count, kTraceWarpsPerSm));
     const unsigned blocks = blocks_for(n, lanes, 128);
-    if (s.depth < 32) k_trace_closest<32><<<blocks, 128, 0, stream>>>(s, rays, n, lanes, eps, ids, ts);
-    else k_trace_closest<kStack><<<blocks, 128, 0, stream>>>(s, rays, n, lanes, eps, ids, ts);
+    const bool small = s.depth < 32, grid = s.grid_base != 0;
+    const auto kernel = small ? (grid ? k_trace_closest<32, true> : k_trace_closest<32, false>)
+                              : (grid ? k_trace_closest<kStack, true> : k_trace_closest<kStack, false>);
+    kernel<<<blocks, 128, 0, stream>>>(s, rays, n, lanes, eps, ids, ts);
     return cudaGetLastError();
 }
 

@@ -293,7 +293,7 @@ __device__ __forceinline__ void leaf_range(const DevScene &s, uint32_t node_off,
     }
 }
 
-// kGrid: the culling copy's boxes come from its grid pairs: one 32-byte load
+// kGrid (scenes with grid pairs): the culling copy's boxes come from its grid pairs: one 32-byte load
 // per pair instead of two, for twelve byte permutes more. The divergent walks
 // of ray queries and of the wavefront's extension and occlusion passes, which
 // L1 throughput bounds (83 to 89 % of its peak under ncu), gain: room 1024^2

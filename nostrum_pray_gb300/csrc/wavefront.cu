@@ -154,7 +154,7 @@ __device__ __forceinline__ uint32_t warp_fetch(uint32_t *counter, unsigned idle,
 // (reset by the shade pass). It also empties the next shade pass's output
 // queue and its occlusion-job count (counts[jobs]; the occlusion pass of the
 // previous bounce, which may run beside this one, reads the other slot).
-template <int kStackN>
+template <int kStackN, bool kGrid>
 __global__ void __launch_bounds__(kThreads, kTraceBlocksPerSm) k_wf_extend(DevScene s, PtLaunch L, WavefrontScratch w,
                                                                          int in, int out, int jobs) {
     constexpr unsigned kFull = 0xFFFFFFFFu;
@@ -181,11 +181,11 @@ __global__ void __launch_bounds__(kThreads, kTraceBlocksPerSm) k_wf_extend(DevSc
                 r.dx = d.x, r.dy = d.y, r.dz = d.z;
                 r.ix = 1.0f / d.x, r.iy = 1.0f / d.y, r.iz = 1.0f / d.z;  // (as make_ray gave)
                 has = true;
-                trav_start<kClosest, true>(s, r, 0.f, s.n_refs > 0, T);
+                trav_start<kClosest, kGrid>(s, r, 0.f, s.n_refs > 0, T);
             }
         }
         if (!__any_sync(kFull, has)) break;
-        trav_round<kClosest, true, false>(s, r, L.eps, 0.f, T, S, nullptr);
+        trav_round<kClosest, kGrid, false>(s, r, L.eps, 0.f, T, S, nullptr);
         if (has && !T.active()) {
             w.dir[p].w = T.best_t;
             w.org[p].w = __int_as_float(T.best);
@@ -491,7 +491,10 @@ cudaError_t wavefront_preload_kernels() {
     cudaFuncAttributes a;
     const void *kernels[] = {
         reinterpret_cast<const void *>(k_wf_first<32>),    reinterpret_cast<const void *>(k_wf_first<kStack>),
-        reinterpret_cast<const void *>(k_wf_extend<32>),   reinterpret_cast<const void *>(k_wf_extend<kStack>),
+        reinterpret_cast<const void *>(k_wf_extend<32, false>),
+        reinterpret_cast<const void *>(k_wf_extend<kStack, false>),
+        reinterpret_cast<const void *>(k_wf_extend<32, true>),
+        reinterpret_cast<const void *>(k_wf_extend<kStack, true>),
         reinterpret_cast<const void *>(k_wf_shade<true>),  reinterpret_cast<const void *>(k_wf_shade<false>),
         reinterpret_cast<const void *>(k_wf_occlude<32, false>),
         reinterpret_cast<const void *>(k_wf_occlude<kStack, false>),
@@ -514,6 +517,7 @@ cudaError_t record_wavefront_frame(const DevScene &s, const PtLaunch &L, const W
     const unsigned grid = (unsigned)std::max(1, sm_count) * kTraceBlocksPerSm;
     const unsigned shade_grid = (unsigned)std::max(1, sm_count) * kShadeBlocksPerSm;
     const bool small_stack = s.depth < 32;  // a 32-entry traversal stack suffices
+    const bool on_grid = s.grid_base != 0;
     // With a side stream, bounce b's occlusion pass runs there, beside bounce
     // b + 1's extend pass (they touch different fields and counters: the
     // two alternate occlusion-job counts, counts[2] and counts[5]), so each
@@ -529,8 +533,9 @@ cudaError_t record_wavefront_frame(const DevScene &s, const PtLaunch &L, const W
         for (uint32_t it = 0; it <= L.max_depth && e == cudaSuccess; it++) {
             const int in = (int)(it & 1), out = 1 - in, jobs = (it & 1) ? 5 : 2;
             if (it > 0) {
-                if (small_stack) k_wf_extend<32><<<grid, kThreads, 0, stream>>>(s, L, w, in, out, jobs);
-                else k_wf_extend<kStack><<<grid, kThreads, 0, stream>>>(s, L, w, in, out, jobs);
+                const auto extend = on_grid ? (small_stack ? k_wf_extend<32, true> : k_wf_extend<kStack, true>)
+                                            : (small_stack ? k_wf_extend<32, false> : k_wf_extend<kStack, false>);
+                extend<<<grid, kThreads, 0, stream>>>(s, L, w, in, out, jobs);
                 if (overlap) e = cudaStreamWaitEvent(stream, join, 0);
                 k_wf_shade<false><<<shade_grid, kThreads, 0, stream>>>(s, L, w, in, out, jobs, it, base, Sr, P);
             } else {
@@ -542,8 +547,9 @@ cudaError_t record_wavefront_frame(const DevScene &s, const PtLaunch &L, const W
                 if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
                 occ = side;
             }
-            const auto occlude = it == 0 ? (small_stack ? k_wf_occlude<32, false> : k_wf_occlude<kStack, false>)
-                                         : (small_stack ? k_wf_occlude<32, true> : k_wf_occlude<kStack, true>);
+            const auto occlude = on_grid && it > 0
+                                     ? (small_stack ? k_wf_occlude<32, true> : k_wf_occlude<kStack, true>)
+                                     : (small_stack ? k_wf_occlude<32, false> : k_wf_occlude<kStack, false>);
             occlude<<<grid, kThreads, 0, occ>>>(s, L, w, jobs);
             if (overlap && e == cudaSuccess) e = cudaEventRecord(join, side);
         }

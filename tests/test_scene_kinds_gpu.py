@@ -102,3 +102,26 @@ def test_thin_triangles(oracle, strips, tree):
     ids, ts = trace(native.Scene.from_setup(m, st), rays, st.det_eps)
     assert (want >= 0).sum() > 1000
     assert ((ids != want) | (ts != want_t)).sum() <= 20
+
+
+@pytest.mark.parametrize("tree", ["median", "sah"])
+@pytest.mark.parametrize("n,odd", [(5000, "nan"), (5000, "far"), (3, None)])
+def test_triangles_without_bounds(oracle, n, odd, tree):
+    """A triangle of NaNs among sound ones (no ray hits it) leaves the others
+    their culling hierarchy: frames fetch hardly more triangles than without it.
+    One whose bounds cannot be squared and a hierarchy of a single leaf give
+    the oracle's answers too."""
+    plain = scenes.soup(n, 3)
+    v = {"nan": [np.nan] * 9, "far": [0, 0, 0, 3e38, 0, 0, 0, 3e38, 0], None: []}[odd]
+    m = _mesh(np.concatenate([plain.verts.reshape(-1), np.array(v)]))
+    st = _setup(tree, width=160, height=120)
+    check_frame(oracle, m, st)
+    rng = np.random.default_rng(4)
+    rays = _rays(rng.uniform(-0.5, 1.5, (3000, 3)), rng.uniform(0, 1, (3000, 3)))
+    want, want_t = oracle.OracleScene.from_setup(m, st).trace(rays, st.det_eps)
+    sc = native.Scene.from_setup(m, st)
+    ids, ts = trace(sc, rays, st.det_eps)
+    assert ((ids != want) | (ts != want_t)).sum() <= 3
+    if odd == "nan":
+        of = [native.Scene.from_setup(x, st).render_rt_counts(st)[3] for x in (m, plain)]
+        assert of[0] < 3 * of[1]
