@@ -57,7 +57,8 @@ struct DeviceImage {
 // 2p and 2p + 1; pair 0 is unused). Every box is rounded outwards by one to
 // two cells: one cell more than the grid needs, for the rounding of the
 // distances that the kernels compute from grid steps (slab_grid). leaf_word:
-// the device's word of a leaf node. False: the boxes do not fit a grid.
+// the device's word of a leaf node. False: the boxes do not fit a grid, or grow
+// too much on one.
 struct GridImage {
     std::vector<GPair> pairs;
     float org[3] = {0.f, 0.f, 0.f}, scale = 1.f;

@@ -197,6 +197,47 @@ static size_t line_triangles(const DeviceImage &img, const Ray &r) {
     return tris;
 }
 
+// grid <half-width>: whether the cube's scene as in mixed_mode, on a floor of
+// that half-width, gets grid pairs; how much wider than the boxes they are
+// (triangles per ray on the grid's boxes over those on the whole nodes').
+static int grid_mode(float half) {
+    auto verts = soup(30000, 0.01, 4);
+    const float h = half, q[18] = {-h, 0, -h, -h, 0, h, h, 0, h, -h, 0, -h, h, 0, h, h, 0, -h};
+    verts.insert(verts.end(), q, q + 18);
+    const auto pre = precompute_triangles(verts.data(), verts.size() / 9, 0);
+    const BuiltTree tree = build_tree(pre, TreeOptions{});
+    const CullBvh bvh = build_cull_bvh(pre, 4, 0);
+    DeviceImage img;
+    flatten_for_device(tree, pre, &bvh, img);
+    GridImage grid;
+    const bool made = grid_for_device(img.cull, [](const GNode &n) { return n.a; }, grid);
+    double ratio = 1.0;
+    if (made) {
+        DeviceImage wide = img;
+        for (size_t p = 1; p < grid.pairs.size(); p++)
+            for (int c = 0; c < 2; c++) {
+                const uint32_t *w = c ? grid.pairs[p].q1 : grid.pairs[p].q0;
+                const uint32_t s[6] = {w[0] & 0xFFFF, w[0] >> 16, w[1] & 0xFFFF, w[1] >> 16, w[2] & 0xFFFF, w[2] >> 16};
+                GNode &n = wide.cull[2 * p + c];
+                for (int k = 0; k < 3; k++) {
+                    n.lo[k] = grid.org[k] + (float)(s[k] / (double)grid.scale);
+                    n.hi[k] = grid.org[k] + (float)(s[3 + k] / (double)grid.scale);
+                }
+            }
+        std::mt19937 g(5);
+        std::uniform_real_distribution<double> u(-1, 2);
+        size_t a = 0, b = 0;
+        for (int i = 0; i < 2000; i++) {
+            const double o[3] = {u(g), u(g), u(g)}, p[3] = {u(g), u(g), u(g)};
+            const Ray r = ray_to(o, p);
+            a += line_triangles(img, r), b += line_triangles(wide, r);
+        }
+        ratio = (double)b / a;
+    }
+    std::printf("made %d ratio %.3f\n", made ? 1 : 0, ratio);
+    return 0;
+}
+
 // slivers <strips> <leaf size>: 30 cylinders of thin strips (two triangles
 // each); triangles per ray as above.
 static int slivers_mode(int strips, int leaf_size) {
@@ -268,5 +309,6 @@ int main(int argc, char **argv) {
     if (mode == "owners") return owners_mode((size_t)std::atoll(argv[2]));
     if (mode == "mixed") return mixed_mode((float)std::atof(argv[2]));
     if (mode == "slivers") return slivers_mode(std::atoi(argv[2]), std::atoi(argv[3]));
+    if (mode == "grid") return grid_mode((float)std::atof(argv[2]));
     return 2;
 }

@@ -78,3 +78,13 @@ def test_thin_triangles(cull_check, strips, leaf):
     r = cull_check("slivers", strips, leaf)
     assert r.returncode == 0, r.stderr
     assert float(r.stdout.split()[1]) < 40
+
+
+@pytest.mark.parametrize("half,made", [(1, True), (3, True), (300, False), (30_000, False)])
+def test_grid_only_where_it_fits_the_boxes(cull_check, half, made):
+    """Grid pairs are made where the scene's 16-bit steps are fine enough for its
+    boxes, and then cost a ray hardly any more triangles."""
+    r = cull_check("grid", half)
+    assert r.returncode == 0, r.stderr
+    v = dict(zip(r.stdout.split()[::2], map(float, r.stdout.split()[1::2])))
+    assert bool(v["made"]) == made and v["ratio"] < 1.5
