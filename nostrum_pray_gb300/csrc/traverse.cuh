@@ -246,8 +246,8 @@ struct Trav {
     // node's first child, or a leaf (kLeafFlag; culling copy: count and first
     // record, exact copy: its node)
     uint32_t w, lw;
-    uint32_t node_off;  // 0: the exact copy, else the culling copy's nodes or grid pairs (finite inverse
-                        // direction, near origin)
+    uint32_t node_off;  // 0: the exact copy, else the culling copy's nodes or (kGrid) its grid pairs (finite
+                        // inverse direction, near origin)
     float cur_tn, leaf_tn, limit, back;  // grid pairs: in cells
     float best_t;
     float nox, noy, noz;  // culling copy: -origin / direction (slab_fma), or slab_grid's
@@ -293,8 +293,15 @@ __device__ __forceinline__ void leaf_range(const DevScene &s, uint32_t node_off,
     }
 }
 
-// kGrid (scenes with grid pairs): the culling copy's boxes come from its grid pairs: one 32-byte load
-// per pair instead of two, for twelve byte permutes more. The divergent walks
+// Whether the walk tests boxes in FMA form (culling copy; kGrid: grid pairs).
+template <bool kGrid>
+__device__ __forceinline__ bool fast_boxes(const DevScene &s, const Trav &T) {
+    return kGrid ? T.node_off == s.grid_base : T.node_off != 0u;
+}
+
+// kGrid (scenes with grid pairs): the culling copy's boxes come from its grid
+// pairs: one 32-byte load per pair instead of two, for twelve byte permutes
+// more. The divergent walks
 // of ray queries and of the wavefront's extension and occlusion passes, which
 // L1 throughput bounds (83 to 89 % of its peak under ncu), gain: room 1024^2
 // at 16 spp 37.43 -> 34.00 ms, 300k closest hits 178 -> 168 us, 100k occlusion
@@ -318,12 +325,14 @@ __device__ __forceinline__ void trav_start(const DevScene &s, const RayF &r, flo
     }
     const float cx = r.ox - s.cull_c[0], cy = r.oy - s.cull_c[1], cz = r.oz - s.cull_c[2];
     if (kGrid) {
-        // (2^23 inverses, and 2^20 cells of inverses, stay finite)
+        // 2^23 inverses, and 2^20 cells of inverses, stay finite; larger ones
+        // walk the culling copy's nodes in the subtraction form (100k rays in
+        // the room with one inverse of 1e33: 209 us, on the exact copy 1,296)
         constexpr float kMaxInv = 1e30f;
-        const bool cull = fabsf(r.ix) < kMaxInv && fabsf(r.iy) < kMaxInv && fabsf(r.iz) < kMaxInv &&
-                          cx * cx + cy * cy + cz * cz <= s.cull_r2;
-        T.node_off = cull ? s.grid_base : 0u;
-        T.finite = cull || (isfinite(r.ix) && isfinite(r.iy) && isfinite(r.iz));
+        const bool near = cx * cx + cy * cy + cz * cz <= s.cull_r2;
+        const bool grid = near && fabsf(r.ix) < kMaxInv && fabsf(r.iy) < kMaxInv && fabsf(r.iz) < kMaxInv;
+        T.finite = grid || (isfinite(r.ix) && isfinite(r.iy) && isfinite(r.iz));
+        T.node_off = grid ? s.grid_base : near && T.finite ? s.n_nodes : 0u;
     } else {
         T.node_off = (T.finite && isfinite(T.nox) && isfinite(T.noy) && isfinite(T.noz) &&
                       cx * cx + cy * cy + cz * cz <= s.cull_r2)
@@ -332,7 +341,7 @@ __device__ __forceinline__ void trav_start(const DevScene &s, const RayF &r, flo
     }
     if (valid) {
         float tn, tf;
-        const GNode *root = s.nodes + (kGrid ? (T.node_off ? s.n_nodes : 0u) : T.node_off);
+        const GNode *root = s.nodes + (T.node_off ? s.n_nodes : 0u);
         float4 rlo, rhi;
         ldg_node(root, rlo, rhi);
         if (slab(rlo, rhi, r, tn, tf)) {
@@ -340,7 +349,7 @@ __device__ __forceinline__ void trav_start(const DevScene &s, const RayF &r, flo
             if (!T.node_off && (__float_as_uint(rhi.w) & kLeafFlag)) T.w = kLeafFlag;  // (node 0)
             T.cur_tn = tn;
             T.have_node = true;
-            if (kGrid && T.node_off) {
+            if (kGrid && fast_boxes<kGrid>(s, T)) {
                 if (!(T.w & kLeafFlag)) T.w /= 2;
                 T.cur_tn *= s.grid_scale, T.limit *= s.grid_scale, T.back *= s.grid_scale;
                 constexpr float kBias = 8388608.f;
@@ -371,7 +380,7 @@ __device__ __forceinline__ void trav_round(const DevScene &s, const RayF &r, flo
             float tn0, tf0, tn1, tf1;
             bool v0, v1;
             // entered: tn <= tf, not beyond the best hit, not behind the origin
-            if (T.node_off) {
+            if (fast_boxes<kGrid>(s, T)) {
                 if (kGrid) {
                     slab_grid(l0.x, l0.y, l0.z, r, T.nox, T.noy, T.noz, tn0, tf0);
                     slab_grid(h0.x, h0.y, h0.z, r, T.nox, T.noy, T.noz, tn1, tf1);
@@ -388,8 +397,10 @@ __device__ __forceinline__ void trav_round(const DevScene &s, const RayF &r, flo
                 }
                 v0 = slab(l0, h0, r, T.finite, tn0, tf0) && tn0 <= T.limit && tf0 >= T.back;
                 v1 = slab(l1, h1, r, T.finite, tn1, tf1) && tn1 <= T.limit && tf1 >= T.back;
-                if (__float_as_uint(h0.w) & kLeafFlag) w0 = kLeafFlag | T.w;
-                if (__float_as_uint(h1.w) & kLeafFlag) w1 = kLeafFlag | (T.w + 1);
+                if (!kGrid || !T.node_off) {
+                    if (__float_as_uint(h0.w) & kLeafFlag) w0 = kLeafFlag | T.w;
+                    if (__float_as_uint(h1.w) & kLeafFlag) w1 = kLeafFlag | (T.w + 1);
+                }
             }
             if (v0 && v1) {
                 const bool first0 = tn0 <= tn1;
@@ -448,7 +459,7 @@ __device__ __forceinline__ void trav_round(const DevScene &s, const RayF &r, flo
                                 T.best = (int)i;
                                 T.best_key = key;
                                 T.limit = t * kPruneRel;
-                                if (kGrid && T.node_off) T.limit *= s.grid_scale;
+                                if (kGrid && fast_boxes<kGrid>(s, T)) T.limit *= s.grid_scale;
                             }
                         }
                     }

@@ -125,3 +125,45 @@ def test_triangles_without_bounds(oracle, n, odd, tree):
     if odd == "nan":
         of = [native.Scene.from_setup(x, st).render_rt_counts(st)[3] for x in (m, plain)]
         assert of[0] < 3 * of[1]
+
+
+@pytest.mark.parametrize("grid", [True, False])
+def test_inverses_beyond_the_grid(oracle, grid):
+    """Directions so close to an axis that an inverse lies between the largest
+    that the grid serves and the largest float: the oracle's hits, at the cost
+    of other near-axis rays (whole nodes of the culling hierarchy, not the
+    reference's leaves one triangle after another)."""
+    m = scenes.room(grid=20)
+    if not grid:
+        m = _mesh(np.concatenate([m.verts, _floor(500) - [0, 5, 0] * 3]))
+    st = scenes.room_setup()
+    rng = np.random.default_rng(6)
+    n = 60_000
+    o = rng.uniform([-0.9, 0.1, -0.9], [0.9, 1.8, 0.9], (n, 3)).astype(np.float32)
+    d = rng.normal(size=(n, 3))
+    d[:, 1] = 0
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    sc = native.Scene.from_setup(m, st)
+    orc = oracle.OracleScene.from_setup(m, st)
+    times = []
+    for y in (1e-20, 2e-31, 1e-35, 1e-37):
+        d[:, 1] = y * rng.choice([-1, 1], n)
+        d32 = d.astype(np.float32)
+        rays = np.concatenate([o, d32, np.float32(1) / d32], 1).astype(np.float32)
+        assert np.isfinite(rays).all()
+        part = rays[:2000]
+        want, want_t = orc.trace(part, st.det_eps)
+        ids, ts = trace(sc, part, st.det_eps)
+        assert ((ids != want) | (ts != want_t)).sum() <= 2
+        r = torch.from_numpy(rays).cuda()
+        out = torch.empty(n, dtype=torch.int32, device="cuda"), torch.empty(n, device="cuda")
+        best = 1e9
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            sc.trace_closest(r, st.det_eps, *out)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        times.append(best)
+    assert max(times[1:]) < 2.5 * times[0], times
