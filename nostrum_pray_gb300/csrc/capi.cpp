@@ -502,7 +502,7 @@ pray_status pray_host_tree_device_layout(const pray_host_tree *t, int32_t leaf_r
         if (!validate_device_image(img, bad)) return set_error(PRAY_ERR_UNSUPPORTED, "device layout: " + bad);
         out[0] = img.nodes.size() + img.cull.size();
         out[1] = img.refs;
-        out[2] = img.tris.size() - img.refs;
+        out[2] = img.culled();
         out[3] = img.cull.size();
         return PRAY_OK;
     })

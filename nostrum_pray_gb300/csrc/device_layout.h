@@ -11,16 +11,16 @@
 // the voxel for the SAH tree) so the kernels apply the reference's slab test
 // to exactly the boxes the reference tests.
 //
-// Triangle references: 48 bytes each, one per leaf entry, in depth-first leaf
-// order (a triangle referenced by two SAH leaves is stored twice). The
-// position of a reference in this array is the reference's depth-first visit
-// order, which breaks distance ties.
+// Triangle records, 48 bytes each:
 //   v0 = (a.xyz, triangle id as bits), e1 = (b - a, key), e2 = (c - a, owner)
-// key: the position; owner: kNoOwner. After the references come the culling
-// copy's triangles, each once, in its leaf order: with one owner (a leaf of
-// the exact copy) owner is that leaf's node and key its position, with more
+// First the culling copy's triangles, each once, in its leaf order (first, so
+// that its leaves' words number nothing else): with one owner (a leaf of the
+// exact copy) owner is that leaf's node and key its position there, with more
 // owner is kOwnerList | the entries of its list (GOwner) and key the first
-// entry's index.
+// entry's index. Then the references of the exact copy, one per leaf entry, in
+// depth-first leaf order (a triangle in two SAH leaves is stored twice): key is
+// the reference's position in this order, which breaks distance ties, owner
+// kNoOwner.
 // Shading records: per triangle id, normal (w: 1 for emitters) and colour.
 #pragma once
 
@@ -30,8 +30,12 @@ namespace pray_gpu {
 
 constexpr uint32_t kLeafFlag = 0x80000000u;
 // Device word of a culling leaf: kLeafFlag | (count - 1) << kCullCountShift |
-// first record (counts up to 4, records below 2^kCullCountShift).
+// first record (counts up to 4, records below 2^kCullCountShift; kernels number
+// all records in an int).
 constexpr int kCullCountShift = 29;
+constexpr bool cull_records_fit(uint64_t refs, uint64_t tris) {
+    return tris < (1ull << kCullCountShift) && refs + tris < (1ull << 31);
+}
 constexpr uint32_t kOwnerList = 0x80000000u, kNoOwner = 0x7FFFFFFFu;
 constexpr int kMaxTreeDepth = 30;        // deepest reference tree the API accepts
 constexpr int kMaxTraversalDepth = 62;   // deepest device hierarchy (reference tree or culling copy)

@@ -155,16 +155,16 @@ struct Flattener {
     const BuiltTree &t;
     const std::vector<TriPre> &pre;
     DeviceImage &out;
+    size_t culled, at = 0;              // records of the culling copy, references placed
     std::vector<uint32_t> first_pos{};  // of each node of the exact copy: its first reference's position
 
-    void put_tri(uint32_t tri, uint32_t key, uint32_t owner) {
+    void put_tri(size_t at, uint32_t tri, uint32_t key, uint32_t owner) {
         const TriPre &p = pre[tri];
-        GTri g;
+        GTri &g = out.tris[at];
         for (int k = 0; k < 3; k++) g.v0[k] = p.a[k], g.e1[k] = p.ab[k], g.e2[k] = p.ac[k];
         std::memcpy(&g.v0[3], &tri, 4);
         std::memcpy(&g.e1[3], &key, 4);
         std::memcpy(&g.e2[3], &owner, 4);
-        out.tris.push_back(g);
     }
 
     // Reference node p into slot, its subtree after it; leaves in depth-first
@@ -172,17 +172,18 @@ struct Flattener {
     void put(int32_t p, uint32_t slot, std::vector<uint32_t> &leaf_of) {
         const FlatNode &n = t.nodes[p];
         first_pos.resize(out.nodes.size());
-        first_pos[slot] = (uint32_t)out.tris.size();
+        first_pos[slot] = (uint32_t)at;
         GNode g;
         for (int k = 0; k < 3; k++) g.lo[k] = n.box.lo[k], g.hi[k] = n.box.hi[k];
         g.a = 0;
         g.b = 0;
         if (n.left < 0) {
-            g.a = (uint32_t)out.tris.size();
+            g.a = (uint32_t)(culled + at);
             g.b = kLeafFlag | n.count;
             for (uint32_t i = n.first; i < n.first + n.count; i++) {
-                put_tri(t.refs[i], i, kNoOwner);
+                put_tri(culled + at, t.refs[i], i, kNoOwner);
                 leaf_of[i] = slot;
+                at++;
             }
             out.nodes[slot] = g;
             return;
@@ -262,33 +263,35 @@ struct Flattener {
 void flatten_for_device(const BuiltTree &t, const std::vector<TriPre> &pre, const CullBvh *bvh, DeviceImage &out) {
     out = DeviceImage{};
     out.nodes.assign(2, GNode{});
-    out.tris.reserve(t.refs.size() + (bvh ? pre.size() : 0));
-    Flattener f{t, pre, out};
     const Aabb &root = t.nodes[0].box;
     double d2 = 0.0;
     for (int k = 0; k < 3; k++) d2 += ((double)root.hi[k] - root.lo[k]) * ((double)root.hi[k] - root.lo[k]);
     const float diag = (float)std::sqrt(d2);
     const bool sized = !t.refs.empty() && std::isfinite(diag);
+    out.refs = t.refs.size();
+    // (no culling copy where its leaves' words could not hold the records' numbers)
+    const bool cull = bvh && sized && cull_records_fit(out.refs, pre.size());
+    const size_t culled = cull ? pre.size() : 0;
+    out.tris.resize(culled + out.refs);
+    Flattener f{t, pre, out, culled};
     std::vector<uint32_t> leaf_of(t.refs.size());
     f.put(0, 0, leaf_of);
-    out.refs = out.tris.size();
-    // (no culling copy where its leaves' words could not hold the records' numbers)
-    if (!bvh || !sized || out.refs + pre.size() >= (1ull << kCullCountShift)) return;
+    if (!cull) return;
     // each triangle's references, in depth-first order
     std::vector<uint32_t> first(pre.size() + 1, 0);
     for (uint32_t tri : t.refs) first[tri + 1]++;
     for (size_t i = 0; i < pre.size(); i++) first[i + 1] += first[i];
     std::vector<uint32_t> at(first.begin(), first.end() - 1), of(t.refs.size());
     for (uint32_t i = 0; i < (uint32_t)t.refs.size(); i++) of[at[t.refs[i]]++] = i;
-    for (uint32_t tri : bvh->order) {
-        const uint32_t a = first[tri], n = first[tri + 1] - a;
+    for (size_t i = 0; i < culled; i++) {
+        const uint32_t tri = bvh->order[i], a = first[tri], n = first[tri + 1] - a;
         if (n == 1) {
-            f.put_tri(tri, of[a], leaf_of[of[a]]);
+            f.put_tri(i, tri, of[a], leaf_of[of[a]]);
             continue;
         }
         const size_t list = out.owners.size();
         f.put_owners(of.data() + a, n, 0, list, leaf_of, true);
-        f.put_tri(tri, (uint32_t)list, kOwnerList | (uint32_t)(out.owners.size() - list));
+        f.put_tri(i, tri, (uint32_t)list, kOwnerList | (uint32_t)(out.owners.size() - list));
     }
     out.cull = bvh->nodes;
     double scanned = 0.0;
@@ -320,10 +323,7 @@ void flatten_for_device(const BuiltTree &t, const std::vector<TriPre> &pre, cons
                 grow(g, it->second);
         }
     }
-    for (GNode &g : out.cull) {
-        if (g.b & kLeafFlag) g.a += (uint32_t)out.refs;
-        region.pad(g, g);
-    }
+    for (GNode &g : out.cull) region.pad(g, g);
 }
 
 bool grid_for_device(const std::vector<GNode> &cull, uint32_t (*leaf_word)(const GNode &), GridImage &out) {
@@ -447,10 +447,10 @@ bool validate_nodes(const std::vector<GNode> &nodes, uint64_t begin, uint64_t en
 
 bool validate_device_image(const DeviceImage &img, std::string &why, int *max_depth) {
     int deepest = 0;
-    if (!validate_nodes(img.nodes, 0, img.refs, why, deepest)) return false;
+    if (!validate_nodes(img.nodes, img.culled(), img.tris.size(), why, deepest)) return false;
     if (!img.cull.empty()) {
-        if (!validate_nodes(img.cull, img.refs, img.tris.size(), why, deepest)) return false;
-        for (uint64_t i = img.refs; i < img.tris.size(); i++) {
+        if (!validate_nodes(img.cull, 0, img.culled(), why, deepest)) return false;
+        for (uint64_t i = 0; i < img.culled(); i++) {
             uint32_t key, owner;
             std::memcpy(&key, &img.tris[i].e1[3], 4);
             std::memcpy(&owner, &img.tris[i].e2[3], 4);

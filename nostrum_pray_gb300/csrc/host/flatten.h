@@ -48,8 +48,9 @@ struct DeviceImage {
     std::vector<GNode> cull;    // the culling copy (child indices from its own start); empty: none
     float cull_center[3] = {0.f, 0.f, 0.f};
     float cull_radius2 = -1.f;  // origins within sqrt of this of cull_center use the culling copy
-    std::vector<GTri> tris;     // leaf references of the exact copy, then the triangles of the culling copy
-    uint64_t refs = 0;          // the former
+    std::vector<GTri> tris;     // triangles of the culling copy, then leaf references of the exact copy
+    uint64_t refs = 0;          // the latter
+    uint64_t culled() const { return tris.size() - refs; }
     std::vector<GOwner> owners; // owner lists of triangles with more than one
 };
 

@@ -145,7 +145,7 @@ static int owners_mode(size_t n) {
     size_t leaves = 0, tests = 0, most = 0, hits = 0, wrong = 0;
     const int kRays = 20000;
     for (uint32_t tri = (uint32_t)n; tri < n + 2; tri++) {
-        size_t at = img.refs;
+        size_t at = 0;
         while (word(img.tris[at].v0[3]) != tri) at++;
         const uint32_t first = word(img.tris[at].e1[3]), owner = word(img.tris[at].e2[3]), count = owner & 0x7FFFFFFFu;
         if (!(owner & kOwnerList)) return std::printf("no list\n"), 1;
@@ -154,7 +154,7 @@ static int owners_mode(size_t n) {
             const GNode &l = img.nodes[i];
             if (i == 1 || !(l.b & kLeafFlag)) continue;
             for (uint32_t k = l.a; k < l.a + (l.b & ~kLeafFlag); k++)
-                if (word(img.tris[k].v0[3]) == tri) all.push_back({k, i});
+                if (word(img.tris[k].v0[3]) == tri) all.push_back({k - (uint32_t)img.culled(), i});
         }
         std::sort(all.begin(), all.end());
         leaves += all.size();
@@ -302,6 +302,12 @@ static int mixed_mode(float half) {
     return 0;
 }
 
+// fits <references> <triangles>: whether such a scene gets a culling copy.
+static int fits_mode(uint64_t refs, uint64_t tris) {
+    std::printf("fits %d\n", cull_records_fit(refs, tris) ? 1 : 0);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string mode = argc > 1 ? argv[1] : "";
     if (mode == "threads") return threads_mode(std::atoi(argv[2]));
@@ -310,5 +316,6 @@ int main(int argc, char **argv) {
     if (mode == "mixed") return mixed_mode((float)std::atof(argv[2]));
     if (mode == "slivers") return slivers_mode(std::atoi(argv[2]), std::atoi(argv[3]));
     if (mode == "grid") return grid_mode((float)std::atof(argv[2]));
+    if (mode == "fits") return fits_mode(std::strtoull(argv[2], nullptr, 0), std::strtoull(argv[3], nullptr, 0));
     return 2;
 }

@@ -69,6 +69,14 @@ def test_fine_detail_in_a_large_scene(cull_check, half):
     assert large["tris"] < 4 * small["tris"]
 
 
+@pytest.mark.parametrize("refs,tris,fits", [(2 ** 30, 2 ** 28, 1), (2 ** 30 + 2 ** 29, 2 ** 29 - 1, 1),
+                                            (2 ** 29, 2 ** 29, 0), (2 ** 31 - 2 ** 20, 2 ** 20, 0)])
+def test_large_scenes_are_culled(cull_check, refs, tris, fits):
+    """The culling copy's limit is its own triangles', not that of all records:
+    its records come first."""
+    assert cull_check("fits", refs, tris).stdout.split() == ["fits", str(fits)]
+
+
 @pytest.mark.parametrize("leaf", [8, 32, 10 ** 6])
 @pytest.mark.parametrize("strips", [40, 300, 2000])
 def test_thin_triangles(cull_check, strips, leaf):
