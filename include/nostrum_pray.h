@@ -197,7 +197,8 @@ pray_status pray_trace_closest_host(pray_scene *s, const float *rays_host, uint6
  * mask of the lanes whose own box tests passed, for the primary and the
  * occlusion rays (PACKETS) or for the primary rays only (PRIMARY_PACKETS);
  * all return the same hits. AUTO (the default) times the three on the
- * scene's first ray-traced frame and keeps the fastest. */
+ * scene's first ray-traced frame and keeps the fastest, separately for frames
+ * large enough to fill the GPU and for smaller ones. */
 typedef enum {
     PRAY_TRAVERSAL_AUTO = -1,
     PRAY_TRAVERSAL_LANES = 0,
@@ -205,7 +206,8 @@ typedef enum {
     PRAY_TRAVERSAL_PRIMARY_PACKETS = 2
 } pray_traversal;
 pray_status pray_scene_set_traversal(pray_scene *s, int32_t traversal);
-/* The traversal in use (PRAY_TRAVERSAL_AUTO until the first frame chose). */
+/* The traversal set, or the one that the last frame chose
+ * (PRAY_TRAVERSAL_AUTO before the first frame). */
 pray_status pray_scene_traversal(const pray_scene *s, int32_t *traversal);
 
 /* One ray-traced frame into device memory: rgb_dev height x width x 3 bytes,
@@ -213,8 +215,10 @@ pray_status pray_scene_traversal(const pray_scene *s, int32_t *traversal);
  * may be NULL) receive the primary hits. counters_dev (may be NULL) is
  * incremented by [primary rays, occlusion rays]. Under PRAY_TRAVERSAL_AUTO
  * the scene's first ray-traced frame (this call, pray_render_rt_host or
- * pray_render_rt_counts) renders the frame seven times to time the three
- * traversals, and synchronises. */
+ * pray_render_rt_counts), and the first one that fills the GPU or does not if
+ * that one was of the other kind, renders the frame seven times to time the
+ * three traversals, and synchronises (while the stream is captured the second
+ * takes the first's choice). */
 pray_status pray_render_rt(pray_scene *s, const pray_rt_params *p, uint8_t *rgb_dev, int32_t *ids_dev,
                            float *t_dev, unsigned long long *counters_dev, void *stream);
 

@@ -106,6 +106,9 @@ struct pray_scene {
     uint32_t grid_base = 0;
     float grid_org[3] = {0.f, 0.f, 0.f}, grid_scale = 1.f;
     std::atomic<int> rt_packets{PRAY_TRAVERSAL_AUTO};  // pray_traversal of the ray-traced frames
+    // under AUTO: what was the fastest for frames that give a warp all 32 lanes
+    // [0] or fewer [1], and what the last frame used
+    std::atomic<int> rt_choice[2] = {PRAY_TRAVERSAL_AUTO, PRAY_TRAVERSAL_AUTO}, rt_last{PRAY_TRAVERSAL_AUTO};
     uint64_t device_bytes = 0;
     // wavefront path tracer: scratch (path pool, queues), private stream,
     // events and the captured frame graph
@@ -232,11 +235,25 @@ pray_status check_params(const pray_rt_params *p) {
 // A ray-traced frame with the scene's traversal. The first frame of a scene
 // renders with each traversal (per lane, packets, packets for the primary
 // rays only) twice, times the second of each pair and keeps the fastest for
-// the scene (the frames are identical; coherent surfaces favour packets,
+// the scene's frames that fill the GPU or for those that do not, whichever it
+// is itself (the frames are identical; coherent surfaces favour packets,
 // occlusion rays from the scattered hits of a triangle soup the per-lane
-// walk); it synchronises `stream`.
+// walk, and so do warps with few lanes at work: a 96 x 64 frame of the
+// 1.31M-triangle sphere takes 201 us per lane, 264 in packets, 1080p 801 and
+// 751); it synchronises `stream`. While a stream is captured, which rules that
+// out, an untimed kind of frame takes the other's choice.
 cudaError_t render_rt(pray_scene *s, RtLaunch L, cudaStream_t stream) {
-    if (s->rt_packets.load() < 0) {
+    L.packets = s->rt_packets.load();
+    if (L.packets >= 0) return launch_render_rt(s->view(), L, s->sm_count, stream);
+    const int kind = rt_few_lanes(L.cam, s->sm_count) ? 1 : 0;
+    int choice = s->rt_choice[kind].load();
+    if (choice < 0 && s->rt_choice[1 - kind].load() >= 0) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        const cudaError_t e = cudaStreamIsCapturing(stream, &capture);
+        if (e != cudaSuccess) return e;
+        if (capture != cudaStreamCaptureStatusNone) choice = s->rt_choice[1 - kind].load();
+    }
+    if (choice < 0) {
         constexpr int kModes = 3;
         const int modes[kModes] = {PRAY_TRAVERSAL_LANES, PRAY_TRAVERSAL_PACKETS, PRAY_TRAVERSAL_PRIMARY_PACKETS};
         RtLaunch C = L;
@@ -264,9 +281,11 @@ cudaError_t render_rt(pray_scene *s, RtLaunch L, cudaStream_t stream) {
         for (cudaEvent_t x : ev)
             if (x) cudaEventDestroy(x);
         if (e != cudaSuccess) return e;
-        s->rt_packets.store(modes[best]);
+        choice = modes[best];
+        s->rt_choice[kind].store(choice);
     }
-    L.packets = s->rt_packets.load();
+    s->rt_last.store(choice);
+    L.packets = choice;
     return launch_render_rt(s->view(), L, s->sm_count, stream);
 }
 
@@ -683,12 +702,15 @@ pray_status pray_scene_set_traversal(pray_scene *s, int32_t traversal) {
         return set_error(PRAY_ERR_INVALID_ARGUMENT,
                          "traversal must be PRAY_TRAVERSAL_AUTO, _LANES, _PACKETS or _PRIMARY_PACKETS");
     s->rt_packets.store(traversal);
+    for (auto &c : s->rt_choice) c.store(PRAY_TRAVERSAL_AUTO);
+    s->rt_last.store(PRAY_TRAVERSAL_AUTO);
     return PRAY_OK;
 }
 
 pray_status pray_scene_traversal(const pray_scene *s, int32_t *traversal) {
     if (!s || !traversal) return set_error(PRAY_ERR_INVALID_ARGUMENT, "NULL argument");
-    *traversal = s->rt_packets.load();
+    const int set = s->rt_packets.load();
+    *traversal = set >= 0 ? set : s->rt_last.load();
     return PRAY_OK;
 }
 

@@ -257,6 +257,10 @@ cudaError_t launch_trace_closest(const DevScene &s, const float *rays, uint64_t 
     return cudaGetLastError();
 }
 
+bool rt_few_lanes(const CameraConsts &cam, int sm_count) {
+    return lanes_for(dev::warp_tiles(cam.width, cam.height) * 32, resident(sm_count, kFrameWarpsPerSm)) < 32;
+}
+
 cudaError_t launch_render_rt(const DevScene &s, const RtLaunch &launch, int sm_count, cudaStream_t stream) {
     RtLaunch L = launch;
     const uint64_t slots = warp_tiles(L.cam.width, L.cam.height) * 32;

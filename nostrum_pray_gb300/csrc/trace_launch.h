@@ -123,5 +123,7 @@ cudaError_t launch_trace_closest(const DevScene &s, const float *rays, uint64_t 
                                  float *ts, int sm_count, cudaStream_t stream);
 
 cudaError_t launch_render_rt(const DevScene &s, const RtLaunch &L, int sm_count, cudaStream_t stream);
+// Whether such a frame gives each warp fewer than 32 pixels (lanes_for, per-lane walk).
+bool rt_few_lanes(const CameraConsts &cam, int sm_count);
 
 }  // namespace pray_gpu

@@ -167,3 +167,39 @@ def test_inverses_beyond_the_grid(oracle, grid):
             best = min(best, a.elapsed_time(b))
         times.append(best)
     assert max(times[1:]) < 2.5 * times[0], times
+
+
+def test_traversal_is_timed_for_each_kind_of_frame(oracle):
+    """Under AUTO the first frame that fills the GPU and the first smaller one
+    are each timed (the call waits for the stream), whichever comes first, later
+    ones are not; a captured frame takes what there is."""
+    m = scenes.soup(2_000, 1)
+    small, large = scenes.soup_setup(64, 48), scenes.soup_setup(1024, 768)
+    rgb = {id(st): torch.empty((st.height, st.width, 3), dtype=torch.uint8, device="cuda") for st in (small, large)}
+
+    def waits(sc, st):
+        """Whether the call returns only after work queued before it."""
+        torch.cuda.synchronize()
+        torch.cuda._sleep(int(1e8))  # some 50 ms
+        queued = torch.cuda.Event()
+        queued.record()
+        sc.render_rt(st, rgb[id(st)])
+        waited = queued.query()
+        torch.cuda.synchronize()
+        return waited
+
+    for first, second in ((small, large), (large, small)):
+        sc = native.Scene.from_setup(m, small)
+        assert waits(sc, first) and not waits(sc, first)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            sc.render_rt(second, rgb[id(second)])
+        g.replay()
+        torch.cuda.synchronize()
+        captured = rgb[id(second)].clone()
+        assert waits(sc, second) and not waits(sc, second) and not waits(sc, first)
+        assert torch.equal(captured, rgb[id(second)])
+        sc.set_traversal(native.TRAVERSAL_AUTO)
+        assert sc.traversal() == native.TRAVERSAL_AUTO and waits(sc, first)
+        sc.set_traversal(native.TRAVERSAL_LANES)
+        assert not waits(sc, first) and sc.traversal() == native.TRAVERSAL_LANES
