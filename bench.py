@@ -396,6 +396,13 @@ def _timed_frames(fn, steps, warmup, flush):
     return sum(a.elapsed_time(b) for a, b in zip(starts, ends))
 
 
+def traced_rays(segments, frames, shared):
+    """Rays that the kernels traced of a path-traced frame's segments: where
+    they trace the camera ray of a pixel once (`shared`), the segments still
+    count it for each sample. frames: (pixels, samples per pixel)."""
+    return segments - sum(px * (spp - 1) for px, spp in frames) if shared else segments
+
+
 def run_pt(args):
     """Path tracing of the closed room (next-event estimation + Russian
     roulette after depth 3), 1024x1024, 64 spp, depth 8."""
@@ -414,6 +421,8 @@ def run_pt(args):
     sc.render_pt(p, rgb, counters=cnt)
     torch.cuda.synchronize()
     paths, segs = int(cnt[0]), int(cnt[1])
+    # the wavefront traces a pixel's camera ray once for all of its samples
+    traced = traced_rays(segs, [(st.width * st.height, spp)], args.scheduler == "wavefront")
     ms = _timed_frames(lambda: sc.render_pt(p, rgb), args.steps, args.warmup, flush)
     sec = ms / 1e3
     cpu = None
@@ -439,7 +448,8 @@ def run_pt(args):
             "config": {"workload": f"closed room {mesh.n} triangles, 1024x1024, {spp} spp, depth 8, NEE + "
                                    f"Russian roulette after depth 3, {args.scheduler} scheduler",
                        "l2": "flushed between steps"},
-            "mrays_per_s": round(segs * args.steps / sec / 1e6, 2), "segments_per_frame": segs, "cpu_baseline": cpu}
+            "mrays_per_s": round(traced * args.steps / sec / 1e6, 2), "segments_per_frame": segs,
+            "traced_rays_per_frame": traced, "cpu_baseline": cpu}
     sc.close()
     return line
 
@@ -467,6 +477,8 @@ def run_batch(args):
     b.render(cnt)
     torch.cuda.synchronize()
     paths, segs = int(cnt[0]), int(cnt[1])
+    # (as the Kajiya estimator's kernels do)
+    traced = traced_rays(segs, [(st.width * st.height, spp) for _, st in items], True)
     flush = torch.empty(L2_FLUSH_BYTES, dtype=torch.uint8, device="cuda")
     ms = _timed_frames(lambda: b.render(), args.steps, args.warmup, flush)
     sec = ms / 1e3
@@ -478,7 +490,8 @@ def run_batch(args):
                                    "one persistent graph-captured launch", "tuned": cfg.as_dict(),
                        "tuning_s": round(tune_s, 2), "scene_build_s": round(build_s, 2),
                        "l2": "flushed between steps"},
-            "mrays_per_s": round(segs * args.steps / sec / 1e6, 2), "segments_per_frame": segs}
+            "mrays_per_s": round(traced * args.steps / sec / 1e6, 2), "segments_per_frame": segs,
+            "traced_rays_per_frame": traced}
     del b
     for sc in scs:
         sc.close()
@@ -688,7 +701,7 @@ def run_denoise_infer(args):
     e2e_ms = _timed_frames(e2e_step, args.steps, args.warmup, flush)
     stream.synchronize()
     flops = D.forward_flops(res, res, nb)
-    nbytes = D.forward_bytes(res, res, nb)
+    nbytes = D.inference_bytes(res, res, nb)
     per = ms / args.steps / 1e3
     peak, peak_kind = measured_bf16()
     hbm, hbm_kind = measured_peaks()
@@ -714,9 +727,7 @@ def run_denoise_infer(args):
                        "launch": "one CUDA graph per call (recorded by the first call)"},
             "e2e": {"value": round(nb * args.steps / (e2e_ms / 1e3), 2), "unit": "frames/s",
                     "h2d_bytes_per_step": rad.numel() * 4 + feat.numel() * 2, "d2h_bytes_per_step": out.numel() * 4},
-            "gpu_launches": D.denoise_launches(res, res, nb, tensor_cores=not args.dn_cuda_cores,
-                                               sm_count=torch.cuda.get_device_properties(0).multi_processor_count)
-            * args.steps,
+            "gpu_launches": D.inference_launches(not args.dn_cuda_cores) * args.steps,
             "roofline": ({"bound": "hbm", "achieved": round(gbs, 1), "peak": hbm, "unit": "GB/s",
                           "frac": round(gbs / hbm, 4), "peak_kind": f"{hbm_kind} HBM copy bandwidth"}
                          if intensity < ridge else

@@ -79,9 +79,8 @@ def forward_bytes(h: int, w: int, n: int = 1) -> int:
     output), the second convolutions of levels 4-1 their output upsampled
     into the next concatenation (4 pixels each), the output convolution the
     log-space and the final radiance (FP32) after reading 3 channels of the
-    input and the albedo; the others their output. (Inference does not store
-    the log-space radiance: its 12 bytes per pixel, 1 % of the sum, are counted
-    all the same.)"""
+    input and the albedo; the others their output. (A training forward pass
+    stores the log-space radiance; inference does not: inference_bytes.)"""
     px0 = n * h * w
     total = px0 * (12 + 14 + 32)
     for i, (ci, co, l) in enumerate(CONVS):
@@ -100,15 +99,25 @@ def forward_bytes(h: int, w: int, n: int = 1) -> int:
     return total
 
 
+def inference_bytes(h: int, w: int, n: int = 1) -> int:
+    """forward_bytes without the log-space radiance (12 bytes per pixel), which
+    inference does not store."""
+    return forward_bytes(h, w, n) - 12 * n * h * w
+
+
+def inference_launches(tensor_cores: bool = True) -> int:
+    """Kernels that one pray_denoise call launches, whatever the size. Tensor
+    cores: input packing and the 19 convolutions, whose epilogues do the rest.
+    CUDA cores: besides, 4 poolings, 4 upsample-concatenations, the residual
+    add and the output transform, a kernel each."""
+    return 1 + len(CONVS) + (0 if tensor_cores else 4 + 4 + 2)
+
+
 def denoise_launches(h: int, w: int, n: int = 1, sm_count: int = 152, tensor_cores: bool = True) -> int:
-    """Kernels one pray_denoise call launches, at most. On the CUDA cores:
-    input packing, 4 poolings, 4 upsample-concatenations, the 19 convolutions,
-    the residual add and the output transform. On the tensor cores the
-    poolings, concatenations, residual and output transform are stores of the
-    convolutions' epilogues: input packing and the 19 convolutions, 20 launches
-    at every size. The bound is larger where the output convolution has fewer
-    than two 16x8-pixel tiles per SM (it allows that one a finalize kernel and
-    separate residual and output kernels)."""
+    """An upper bound of inference_launches, which is what runs: it allows the
+    output convolution of small frames (fewer than two 16x8-pixel tiles per SM)
+    a finalize kernel and separate residual and output kernels, which earlier
+    versions launched."""
     convs, split = 0, False
     for _, co, l in CONVS:
         tiles = n * -(-(w >> l) // 8) * -(-(h >> l) // 16)
