@@ -55,7 +55,10 @@ typedef struct {
                                       included; 0 = all */
     int32_t leaf_refine;           /* device layout only: most triangles per leaf (at most 4) of the conservative
                                       hierarchy that the kernels cull with (8; 0 = off, they walk the reference's
-                                      tree itself). Results are unchanged. */
+                                      tree itself). Results are unchanged where the sine of a triangle's smallest
+                                      angle times that of the ray's angle to its plane is 1/50 or more; beyond that
+                                      (grazing rays, slivers) a reported distance is rounding noise, and the walk
+                                      may settle on another of the hits in a few rays of 100,000. */
 } pray_tree_options;
 
 /* Ray-tracing frame parameters: the scene JSON's camera, lights and

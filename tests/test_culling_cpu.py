@@ -96,3 +96,22 @@ def test_grid_only_where_it_fits_the_boxes(cull_check, half, made):
     assert r.returncode == 0, r.stderr
     v = dict(zip(r.stdout.split()[::2], map(float, r.stdout.split()[1::2])))
     assert bool(v["made"]) == made and v["ratio"] < 1.5
+
+
+@pytest.mark.parametrize("tree", ["median", "sah"])
+@pytest.mark.parametrize("refine", [0, 1, 4, 8])
+def test_device_layout_holds_every_triangle(tree, refine):
+    """The culling hierarchy of a device layout holds every triangle once and
+    has nodes of its own; with refinement off there is none."""
+    from nostrum_pray_gb300 import native, scenes
+    st = scenes.soup_setup()
+    st.tree = tree
+    m = scenes.soup(2000, 1)
+    h = native.HostTree(m, native.tree_options(st))
+    nodes, refs, tris, cull = (int(x) for x in h.device_layout(refine))
+    stats = [int(x) for x in h.tree_stats()]
+    assert refs == stats[4]
+    if refine == 0:
+        assert (tris, cull) == (0, 0)
+    else:
+        assert tris == m.n and 2 * m.n // min(refine, 4) <= cull <= 2 * m.n and nodes > cull
