@@ -54,7 +54,6 @@ void Denoiser::release() {
     for (void *p : owned_) cudaFree(p);
     owned_.clear();
     act_.clear();
-    grad_.clear();
     cap_pixels_ = 0;
 }
 
@@ -184,7 +183,6 @@ cudaError_t Denoiser::ensure(int n, int h, int w) {
     owned_ = keep;
     generation_++;
     act_.clear();
-    grad_.clear();
     cap_pixels_ = 0;  // until every buffer below is there
     n_ = n, h_ = h, w_dim_ = w;
     cudaError_t e;

@@ -72,7 +72,6 @@ class Denoiser {
 
     std::vector<Conv> convs_;
     std::vector<Buf> act_;
-    std::vector<float *> grad_;
     std::vector<void *> owned_;
     size_t n_params_ = 0, cap_pixels_ = 0;
     int n_ = 0, h_ = 0, w_dim_ = 0, step_ = 0;

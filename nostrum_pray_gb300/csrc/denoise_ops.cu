@@ -442,10 +442,6 @@ cudaError_t relu_mask(const __nv_bfloat16 *y, const float *g, float *out, size_t
     k_relu_mask<<<blocks_for(n), 256, 0, st>>>(y, g, out, n);
     return cudaGetLastError();
 }
-cudaError_t bias_grad(const float *g, float *db, size_t pixels, int c, cudaStream_t st) {
-    k_bias_grad<<<c, 256, 0, st>>>(g, db, pixels, c);
-    return cudaGetLastError();
-}
 cudaError_t avgpool(const __nv_bfloat16 *x, __nv_bfloat16 *y, int n, int h, int w, int c, cudaStream_t st) {
     k_avgpool<<<blocks_for((size_t)n * h * w * c / 4), 256, 0, st>>>(x, y, n, h, w, c);
     return cudaGetLastError();

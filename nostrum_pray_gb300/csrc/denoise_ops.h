@@ -27,7 +27,7 @@ struct TcConvPlan {
     int n, h, w, cin, cout, npad, relu;
     int tiles_x, tiles_y, tiles;
     int nsplit, npad_full;        // output-channel chunks of npad channels each, of npad_full
-    int grid, per_sm;             // persistent CTAs of each chunk, and the CTAs per SM it was planned for
+    int grid;                     // persistent CTAs of each chunk
     int ring, wstages;            // halo slots; weight slots of a tap each (9: all resident)
     int acc_slots, acc_stride, tmem_cols;
     int grad;                     // planned for TcFuse::grad
@@ -156,8 +156,6 @@ cudaError_t conv3x3_forward(const __nv_bfloat16 *x, const __nv_bfloat16 *w, cons
 cudaError_t conv3x3_backward(const __nv_bfloat16 *x, const __nv_bfloat16 *w, const float *gpre, float *dx, float *dw,
                              float *db, int n, int h, int wd, int cin, int cout, cudaStream_t st);
 cudaError_t relu_mask(const __nv_bfloat16 *y, const float *g, float *out, size_t n, cudaStream_t st);
-// db[c] += sum over pixels of g[p][c]
-cudaError_t bias_grad(const float *g, float *db, size_t pixels, int c, cudaStream_t st);
 cudaError_t avgpool(const __nv_bfloat16 *x, __nv_bfloat16 *y, int n, int h, int w, int c, cudaStream_t st);
 cudaError_t avgpool_backward(const float *gy, float *gx, int n, int h, int w, int c, cudaStream_t st);
 cudaError_t upsample_backward(const float *gy, float *gx, int n, int h, int w, int c, int cy, cudaStream_t st);

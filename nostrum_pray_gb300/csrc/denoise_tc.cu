@@ -1392,7 +1392,6 @@ cudaError_t tc_conv_plan(TcConvPlan &p, const __nv_bfloat16 *x, int n, int h, in
                     best = cost;
                     p.npad = cw, p.nsplit = nsplit, p.grid = (int)ctas, p.wstages = wst, p.ring = (int)ring;
                     p.acc_slots = acc, p.acc_stride = stride, p.tmem_cols = cols;
-                    p.per_sm = per_sm;
                 }
                 break;  // fewer weight slots never help
             }
