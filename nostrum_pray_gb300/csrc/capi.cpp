@@ -585,7 +585,9 @@ pray_status pray_scene_create(const float *verts, const float *colors, const uin
             return n ? g.a | kLeafFlag | (n - 1) << kCullCountShift : g.a;
         };
         GridImage grid;
-        const bool on_grid = grid_for_device(img.cull, leaf_word, grid);
+        // (kernels number nodes and pairs in 31 bits)
+        const bool on_grid = gnodes.size() + 2 * img.cull.size() < (1ull << 31) &&
+                             grid_for_device(img.cull, leaf_word, grid);
         gnodes.reserve(gnodes.size() + img.cull.size() + grid.pairs.size());
         for (GNode g : img.cull) {
             if (g.b & kLeafFlag) g.a = leaf_word(g);

@@ -247,7 +247,8 @@ struct Trav {
     // record, exact copy: its node)
     uint32_t w, lw;
     uint32_t node_off;  // 0: the exact copy, else the culling copy's nodes or (kGrid) its grid pairs (finite
-                        // inverse direction, near origin)
+                        // inverse direction, near origin); kGrid: kLeafFlag | the culling copy's nodes, for the
+                        // subtraction form
     float cur_tn, leaf_tn, limit, back;  // grid pairs: in cells
     float best_t;
     float nox, noy, noz;  // culling copy: -origin / direction (slab_fma), or slab_grid's
@@ -296,7 +297,7 @@ __device__ __forceinline__ void leaf_range(const DevScene &s, uint32_t node_off,
 // Whether the walk tests boxes in FMA form (culling copy; kGrid: grid pairs).
 template <bool kGrid>
 __device__ __forceinline__ bool fast_boxes(const DevScene &s, const Trav &T) {
-    return kGrid ? T.node_off == s.grid_base : T.node_off != 0u;
+    return kGrid ? (int)T.node_off > 0 : T.node_off != 0u;
 }
 
 // kGrid (scenes with grid pairs): the culling copy's boxes come from its grid
@@ -332,7 +333,7 @@ __device__ __forceinline__ void trav_start(const DevScene &s, const RayF &r, flo
         const bool near = cx * cx + cy * cy + cz * cz <= s.cull_r2;
         const bool grid = near && fabsf(r.ix) < kMaxInv && fabsf(r.iy) < kMaxInv && fabsf(r.iz) < kMaxInv;
         T.finite = grid || (isfinite(r.ix) && isfinite(r.iy) && isfinite(r.iz));
-        T.node_off = grid ? s.grid_base : near && T.finite ? s.n_nodes : 0u;
+        T.node_off = grid ? s.grid_base : near && T.finite ? s.n_nodes | kLeafFlag : 0u;
     } else {
         T.node_off = (T.finite && isfinite(T.nox) && isfinite(T.noy) && isfinite(T.noz) &&
                       cx * cx + cy * cy + cz * cz <= s.cull_r2)
@@ -372,7 +373,7 @@ __device__ __forceinline__ void trav_round(const DevScene &s, const RayF &r, flo
         if (!__any_sync(kFull, interior && !T.have_leaf)) break;
         if (interior) {
             if (kCount) fc->pairs++;
-            const GNode *c = s.nodes + (T.w + T.node_off);
+            const GNode *c = s.nodes + (kGrid ? T.w + (T.node_off & ~kLeafFlag) : T.w + T.node_off);
             float4 l0, h0, l1, h1;
             ldg_node(c, l0, h0);
             if (!kGrid) ldg_node(c + 1, l1, h1);
