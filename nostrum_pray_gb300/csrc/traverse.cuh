@@ -295,9 +295,10 @@ __device__ __forceinline__ void leaf_range(const DevScene &s, uint32_t node_off,
 }
 
 // Whether the walk tests boxes in FMA form (culling copy; kGrid: grid pairs).
-template <bool kGrid>
+template <int kMode, bool kGrid>
 __device__ __forceinline__ bool fast_boxes(const DevScene &s, const Trav &T) {
-    return kGrid ? (int)T.node_off > 0 : T.node_off != 0u;
+    if (!kGrid) return T.node_off != 0u;
+    return kMode == kClosest ? (int)T.node_off > 0 : T.node_off == s.grid_base;
 }
 
 // kGrid (scenes with grid pairs): the culling copy's boxes come from its grid
@@ -333,7 +334,7 @@ __device__ __forceinline__ void trav_start(const DevScene &s, const RayF &r, flo
         const bool near = cx * cx + cy * cy + cz * cz <= s.cull_r2;
         const bool grid = near && fabsf(r.ix) < kMaxInv && fabsf(r.iy) < kMaxInv && fabsf(r.iz) < kMaxInv;
         T.finite = grid || (isfinite(r.ix) && isfinite(r.iy) && isfinite(r.iz));
-        T.node_off = grid ? s.grid_base : near && T.finite ? s.n_nodes | kLeafFlag : 0u;
+        T.node_off = grid ? s.grid_base : near && T.finite ? s.n_nodes | (kMode == kClosest ? kLeafFlag : 0u) : 0u;
     } else {
         T.node_off = (T.finite && isfinite(T.nox) && isfinite(T.noy) && isfinite(T.noz) &&
                       cx * cx + cy * cy + cz * cz <= s.cull_r2)
@@ -350,7 +351,7 @@ __device__ __forceinline__ void trav_start(const DevScene &s, const RayF &r, flo
             if (!T.node_off && (__float_as_uint(rhi.w) & kLeafFlag)) T.w = kLeafFlag;  // (node 0)
             T.cur_tn = tn;
             T.have_node = true;
-            if (kGrid && fast_boxes<kGrid>(s, T)) {
+            if (kGrid && fast_boxes<kMode, kGrid>(s, T)) {
                 if (!(T.w & kLeafFlag)) T.w /= 2;
                 T.cur_tn *= s.grid_scale, T.limit *= s.grid_scale, T.back *= s.grid_scale;
                 constexpr float kBias = 8388608.f;
@@ -373,7 +374,7 @@ __device__ __forceinline__ void trav_round(const DevScene &s, const RayF &r, flo
         if (!__any_sync(kFull, interior && !T.have_leaf)) break;
         if (interior) {
             if (kCount) fc->pairs++;
-            const GNode *c = s.nodes + (kGrid ? T.w + (T.node_off & ~kLeafFlag) : T.w + T.node_off);
+            const GNode *c = s.nodes + (kGrid && kMode == kClosest ? T.w + (T.node_off & ~kLeafFlag) : T.w + T.node_off);
             float4 l0, h0, l1, h1;
             ldg_node(c, l0, h0);
             if (!kGrid) ldg_node(c + 1, l1, h1);
@@ -381,7 +382,7 @@ __device__ __forceinline__ void trav_round(const DevScene &s, const RayF &r, flo
             float tn0, tf0, tn1, tf1;
             bool v0, v1;
             // entered: tn <= tf, not beyond the best hit, not behind the origin
-            if (fast_boxes<kGrid>(s, T)) {
+            if (fast_boxes<kMode, kGrid>(s, T)) {
                 if (kGrid) {
                     slab_grid(l0.x, l0.y, l0.z, r, T.nox, T.noy, T.noz, tn0, tf0);
                     slab_grid(h0.x, h0.y, h0.z, r, T.nox, T.noy, T.noz, tn1, tf1);
@@ -460,7 +461,7 @@ __device__ __forceinline__ void trav_round(const DevScene &s, const RayF &r, flo
                                 T.best = (int)i;
                                 T.best_key = key;
                                 T.limit = t * kPruneRel;
-                                if (kGrid && fast_boxes<kGrid>(s, T)) T.limit *= s.grid_scale;
+                                if (kGrid && fast_boxes<kMode, kGrid>(s, T)) T.limit *= s.grid_scale;
                             }
                         }
                     }
