@@ -15,9 +15,8 @@ namespace {
 using namespace dev;
 
 // Modes 0 and 1 bounce by bounce (pt_sync). The per-lane state machine
-// that the batch kernel runs for mode 0 measured slower here: 176.6 against
-// 194.7 Msamples/s on the closed room, 653 against 863 on a 20k-triangle
-// sphere (at 8 blocks of 128 threads per SM, 64 registers).
+// that the batch kernel runs for mode 0 measured slower here: a room at 401 x
+// 299 and 8 spp 2,368 us against 2,044.
 // Pixels of the frame in warp-tile order (pixel_of) from a counter: the lanes
 // of a warp whose pixel is done take the next slots together (one atomic), so
 // they do not wait for the warp's longest path. Warp-uniform state.
@@ -41,14 +40,14 @@ struct FrameSrc {
 };
 
 // kRefill (mode 1): a persistent grid whose lanes take pixels from the
-// frame's counter (512^2 at 1 spp: 1.68 -> 1.49 ms; room 1024^2 at 64 spp
-// unchanged). Mode 0 keeps one pixel per lane: refilled, it measured 6 %
-// slower on the room. kBlocks: resident blocks per SM (the register cap).
-// Long frames run 10 (48 registers); a frame of fewer paths than two rounds
-// of those lanes is bound by its last paths, which run faster with more
-// registers and fewer spills: 8 blocks (64 registers) take 512^2 at 1 spp
-// from 1.231 to 1.186 ms, where the 1024^2 x 64-spp room drops from 200.2
-// to 191.0 Msamples/s.
+// frame's counter (512^2 at 1 spp: 925 -> 806 us; room 1024^2 at 16 spp 48.8 ->
+// 47.3 ms). Mode 0 keeps one pixel per lane: refilled, 401 x 299 at 8 spp took
+// 2,022 us against 2,044, but 1024 x 768 at 2 spp 2,713 against 2,595. kBlocks:
+// resident blocks per SM (the register cap). Long frames run 10 (48
+// registers); a frame of fewer paths than two rounds of those lanes is bound by
+// its last paths, which run faster with more registers and fewer spills: 512^2
+// at 1 spp takes 852 us with 10 blocks and 806 with 8 (64 registers), the 1024^2
+// room at 16 spp 47.3 ms with either.
 template <bool kRefill, int kBlocks>
 __global__ void __launch_bounds__(128, kBlocks) k_render_pt(DevScene s, PtLaunch L) {
     constexpr unsigned kFull = 0xFFFFFFFFu;

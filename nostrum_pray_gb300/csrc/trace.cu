@@ -87,11 +87,10 @@ __global__ void __launch_bounds__(128) k_trace_closest(DevScene s, const float *
 // occlusion rays as a packet (traverse_coherent).
 // Resident blocks per SM (the register cap): the all-packet walk (one
 // shared-memory stack per warp) gains from more warps in flight despite
-// some spills (1.31M sphere: 8 / 9 / 10 blocks 1.660 / 1.626 /
-// 1.616 ms per frame); per-lane and primary-packet walks lose from them.
-// Smaller blocks, so that a warp's slot frees without waiting for the
-// block's other warps, measured slower: 64 x 20 1.68 ms, 32 x 32 1.63 ms,
-// 64 x 16 1.74 ms against 1.61 ms for 128 x 10.
+// some spills (1.31M sphere at 1080p, 128 threads x 8 / 9 / 10 / 11 blocks: 1,207
+// / 1,170 / 1,170 / 1,206 us per frame); per-lane and primary-packet walks lose
+// from them. Smaller blocks, whose warps' slots free one by one: 64 x 16 1,232,
+// 64 x 20 1,203, 32 x 32 1,138 (not taken: measured on this scene alone).
 constexpr int kPacketBlocks = 10, kPacketThreads = 128;
 
 template <bool kCount, int kStackN, bool kPrimPacket, bool kShadowPacket>

@@ -5,10 +5,15 @@
 // reference's scalar build compiled without FMA contraction.
 //
 // Traversal: one ray per thread, iterative, with a short per-thread stack.
-// Both children of a node are fetched together (one 64-byte pair) and tested
-// with the reference's infinite-line slab test (BoundingBox::intersect,
-// include/geometry.h:151-164); the nearer is entered first and the farther
-// pushed. Instead of the reference's visit-everything depth-first order
+// Both children of a node are fetched together and tested; the nearer is
+// entered first and the farther pushed. Rays with finite inverse directions
+// and origins near the scene walk the culling copy (host/flatten.h): its boxes
+// are padded and tested in FMA form (slab_fma, slab_grid), each triangle
+// stands there once, and a hit counts if a leaf of the reference's tree that
+// holds the triangle passes the reference's infinite-line slab test
+// (BoundingBox::intersect, include/geometry.h:151-164; owned). The others walk
+// the exact copy, the reference's tree, with that test at every box. Instead of
+// the reference's visit-everything depth-first order
 // (KDTree::intersectRecursive, src/kd_tree.cpp:237-279), boxes that start
 // beyond the best hit found so far are skipped: the result is the
 // lexicographic minimum of (distance, depth-first reference position) over
@@ -303,11 +308,11 @@ __device__ __forceinline__ bool fast_boxes(const DevScene &s, const Trav &T) {
 
 // kGrid (scenes with grid pairs): the culling copy's boxes come from its grid
 // pairs: one 32-byte load per pair instead of two, for twelve byte permutes
-// more. The divergent walks
-// of ray queries and of the wavefront's extension and occlusion passes, which
-// L1 throughput bounds (83 to 89 % of its peak under ncu), gain: room 1024^2
-// at 16 spp 37.43 -> 34.00 ms, 300k closest hits 178 -> 168 us, 100k occlusion
-// rays 105 -> 98 us. The others are bound by instruction issue or registers
+// more. The divergent walks of ray queries and of the wavefront's extension and
+// occlusion passes, which whole nodes bind to L1 throughput (83 to 89 % of its
+// peak under ncu), gain: room 1024^2 at 16 spp 37.43 -> 34.00 ms, 300k closest
+// hits 178 -> 168 us, 100k occlusion rays 105 -> 98 us. The others are bound by
+// instruction issue or registers
 // and lose (per-pixel paths of 512^2 at 1 spp 832 -> 950 us, 12 scenes 6.18 ->
 // 6.44 ms) and keep whole nodes.
 template <int kMode, bool kGrid>
@@ -495,8 +500,8 @@ __device__ __forceinline__ int traverse(const DevScene &s, const RayF &r, float 
 // so it returns the same lexicographic minimum as traverse(); only the order
 // of visits differs (the warp enters first the child that is nearer for most
 // of the lanes entering both), and a lane whose bound shrank after a node was
-// pushed still visits it (testing a popped node's box again measured slower:
-// 2,571 against 2,682 Mrays/s on the 1.31M sphere). Box tests run in FMA
+// pushed still visits it (a popped node's box is not at hand: only its word is
+// on the stack). Box tests run in FMA
 // form (slab_fma). Only for warps whose valid lanes all use the culling
 // copy.
 template <bool kAny, bool kCount, int kStackN>
